@@ -29,15 +29,15 @@
 //               exceeds it by more than 2^8 (any fixed reference gives the same quotient;
 //               float32 has the range), so the pass over O that a new maximum costs is rare.
 //
-// Why two lanes and four issuing threads: a thread needs 55 ns and more to issue one
-// tcgen05.mma, whatever its size, while the tensor pipe finishes a product of 64 or 128
-// columns in 30 to 35 ns (measured: one to four threads issuing side by side each keep their
-// own rate until the pipe is full); one softmax group alone leaves its four schedulers waiting
-// on the latencies of tensor-memory loads and stores and on the exponential unit; and what a
-// CTA spends before its first and after its last tile (about 12 us: some 3 us until its first
-// loads from global memory are back, queries and page table alike, then first pages, rewrite,
-// the chain of first products; at the end the last product and the output) is spent once for
-// 256 rows, and every key tile is fetched and rewritten once for them.
+// Why two lanes and four issuing threads: one softmax group alone leaves its four schedulers
+// waiting on the latencies of tensor-memory loads and stores and on the exponential unit, and two
+// groups need products issued for both; and what a CTA spends before its first and after its last
+// tile (about 12 us: some 3 us until its first loads from global memory are back, queries and
+// page table alike, then first pages, rewrite, the chain of first products; at the end the last
+// product and the output) is spent once for 256 rows, and every key tile is fetched and rewritten
+// once for them.  The issuing threads are picked by elect.sync: behind `lane == 0` a thread
+// needed 55 ns to issue a product of any size (2,048 tokens, 32 heads of 128: 129 us a layer in
+// place, 108 with elect.sync).
 //
 // Operand layouts.  Nothing is swizzled: every operand is made of "core matrices" of 8 rows
 // x 16 bytes (128 contiguous bytes), which is exactly what a page block of the cache is made
@@ -265,7 +265,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
     // Each as far ahead as its own ring allows: the keys of a tile are wanted well before
     // its values (they are rewritten, then multiplied, then the softmax runs), and one ring
     // must not hold up the other.
-    if (lane == 0) {
+    if (elect_one()) {
       const bool values = warp == WARP_VALUES;
       const int stages = values ? V_STAGES : K_STAGES;
       uint64_t* full = values ? v_full : k_full;
@@ -395,7 +395,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
     }
   } else if (warp == WARP_SCORES || warp == WARP_SCORES + 1) {
     // ------------------------------------------------------------ score products
-    if (lane == 0) {
+    if (elect_one()) {
       constexpr uint32_t idesc_scores = make_idesc(BLOCK_M, BLOCK_N);
       // Descriptors differ from product to product only in their start address (the low 14
       // bits, in units of 16 bytes): build one of each kind and add offsets.
@@ -436,7 +436,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
     }
   } else if (warp == WARP_OUTPUT || warp == WARP_OUTPUT + 1) {
     // ----------------------------------------------------------- output products
-    if (lane == 0) {
+    if (elect_one()) {
       const int l = warp - WARP_OUTPUT;
       const int my_tiles = lane_tiles(l);
       constexpr uint32_t idesc_output = make_idesc_b_mn_major(BLOCK_M, D);
