@@ -28,6 +28,7 @@ SOURCES = (
     "hx_recurrent.cu",
     "hx_matrix_lstm.cu",
     "hx_state_chunks.cu",
+    "hx_delta_chunks.cu",
     "hx_map_attention.cu",
     "hx_gated_recurrence.cu",
     "hx_rotary_norm.cu",

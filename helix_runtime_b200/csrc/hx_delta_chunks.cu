@@ -1,0 +1,683 @@
+// The gated delta rule in prompts, 64 tokens at a time on the tensor cores (bfloat16 rows):
+//
+//     S_t = e^(d_t) S_(t-1) + k_t u_t',   u_t = beta_t (v_t - e^(d_t) S_(t-1)' k_t),   o_t = S_t' q_t
+//
+// with queries and keys divided by their lengths (or scaled by constants).  Inside a chunk that
+// starts from S_0, with L_t the sum of d up to t, the u_t solve a triangular system:
+//
+//     (1 + A) U = R,    A_ts = beta_t (k_t . k_s) e^(L_t - L_s)  (s < t),
+//                       R_t  = beta_t v_t - beta_t e^(L_t) S_0' k_t
+//     o_t  = e^(L_t) S_0' q_t + sum_(s <= t) P_ts u_s,   P_ts = (q_t . k_s) e^(L_t - L_s)
+//     S_64 = e^(L_64) S_0 + sum_s e^(L_64 - L_s) k_s u_s'
+//
+// Every exponent is a difference of decays between two tokens of the chunk, never positive.
+//
+//   * delta_weights_kernel, all chunks at once: T = (1 + A)^-1 by forward substitution in float32,
+//     P, and the factors of a token.
+//   * delta_states_kernel, one CTA per (request, head, block of columns), chunk after chunk: a
+//     warp keeps S' for 16 columns in registers as accumulators of mma.sync, whose layout is also
+//     that of an A operand, so S' goes into S' K' and S' Q', R' into R' T', U' into U' P' and
+//     U' K without leaving the registers.  The next chunk's rows are on their way meanwhile.
+//
+// Queries, keys and values go in as they are stored; what the scan holds in float32 (S, R, U, T,
+// P) goes into the products as three bfloat16 terms, 24 bits; lengths and decays multiply the
+// float32 sums.  The products of the small terms are summed before those of the large ones,
+// which are then the only ones whose rounding counts.
+//
+// The scan walks a token in 0.6 us whatever the chip could do beside it (a chain of two dot
+// products over the state); a chunk is a chain of about 800 products a warp, which is what bounds
+// it now.  Measured (one B200, 32 heads of 128 by 128): a portion of 1,000 tokens 1,030 -> 198 us,
+// eight of 256 1,092 -> 225, one of 64 73 -> 42; errors against 64 bits 2.7e-7 (outputs) and 2.6e-7
+// (state) where the scan has 2.3e-7 and 2.2e-7, and the layer's outputs are 0.0031 off either way.
+#include "hx_mma.cuh"
+#include "hx_scan.cuh"
+
+namespace {
+
+constexpr int CHUNK = 64;
+constexpr int ROW_PAD = 8;             // elements behind a staged row: rows start on different banks
+constexpr int TERMS = 3;
+constexpr int WEIGHT_COLUMNS = 2 * TERMS * CHUNK;      // a token's row of T, then of P, three terms each
+constexpr int WEIGHT_STRIDE = WEIGHT_COLUMNS + ROW_PAD;
+
+struct DeltaArgs {
+  const __nv_bfloat16* q;    // [tokens, ld_q], already offset; qk_heads * dim columns
+  const __nv_bfloat16* k;
+  const __nv_bfloat16* v;    // heads * vdim columns
+  int ld_q, ld_k, ld_v;
+  const __nv_bfloat16* decay_in;      // as in LinearStateArgs
+  const __nv_bfloat16* beta_in;
+  int ld_gates;
+  const float* a_log;
+  const float* dt_bias;
+  const float* fixed_decay_m1;
+  int unit_norm;
+  float unit_eps, q_scale, k_scale;
+  __nv_bfloat16* weights;    // [heads, rows, WEIGHT_COLUMNS]
+  float4* factors;           // [heads, rows]: of S' q, of S' k, of v, of u k'
+  float* total;              // [heads, rows]: e^(L_64) at a chunk's first token
+  int rows;
+  float* state;
+  long long state_stride;
+  int head_stride;
+  float* o;                  // [tokens, heads * vdim]
+  const int* request_start;
+  const int* request_slot;
+  int requests, heads, qk_heads, dim, vdim, parts, column_warps;
+};
+
+// two neighbouring values in three bfloat16 terms, a word each
+__device__ __forceinline__ void split_terms(float x0, float x1, uint32_t& t0, uint32_t& t1,
+                                            uint32_t& t2) {
+  const __nv_bfloat162 high = __floats2bfloat162_rn(x0, x1);
+  const float2 h = __bfloat1622float2(high);
+  x0 -= h.x;
+  x1 -= h.y;
+  const __nv_bfloat162 middle = __floats2bfloat162_rn(x0, x1);
+  const float2 m = __bfloat1622float2(middle);
+  t0 = *reinterpret_cast<const uint32_t*>(&high);
+  t1 = *reinterpret_cast<const uint32_t*>(&middle);
+  t2 = hx_pack_bf16(x0 - m.x, x1 - m.y);
+}
+
+// The A operand of products over step `step`'s sixteen coordinates from two neighbouring
+// accumulator tiles: all three terms, or the first one only (made anew, in volatile assembly:
+// otherwise the compiler keeps the first terms of a whole pass over the state in registers that
+// it does not have).
+template <int TILES>
+__device__ __forceinline__ void operand_terms(const float (&x)[TILES][4], int step, uint32_t (&t0)[4],
+                                              uint32_t (&t1)[4], uint32_t (&t2)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int tile = 2 * step + (i >> 1), j = 2 * (i & 1);
+    split_terms(x[tile][j], x[tile][j + 1], t0[i], t1[i], t2[i]);
+  }
+}
+template <int TILES>
+__device__ __forceinline__ void operand_high(const float (&x)[TILES][4], int step, uint32_t (&t0)[4]) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int tile = 2 * step + (i >> 1), j = 2 * (i & 1);
+    asm volatile("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(t0[i]) : "f"(x[tile][j + 1]), "f"(x[tile][j]));
+  }
+}
+
+// PIECES 16-byte pieces of each of 64 rows into shared memory (those in front of `columns`); rows
+// from `live` on are zeros
+template <int PIECES>
+__device__ __forceinline__ void copy_rows(__nv_bfloat16* dst, int stride, const __nv_bfloat16* src,
+                                          size_t ld, int columns, int live) {
+  for (int i = threadIdx.x; i < CHUNK * PIECES; i += blockDim.x) {
+    const int row = i / PIECES, piece = i - row * PIECES;
+    const bool there = row < live;
+    if (8 * piece < columns)
+      hx_cp_async_16(hx_shared_address(dst + row * stride + 8 * piece),
+                     there ? src + row * ld + 8 * piece : src, there ? 16 : 0);
+  }
+}
+
+// zeros behind the copied columns, once: the copies never touch them
+__device__ __forceinline__ void clear_columns(__nv_bfloat16* dst, int stride, int from, int to) {
+  const int width = to - from;
+  for (int i = threadIdx.x; i < CHUNK * width; i += blockDim.x) {
+    const int row = i / width;
+    dst[row * stride + from + i - row * width] = __float2bfloat16_rn(0.0f);
+  }
+}
+
+constexpr int SOLVE_STRIDE = CHUNK + 4;
+
+// Shared memory of delta_weights_kernel: queries, keys, A transposed, T.
+int weights_shared(int padded) {
+  return 2 * 2 * CHUNK * (padded + ROW_PAD) + 2 * 4 * CHUNK * SOLVE_STRIDE;
+}
+
+// grid (chunks of the step, heads), 128 threads: a warp takes 16 of the chunk's tokens
+template <int STEPS>
+__global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
+  constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
+  extern __shared__ uint4 shared_pieces[];
+  __shared__ float level_hi[CHUNK], level_lo[CHUNK], q_length[CHUNK], k_length[CHUNK], write[CHUNK];
+  hx_pdl_prologue();
+  int chunk, chunks;
+  const int request = hx_find_query_tile(a.request_start, a.requests, 1, CHUNK, blockIdx.x, chunk, chunks);
+  if (request < 0) return;
+  const int head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
+  const int first = a.request_start[request] + chunk * CHUNK;
+  const int live = min(CHUNK, a.request_start[request + 1] - first);
+  __nv_bfloat16* queries = reinterpret_cast<__nv_bfloat16*>(shared_pieces);
+  __nv_bfloat16* keys = queries + CHUNK * STRIDE;
+  float* system = reinterpret_cast<float*>(keys + CHUNK * STRIDE);      // [s][t]: A
+  float* solution = system + CHUNK * SOLVE_STRIDE;                      // [t][s]: T
+  copy_rows<2 * STEPS>(queries, STRIDE, a.q + static_cast<size_t>(first) * a.ld_q + qk_head * a.dim, a.ld_q, a.dim, live);
+  copy_rows<2 * STEPS>(keys, STRIDE, a.k + static_cast<size_t>(first) * a.ld_k + qk_head * a.dim, a.ld_k, a.dim, live);
+  hx_cp_async_commit();
+  if (PADDED > a.dim) {
+    clear_columns(queries, STRIDE, a.dim, PADDED);
+    clear_columns(keys, STRIDE, a.dim, PADDED);
+  }
+  const size_t rows = static_cast<size_t>(head) * a.rows + first;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  if (warp == 0) {
+    // sums of the decays' logarithms, two neighbouring tokens a lane, in double: their
+    // differences are what counts
+    float d[2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int t = 2 * lane + i;
+      d[i] = 0.0f;
+      float beta = 0.0f;
+      if (t < live) {
+        const size_t gate = static_cast<size_t>(first + t) * a.ld_gates + head;
+        d[i] = a.decay_in != nullptr
+                   ? -expf(a.a_log[head]) * softplus(__bfloat162float(a.decay_in[gate]) + a.dt_bias[head])
+                   : log1pf(a.fixed_decay_m1[head]);
+        beta = hx_sigmoid(__bfloat162float(a.beta_in[gate]));
+      }
+      write[t] = beta;
+    }
+    double sum = static_cast<double>(d[0]) + static_cast<double>(d[1]);
+#pragma unroll
+    for (int offset = 1; offset < 32; offset <<= 1) {
+      const double other = __shfl_up_sync(0xffffffffu, sum, offset);
+      if (lane >= offset) sum += other;
+    }
+    const double before = sum - static_cast<double>(d[1]);
+    level_hi[2 * lane] = static_cast<float>(before);
+    level_lo[2 * lane] = static_cast<float>(before - static_cast<double>(static_cast<float>(before)));
+    level_hi[2 * lane + 1] = static_cast<float>(sum);
+    level_lo[2 * lane + 1] = static_cast<float>(sum - static_cast<double>(static_cast<float>(sum)));
+  }
+  hx_cp_async_wait<0>();
+  __syncthreads();
+  // what lengths and scales make of a query and a key
+  for (int i = 0; i < 16; ++i) {
+    const int t = 16 * warp + i;
+    float fq = a.q_scale, fk = a.k_scale;
+    if (a.unit_norm) {
+      float sq = 0.0f, sk = 0.0f;
+      for (int e = 2 * lane; e < PADDED; e += 64) {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(queries + t * STRIDE + e));
+        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(keys + t * STRIDE + e));
+        sq = fmaf(x.x, x.x, fmaf(x.y, x.y, sq));
+        sk = fmaf(y.x, y.x, fmaf(y.y, y.y, sk));
+      }
+#pragma unroll
+      for (int offset = 16; offset > 0; offset >>= 1) {
+        sq += __shfl_xor_sync(0xffffffffu, sq, offset);
+        sk += __shfl_xor_sync(0xffffffffu, sk, offset);
+      }
+      fq /= sqrtf(sq + a.unit_eps);
+      fk /= sqrtf(sk + a.unit_eps);
+    }
+    if (lane == 0) {
+      q_length[t] = fq;
+      k_length[t] = fk;
+    }
+  }
+  __syncthreads();
+  // e^(L_t - L_s)
+  auto faded = [&](int t, int s) {
+    return expf((level_hi[t] - level_hi[s]) + (level_lo[t] - level_lo[s]));
+  };
+  if (threadIdx.x < live) {
+    const int t = threadIdx.x;
+    const float level = expf(level_hi[t] + level_lo[t]);
+    a.factors[rows + t] = make_float4(q_length[t] * level, write[t] * k_length[t] * level, write[t],
+                                      k_length[t] * faded(CHUNK - 1, t));
+    if (t == 0) a.total[rows] = expf(level_hi[CHUNK - 1] + level_lo[CHUNK - 1]);
+  }
+  // sums of tokens 16 warp .. + 15 against the tiles of 8 tokens that do not lie behind them
+  float qk[8][4], kk[8][4];
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) qk[n][j] = kk[n][j] = 0.0f;
+  const int tiles = 2 * warp + 2;
+  const int matrix = lane >> 3, in_matrix = lane & 7;
+  const uint32_t a_row = 2 * ((16 * warp + (matrix & 1) * 8 + in_matrix) * STRIDE + (matrix >> 1) * 8);
+  const uint32_t q_at = hx_shared_address(queries) + a_row, k_at = hx_shared_address(keys) + a_row;
+  const uint32_t b_at = hx_shared_address(keys + ((matrix >> 1) * 8 + in_matrix) * STRIDE + (matrix & 1) * 8);
+#pragma unroll
+  for (int step = 0; step < STEPS; ++step) {
+    uint32_t qf[4], kf[4];
+    hx_ldmatrix_x4(qf, q_at + 32 * step);
+    hx_ldmatrix_x4(kf, k_at + 32 * step);
+#pragma unroll
+    for (int n = 0; n < 8; n += 2) {
+      if (n < tiles) {
+        uint32_t b[4];
+        hx_ldmatrix_x4(b, b_at + 2 * (8 * n * STRIDE + 16 * step));
+        hx_mma_bf16(qk[n], qf, b[0], b[1]);
+        hx_mma_bf16(qk[n + 1], qf, b[2], b[3]);
+        hx_mma_bf16(kk[n], kf, b[0], b[1]);
+        hx_mma_bf16(kk[n + 1], kf, b[2], b[3]);
+      }
+    }
+  }
+  const int row = lane >> 2, column = 2 * (lane & 3);
+#pragma unroll
+  for (int half = 0; half < 2; ++half) {
+    const int t = 16 * warp + row + 8 * half;
+    __nv_bfloat16* out = a.weights + (rows + min(t, live - 1)) * WEIGHT_COLUMNS + TERMS * CHUNK;
+#pragma unroll
+    for (int n = 0; n < 8; ++n) {
+      const int s = 8 * n + column;
+      float p[2] = {0.0f, 0.0f};
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        float held = 0.0f;
+        if (s + i <= t) {
+          const float fade = faded(t, s + i) * k_length[s + i];
+          p[i] = qk[n][2 * half + i] * (q_length[t] * fade);
+          if (s + i < t) held = kk[n][2 * half + i] * (write[t] * k_length[t] * fade);
+        }
+        system[(s + i) * SOLVE_STRIDE + t] = held;
+      }
+      if (t < live) {
+        uint32_t t0, t1, t2;
+        split_terms(p[0], p[1], t0, t1, t2);
+        *reinterpret_cast<uint32_t*>(out + s) = t0;
+        *reinterpret_cast<uint32_t*>(out + CHUNK + s) = t1;
+        *reinterpret_cast<uint32_t*>(out + 2 * CHUNK + s) = t2;
+      }
+    }
+  }
+  __syncthreads();
+  if (threadIdx.x < CHUNK) {
+    // a column of T a thread, sixteen rows at a time: what the rows in front of them leave, then
+    // the rows among themselves
+    const int j = threadIdx.x;
+#pragma unroll 1
+    for (int block = 0; block < CHUNK / 16; ++block) {
+      float x[16];
+#pragma unroll
+      for (int r = 0; r < 16; ++r) x[r] = 16 * block + r == j ? 1.0f : 0.0f;
+      if (16 * (block + 1) > (warp << 5)) {      // else all the warp's columns are zero here
+#pragma unroll 2
+        for (int s = warp << 5; s < 16 * block; ++s) {
+          const float known = solution[s * SOLVE_STRIDE + j];
+          const float4* held = reinterpret_cast<const float4*>(system + s * SOLVE_STRIDE + 16 * block);
+#pragma unroll
+          for (int r = 0; r < 4; ++r) {
+            const float4 h = held[r];
+            x[4 * r] = fmaf(-h.x, known, x[4 * r]);
+            x[4 * r + 1] = fmaf(-h.y, known, x[4 * r + 1]);
+            x[4 * r + 2] = fmaf(-h.z, known, x[4 * r + 2]);
+            x[4 * r + 3] = fmaf(-h.w, known, x[4 * r + 3]);
+          }
+        }
+#pragma unroll
+        for (int s = 0; s < 15; ++s) {
+          const float* held = system + (16 * block + s) * SOLVE_STRIDE + 16 * block;
+#pragma unroll
+          for (int r = s + 1; r < 16; ++r) x[r] = fmaf(-held[r], x[s], x[r]);
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < 16; ++r) solution[(16 * block + r) * SOLVE_STRIDE + j] = x[r];
+    }
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < live * (CHUNK / 2); i += 128) {
+    const int t = i / (CHUNK / 2), s = 2 * (i - t * (CHUNK / 2));
+    const float2 x = *reinterpret_cast<const float2*>(solution + t * SOLVE_STRIDE + s);
+    __nv_bfloat16* out = a.weights + (rows + t) * WEIGHT_COLUMNS + s;
+    uint32_t t0, t1, t2;
+    split_terms(x.x, x.y, t0, t1, t2);
+    *reinterpret_cast<uint32_t*>(out) = t0;
+    *reinterpret_cast<uint32_t*>(out + CHUNK) = t1;
+    *reinterpret_cast<uint32_t*>(out + 2 * CHUNK) = t2;
+  }
+}
+
+// Shared memory of delta_states_kernel: two stages of [queries | keys | weights | values | factors |
+// total].
+struct DeltaLayout {
+  int rows_bytes, stage_bytes, bytes;
+  __host__ __device__ DeltaLayout(int padded, int column_warps) {
+    rows_bytes = 2 * CHUNK * (2 * (padded + ROW_PAD) + WEIGHT_STRIDE + 16 * column_warps + ROW_PAD);
+    stage_bytes = rows_bytes + 16 * (CHUNK + 1);
+    bytes = 2 * stage_bytes;
+  }
+};
+
+__device__ __forceinline__ void copy_4(uint32_t dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+}
+
+// sums = x' w', with x' [16 columns x 64 tokens s] in accumulators and w [t][s] of three terms in
+// rows of the staged weights; w_ts is zero for t < s.  Six products carry 24 bits.
+__device__ __forceinline__ void triangular_product(float (&sums)[8][4], const float (&x)[8][4],
+                                                   uint32_t weights_at) {
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sums[n][j] = 0.0f;
+#pragma unroll
+  for (int step = 0; step < CHUNK / 16; ++step) {
+    uint32_t x0[4], x1[4], x2[4];
+    operand_terms(x, step, x0, x1, x2);
+#pragma unroll
+    for (int n = 2 * step; n < 8; n += 2) {
+      uint32_t w0[4], w1[4], w2[4];
+      const uint32_t at = weights_at + 2 * (8 * n * WEIGHT_STRIDE + 16 * step);
+      hx_ldmatrix_x4(w0, at);
+      hx_ldmatrix_x4(w1, at + 2 * CHUNK);
+      hx_ldmatrix_x4(w2, at + 4 * CHUNK);
+      hx_mma_bf16(sums[n], x2, w0[0], w0[1]);
+      hx_mma_bf16(sums[n + 1], x2, w0[2], w0[3]);
+      hx_mma_bf16(sums[n], x0, w2[0], w2[1]);
+      hx_mma_bf16(sums[n + 1], x0, w2[2], w2[3]);
+      hx_mma_bf16(sums[n], x1, w1[0], w1[1]);
+      hx_mma_bf16(sums[n + 1], x1, w1[2], w1[3]);
+      hx_mma_bf16(sums[n], x1, w0[0], w0[1]);
+      hx_mma_bf16(sums[n + 1], x1, w0[2], w0[3]);
+      hx_mma_bf16(sums[n], x0, w1[0], w1[1]);
+      hx_mma_bf16(sums[n + 1], x0, w1[2], w1[3]);
+    }
+  }
+#pragma unroll
+  for (int step = 0; step < CHUNK / 16; ++step) {
+    uint32_t x0[4];
+    operand_high(x, step, x0);
+#pragma unroll
+    for (int n = 2 * step; n < 8; n += 2) {
+      uint32_t w0[4];
+      hx_ldmatrix_x4(w0, weights_at + 2 * (8 * n * WEIGHT_STRIDE + 16 * step));
+      hx_mma_bf16(sums[n], x0, w0[0], w0[1]);
+      hx_mma_bf16(sums[n + 1], x0, w0[2], w0[3]);
+    }
+  }
+}
+
+// grid (requests, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
+template <int STEPS>
+__global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a) {
+  constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
+  extern __shared__ uint4 shared_pieces[];
+  hx_pdl_prologue();
+  const int request = blockIdx.x, head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
+  const int start = a.request_start[request];
+  const int count = a.request_start[request + 1] - start;
+  if (count <= 0) return;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int row = lane >> 2, pair = 2 * (lane & 3);
+  const int matrix = lane >> 3, in_matrix = lane & 7;
+  const int block_columns = 16 * a.column_warps;
+  const int column0 = blockIdx.z * block_columns;
+  const int copied = min(a.vdim - column0, block_columns);
+  const int value_stride = block_columns + ROW_PAD;
+  const DeltaLayout layout(PADDED, a.column_warps);
+  char* base = reinterpret_cast<char*>(shared_pieces);
+  auto queries_of = [&](int stage) { return reinterpret_cast<__nv_bfloat16*>(base + stage * layout.stage_bytes); };
+  auto fetch = [&](int chunk, int stage) {
+    const size_t first = start + chunk * CHUNK;
+    const int live = min(CHUNK, count - chunk * CHUNK);
+    const size_t rows = static_cast<size_t>(head) * a.rows + first;
+    __nv_bfloat16* queries = queries_of(stage);
+    __nv_bfloat16* keys = queries + CHUNK * STRIDE;
+    __nv_bfloat16* weights = keys + CHUNK * STRIDE;
+    __nv_bfloat16* values = weights + CHUNK * WEIGHT_STRIDE;
+    copy_rows<2 * STEPS>(queries, STRIDE, a.q + first * a.ld_q + qk_head * a.dim, a.ld_q, a.dim, live);
+    copy_rows<2 * STEPS>(keys, STRIDE, a.k + first * a.ld_k + qk_head * a.dim, a.ld_k, a.dim, live);
+    copy_rows<WEIGHT_COLUMNS / 8>(weights, WEIGHT_STRIDE, a.weights + rows * WEIGHT_COLUMNS, WEIGHT_COLUMNS,
+                                  WEIGHT_COLUMNS, live);
+    {
+      // a warp brings its own 16 columns of the values
+      const __nv_bfloat16* from = a.v + first * a.ld_v + head * a.vdim + column0;
+      const int column = 16 * warp + 8 * (lane & 1);
+      if (column < copied) {
+#pragma unroll
+        for (int t = lane >> 1; t < CHUNK; t += 16)
+          hx_cp_async_16(hx_shared_address(values + t * value_stride + column),
+                         t < live ? from + static_cast<size_t>(t) * a.ld_v + column : from, t < live ? 16 : 0);
+      }
+    }
+    const uint32_t factors = hx_shared_address(base + stage * layout.stage_bytes + layout.rows_bytes);
+    for (int t = threadIdx.x; t < CHUNK; t += blockDim.x)
+      hx_cp_async_16(factors + 16 * t, a.factors + rows + (t < live ? t : 0), t < live ? 16 : 0);
+    if (threadIdx.x == 0) copy_4(factors + 16 * CHUNK, a.total + rows);
+    hx_cp_async_commit();
+  };
+  // what the copies leave alone
+  for (int stage = 0; stage < 2; ++stage) {
+    __nv_bfloat16* queries = queries_of(stage);
+    if (PADDED > a.dim) {
+      clear_columns(queries, STRIDE, a.dim, PADDED);
+      clear_columns(queries + CHUNK * STRIDE, STRIDE, a.dim, PADDED);
+    }
+    if (copied < block_columns)
+      clear_columns(queries + CHUNK * (2 * STRIDE + WEIGHT_STRIDE), value_stride, copied, block_columns);
+  }
+  fetch(0, 0);
+
+  // the warp's part of S': columns my_column (+ 8), key coordinates 8 n + pair (+ 1)
+  float* s_state = a.state + static_cast<size_t>(a.request_slot[request]) * a.state_stride +
+                   static_cast<size_t>(head) * a.head_stride;
+  const int lanes = a.vdim * a.parts;
+  const int my_column = column0 + 16 * warp + row;
+  float S[2 * STEPS][4];
+#pragma unroll
+  for (int n = 0; n < 2 * STEPS; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = my_column + 8 * (j >> 1), d = 8 * n + pair + (j & 1);
+      S[n][j] = c < a.vdim && d < a.dim
+                    ? s_state[static_cast<size_t>(d & 15) * lanes + c * a.parts + (d >> 4)] : 0.0f;
+    }
+  // offsets of the lane's rows in the operands
+  const uint32_t row_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * STRIDE + (matrix & 1) * 8);
+  const uint32_t key_lane = 2 * (((matrix & 1) * 8 + in_matrix) * STRIDE + (matrix >> 1) * 8);
+  const uint32_t weight_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * WEIGHT_STRIDE + (matrix & 1) * 8);
+  const uint32_t value_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * value_stride + 16 * warp + (matrix & 1) * 8);
+  const int chunks = (count + CHUNK - 1) / CHUNK;
+  for (int chunk = 0; chunk < chunks; ++chunk) {
+    const int stage = chunk & 1;
+    hx_cp_async_wait<0>();
+    __syncthreads();
+    if (chunk + 1 < chunks) fetch(chunk + 1, stage ^ 1);
+    const uint32_t queries = hx_shared_address(queries_of(stage));
+    const uint32_t keys = queries + 2 * CHUNK * STRIDE;
+    const uint32_t weights = keys + 2 * CHUNK * STRIDE;
+    const uint32_t values = weights + 2 * CHUNK * WEIGHT_STRIDE;
+    const float4* factors = reinterpret_cast<const float4*>(base + stage * layout.stage_bytes + layout.rows_bytes);
+
+    // S_0' q and S_0' k of all tokens, [16 columns x 64 tokens] each
+    float out[8][4], rest[8][4];
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) out[n][j] = rest[n][j] = 0.0f;
+#pragma unroll
+    for (int step = 0; step < STEPS; ++step) {
+      uint32_t s0[4], s1[4], s2[4];
+      operand_terms(S, step, s0, s1, s2);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t kf[4], qf[4];
+        hx_ldmatrix_x4(kf, keys + row_lane + 2 * (8 * n * STRIDE + 16 * step));
+        hx_ldmatrix_x4(qf, queries + row_lane + 2 * (8 * n * STRIDE + 16 * step));
+        hx_mma_bf16(rest[n], s2, kf[0], kf[1]);
+        hx_mma_bf16(rest[n + 1], s2, kf[2], kf[3]);
+        hx_mma_bf16(out[n], s2, qf[0], qf[1]);
+        hx_mma_bf16(out[n + 1], s2, qf[2], qf[3]);
+        hx_mma_bf16(rest[n], s1, kf[0], kf[1]);
+        hx_mma_bf16(rest[n + 1], s1, kf[2], kf[3]);
+        hx_mma_bf16(out[n], s1, qf[0], qf[1]);
+        hx_mma_bf16(out[n + 1], s1, qf[2], qf[3]);
+      }
+    }
+#pragma unroll
+    for (int step = 0; step < STEPS; ++step) {
+      uint32_t s0[4];
+      operand_high(S, step, s0);
+#pragma unroll
+      for (int n = 0; n < 8; n += 2) {
+        uint32_t kf[4], qf[4];
+        hx_ldmatrix_x4(kf, keys + row_lane + 2 * (8 * n * STRIDE + 16 * step));
+        hx_ldmatrix_x4(qf, queries + row_lane + 2 * (8 * n * STRIDE + 16 * step));
+        hx_mma_bf16(rest[n], s0, kf[0], kf[1]);
+        hx_mma_bf16(rest[n + 1], s0, kf[2], kf[3]);
+        hx_mma_bf16(out[n], s0, qf[0], qf[1]);
+        hx_mma_bf16(out[n + 1], s0, qf[2], qf[3]);
+      }
+    }
+    // R: what the values leave to be written
+#pragma unroll
+    for (int step = 0; step < CHUNK / 16; ++step) {
+      uint32_t v[4];      // in the order of two neighbouring accumulator tiles
+      hx_ldmatrix_x4_trans(v, values + value_lane + 2 * (16 * step * value_stride));
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        const int n = 2 * step + i;
+        const float4 f0 = factors[8 * n + pair], f1 = factors[8 * n + pair + 1];
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[2 * i + half]));
+          rest[n][2 * half] = fmaf(f0.z, x.x, -f0.y * rest[n][2 * half]);
+          rest[n][2 * half + 1] = fmaf(f1.z, x.y, -f1.y * rest[n][2 * half + 1]);
+          out[n][2 * half] *= f0.x;
+          out[n][2 * half + 1] *= f1.x;
+        }
+      }
+    }
+    float u[8][4];
+    triangular_product(u, rest, weights + weight_lane);
+    triangular_product(rest, u, weights + weight_lane + 2 * TERMS * CHUNK);
+    {
+      const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int t = 8 * n + pair + (j & 1), c = my_column + 8 * (j >> 1);
+          if (t < live && c < a.vdim)
+            a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j] + rest[n][j];
+        }
+    }
+    // the state behind the chunk
+    const float total = factors[CHUNK].x;
+#pragma unroll
+    for (int n = 0; n < 2 * STEPS; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) S[n][j] *= total;
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) u[n][j] *= factors[8 * n + pair + (j & 1)].w;
+#pragma unroll
+    for (int step = 0; step < CHUNK / 16; ++step) {
+      uint32_t u0[4], u1[4], u2[4];
+      operand_terms(u, step, u0, u1, u2);
+#pragma unroll
+      for (int n = 0; n < STEPS; ++n) {
+        uint32_t b[4];
+        hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * n));
+        hx_mma_bf16(S[2 * n], u2, b[0], b[1]);
+        hx_mma_bf16(S[2 * n + 1], u2, b[2], b[3]);
+        hx_mma_bf16(S[2 * n], u1, b[0], b[1]);
+        hx_mma_bf16(S[2 * n + 1], u1, b[2], b[3]);
+        hx_mma_bf16(S[2 * n], u0, b[0], b[1]);
+        hx_mma_bf16(S[2 * n + 1], u0, b[2], b[3]);
+      }
+    }
+  }
+#pragma unroll
+  for (int n = 0; n < 2 * STEPS; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = my_column + 8 * (j >> 1), d = 8 * n + pair + (j & 1);
+      if (c < a.vdim && d < a.dim)
+        s_state[static_cast<size_t>(d & 15) * lanes + c * a.parts + (d >> 4)] = S[n][j];
+    }
+}
+
+template <int STEPS>
+int launch_delta(const DeltaArgs& a, int tiles, cudaStream_t stream) {
+  const int shared = DeltaLayout(16 * STEPS, a.column_warps).bytes, first = weights_shared(16 * STEPS);
+  if (cudaFuncSetAttribute(delta_weights_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           first) != cudaSuccess ||
+      cudaFuncSetAttribute(delta_states_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                           227 * 1024) != cudaSuccess) {
+    cudaGetLastError();
+    hx_set_error("hx_delta_chunks: the device refuses %d bytes of shared memory", shared);
+    return HX_ERR_LAUNCH;
+  }
+  hx_launch(delta_weights_kernel<STEPS>, dim3(tiles, a.heads), 128, first, stream, a);
+  const int block_columns = 16 * a.column_warps;
+  hx_launch(delta_states_kernel<STEPS>, dim3(a.requests, a.heads, (a.vdim + block_columns - 1) / block_columns),
+            32 * a.column_warps, shared, stream, a);
+  return HX_OK;
+}
+
+}  // namespace
+
+// 1: heads of these sizes run here (bfloat16); else they take the token-by-token scan.
+HX_API int hx_delta_chunks_supports(int dim, int vdim) {
+  return dim > 0 && vdim > 0 && dim % 8 == 0 && vdim % 8 == 0 && dim <= 128 ? 1 : 0;
+}
+
+// Bytes of scratch for a step of `tokens` tokens.
+HX_API long long hx_delta_chunks_scratch(int heads, int tokens) {
+  return static_cast<long long>(heads) * tokens * (2 * WEIGHT_COLUMNS + 16 + 4);
+}
+
+// See the head of this file.  q, k [tokens, qk_heads * dim] and v [tokens, heads * vdim] bfloat16
+// rows on 16 bytes; decay_in, beta_in, a_log, dt_bias, fixed_decay_m1, the scales, the state and o
+// as for hx_linear_state_scan with its delta rule and without a rotation.  scratch:
+// hx_delta_chunks_scratch bytes on 16 bytes.  tiles: at least the chunks of 64 tokens in the step,
+// counted request by request.
+HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                           const void* decay_in, const void* beta_in, int ld_gates,
+                           const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
+                           int unit_norm, float unit_eps, float q_scale, float k_scale,
+                           void* scratch, float* state, long long state_stride, int head_stride,
+                           float* o, const int* request_start, const int* request_slot,
+                           int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
+                           int vdim, cudaStream_t stream) {
+  HX_REQUIRE(hx_delta_chunks_supports(dim, vdim), "hx_delta_chunks: heads of %d by %d are not supported",
+             dim, vdim);
+  HX_REQUIRE(requests >= 0 && tokens >= requests && tiles >= requests && heads > 0 && heads <= 65535 &&
+                 qk_heads > 0 && heads % qk_heads == 0,
+             "hx_delta_chunks: bad sizes");
+  HX_REQUIRE(ld_q % 8 == 0 && ld_k % 8 == 0 && ld_v % 8 == 0 && ld_q >= qk_heads * dim &&
+                 ld_k >= qk_heads * dim && ld_v >= heads * vdim && ld_gates >= heads,
+             "hx_delta_chunks: bad strides");
+  HX_REQUIRE(((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(k) |
+               reinterpret_cast<uintptr_t>(v) | reinterpret_cast<uintptr_t>(scratch)) & 15) == 0,
+             "hx_delta_chunks: rows are not 16-byte aligned");
+  HX_REQUIRE(beta_in != nullptr && scratch != nullptr &&
+                 (decay_in != nullptr ? (a_log != nullptr && dt_bias != nullptr) : fixed_decay_m1 != nullptr),
+             "hx_delta_chunks: gates missing");
+  HX_REQUIRE(head_stride >= state_floats(vdim, dim), "hx_delta_chunks: a head's state takes %d floats, not %d",
+             state_floats(vdim, dim), head_stride);
+  if (requests == 0) return HX_OK;
+  // four warps of 16 columns a CTA, one for each quarter of an SM (the staged chunks leave room for
+  // one CTA); eight where there are more CTAs than SMs, so that a chunk is staged for twice as many
+  const int sms = hx_device_sm_count();
+  if (sms <= 0) return HX_ERR_LAUNCH;
+  const long long ctas = static_cast<long long>(requests) * heads * ((vdim + 63) / 64);
+  const int column_warps = vdim > 64 && ctas > sms ? 8 : vdim > 32 ? 4 : (vdim + 15) / 16;
+  const size_t rows = static_cast<size_t>(heads) * tokens;
+  float4* factors = static_cast<float4*>(scratch);
+  __nv_bfloat16* weights = reinterpret_cast<__nv_bfloat16*>(factors + rows);
+  float* total = reinterpret_cast<float*>(weights + rows * WEIGHT_COLUMNS);
+  const DeltaArgs a{static_cast<const __nv_bfloat16*>(q), static_cast<const __nv_bfloat16*>(k),
+                    static_cast<const __nv_bfloat16*>(v), ld_q, ld_k, ld_v,
+                    static_cast<const __nv_bfloat16*>(decay_in), static_cast<const __nv_bfloat16*>(beta_in),
+                    ld_gates, a_log, dt_bias, fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, weights,
+                    factors, total, tokens, state, state_stride, head_stride, o, request_start, request_slot,
+                    requests, heads, qk_heads, dim, vdim, parts_for(dim), column_warps};
+  int rc;
+  switch ((dim + 15) / 16) {
+    case 1: case 2: rc = launch_delta<2>(a, tiles, stream); break;
+    case 3: case 4: rc = launch_delta<4>(a, tiles, stream); break;
+    case 5: case 6: rc = launch_delta<6>(a, tiles, stream); break;
+    default: rc = launch_delta<8>(a, tiles, stream); break;
+  }
+  if (rc != HX_OK) return rc;
+  hx_count_launches(1);
+  HX_CHECK_LAUNCH("hx_delta_chunks");
+  return HX_OK;
+}

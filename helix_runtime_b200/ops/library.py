@@ -315,6 +315,15 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_float, _c_ptr, _c_ptr,
         _c_ptr, _c_int, _c_int, _c_float, _c_float, _c_ptr, _c_float, _c_ptr, _c_longlong, _c_ptr,
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
+    library.hx_delta_chunks_supports.argtypes = [_c_int, _c_int]
+    library.hx_delta_chunks_supports.restype = _c_int
+    library.hx_delta_chunks_scratch.argtypes = [_c_int, _c_int]
+    library.hx_delta_chunks_scratch.restype = _c_longlong
+    library.hx_delta_chunks.argtypes = [
+        _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr,
+        _c_ptr, _c_int, _c_float, _c_float, _c_float, _c_ptr, _c_ptr, _c_longlong, _c_int, _c_ptr,
+        _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
+    library.hx_delta_chunks.restype = _c_int
     library.hx_state_chunks_supports.argtypes = [_c_int, _c_int]
     library.hx_state_chunks_scratch.argtypes = [_c_int, _c_int]
     library.hx_state_chunks_scratch.restype = _c_longlong
@@ -1285,6 +1294,51 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
         float(unit_eps), float(q_scale), float(k_scale), state.data_ptr(), state.stride(0),
         head_stride, o.data_ptr(), request_start.data_ptr(), request_slot.data_ptr(), requests,
         q.shape[0] if tokens is None else tokens, heads, qk_heads, dim, vdim, _stream()))
+
+
+def delta_chunks_supports(dim: int, vdim: int) -> bool:
+    """Whether :func:`delta_chunks` takes heads of these sizes."""
+    return bool(lib().hx_delta_chunks_supports(dim, vdim))
+
+
+def delta_chunks_scratch(heads: int, tokens: int) -> int:
+    """Bytes of the scratch of :func:`delta_chunks`."""
+    return lib().hx_delta_chunks_scratch(heads, tokens)
+
+
+def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch.Tensor,
+                 o: torch.Tensor, scratch: torch.Tensor, request_start: torch.Tensor,
+                 request_slot: torch.Tensor, requests: int, tokens: int, tiles: int, heads: int,
+                 qk_heads: int, dim: int, vdim: int, *, beta_in: torch.Tensor,
+                 decay_in: Optional[torch.Tensor] = None, a_log: Optional[torch.Tensor] = None,
+                 dt_bias: Optional[torch.Tensor] = None,
+                 fixed_decay_m1: Optional[torch.Tensor] = None, unit_norm: bool = False,
+                 unit_eps: float = 0.0, q_scale: float = 1.0, k_scale: float = 1.0) -> None:
+    """The ``delta`` rule of :func:`linear_state_scan` without a rotation, 64 tokens at a time on
+    the tensor cores (bfloat16 rows on 16 bytes); arguments as there.  ``scratch``:
+    :func:`delta_chunks_scratch` bytes; ``tiles``: :func:`recurrence_tiles` of the step."""
+    _need(state, torch.float32, "state")
+    _need(o, torch.float32, "o")
+    for tensor in (q, k, v, beta_in):
+        _need(tensor, torch.bfloat16, "a bfloat16 argument")
+        assert tensor.stride(-1) == 1
+    assert o.is_contiguous() and o.shape[1] == heads * vdim
+    head_stride = scan_state_floats(vdim, dim)
+    assert state.shape[1] >= heads * head_stride
+    assert decay_in is None or (decay_in.dtype == q.dtype and decay_in.stride(-1) == 1
+                                and decay_in.stride(0) == beta_in.stride(0))
+    for name, tensor in (("a_log", a_log), ("dt_bias", dt_bias),
+                         ("fixed_decay_m1", fixed_decay_m1)):
+        if tensor is not None:
+            _need(tensor, torch.float32, name)
+    assert scratch.numel() * scratch.element_size() >= delta_chunks_scratch(heads, tokens)
+    _check(lib().hx_delta_chunks(
+        q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
+        _ptr(decay_in), beta_in.data_ptr(), beta_in.stride(0), _ptr(a_log), _ptr(dt_bias),
+        _ptr(fixed_decay_m1), 1 if unit_norm else 0, float(unit_eps), float(q_scale),
+        float(k_scale), scratch.data_ptr(), state.data_ptr(), state.stride(0), head_stride,
+        o.data_ptr(), request_start.data_ptr(), request_slot.data_ptr(), requests, tokens, tiles,
+        heads, qk_heads, dim, vdim, _stream()))
 
 
 # ------------------------------------------------------------- gated residual connection

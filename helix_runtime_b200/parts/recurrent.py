@@ -362,6 +362,19 @@ class LinearState(Mixer):
             self.rotary_dims = dims
             self.rotary_layout = ops.ROTARY_LAYOUTS[self.rotary.get("layout", "halves")]
 
+    # The chunks' two kernels take about as long for one portion of up to 64 tokens as the scan
+    # for 35 (32 heads of 128 by 128: 43 us against 39 for 32 tokens, 73 for 64); with more
+    # requests they win earlier (16 portions of 32: 149 us against 258).
+    CHUNKS_FROM_TOKENS = 32
+
+    def runs_in_chunks(self, ctx: StepContext, qkv: torch.Tensor) -> bool:
+        """Whether the recurrence takes this step 64 tokens at a time on the tensor cores: the
+        delta rule in bfloat16 without a rotation (turned queries and keys are float32 numbers
+        that no stored row holds), for a step with a prompt portion in it."""
+        return (self.rule == "delta" and not self.rotary_dims and ctx.dtype == torch.bfloat16
+                and ctx.max_query_len >= self.CHUNKS_FROM_TOKENS and qkv.stride(0) % 8 == 0
+                and ops.delta_chunks_supports(self.head_dim, self.value_dim))
+
     def weight_bytes(self) -> int:
         return self.w_in.nbytes() + self.w_o.nbytes()
 
@@ -384,20 +397,30 @@ class LinearState(Mixer):
                               n, True,
                               ctx.token_request, ctx.request_slot, ctx.request_start)
         learned = self.fixed_decay is None
-        ops.linear_state_scan(
-            qkv[:, :self.qk_width], qkv[:, self.qk_width:2 * self.qk_width],
-            qkv[:, 2 * self.qk_width:self.filtered],
-            _state_piece(cache, self.filter_state, self.matrix_state), o, ctx.request_start,
-            ctx.request_slot, ctx.n_requests, self.heads, self.qk_heads, self.head_dim,
-            self.value_dim, delta=self.rule == "delta",
+        q, k, v = (qkv[:, begin:end] for begin, end in
+                   ((0, self.qk_width), (self.qk_width, 2 * self.qk_width),
+                    (2 * self.qk_width, self.filtered)))
+        state = _state_piece(cache, self.filter_state, self.matrix_state)
+        gates = dict(
             decay_in=rows[:, self.decay_at:self.decay_at + self.heads] if learned else None,
             beta_in=rows[:, self.beta_at:self.beta_at + self.heads] if self.rule == "delta" else None,
-            a_log=self.a_log, dt_bias=self.dt_bias, fixed_decay=self.decay,
-            fixed_decay_m1=self.decay_m1,
-            positions=ctx.positions if self.rotary_dims else None, freq=self.freq,
-            freq_exact=self.freq_exact, rotary_dim=self.rotary_dims,
-            rotary_layout=self.rotary_layout, unit_norm=self.unit_norm, unit_eps=self.unit_eps,
-            q_scale=self.q_scale, k_scale=self.k_scale, tokens=n)
+            a_log=self.a_log, dt_bias=self.dt_bias, fixed_decay_m1=self.decay_m1,
+            unit_norm=self.unit_norm, unit_eps=self.unit_eps, q_scale=self.q_scale,
+            k_scale=self.k_scale)
+        if self.runs_in_chunks(ctx, qkv):
+            scratch = ctx.workspace.get(
+                f"linear_state.chunks/{self.heads}",
+                (ops.delta_chunks_scratch(self.heads, ctx.capacity),), torch.uint8)
+            ops.delta_chunks(q, k, v, state, o, scratch, ctx.request_start, ctx.request_slot,
+                             ctx.n_requests, n, ops.recurrence_tiles(ctx.host_query_lengths),
+                             self.heads, self.qk_heads, self.head_dim, self.value_dim, **gates)
+        else:
+            ops.linear_state_scan(
+                q, k, v, state, o, ctx.request_start, ctx.request_slot, ctx.n_requests, self.heads,
+                self.qk_heads, self.head_dim, self.value_dim, delta=self.rule == "delta",
+                fixed_decay=self.decay, positions=ctx.positions if self.rotary_dims else None,
+                freq=self.freq, freq_exact=self.freq_exact, rotary_dim=self.rotary_dims,
+                rotary_layout=self.rotary_layout, tokens=n, **gates)
         ops.gated_group_norm(o, rows[:, self.gate_at:self.gate_at + self.v_width], self.norm, gated,
                              n, self.heads, self.eps, gate_after=True)
         project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)

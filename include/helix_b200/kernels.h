@@ -402,6 +402,19 @@ int hx_state_chunks(const void* q, const void* k, const void* v, int ld, float* 
                     const int* request_start, const int* request_slot, int requests, int tiles,
                     int heads, int dim, int vdim, cudaStream_t stream);
 
+/* the delta rule of hx_linear_state_scan (no rotation) 64 tokens at a time on the tensor cores
+ * (bfloat16, heads of up to 128 by any multiple of 8): scratch of hx_delta_chunks_scratch bytes;
+ * tiles: at least the step's chunks of 64 tokens, counted request by request */
+int hx_delta_chunks_supports(int dim, int vdim);
+long long hx_delta_chunks_scratch(int heads, int tokens);
+int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                    const void* decay_in, const void* beta_in, int ld_gates, const float* a_log,
+                    const float* dt_bias, const float* fixed_decay_m1, int unit_norm,
+                    float unit_eps, float q_scale, float k_scale, void* scratch, float* state,
+                    long long state_stride, int head_stride, float* o, const int* request_start,
+                    const int* request_slot, int requests, int tokens, int tiles, int heads,
+                    int qk_heads, int dim, int vdim, cudaStream_t stream);
+
 /* ---- attention over a cached latent ----------------------------------------------------- */
 /* down [tokens][q_rank + kv_rank + rot] float32: both latents RMS-normed with a weight; the
  * query latent goes to query_latent; the key row [c | rot(kr) | 0..] and the value row

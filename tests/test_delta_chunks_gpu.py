@@ -1,0 +1,111 @@
+"""The delta rule by chunks of 64 tokens against the recurrence in double, token by token: outputs
+and the state left behind, at the edges of chunks, head sizes and column blocks."""
+from __future__ import annotations
+
+import numpy as np
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+def rounded(array):
+    return torch.tensor(np.asarray(array), dtype=torch.float32).to(torch.bfloat16).cuda()
+
+
+def plain(q, k, v, beta, log_decay, state):
+    """``q, k [T, H, D]``, ``v [T, H, V]``, state ``[H, D, V]``, all double."""
+    out = np.zeros((q.shape[0], q.shape[1], v.shape[2]))
+    for t in range(q.shape[0]):
+        state = np.exp(log_decay[t])[:, None, None] * state
+        u = beta[t][:, None] * (v[t] - np.einsum("hdv,hd->hv", state, k[t]))
+        state = state + k[t][:, :, None] * u[:, None]
+        out[t] = np.einsum("hdv,hd->hv", state, q[t])
+    return out, state
+
+
+def packed_state(state, per_head):
+    """``[H, D, V]`` as a request's state row keeps it: [row % 16][column][row / 16]."""
+    heads, dim, vdim = state.shape
+    parts = per_head // (16 * vdim)
+    wide = np.zeros((heads, 16 * parts, vdim))
+    wide[:, :dim] = state
+    return wide.reshape(heads, parts, 16, vdim).transpose(0, 2, 3, 1).reshape(heads, -1)
+
+
+@pytest.mark.parametrize("unit", [True, False])
+@pytest.mark.parametrize("heads,qk_heads,dim,vdim,lengths", [
+    (4, 2, 128, 128, (64, 1, 129)),        # whole chunks, a single token, one token over
+    (2, 2, 120, 136, (65, 63)),            # padded keys, a second block of columns
+    (3, 1, 48, 40, (200,)),
+    (2, 1, 8, 8, (1, 16, 17, 2)),          # the smallest heads
+    (40, 40, 64, 128, (3, 70, 1, 5)),      # more blocks than SMs: eight warps of columns
+])
+def test_chunks_against_the_recurrence(heads, qk_heads, dim, vdim, lengths, unit):
+    from helix_runtime_b200.ops import library as ops
+    rng = np.random.default_rng(dim + vdim + unit)
+    tokens = sum(lengths)
+    q, k = (rounded(rng.normal(size=(tokens, qk_heads * dim))) for _ in range(2))
+    v = rounded(rng.normal(size=(tokens, heads * vdim)))
+    gates = rounded(rng.normal(size=(tokens, 2 * heads)) * 2.0)
+    a_log = rng.uniform(np.log(0.01), np.log(4.0), size=heads).astype(np.float32)
+    dt_bias = rng.uniform(-3.0, 2.0, size=heads).astype(np.float32)
+    fixed = (1.0 - 2.0 ** -rng.uniform(2.0, 9.0, size=heads)).astype(np.float32)
+    per_head = ops.scan_state_floats(vdim, dim)
+    slots = [int(s) for s in rng.permutation(len(lengths) + 2)[:len(lengths)]]
+    before = rng.normal(size=(len(lengths), heads, dim, vdim)).astype(np.float32)
+    state = torch.full((len(lengths) + 2, heads * per_head + 3), 7.0, device="cuda")
+    for r, slot in enumerate(slots):
+        state[slot, :heads * per_head] = torch.tensor(
+            packed_state(before[r], per_head).reshape(-1), dtype=torch.float32)
+    o = torch.full((tokens, heads * vdim), float("nan"), device="cuda")
+    scratch = torch.full((ops.delta_chunks_scratch(heads, tokens) // 4 + 1,), float("nan"),
+                         device="cuda")
+    starts = np.concatenate([[0], np.cumsum(lengths)]).astype(np.int32)
+    options = dict(unit_norm=True, unit_eps=1e-6, q_scale=dim ** -0.5) if unit else \
+        dict(q_scale=0.5, k_scale=0.9 * dim ** -0.5)
+    if unit:
+        options.update(decay_in=gates[:, heads:], a_log=torch.tensor(a_log).cuda(),
+                       dt_bias=torch.tensor(dt_bias).cuda())
+    else:
+        options.update(fixed_decay_m1=torch.tensor(fixed - 1.0).cuda())
+    ops.delta_chunks(q, k, v, state, o, scratch, torch.tensor(starts).cuda(),
+                     torch.tensor(slots, dtype=torch.int32).cuda(), len(lengths), tokens,
+                     ops.recurrence_tiles(lengths), heads, qk_heads, dim, vdim,
+                     beta_in=gates[:, :heads], **options)
+    qd, kd, vd, gd = (t.double().cpu().numpy() for t in (q, k, v, gates))
+    qd, kd = (x.reshape(tokens, qk_heads, dim) for x in (qd, kd))
+    if unit:
+        qd = qd / np.sqrt((qd * qd).sum(-1, keepdims=True) + 1e-6) * dim ** -0.5
+        kd = kd / np.sqrt((kd * kd).sum(-1, keepdims=True) + 1e-6)
+        log_decay = -np.exp(a_log.astype(np.float64)) * np.logaddexp(0.0, gd[:, heads:] + dt_bias)
+    else:
+        qd, kd = qd * 0.5, kd * np.float32(0.9 * dim ** -0.5)
+        log_decay = np.broadcast_to(np.log(fixed.astype(np.float64)), (tokens, heads))
+    share = heads // qk_heads
+    qd, kd = np.repeat(qd, share, 1), np.repeat(kd, share, 1)
+    beta = 1.0 / (1.0 + np.exp(-gd[:, :heads]))
+    got_state = state.cpu().numpy()
+    for r, slot in enumerate(slots):
+        rows = slice(starts[r], starts[r + 1])
+        want, after = plain(qd[rows], kd[rows], vd.reshape(tokens, heads, vdim)[rows], beta[rows],
+                            log_decay[rows], before[r].astype(np.float64))
+        # a chain of at most four float32 sums of up to 128 terms, each with a relative error of
+        # 128 * 2^-24 at worst and some sqrt(128) * 2^-24 in earnest; the writes of a chunk
+        # depend on one another, which multiplies it by a few
+        bound = 8 * 128 ** 0.5 * 2.0 ** -24
+        got = o[rows].cpu().numpy().reshape(want.shape)
+        assert np.isfinite(got).all()
+        assert np.linalg.norm(got - want) <= bound * np.linalg.norm(want)
+        error = got_state[slot, :heads * per_head] - packed_state(after, per_head).reshape(-1)
+        assert np.linalg.norm(error) <= bound * np.linalg.norm(after)
+        assert (got_state[slot, heads * per_head:] == 7.0).all()
+    untouched = [s for s in range(len(lengths) + 2) if s not in slots]
+    assert (got_state[untouched] == 7.0).all()
+
+
+def test_refusals():
+    from helix_runtime_b200.ops import library as ops
+    assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
+    assert not ops.delta_chunks_supports(136, 8) and not ops.delta_chunks_supports(20, 8)
+    assert not ops.delta_chunks_supports(16, 12)
