@@ -36,8 +36,10 @@
 // page table alike, then first pages, rewrite, the chain of first products; at the end the last
 // product and the output) is spent once for 256 rows, and every key tile is fetched and rewritten
 // once for them.  The issuing threads are picked by elect.sync: behind `lane == 0` a thread
-// needed 55 ns to issue a product of any size (2,048 tokens, 32 heads of 128: 129 us a layer in
-// place, 108 with elect.sync).
+// needed 55 ns to issue a product of any size.  Measured (2,048 tokens, 32 heads of 128, in place): 129
+// us a layer, 108 with elect.sync, 87 with the softmax's arithmetic in pairs (its instructions are
+// what bounds the kernel).  Wide heads (2,048 tokens, 32 heads of 256 over one cached row, window
+// 1,024): 610 us on mma.sync, 133 here.
 //
 // Operand layouts.  Nothing is swizzled: every operand is made of "core matrices" of 8 rows
 // x 16 bytes (128 contiguous bytes), which is exactly what a page block of the cache is made
@@ -58,13 +60,8 @@
 namespace {
 
 constexpr int BLOCK_M = 128;   // query rows per lane (the MMA's M)
-constexpr int LANES = 2;       // lanes per CTA: 256 query rows
 constexpr int BLOCK_N = 64;    // keys per tile
-constexpr int K_STAGES = 2;    // key tiles in shared memory as they land (rewritten at once)
-constexpr int V_STAGES = 4;    // value tiles in shared memory (held until both products are done)
-constexpr int KEY_BUFFERS = 3; // rewritten key tiles in shared memory
 constexpr int S_BUFFERS = 2;   // score tiles in tensor memory per lane
-constexpr int THREADS = 512;
 constexpr int WARP_KEYS = 0, WARP_VALUES = 1, WARP_REWRITE = 2, WARP_SCORES = 3, WARP_OUTPUT = 5,
               WARP_SOFTMAX = 8;
 constexpr int GROUP_STRIDE = 128;             // bytes from one 8-row core matrix to the next row group
@@ -100,25 +97,68 @@ struct TcPrefillArgs {
   const float* slopes = nullptr;
   int chunk = 0;          // > 0: positions see each other only inside chunks of this many
   float softcap = 0.0f;   // > 0: the scaled score s becomes softcap * tanh(s / softcap)
+  int pack = 1;           // packed kernels: the query heads of a key/value head, side by side in
+                          // a tile's rows, token by token; the grid's x counts key/value heads
 };
 
+// Heads of up to 128: two lanes.  Wider ones: tensor memory holds the output of one lane, shared
+// memory its queries and fewer tiles, and four warps share the rewriting of a tile, which is
+// twice as large for half the rows.
 template <int D>
 struct TcConfig {
+  static constexpr int kLanes = D <= 128 ? 2 : 1;
+  static constexpr int kKeyStages = D <= 128 ? 2 : 1;      // key tiles in shared memory as they land
+  static constexpr int kValueStages = D <= 128 ? 4 : 2;    // value tiles, held until multiplied
+  static constexpr int kKeyBuffers = D <= 128 ? 3 : 2;     // rewritten key tiles
+  static constexpr int kRewriters = D <= 128 ? 1 : 4;
+  static constexpr int kThreads = 256 + 128 * kLanes;
   static constexpr int kQBytes = BLOCK_M * D * 2;              // per lane
   static constexpr int kHalfBytes = BLOCK_N * D * 2;          // keys (or values) of a tile
   static constexpr int kSmemBytes =
-      LANES * kQBytes + (K_STAGES + V_STAGES + KEY_BUFFERS) * kHalfBytes + 1024 + 512;
+      kLanes * kQBytes + (kKeyStages + kValueStages + kKeyBuffers) * kHalfBytes + 1024 + 512;
   static constexpr int kScoreColumns = BLOCK_N;               // per score buffer
   static constexpr int kLowTermColumn = BLOCK_N / 2;          // P: hi in columns [0, 32), lo after
-  static constexpr int kOutputColumn = LANES * S_BUFFERS * BLOCK_N;   // lane 0's O; lane 1's follows
+  static constexpr int kOutputColumn = kLanes * S_BUFFERS * BLOCK_N;  // lane 0's O; lane 1's follows
   static constexpr int kTmemColumns = 512;
-  static_assert(LANES * (S_BUFFERS * BLOCK_N + D) <= 512, "tensor memory has 512 columns");
+  static_assert(kLanes * (S_BUFFERS * BLOCK_N + D) <= 512, "tensor memory has 512 columns");
+  static_assert(kSmemBytes <= 227 * 1024, "a CTA has 227 KB of shared memory");
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
   return y;
+}
+
+// Two float32 operations in one instruction, each rounded as its scalar form; and the largest of
+// three.  The softmax is bound by the instructions it issues: these take half of them off.
+__device__ __forceinline__ uint64_t pair_of(float low, float high) {
+  uint64_t pair;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(pair) : "f"(low), "f"(high));
+  return pair;
+}
+__device__ __forceinline__ void halves_of(uint64_t pair, float& low, float& high) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(pair));
+}
+__device__ __forceinline__ uint64_t pair_fma(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  return r;
+}
+__device__ __forceinline__ uint64_t pair_add(uint64_t x, uint64_t y) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+  return r;
+}
+__device__ __forceinline__ float max_of_3(float x, float y, float z) {
+  float r;
+  asm("max.f32 %0, %1, %2, %3;" : "=f"(r) : "f"(x), "f"(y), "f"(z));
+  return r;
+}
+
+__device__ __forceinline__ uint32_t pack_bf16(float low, float high) {
+  const __nv_bfloat162 pair = __floats2bfloat162_rn(low, high);
+  return *reinterpret_cast<const uint32_t*>(&pair);
 }
 
 __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_t bytes,
@@ -129,18 +169,26 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
-template <int D>
-__global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPrefillArgs a) {
+template <int D, bool PACKED>
+__global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc_kernel(
+    TcPrefillArgs a) {
   using Config = TcConfig<D>;
+  constexpr int LANES = Config::kLanes, THREADS = Config::kThreads;
+  constexpr int K_STAGES = Config::kKeyStages, V_STAGES = Config::kValueStages;
+  constexpr int KEY_BUFFERS = Config::kKeyBuffers, REWRITERS = Config::kRewriters;
   constexpr int kDSteps = D / 16;      // k-steps of Q K^T
   hx_pdl_trigger();
 
   // which request and which 256-row tile of it is this CTA?  The last rows of a request see
   // the most keys: their CTAs are started first (the grid is walked heads first, then tiles),
   // so the short ones fill the gaps at the end.
+  // A row is a token of one head, or with PACKED one of the `pack` heads of a token.
+  const int pack = PACKED ? a.pack : 1;
+  auto token_of = [&](int row) { return PACKED ? row / pack : row; };
+  const int tile_tokens = token_of(LANES * BLOCK_M);
   int tile_in_request = 0, tiles_of_request = 0;
   const int request = hx_find_query_tile(a.request_start, a.requests, a.min_query_len,
-                                         LANES * BLOCK_M, blockIdx.y, tile_in_request,
+                                         tile_tokens, blockIdx.y, tile_in_request,
                                          tiles_of_request);
   tile_in_request = tiles_of_request - 1 - tile_in_request;
   if (request < 0) return;      // before any barrier or allocation: the whole CTA leaves
@@ -167,31 +215,33 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int head = blockIdx.x;
-  const int kv_head = head / (a.heads / a.kv_heads);
+  const int head0 = PACKED ? blockIdx.x * pack : blockIdx.x;      // of a token's first row
+  const int kv_head = PACKED ? blockIdx.x : blockIdx.x / (a.heads / a.kv_heads);
+  auto head_of = [&](int row, int token) { return PACKED ? head0 + row - token * pack : head0; };
   const int q_begin = a.request_start[request];
   const int q_len = a.request_start[request + 1] - q_begin;
   const int context = a.request_context[request];
-  const int row0 = tile_in_request * LANES * BLOCK_M;         // first query row of the CTA
-  const int rows_here = min(LANES * BLOCK_M, q_len - row0);
-  const int last_key = context + row0 + rows_here - 1;        // last key any row here sees
+  const int token0 = tile_in_request * tile_tokens;           // first token of the CTA's rows
+  const int tokens_here = min(tile_tokens, q_len - token0);
+  const int rows_here = PACKED ? tokens_here * pack : tokens_here;
+  const int last_key = context + token0 + tokens_here - 1;    // last key any row here sees
   // With a window or chunks the CTA walks the key tiles that hold kept first keys and then the
   // tiles from the one with the first key its FIRST row sees; `skipped` tiles lie
   // between the two runs.  Every loop below counts TURNS: turn t works on key tile
   // tile_at(t); rings and barriers go by turns, positions and pages by key tiles.  Keys from
   // keep_first up to first_needed are seen by no row of the CTA: their pages may have been
   // given back and are not read.
-  const int first_needed = hx_first_seen(context + row0, a.window, a.chunk);
+  const int first_needed = hx_first_seen(context + token0, a.window, a.chunk);
   const int kept_tiles =
       a.window > 0 ? min((a.keep_first + BLOCK_N - 1) / BLOCK_N, first_needed / BLOCK_N) : 0;
   const int skipped = first_needed / BLOCK_N - kept_tiles;
   auto tile_at = [&](int turn) { return turn < kept_tiles ? turn : turn + skipped; };
   const int n_tiles = last_key / BLOCK_N + 1 - skipped;       // turns somebody here takes
-  // lane l has rows [row0 + 128 l, ...) and takes the turns before lane_tiles(l); lane 1 may be empty
+  // lane l has rows [128 l, ...) of the CTA's and takes the turns before lane_tiles(l); lane 1 may be empty
   auto lane_rows = [&](int l) { return max(0, min(BLOCK_M, rows_here - l * BLOCK_M)); };
   auto lane_tiles = [&](int l) {
     const int rows = lane_rows(l);
-    return rows > 0 ? (context + row0 + l * BLOCK_M + rows - 1) / BLOCK_N + 1 - skipped : 0;
+    return rows > 0 ? (context + token0 + token_of(l * BLOCK_M + rows - 1)) / BLOCK_N + 1 - skipped : 0;
   };
   const int page_size = a.page_size;
   const int pages_per_tile = BLOCK_N / page_size;
@@ -201,7 +251,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
   if (threadIdx.x == 0) {
     for (int s = 0; s < K_STAGES; ++s) {
       mbar_init(&k_full[s], 1);
-      mbar_init(&k_empty[s], 1);
+      mbar_init(&k_empty[s], REWRITERS);
     }
     for (int s = 0; s < V_STAGES; ++s) mbar_init(&v_full[s], 1);
     for (int s = 0; s < LANES * V_STAGES; ++s) mbar_init(&v_empty[s], 1);
@@ -210,7 +260,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
       mbar_init(&p_full[b], 4);   // one arrival per softmax warp of the lane
       mbar_init(&o_full[b], 1);
     }
-    for (int b = 0; b < KEY_BUFFERS; ++b) mbar_init(&k_ready[b], 1);
+    for (int b = 0; b < KEY_BUFFERS; ++b) mbar_init(&k_ready[b], REWRITERS);
     for (int b = 0; b < LANES * KEY_BUFFERS; ++b) mbar_init(&k_done[b], 1);
     mbar_init(q_ready, THREADS / 32 - WARP_SCORES);      // one arrival per warp that loads queries
     *failed = 0;
@@ -240,10 +290,12 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
       const int row = index / (D / 8);      // among the CTA's 256
       const int piece = index - row * (D / 8);
       values[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (index < kPieces && row < rows_here)
+      if (index < kPieces && row < rows_here) {
+        const int token = token_of(row);
         values[i] = *reinterpret_cast<const uint4*>(
-            a.q + static_cast<size_t>(q_begin + row0 + row) * a.ldq + static_cast<size_t>(head) * D +
-            piece * 8);
+            a.q + static_cast<size_t>(q_begin + token0 + token) * a.ldq +
+            static_cast<size_t>(head_of(row, token)) * D + piece * 8);
+      }
     }
 #pragma unroll
     for (int i = 0; i < kPerThread; ++i) {
@@ -328,12 +380,20 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
         for (int p = 0; p < 4; ++p) pages[p] = next_pages[p];
       }
     }
-  } else if (warp == WARP_REWRITE) {
+  } else if (warp == WARP_REWRITE ||
+             (REWRITERS == 4 && (warp == WARP_SCORES + 1 || warp == WARP_OUTPUT + 1 ||
+                                 warp == WARP_SOFTMAX - 1))) {
     // ------------------------------------------------------ keys, piece by piece
     // The score product wants all 64 keys of the tile at one stride, but every page block
     // holds its own keys piece-major: this warp rewrites a landed tile as
     // [piece][64 keys][16 bytes] into buffer tile % KEY_BUFFERS.
     bool ok = true;
+    // this warp's share of the pieces
+    constexpr int kShare = D / 8 / REWRITERS;
+    const int first_piece = REWRITERS == 1 || warp == WARP_REWRITE ? 0
+                            : warp == WARP_SCORES + 1              ? kShare
+                            : warp == WARP_OUTPUT + 1              ? 2 * kShare
+                                                                   : 3 * kShare;
     // where keys `lane` and `lane + 32` of a tile sit inside the landed page blocks
     const uint32_t source_low = (lane / page_size) * page_bytes + (lane % page_size) * 16;
     const uint32_t source_high =
@@ -358,16 +418,18 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
       }
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) break;
-      const uint32_t source = smem_u32(k_stages + (tile % K_STAGES) * Config::kHalfBytes);
+      const uint32_t source = smem_u32(k_stages + (tile % K_STAGES) * Config::kHalfBytes) +
+                              first_piece * piece_stride;
       const uint32_t target =
-          smem_u32(keys_by_piece + (tile % KEY_BUFFERS) * Config::kHalfBytes) + lane * 16;
+          smem_u32(keys_by_piece + (tile % KEY_BUFFERS) * Config::kHalfBytes) + lane * 16 +
+          first_piece * (BLOCK_N * 16);
       // eight pieces at a time: all their loads are in flight before the first store
 #pragma unroll
-      for (int piece0 = 0; piece0 < D / 8; piece0 += 8) {
+      for (int piece0 = 0; piece0 < kShare; piece0 += 8) {
         uint4 low[8], high[8];
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          if (piece0 + i >= D / 8) continue;      // (a head of 112: fourteen pieces)
+          if (piece0 + i >= kShare) continue;      // (a head of 112: fourteen pieces)
           asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
                        : "=r"(low[i].x), "=r"(low[i].y), "=r"(low[i].z), "=r"(low[i].w)
                        : "r"(source + source_low + (piece0 + i) * piece_stride));
@@ -377,7 +439,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
         }
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
-          if (piece0 + i >= D / 8) continue;
+          if (piece0 + i >= kShare) continue;
           asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(
                            target + (piece0 + i) * (BLOCK_N * 16)),
                        "r"(low[i].x), "r"(low[i].y), "r"(low[i].z), "r"(low[i].w) : "memory");
@@ -393,7 +455,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
         mbar_arrive(&k_empty[tile % K_STAGES]);      // the landed copy may be overwritten
       }
     }
-  } else if (warp == WARP_SCORES || warp == WARP_SCORES + 1) {
+  } else if (warp >= WARP_SCORES && warp < WARP_SCORES + LANES) {
     // ------------------------------------------------------------ score products
     if (elect_one()) {
       constexpr uint32_t idesc_scores = make_idesc(BLOCK_M, BLOCK_N);
@@ -434,7 +496,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
         umma_commit(&k_done[l * KEY_BUFFERS + tile % KEY_BUFFERS]);
       }
     }
-  } else if (warp == WARP_OUTPUT || warp == WARP_OUTPUT + 1) {
+  } else if (warp >= WARP_OUTPUT && warp < WARP_OUTPUT + LANES) {
     // ----------------------------------------------------------- output products
     if (elect_one()) {
       const int l = warp - WARP_OUTPUT;
@@ -486,13 +548,18 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
     const int group_thread = threadIdx.x - (WARP_SOFTMAX + 4 * l) * 32;      // 0..127
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     const uint32_t output_base = lane_base + Config::kOutputColumn + l * D;
-    const int q_position = context + row0 + l * BLOCK_M + row;      // the last key this row sees
+    const int my_token = token_of(l * BLOCK_M + row);
+    const int head = min(head_of(l * BLOCK_M + row, my_token), a.heads - 1);
+    const int q_position = context + token0 + my_token;             // the last key this row sees
     float row_max = -INFINITY;      // the reference of this row's exponentials, in log2 units
     float row_sum = 0.0f;
     const float scale_log2 = a.scale * 1.4426950408889634f;
     const int row_first = hx_first_seen(q_position, a.window, a.chunk);     // first key this row sees
     // a slope per position of distance, in the same log2 units (0: none)
     const float slope_log2 = a.slopes != nullptr ? a.slopes[head] * 1.4426950408889634f : 0.0f;
+    const bool plain_scores = a.softcap <= 0.0f && a.slopes == nullptr && a.scale > 0.0f;
+    const float factor = plain_scores ? scale_log2 : 1.0f;
+    const uint64_t factor_pair = pair_of(factor, factor), minus_one = pair_of(-1.0f, -1.0f);
     bool ok = true;
 
     // One lane waits and looks at the failure flag, all lanes get the same answer (what
@@ -526,9 +593,11 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
 #pragma unroll
           for (int i = 0; i < 16; ++i) p[c * 16 + i] = __uint_as_float(r[c][i]);
       }
+      // plain scores stay as they are until the exponential, whose argument is one multiply-add
+      // (a positive factor does not change which is the largest); the others are scaled here
       if (a.softcap > 0.0f) {
         hx_level_off_fast(p, a.scale / a.softcap, a.softcap * 1.4426950408889634f);
-      } else {
+      } else if (!plain_scores) {
 #pragma unroll
         for (int i = 0; i < BLOCK_N; ++i) p[i] *= scale_log2;
       }
@@ -550,12 +619,16 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
         for (int i = 0; i < BLOCK_N; ++i)
           if (key0 + i < row_first && key0 + i >= a.keep_first) p[i] = -INFINITY;
       }
-      float part_max[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+      float part_max[4];
 #pragma unroll
-      for (int i = 0; i < BLOCK_N; i += 4)
+      for (int u = 0; u < 4; ++u) part_max[u] = max_of_3(p[u], p[u + 4], p[u + 8]);
 #pragma unroll
-        for (int u = 0; u < 4; ++u) part_max[u] = fmaxf(part_max[u], p[i + u]);
-      const float tile_max = fmaxf(fmaxf(part_max[0], part_max[1]), fmaxf(part_max[2], part_max[3]));
+      for (int i = 12; i + 8 <= BLOCK_N; i += 8)
+#pragma unroll
+        for (int u = 0; u < 4; ++u) part_max[u] = max_of_3(part_max[u], p[i + u], p[i + 4 + u]);
+#pragma unroll
+      for (int u = 0; u < 4; ++u) part_max[u] = fmaxf(part_max[u], p[BLOCK_N - 4 + u]);
+      const float tile_max = factor * fmaxf(max_of_3(part_max[0], part_max[1], part_max[2]), part_max[3]);
       // without a window key 0 is visible to every row and the reference is finite from the
       // first tile on; with one a row may see nothing of the CTA's first tiles and keeps
       // -inf as its reference (and zeros as its probabilities) until it does
@@ -590,31 +663,38 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
           if (both) tmem_store16_raw(output_base + d0 + 16, r1);
         }
       }
-      float part_sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+      uint64_t part_sum[4] = {0, 0, 0, 0};
       const float reference = row_max == -INFINITY ? 0.0f : row_max;
+      const uint64_t reference_pair = pair_of(-reference, -reference);
 #pragma unroll
-      for (int i = 0; i < BLOCK_N; i += 4)
-#pragma unroll
-        for (int u = 0; u < 4; ++u) {
-          p[i + u] = fast_exp2(p[i + u] - reference);
-          part_sum[u] += p[i + u];
-        }
-      row_sum += (part_sum[0] + part_sum[1]) + (part_sum[2] + part_sum[3]);
+      for (int i = 0; i < BLOCK_N; i += 2) {
+        float x0, x1;
+        halves_of(pair_fma(pair_of(p[i], p[i + 1]), factor_pair, reference_pair), x0, x1);
+        p[i] = fast_exp2(x0);
+        p[i + 1] = fast_exp2(x1);
+        part_sum[(i / 2) % 4] = pair_add(part_sum[(i / 2) % 4], pair_of(p[i], p[i + 1]));
+      }
+      {
+        float low, high;
+        halves_of(pair_add(pair_add(part_sum[0], part_sum[1]), pair_add(part_sum[2], part_sum[3])), low,
+                  high);
+        row_sum += low + high;
+      }
 
-      // ---- P = hi + lo over the scores just read: hi is p cut to its upper 16 bits (a
-      // bfloat16 exactly), lo is p - hi (exact in float32) cut the same way: together 16
-      // bits of p.  Two keys per column, the earlier key in the lower half.
+      // ---- P = hi + lo over the scores just read: hi is p rounded to bfloat16, lo is p - hi
+      // (exact in float32) rounded the same way: together 16 bits of p.  Two keys per column,
+      // the earlier key in the lower half.
 #pragma unroll
       for (int c = 0; c < 2; ++c) {
         uint32_t hi[16], lo[16];
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           const float p0 = p[c * 32 + 2 * i], p1 = p[c * 32 + 2 * i + 1];
-          const uint32_t x0 = __float_as_uint(p0), x1 = __float_as_uint(p1);
-          const float rest0 = p0 - __uint_as_float(x0 & 0xffff0000u);
-          const float rest1 = p1 - __uint_as_float(x1 & 0xffff0000u);
-          hi[i] = __byte_perm(x0, x1, 0x7632);
-          lo[i] = __byte_perm(__float_as_uint(rest0), __float_as_uint(rest1), 0x7632);
+          hi[i] = pack_bf16(p0, p1);
+          float rest0, rest1;
+          halves_of(pair_fma(pair_of(__uint_as_float(hi[i] << 16), __uint_as_float(hi[i] & 0xffff0000u)),
+                             minus_one, pair_of(p0, p1)), rest0, rest1);
+          lo[i] = pack_bf16(rest0, rest1);
         }
         tmem_store16_raw(score_base + c * 16, hi);
         tmem_store16_raw(score_base + Config::kLowTermColumn + c * 16, lo);
@@ -668,7 +748,7 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
           inverse = keep / (row_sum * keep + fast_exp2(sink_log2 - top));
         }
         __nv_bfloat16* out = a.out +
-                             static_cast<size_t>(q_begin + row0 + l * BLOCK_M + row) * a.ldo +
+                             static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
                              static_cast<size_t>(head) * D;
 #pragma unroll
         for (int d0 = 0; d0 < D; d0 += 32) {
@@ -704,12 +784,12 @@ __global__ __launch_bounds__(THREADS, 1) void prefill_attention_tc_kernel(TcPref
   }
 }
 
-template <int D>
+template <int D, bool PACKED = false>
 int launch(const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
   using Config = TcConfig<D>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(prefill_attention_tc_kernel<D>,
+    if (cudaFuncSetAttribute(prefill_attention_tc_kernel<D, PACKED>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Config::kSmemBytes) != cudaSuccess) {
       cudaGetLastError();
@@ -719,8 +799,8 @@ int launch(const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
     }
     configured = true;
   }
-  hx_launch(prefill_attention_tc_kernel<D>, dim3(a.heads, tiles), THREADS, Config::kSmemBytes,
-            stream, a);
+  hx_launch(prefill_attention_tc_kernel<D, PACKED>, dim3(PACKED ? a.heads / a.pack : a.heads, tiles),
+            Config::kThreads, Config::kSmemBytes, stream, a);
   return HX_OK;
 }
 
@@ -812,4 +892,63 @@ HX_API int hx_prefill_attention_tc(const void* q, int ldq, const void* k_cache,
                                           table_stride, out, ldo, requests, tile_bound, heads,
                                           kv_heads, head_dim, page_size, num_pages, scale,
                                           min_query_len, 0, 0, status, stream);
+}
+
+// Tokens of a query tile of hx_prefill_attention_tc_packed; 0 where it does not apply.  It is for
+// the heads that hx_prefill_attention_tc_supports leaves out (160 to 256 in steps of 32).
+HX_API int hx_prefill_attention_tc_packed_tokens(int heads, int kv_heads, int head_dim, int page_size) {
+  if (heads <= 0 || kv_heads <= 0 || heads % kv_heads != 0) return 0;
+  // as many heads side by side as the mma.sync kernel takes
+  if (heads / kv_heads < 2 || heads / kv_heads > BLOCK_M / 2) return 0;
+  if (head_dim < 160 || head_dim > 256 || head_dim % 32 != 0) return 0;
+  if (page_size != 16 && page_size != 32 && page_size != 64) return 0;
+  return BLOCK_M / (heads / kv_heads);
+}
+
+// The arguments of hx_prefill_attention_tc_biased, for heads of 160 to 256 in steps of 32: a tile's
+// 128 rows are the query heads of a key/value head, side by side, of
+// hx_prefill_attention_tc_packed_tokens tokens; tile_bound bounds the number of such tiles.
+HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_cache,
+                                          const void* v_cache, const int* request_start,
+                                          const int* request_context,
+                                          const int* request_table_row, const int* block_tables,
+                                          int table_stride, void* out, int ldo, int requests,
+                                          int tile_bound, int heads, int kv_heads, int head_dim,
+                                          int page_size, int num_pages, float scale,
+                                          int min_query_len, int window, int keep_first,
+                                          const float* sinks, const float* slopes, int chunk,
+                                          float softcap, int* status, cudaStream_t stream) {
+  HX_REQUIRE(chunk >= 0 && softcap >= 0.0f, "hx_prefill_attention_tc_packed: bad chunk or softcap");
+  HX_REQUIRE(window >= 0 && keep_first >= 0, "hx_prefill_attention_tc_packed: bad window");
+  if (window == 0) keep_first = 0;
+  HX_REQUIRE(hx_prefill_attention_tc_packed_tokens(heads, kv_heads, head_dim, page_size) > 0,
+             "hx_prefill_attention_tc_packed: %d heads of %d on %d with pages of %d are not supported",
+             heads, head_dim, kv_heads, page_size);
+  HX_REQUIRE(requests >= 0 && tile_bound >= 0, "hx_prefill_attention_tc_packed: bad sizes");
+  HX_REQUIRE(tile_bound <= 65535, "hx_prefill_attention_tc_packed: too many query tiles");
+  HX_REQUIRE(num_pages > 0 && table_stride > 0, "hx_prefill_attention_tc_packed: bad cache geometry");
+  HX_REQUIRE(status != nullptr, "hx_prefill_attention_tc_packed: status word missing");
+  HX_REQUIRE(ldq % 8 == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
+                 (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 &&
+                 (reinterpret_cast<uintptr_t>(v_cache) & 15) == 0 &&
+                 (reinterpret_cast<uintptr_t>(out) & 15) == 0,
+             "hx_prefill_attention_tc_packed: operands must be 16-byte aligned, row strides multiples "
+             "of 8");
+  if (requests == 0 || tile_bound == 0) return HX_OK;
+  TcPrefillArgs a{static_cast<const __nv_bfloat16*>(q), ldq,
+                  static_cast<const __nv_bfloat16*>(k_cache),
+                  static_cast<const __nv_bfloat16*>(v_cache), request_start, request_context,
+                  request_table_row, block_tables, table_stride, static_cast<__nv_bfloat16*>(out),
+                  ldo, requests, heads, kv_heads, page_size, num_pages, scale, min_query_len, status,
+                  window, keep_first, sinks, slopes, chunk, softcap, heads / kv_heads};
+  int rc;
+  switch (head_dim) {
+    case 160: rc = launch<160, true>(a, tile_bound, stream); break;
+    case 192: rc = launch<192, true>(a, tile_bound, stream); break;
+    case 224: rc = launch<224, true>(a, tile_bound, stream); break;
+    default: rc = launch<256, true>(a, tile_bound, stream); break;
+  }
+  if (rc != HX_OK) return rc;
+  HX_CHECK_LAUNCH("hx_prefill_attention_tc_packed");
+  return HX_OK;
 }

@@ -30,6 +30,7 @@
 
 #include <cuda.h>
 
+#include <cmath>
 #include <mutex>
 #include <type_traits>
 #include <unordered_map>
@@ -392,6 +393,12 @@ struct PersistentArgs {
   const float* gate_bias = nullptr;
   const float* up_bias = nullptr;
   float softcap = 0.0f;       // float32 store: see level_off
+  int tail_ctas = 0;          // CTAs that share the tiles behind the whole rounds
+  // One small product per head (heads > 1): the feature tiles come head by head, head_tiles of
+  // them; head h multiplies the columns of x from h * head_x on with the rows of the weights from
+  // h * features on and writes its `features` columns from h * head_out on.
+  int heads = 1;
+  int head_tiles = 0, head_x = 0, head_out = 0;
 };
 
 // What a CTA works on at a time: a tile, or (`partial`) a run of k-blocks of a tile that
@@ -404,8 +411,9 @@ struct Unit {
 // The grid walks the tiles round by round.  The last round seldom fills the grid: 256 tiles
 // on 148 CTAs are 1.73 rounds that cost 2.  Where the epilogue ADDS into a float32 output the
 // order of the sum is free, so the tiles of that last round are laid end to end as one list
-// of k-blocks and every CTA takes an equal run of it (one or two pieces of tiles), which it
-// adds to the output with atomic adds; whole tiles keep the plain read-add-store.
+// of k-blocks and the first `tail_ctas` CTAs take an equal run of it each (one or two pieces of
+// tiles), which they add to the output with atomic adds; whole tiles keep the plain
+// read-add-store.
 __device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, Unit& u) {
   const int grid = static_cast<int>(gridDim.x);
   int index;
@@ -417,9 +425,10 @@ __device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, 
     u.partial = false;
   } else {
     const int first = a.whole_rounds * grid;
+    if (static_cast<int>(blockIdx.x) >= a.tail_ctas) return false;
     const long long blocks = static_cast<long long>(a.units - first) * a.k_blocks;
-    const long long begin = blocks * blockIdx.x / grid;
-    const long long end = blocks * (blockIdx.x + 1) / grid;
+    const long long begin = blocks * blockIdx.x / a.tail_ctas;
+    const long long end = blocks * (blockIdx.x + 1) / a.tail_ctas;
     const long long tile = begin / a.k_blocks + (iteration - a.whole_rounds);
     const long long from = max(begin, tile * a.k_blocks);
     const long long to = min(end, (tile + 1) * a.k_blocks);
@@ -724,7 +733,12 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
           if (group < 0) kb_end = unit.kb_begin;
           else group_row0 = group * args.group_rows;
         }
-        const int feature0 = group_row0 + unit.feature_tile * FEATURES;
+        int feature0 = group_row0 + unit.feature_tile * FEATURES, k_first = 0;
+        if (EPI == EPI_STORE_BF16 && args.heads > 1) {
+          const int head = unit.feature_tile / args.head_tiles;
+          feature0 = head * args.features + (unit.feature_tile - head * args.head_tiles) * FEATURES;
+          k_first = head * args.head_x;
+        }
         const int second_half = EPI == EPI_SWIGLU ? args.up_row_offset + feature0 : feature0 + BM;
         const int token0 = unit.token_tile * BM;
         for (int kb = unit.kb_begin; kb < kb_end; ++kb, ++fill) {
@@ -737,8 +751,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
           }
           uint8_t* stage = smem + s * Config::kStageBytes;
           mbar_expect_tx(&full_bar[s], Config::kStageBytes);
-          const int k = kb * BK;
-          tma_load_2d(stage, &map_x, &full_bar[s], k, token0);
+          tma_load_2d(stage, &map_x, &full_bar[s], k_first + kb * BK, token0);
           load_weight_box(stage + Config::kBytesA, &map_w, &full_bar[s], feature0, kb, args.k_tiles);
           load_weight_box(stage + Config::kBytesA + BM * BK * 2, &map_w, &full_bar[s], second_half,
                           kb, args.k_tiles);
@@ -833,6 +846,13 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
                            lane_base + buffer * Config::kBufferColumns,
                            unit.token_tile * BM + quarter * 32 + lane, args.tokens,
                            unit.feature_tile * FEATURES);
+      } else if (EPI == EPI_STORE_BF16 && args.heads > 1) {
+        const int head = unit.feature_tile / args.head_tiles;
+        write_row<EPI>(static_cast<__nv_bfloat16*>(args.out) + static_cast<size_t>(head) * args.head_out,
+                       args.ldo, args.features, lane_base + buffer * Config::kBufferColumns,
+                       unit.token_tile * BM + quarter * 32 + lane, args.tokens,
+                       (unit.feature_tile - head * args.head_tiles) * FEATURES, args.activation,
+                       args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
       } else if (args.tile_group == nullptr || args.tile_group[unit.token_tile] >= 0) {
         write_row<EPI>(args.out, args.ldo, args.features,
                        lane_base + buffer * Config::kBufferColumns,
@@ -996,24 +1016,32 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
     configured = true;
   }
   constexpr int kFeatures = EPI == EPI_SWIGLU ? BM : 2 * BM;
-  const int feature_tiles = (args.features + kFeatures - 1) / kFeatures;
+  args.head_tiles = (args.features + kFeatures - 1) / kFeatures;
+  const int feature_tiles = args.heads * args.head_tiles;
   args.token_tiles = (args.tokens + BM - 1) / BM;
   const long long tiles = static_cast<long long>(args.token_tiles) * feature_tiles;
   HX_REQUIRE(tiles < (1ll << 30), "hx_gemm_tc: too many tiles");
   args.units = static_cast<int>(tiles);
   // The add epilogue shares the last, partly filled round out by k-blocks (see unit_at) when
-  // that pays.  Every piece costs an epilogue of atomic adds (128 KB of them, all CTAs at the
-  // same time), which measured about as much as 30 k-blocks of products: with 2,048 tokens
-  // (108 tiles left for 148 SMs) sharing out gains nothing, with 512 tokens (64 tiles, less
-  // than half the grid) the output and down projections take 20 % and 23 % less time.
+  // that pays.  A piece costs its run of k-blocks and an epilogue of atomic adds, 128 KB of them,
+  // which measured about as much as 8 k-blocks of products alone and 15 more when all SMs add at
+  // the same time; so many CTAs share the tiles that the sum of both is least.  With 2,048 tokens
+  // by [4,096 x 4,096] (108 tiles left for 148 SMs) sharing out gains nothing, with 512 tokens (64
+  // tiles, less than half the grid) it takes 20 % off.
+  // 1,900 tokens by [5,120 x 13,824] leave 4 of 300 tiles: 261 us as a whole round, 195 shared
+  // out among 80 CTAs.
   args.whole_rounds = -1;
   int ctas = args.units < sms ? args.units : sms;
   if (EPI == EPI_ADD_F32 && HX_GEMM_STREAM_K) {
     const int rest = args.units % sms;
-    const long long run = static_cast<long long>(rest) * args.k_blocks / sms;
-    if (rest > 0 && rest * 2 <= sms && run >= 8 && args.k_blocks - run >= 32) {
+    const double blocks = static_cast<double>(rest) * args.k_blocks;
+    int share = static_cast<int>(sqrt(blocks * sms / 15.0));
+    share = share < rest ? rest : share > sms ? sms : share;
+    if (rest > 0 && rest * 2 <= sms &&
+        args.k_blocks - (blocks / share + 8.0 + 15.0 * share / sms) >= 12.0) {
       args.whole_rounds = args.units / sms;
-      ctas = sms;
+      args.tail_ctas = share;
+      ctas = args.whole_rounds > 0 ? sms : share;
     }
   }
   hx_launch(gemm_tc_persistent_kernel<EPI>, ctas, THREADS, Config::kSmemBytes, stream, map_w,
@@ -1270,6 +1298,44 @@ HX_API int hx_gemm_tc_grouped_gated(const void* x, int ldx, int x_capacity_rows,
   return gemm_tc_grouped(x, ldx, x_capacity_rows, w, ldw, group_rows, groups, out, ldo, tokens,
                          features, depth, EPI_SWIGLU, activation, gate_limit, up_row_offset,
                          token_tile, tile_group, status, stream);
+}
+
+// One product per head on the persistent kernel: out[t, h * out_stride + o] = sum_i w[h][o][i] *
+// x[t, h * x_stride + i], x [tokens, ldx], w [heads][out_dim][in_dim], out [tokens, ldo], all bf16.
+// Whole k-blocks only (in_dim a multiple of 64): a box must not reach into the next head's columns.
+HX_API int hx_gemm_tc_heads_supports(int in_dim, int x_stride, int ldx) {
+  return in_dim > 0 && in_dim % BK == 0 && x_stride % 8 == 0 && ldx % 8 == 0;
+}
+
+HX_API int hx_gemm_tc_heads(const void* x, int ldx, int x_capacity_rows, int x_stride, const void* w,
+                            void* out, int ldo, int out_stride, int tokens, int heads, int out_dim,
+                            int in_dim, int* status, cudaStream_t stream) {
+  HX_REQUIRE(tokens >= 0 && heads > 0 && out_dim > 0 && hx_gemm_tc_heads_supports(in_dim, x_stride, ldx),
+             "hx_gemm_tc_heads: heads of %d by %d, %d apart in rows of %d, are not supported", out_dim,
+             in_dim, x_stride, ldx);
+  HX_REQUIRE(static_cast<long long>(heads) * out_dim < (1ll << 31) && x_stride >= 0 &&
+                 ldx >= (heads - 1) * x_stride + in_dim && ldo >= (heads - 1) * out_stride + out_dim,
+             "hx_gemm_tc_heads: bad strides");
+  HX_REQUIRE((reinterpret_cast<uintptr_t>(x) & 15) == 0 && (reinterpret_cast<uintptr_t>(w) & 15) == 0,
+             "hx_gemm_tc_heads: operands must be 16-byte aligned");
+  HX_REQUIRE(x_capacity_rows >= tokens, "hx_gemm_tc_heads: buffer rows %d < tokens %d", x_capacity_rows,
+             tokens);
+  HX_REQUIRE(status != nullptr, "hx_gemm_tc_heads: status word missing");
+  if (tokens == 0) return HX_OK;
+  CUtensorMap map_w, map_x;
+  int rc = get_tensor_map(w, static_cast<uint64_t>(heads) * out_dim, in_dim, in_dim, BM, &map_w);
+  if (rc != HX_OK) return rc;
+  rc = get_tensor_map(x, x_capacity_rows, (heads - 1) * x_stride + in_dim, ldx, BM, &map_x);
+  if (rc != HX_OK) return rc;
+  PersistentArgs args{out, ldo, tokens, out_dim, in_dim, 0, 0, 0, 0, in_dim / BK, status, RopeArgs{}, -1,
+                      HX_GATE_SILU, nullptr, 0};
+  args.heads = heads;
+  args.head_x = x_stride;
+  args.head_out = out_stride;
+  rc = launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, stream);
+  if (rc != HX_OK) return rc;
+  HX_CHECK_LAUNCH("hx_gemm_tc_heads");
+  return HX_OK;
 }
 
 // Fewest tokens hx_gemm_tc_rope_append takes: it exists for the persistent kernel only.

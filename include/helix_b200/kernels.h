@@ -436,6 +436,11 @@ int hx_latent_queries(const void* q, int ld_q, int rot_offset, void* rows, int l
 int hx_head_products(const void* x, int ld_x, int x_stride, const void* w, void* out, int ld_out,
                      int out_stride, int dtype, int tokens, int heads, int out_dim, int in_dim,
                      cudaStream_t stream);
+/* the same on the tensor cores (bfloat16, many tokens): in_dim a multiple of 64, x_stride and ldx of 8 */
+int hx_gemm_tc_heads_supports(int in_dim, int x_stride, int ldx);
+int hx_gemm_tc_heads(const void* x, int ldx, int x_capacity_rows, int x_stride, const void* w,
+                     void* out, int ldo, int out_stride, int tokens, int heads, int out_dim,
+                     int in_dim, int* status, cudaStream_t stream);
 
 /* ---- rotation from positions, normed heads, rotated values + cache append --------------- */
 /* heads are row_dim wide (head_dim / value_dim real coordinates); q_norm, k_norm (both or
@@ -651,6 +656,18 @@ int hx_prefill_attention_tc_biased(const void* q, int ldq, const void* k_cache, 
                                    int window, int keep_first, const float* sinks,
                                    const float* slopes, int chunk, float softcap, int* status,
                                    cudaStream_t stream);
+/* the same for heads of 160 to 256 in steps of 32: a tile's 128 rows are the query heads of a
+ * key/value head, side by side, of hx_prefill_attention_tc_packed_tokens tokens (0: not supported) */
+int hx_prefill_attention_tc_packed_tokens(int heads, int kv_heads, int head_dim, int page_size);
+int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_cache,
+                                   const void* v_cache, const int* request_start,
+                                   const int* request_context, const int* request_table_row,
+                                   const int* block_tables, int table_stride, void* out, int ldo,
+                                   int requests, int tile_bound, int heads, int kv_heads,
+                                   int head_dim, int page_size, int num_pages, float scale,
+                                   int min_query_len, int window, int keep_first,
+                                   const float* sinks, const float* slopes, int chunk,
+                                   float softcap, int* status, cudaStream_t stream);
 /* the tcgen05 kernel with a window and kept first keys (see hx_prefill_attention_windowed) */
 int hx_prefill_attention_tc_windowed(const void* q, int ldq, const void* k_cache,
                                      const void* v_cache, const int* request_start,
