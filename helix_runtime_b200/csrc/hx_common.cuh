@@ -250,21 +250,19 @@ __device__ __forceinline__ int hx_find_query_tile(const int* request_start, int 
 
 // silu(x) = x * sigmoid(x) with the branch-stable sigmoid of the reference
 // (src/kernels/cuda/transformer.cu:68-83).
-__device__ __forceinline__ float hx_silu(float x) {
-  float sigmoid;
-  if (x >= 0.0f) {
-    sigmoid = 1.0f / (1.0f + expf(-x));
-  } else {
-    const float e = expf(x);
-    sigmoid = e / (1.0f + e);
-  }
-  return x * sigmoid;
+// e = exp(-|x|) serves both signs: a branch would have the lanes of a warp take both its sides.
+__device__ __forceinline__ float hx_sigmoid(float x) {
+  const float e = expf(-fabsf(x));
+  return (x >= 0.0f ? 1.0f : e) / (1.0f + e);
 }
+
+__device__ __forceinline__ float hx_silu(float x) { return x * hx_sigmoid(x); }
 
 // The same with the hardware exponential (relative error about 2^-21): for results that are
 // stored in bfloat16 right away.
 __device__ __forceinline__ float hx_silu_fast(float x) {
-  return x >= 0.0f ? __fdividef(x, 1.0f + __expf(-x)) : __fdividef(x * __expf(x), 1.0f + __expf(x));
+  const float e = __expf(-fabsf(x));
+  return __fdividef(x >= 0.0f ? x : x * e, 1.0f + e);
 }
 
 // What a gated feed-forward passes its gate through before the product with the up
@@ -278,12 +276,6 @@ enum HxGateActivation : int {
 };
 constexpr float HX_CLAMPED_SIGMOID_SLOPE = 1.702f;
 
-__device__ __forceinline__ float hx_sigmoid(float x) {
-  if (x >= 0.0f) return 1.0f / (1.0f + expf(-x));
-  const float e = expf(x);
-  return e / (1.0f + e);
-}
-
 __device__ __forceinline__ float hx_gelu_tanh(float z) {
   const float u = 0.7978845608028654f * (z + 0.044715f * z * z * z);
   return z * hx_sigmoid(2.0f * u);
@@ -291,7 +283,8 @@ __device__ __forceinline__ float hx_gelu_tanh(float z) {
 
 __device__ __forceinline__ float hx_gelu_tanh_fast(float z) {
   const float v = 1.5957691216057308f * (z + 0.044715f * z * z * z);
-  return v >= 0.0f ? __fdividef(z, 1.0f + __expf(-v)) : __fdividef(z * __expf(v), 1.0f + __expf(v));
+  const float e = __expf(-fabsf(v));
+  return __fdividef(v >= 0.0f ? z : z * e, 1.0f + e);
 }
 
 __device__ __forceinline__ float hx_gate(float x, int activation) {

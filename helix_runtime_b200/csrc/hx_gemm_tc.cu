@@ -414,21 +414,22 @@ struct Unit {
 // of k-blocks and the first `tail_ctas` CTAs take an equal run of it each (one or two pieces of
 // tiles), which they add to the output with atomic adds; whole tiles keep the plain
 // read-add-store.
-__device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, Unit& u) {
-  const int grid = static_cast<int>(gridDim.x);
+// `worker` of `grid`: a CTA of the grid, or a pair of them.
+__device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, Unit& u, int worker,
+                                        int grid) {
   int index;
   if (a.whole_rounds < 0 || iteration < a.whole_rounds) {
-    index = static_cast<int>(blockIdx.x) + iteration * grid;
+    index = worker + iteration * grid;
     if (index >= a.units) return false;
     u.kb_begin = 0;
     u.kb_end = a.k_blocks;
     u.partial = false;
   } else {
     const int first = a.whole_rounds * grid;
-    if (static_cast<int>(blockIdx.x) >= a.tail_ctas) return false;
+    if (worker >= a.tail_ctas) return false;
     const long long blocks = static_cast<long long>(a.units - first) * a.k_blocks;
-    const long long begin = blocks * blockIdx.x / a.tail_ctas;
-    const long long end = blocks * (blockIdx.x + 1) / a.tail_ctas;
+    const long long begin = blocks * worker / a.tail_ctas;
+    const long long end = blocks * (worker + 1) / a.tail_ctas;
     const long long tile = begin / a.k_blocks + (iteration - a.whole_rounds);
     const long long from = max(begin, tile * a.k_blocks);
     const long long to = min(end, (tile + 1) * a.k_blocks);
@@ -700,6 +701,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
+  const int worker = blockIdx.x, workers = gridDim.x;
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < STAGES; ++s) {
@@ -726,7 +728,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     if (elect_one()) {
       uint32_t fill = 0;      // stages filled so far, over all units
       Unit unit;
-      for (int iteration = 0; unit_at(args, iteration, unit) && !*failed; ++iteration) {
+      for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
         int group_row0 = 0, kb_end = unit.kb_end;
         if (args.tile_group != nullptr) {
           const int group = args.tile_group[unit.token_tile];
@@ -764,7 +766,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       constexpr uint32_t idesc = make_idesc(BM, Config::kRowsB);
       uint32_t drained = 0;      // stages consumed so far, over all units
       Unit unit;
-      for (int iteration = 0; unit_at(args, iteration, unit) && !*failed; ++iteration) {
+      for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
         const int buffer = iteration & 1;
         const uint32_t use = static_cast<uint32_t>(iteration >> 1);
         // the epilogue must have read this accumulator's previous unit (and, for the add
@@ -811,7 +813,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     // add epilogue: the old output of unit `iteration` goes into its accumulator, which is
     // then handed to the MMA warp
     auto prepare = [&](int iteration) {
-      if (EPI != EPI_ADD_F32 || !unit_at(args, iteration, unit)) return;
+      if (EPI != EPI_ADD_F32 || !unit_at(args, iteration, unit, worker, workers)) return;
       const int buffer = iteration & 1;
       if (!unit.partial)      // a piece starts from zero and is added to the output afterwards
         load_row_into_accumulator(static_cast<const float*>(args.out), args.ldo, args.features,
@@ -824,7 +826,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     };
     prepare(0);
     prepare(1);
-    for (int iteration = 0; unit_at(args, iteration, unit) && !*failed; ++iteration) {
+    for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
       const int buffer = iteration & 1;
       const uint32_t use = static_cast<uint32_t>(iteration >> 1);
       bool ok = true;
@@ -877,6 +879,209 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
   if (warp == 1) {
     tc_fence_after();
     tmem_dealloc(tmem_base, Config::kTmemColumns);
+  }
+}
+
+// ------------------------------------------------------------- the same by pairs of CTAs
+//
+// A tile of 128 tokens by 256 weight rows reads 48 KB of operands per k-block, at the tensor cores'
+// rate about what an SM gets from the L2, and every SM multiplies by weights that it has brought in
+// for itself.  Here two CTAs share a tile of 256 tokens: each brings its own 128 tokens and HALF of
+// the weight rows (for SwiGLU: the gate rows, and the up rows), and tcgen05.mma.cta_group::2 reads
+// both halves: 32 KB a k-block and CTA, so six stages instead of four.  The leader (the even CTA)
+// issues the products for both; either CTA's accumulators hold its own 128 tokens, so the epilogues
+// are those of the kernel above.
+// Measured (2,048 tokens, alone, one CTA a tile and pairs): [12,288 x 4,096] 155.8 -> 139.6 us (1,476
+// TFLOP/s), sums by [4,096 x 4,096] 71.3 -> 55.7, gate and up [22,016 x 4,096] 270.3 -> 256.5, sums by
+// [4,096 x 11,008] 173.2 -> 167.9; 512 tokens 54.8 -> 48.2, 25.4 -> 24.6, 90.2 -> 79.9, 66.7 -> 54.5.
+struct PairConfig {
+  static constexpr int kBytesA = BM * BK * 2;    // this CTA's tokens
+  static constexpr int kBytesB = BM * BK * 2;    // its half of the weight rows
+  static constexpr int kStageBytes = kBytesA + kBytesB;
+  static constexpr int kStages = 6;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment*/ + 256 /*barriers*/;
+};
+
+template <int EPI>
+__global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pair_kernel(
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
+    const PersistentArgs args) {
+  using Config = PairConfig;
+  constexpr int STAGES = Config::kStages;
+  constexpr int FEATURES = EPI == EPI_SWIGLU ? BM : 2 * BM;
+  constexpr int kBufferColumns = PersistentConfig::kBufferColumns;
+
+  hx_pdl_trigger();
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Config::kStageBytes);  // leader's count
+  uint64_t* empty_bar = full_bar + STAGES;
+  uint64_t* tmem_full_bar = empty_bar + STAGES;      // [2]
+  uint64_t* tmem_empty_bar = tmem_full_bar + 2;      // [2]: leader's count, of both CTAs' epilogues
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(tmem_empty_bar + 2);
+  volatile int* failed = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+  const int warp = threadIdx.x >> 5;
+  const int lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_rank());
+  const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < STAGES; ++s) {
+      mbar_init(&full_bar[s], 1);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(&tmem_full_bar[b], 1);
+      mbar_init(&tmem_empty_bar[b], 8);      // one arrival per epilogue warp of both CTAs
+    }
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == 1) tmem_alloc_pair(tmem_holder, PersistentConfig::kTmemColumns);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // nothing arrives at the other CTA's barriers before they are there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  hx_pdl_wait();
+
+  if (warp == 0) {
+    // -------------------------------------------------------------- TMA producer
+    if (elect_one()) {
+      uint32_t fill = 0;      // stages filled so far, over all units
+      Unit unit;
+      for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
+        const int feature0 = unit.feature_tile * FEATURES;
+        const int weight_row = rank == 0 ? feature0
+                               : EPI == EPI_SWIGLU ? args.up_row_offset + feature0 : feature0 + BM;
+        const int token0 = unit.token_tile * 2 * BM + rank * BM;
+        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++fill) {
+          const int s = fill % STAGES;
+          if (!mbar_wait(&empty_bar[s], ((fill / STAGES) & 1u) ^ 1u)) {
+            atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
+            *failed = 1;
+            break;
+          }
+          uint8_t* stage = smem + s * Config::kStageBytes;
+          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * Config::kStageBytes);
+          const uint32_t bar = cluster_address(&full_bar[s], 0);
+          tma_load_2d_pair(stage, &map_x, bar, kb * BK, token0);
+          if (args.k_tiles > 0)
+            tma_load_2d_pair(stage + Config::kBytesA, &map_w, bar, 0,
+                             ((weight_row / BM) * args.k_tiles + kb) * BM);
+          else
+            tma_load_2d_pair(stage + Config::kBytesA, &map_w, bar, kb * BK, weight_row);
+        }
+      }
+      // the leader's last arrivals at this CTA's barriers, before the CTA may end
+      for (uint32_t last = fill > STAGES ? fill - STAGES : 0; last < fill && !*failed; ++last)
+        if (!mbar_wait(&empty_bar[last % STAGES], (last / STAGES) & 1u)) {
+          atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
+          *failed = 1;
+        }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issuer
+    if (rank == 0 && elect_one()) {
+      constexpr uint32_t idesc = make_idesc(2 * BM, 2 * BM);
+      uint32_t drained = 0;
+      Unit unit;
+      for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
+        const int buffer = iteration & 1;
+        const uint32_t use = static_cast<uint32_t>(iteration >> 1);
+        if (!mbar_wait_cluster(&tmem_empty_bar[buffer],
+                               EPI == EPI_ADD_F32 ? (use & 1u) : (use & 1u) ^ 1u)) {
+          atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
+          *failed = 1;
+          break;
+        }
+        tc_fence_after();
+        const uint32_t accumulator = tmem_base + buffer * kBufferColumns;
+        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++drained) {
+          const int s = drained % STAGES;
+          if (!mbar_wait_cluster(&full_bar[s], (drained / STAGES) & 1u)) {
+            atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
+            *failed = 1;
+            break;
+          }
+          tc_fence_after();
+          const uint32_t stage = smem_u32(smem + s * Config::kStageBytes);
+          const uint64_t desc_a = make_smem_desc(stage);
+          const uint64_t desc_b = make_smem_desc(stage + Config::kBytesA);
+#pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
+            const uint32_t accumulate =
+                ((EPI == EPI_ADD_F32 && !unit.partial) || kb > unit.kb_begin || k > 0) ? 1u : 0u;
+            umma_bf16_pair(accumulator, desc_a + step, desc_b + step, idesc, accumulate);
+          }
+          umma_commit_pair(&empty_bar[s]);
+        }
+        if (*failed) break;
+        umma_commit_pair(&tmem_full_bar[buffer]);
+      }
+    }
+  } else {
+    // ------------------------------------------------------------------ epilogue
+    const int quarter = warp & 3;
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+    const int row = rank * BM + quarter * 32 + lane;      // of the tile's 256 tokens
+    Unit unit;
+    auto hand_over = [&](int buffer) {
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive_cluster(cluster_address(&tmem_empty_bar[buffer], 0));
+    };
+    auto prepare = [&](int iteration) {
+      if (EPI != EPI_ADD_F32 || !unit_at(args, iteration, unit, worker, workers)) return;
+      const int buffer = iteration & 1;
+      if (!unit.partial)
+        load_row_into_accumulator(static_cast<const float*>(args.out), args.ldo, args.features,
+                                  lane_base + buffer * kBufferColumns, unit.token_tile * 2 * BM + row,
+                                  args.tokens, unit.feature_tile * FEATURES);
+      hand_over(buffer);
+    };
+    prepare(0);
+    prepare(1);
+    for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
+      const int buffer = iteration & 1;
+      const uint32_t use = static_cast<uint32_t>(iteration >> 1);
+      bool ok = true;
+      if (lane == 0) ok = mbar_wait_cluster(&tmem_full_bar[buffer], use & 1u);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) {
+        if (lane == 0) {
+          atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
+          *failed = 1;
+        }
+        break;
+      }
+      tc_fence_after();
+      const uint32_t accumulator = lane_base + buffer * kBufferColumns;
+      const int token = unit.token_tile * 2 * BM + row, feature0 = unit.feature_tile * FEATURES;
+      if constexpr (EPI == EPI_ROPE_APPEND) {
+        write_row_rope(args, accumulator, token, feature0);
+      } else if (EPI == EPI_ADD_F32 && unit.partial) {
+        add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
+                           args.tokens, feature0);
+      } else {
+        write_row<EPI>(args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
+                       args.activation, args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
+      }
+      if (EPI == EPI_ADD_F32) prepare(iteration + 2);
+      else hand_over(buffer);
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // neither CTA's memory is read or arrived at any more
+  if (warp == 1) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, PersistentConfig::kTmemColumns);
   }
 }
 
@@ -995,24 +1200,59 @@ int launch_epilogue(int epilogue, const CUtensorMap& map_w, const CUtensorMap& m
   }
 }
 
+// How `workers` (CTAs, or pairs of them) go through the tiles of a product: the time in k-blocks of
+// a worker, and for the add epilogue how the last, partly filled round is shared out (see unit_at).
+//
+// Sharing a round out pays where little of it is there.  A piece costs its run of k-blocks and an
+// epilogue of atomic adds, 128 KB of them, which measured about as much as 8 k-blocks of products
+// alone and 15 more when all SMs add at the same time; so many workers share the tiles that the
+// sum of both is least.  With 2,048 tokens by [4,096 x 4,096] (108 tiles left for 148 SMs) sharing
+// out gains nothing, with 512 tokens (64 tiles, less than half the grid) it takes 20 % off.
+// 1,900 tokens by [5,120 x 13,824] leave 4 of 300 tiles: 261 us as a whole round, 195 shared out
+// among 80 CTAs.
+double plan_rounds(long long units, int workers, int k_blocks, bool add, int& whole_rounds,
+                   int& tail_workers) {
+  const int rest = static_cast<int>(units % workers);
+  const long long rounds = units / workers;
+  whole_rounds = -1;
+  tail_workers = 0;
+  if (add && HX_GEMM_STREAM_K && rest > 0 && rest * 2 <= workers) {
+    const double blocks = static_cast<double>(rest) * k_blocks;
+    int share = static_cast<int>(sqrt(blocks * workers / 15.0));
+    share = share < rest ? rest : share > workers ? workers : share;
+    const double tail = blocks / share + 8.0 + 15.0 * share / workers;
+    if (k_blocks - tail >= 12.0) {
+      whole_rounds = static_cast<int>(rounds);
+      tail_workers = share;
+      return static_cast<double>(rounds) * k_blocks + tail;
+    }
+  }
+  return static_cast<double>(rounds + (rest > 0 ? 1 : 0)) * k_blocks;
+}
+
+template <typename Kernel>
+bool reserve_shared(Kernel kernel, int bytes) {
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes) == cudaSuccess)
+    return true;
+  hx_set_error("hx_gemm_tc: cannot reserve %d bytes of shared memory", bytes);
+  cudaGetLastError();
+  return false;
+}
+
+#ifndef HX_GEMM_PAIRS
+#define HX_GEMM_PAIRS 1      // 0: every tile is one CTA's
+#endif
+
 template <int EPI>
 int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
                       cudaStream_t stream) {
-  using Config = PersistentConfig;
   static bool configured = false;
-  static int sms = 0;
+  const int sms = hx_device_sm_count();
+  if (sms <= 0) return HX_ERR_LAUNCH;
   if (!configured) {
-    int device = 0;
-    if (cudaFuncSetAttribute(gemm_tc_persistent_kernel<EPI>,
-                             cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             Config::kSmemBytes) != cudaSuccess ||
-        cudaGetDevice(&device) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device) != cudaSuccess ||
-        sms <= 0) {
-      hx_set_error("hx_gemm_tc: cannot reserve %d bytes of shared memory", Config::kSmemBytes);
-      cudaGetLastError();
+    if (!reserve_shared(gemm_tc_persistent_kernel<EPI>, PersistentConfig::kSmemBytes) ||
+        !reserve_shared(gemm_tc_pair_kernel<EPI>, PairConfig::kSmemBytes))
       return HX_ERR_LAUNCH;
-    }
     configured = true;
   }
   constexpr int kFeatures = EPI == EPI_SWIGLU ? BM : 2 * BM;
@@ -1022,29 +1262,32 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   const long long tiles = static_cast<long long>(args.token_tiles) * feature_tiles;
   HX_REQUIRE(tiles < (1ll << 30), "hx_gemm_tc: too many tiles");
   args.units = static_cast<int>(tiles);
-  // The add epilogue shares the last, partly filled round out by k-blocks (see unit_at) when
-  // that pays.  A piece costs its run of k-blocks and an epilogue of atomic adds, 128 KB of them,
-  // which measured about as much as 8 k-blocks of products alone and 15 more when all SMs add at
-  // the same time; so many CTAs share the tiles that the sum of both is least.  With 2,048 tokens
-  // by [4,096 x 4,096] (108 tiles left for 148 SMs) sharing out gains nothing, with 512 tokens (64
-  // tiles, less than half the grid) it takes 20 % off.
-  // 1,900 tokens by [5,120 x 13,824] leave 4 of 300 tiles: 261 us as a whole round, 195 shared
-  // out among 80 CTAs.
-  args.whole_rounds = -1;
-  int ctas = args.units < sms ? args.units : sms;
-  if (EPI == EPI_ADD_F32 && HX_GEMM_STREAM_K) {
-    const int rest = args.units % sms;
-    const double blocks = static_cast<double>(rest) * args.k_blocks;
-    int share = static_cast<int>(sqrt(blocks * sms / 15.0));
-    share = share < rest ? rest : share > sms ? sms : share;
-    if (rest > 0 && rest * 2 <= sms &&
-        args.k_blocks - (blocks / share + 8.0 + 15.0 * share / sms) >= 12.0) {
-      args.whole_rounds = args.units / sms;
-      args.tail_ctas = share;
-      ctas = args.whole_rounds > 0 ? sms : share;
+  int whole_rounds = -1, tail = 0;
+  const double alone = plan_rounds(tiles, sms, args.k_blocks, EPI == EPI_ADD_F32, args.whole_rounds,
+                                   args.tail_ctas);
+  // Pairs, unless their tiles of 256 tokens make the rounds longer by more than the twentieth that a
+  // round is shorter at least (1,900 tokens by [27,648 x 5,120]: 12 rounds against 11, 380 against 375
+  // us); short sums that are all pieces have nothing to win (129 tokens by [4,096 x 4,096]: 18.8
+  // against 17.0 us).
+  const int pair_tiles = (args.tokens + 2 * BM - 1) / (2 * BM), pairs = sms / 2;
+  const long long pair_units = static_cast<long long>(pair_tiles) * feature_tiles;
+  if (HX_GEMM_PAIRS && args.heads == 1 && args.tile_group == nullptr && args.tokens > BM && pairs > 0) {
+    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, whole_rounds,
+                                      tail);
+    const double penalty = whole_rounds == 0 && args.k_blocks < 96 ? 4.0 : 0.0;
+    if (0.95 * paired + penalty <= alone) {
+      args.token_tiles = pair_tiles;
+      args.units = static_cast<int>(pair_units);
+      args.whole_rounds = whole_rounds;
+      args.tail_ctas = tail;
+      const int used = whole_rounds == 0 ? tail : pair_units < pairs ? static_cast<int>(pair_units) : pairs;
+      hx_launch(gemm_tc_pair_kernel<EPI>, 2 * used, THREADS, PairConfig::kSmemBytes, stream, map_w, map_x,
+                args);
+      return HX_OK;
     }
   }
-  hx_launch(gemm_tc_persistent_kernel<EPI>, ctas, THREADS, Config::kSmemBytes, stream, map_w,
+  const int ctas = args.whole_rounds == 0 ? args.tail_ctas : args.units < sms ? args.units : sms;
+  hx_launch(gemm_tc_persistent_kernel<EPI>, ctas, THREADS, PersistentConfig::kSmemBytes, stream, map_w,
             map_x, args);
   return HX_OK;
 }

@@ -934,6 +934,60 @@ void linear_state_scan_kernel(const LinearStateArgs<T> a) {
 // Channels in `groups` equal parts, each divided by its own root mean square (eps inside the
 // root), times a weight.  gate_after = 0: the gate silu(g) multiplies BEFORE the norm
 // (v = y silu(g); out = v / rms(v) * w); 1: after it (out = y / rms(y) * w * silu(g)).
+// A warp a group, four values a load, the group's values in registers between the sum and the
+// store: bfloat16 groups of up to 128 PIECES channels, in fours (1,725 tokens of 32 groups of 128: 59 us
+// with a CTA of 128 threads a group, HX_MEASURED_NORM now).
+template <int PIECES>
+__global__ __launch_bounds__(256) void gated_group_norm_pieces_kernel(
+    const float* __restrict__ y, int ld_y, const __nv_bfloat16* __restrict__ gate, int ld_gate,
+    const float* __restrict__ weight, __nv_bfloat16* __restrict__ out, int ld_out, int width,
+    int groups, long long rows, float eps, int gate_after) {
+  hx_pdl_prologue();
+  const long long index = blockIdx.x * 8ll + (threadIdx.x >> 5);
+  if (index >= rows) return;
+  const long long token = index / groups;
+  const int first = static_cast<int>(index - token * groups) * width, lane = threadIdx.x & 31;
+  const float* yr = y + token * ld_y + first;
+  const __nv_bfloat16* gr = gate + token * ld_gate + first;
+  float4 v[PIECES], g[PIECES];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = 128 * p + 4 * lane;
+    v[p] = g[p] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (c < width) {
+      v[p] = *reinterpret_cast<const float4*>(yr + c);
+      const uint2 packed = *reinterpret_cast<const uint2*>(gr + c);
+      const float2 low = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed.x));
+      const float2 high = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&packed.y));
+      g[p] = make_float4(low.x, low.y, high.x, high.y);
+    }
+  }
+  float sum = 0.0f;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    g[p] = make_float4(hx_silu(g[p].x), hx_silu(g[p].y), hx_silu(g[p].z), hx_silu(g[p].w));
+    if (!gate_after) v[p] = make_float4(v[p].x * g[p].x, v[p].y * g[p].y, v[p].z * g[p].z, v[p].w * g[p].w);
+    sum = fmaf(v[p].x, v[p].x, fmaf(v[p].y, v[p].y, fmaf(v[p].z, v[p].z, fmaf(v[p].w, v[p].w, sum))));
+  }
+#pragma unroll
+  for (int offset = 16; offset > 0; offset >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, offset);
+  const float inverse = 1.0f / sqrtf(sum / static_cast<float>(width) + eps);
+  __nv_bfloat16* o = out + token * ld_out + first;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int c = 128 * p + 4 * lane;
+    if (c >= width) continue;
+    const float4 w = *reinterpret_cast<const float4*>(weight + first + c);
+    float4 r = make_float4(v[p].x * inverse * w.x, v[p].y * inverse * w.y, v[p].z * inverse * w.z,
+                           v[p].w * inverse * w.w);
+    if (gate_after) r = make_float4(r.x * g[p].x, r.y * g[p].y, r.z * g[p].z, r.w * g[p].w);
+    uint2 packed;
+    *reinterpret_cast<__nv_bfloat162*>(&packed.x) = __floats2bfloat162_rn(r.x, r.y);
+    *reinterpret_cast<__nv_bfloat162*>(&packed.y) = __floats2bfloat162_rn(r.z, r.w);
+    *reinterpret_cast<uint2*>(o + c) = packed;
+  }
+}
+
 template <typename T>
 __global__ __launch_bounds__(128) void gated_group_norm_kernel(
     const float* __restrict__ y, int ld_y, const T* __restrict__ gate, int ld_gate,
@@ -1270,6 +1324,18 @@ HX_API int hx_gated_group_norm(const float* y, int ld_y, const void* gate, int l
     hx_launch(gated_group_norm_kernel<float>, grid, 128, 0, stream, y, ld_y,
               static_cast<const float*>(gate), ld_gate, weight, static_cast<float*>(out), ld_out,
               width, eps, gate_after);
+  } else if (dtype == HX_BF16 && width % 4 == 0 && width <= 1024 && ld_y % 4 == 0 &&
+             ld_gate % 4 == 0 && ld_out % 4 == 0 &&
+             ((reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(weight)) & 15) == 0 &&
+             ((reinterpret_cast<uintptr_t>(gate) | reinterpret_cast<uintptr_t>(out)) & 7) == 0) {
+    const long long rows = static_cast<long long>(tokens) * groups;
+    auto kernel = width <= 128   ? gated_group_norm_pieces_kernel<1>
+                  : width <= 256 ? gated_group_norm_pieces_kernel<2>
+                  : width <= 512 ? gated_group_norm_pieces_kernel<4>
+                                 : gated_group_norm_pieces_kernel<8>;
+    hx_launch(kernel, static_cast<unsigned>((rows + 7) / 8), 256, 0, stream, y, ld_y,
+              static_cast<const __nv_bfloat16*>(gate), ld_gate, weight, static_cast<__nv_bfloat16*>(out),
+              ld_out, width, groups, rows, eps, gate_after);
   } else if (dtype == HX_BF16) {
     hx_launch(gated_group_norm_kernel<__nv_bfloat16>, grid, 128, 0, stream, y, ld_y,
               static_cast<const __nv_bfloat16*>(gate), ld_gate, weight,
