@@ -27,13 +27,10 @@
 // Every wait on an mbarrier is bounded; a wait that runs out sets a status bit, the
 // CTA skips its remaining work, frees its tensor memory and returns.
 #include "hx_tcgen05.cuh"
-
-#include <cuda.h>
+#include "hx_tensor_map.cuh"
 
 #include <cmath>
-#include <mutex>
 #include <type_traits>
-#include <unordered_map>
 
 namespace {
 
@@ -394,6 +391,7 @@ struct PersistentArgs {
   const float* up_bias = nullptr;
   float softcap = 0.0f;       // float32 store: see level_off
   int tail_ctas = 0;          // CTAs that share the tiles behind the whole rounds
+  int tail_pieces = 1;        // pairs: the tiles behind the whole rounds are cut into so many pieces
   // One small product per head (heads > 1): the feature tiles come head by head, head_tiles of
   // them; head h multiplies the columns of x from h * head_x on with the rows of the weights from
   // h * features on and writes its `features` columns from h * head_out on.
@@ -406,6 +404,7 @@ struct PersistentArgs {
 struct Unit {
   int token_tile, feature_tile, kb_begin, kb_end;
   bool partial;
+  int pieces, piece;      // pairs: which of so many pieces of the tile's columns
 };
 
 // The grid walks the tiles round by round.  The last round seldom fills the grid: 256 tiles
@@ -418,7 +417,19 @@ struct Unit {
 __device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, Unit& u, int worker,
                                         int grid) {
   int index;
-  if (a.whole_rounds < 0 || iteration < a.whole_rounds) {
+  u.pieces = 1;
+  u.piece = 0;
+  if (a.tail_pieces > 1 && iteration == a.whole_rounds) {
+    if (worker >= (a.units - a.whole_rounds * grid) * a.tail_pieces) return false;
+    index = a.whole_rounds * grid + worker / a.tail_pieces;
+    u.pieces = a.tail_pieces;
+    u.piece = worker % a.tail_pieces;
+    u.kb_begin = 0;
+    u.kb_end = a.k_blocks;
+    u.partial = false;
+  } else if (a.tail_pieces > 1 && iteration > a.whole_rounds) {
+    return false;
+  } else if (a.whole_rounds < 0 || iteration < a.whole_rounds) {
     index = worker + iteration * grid;
     if (index >= a.units) return false;
     u.kb_begin = 0;
@@ -479,25 +490,24 @@ __device__ __forceinline__ void load_row_into_accumulator(const float* out, int 
 }
 
 // This thread's token: `columns` features starting at feature0, 16 at a time, from its lane of
-// the accumulator.  With SwiGLU the accumulator holds 128 gate columns, then 128 up columns.
+// the accumulator.  With SwiGLU the accumulator holds `columns` gate columns, then the up columns.
 template <int EPI>
-__device__ __forceinline__ void write_row(void* out, int ldo, int features, uint32_t lane_address,
+__device__ __forceinline__ void write_row(int columns, void* out, int ldo, int features, uint32_t lane_address,
                                           int token, int tokens, int feature0, int activation,
                                           float gate_limit, const float* gate_bias,
                                           const float* up_bias, float softcap) {
   using Element = typename std::conditional<EPI == EPI_STORE_BF16 || EPI == EPI_SWIGLU,
                                             __nv_bfloat16, float>::type;
-  constexpr int kColumns = EPI == EPI_SWIGLU ? BM : 2 * BM;
   const bool wide = (ldo % (16 / static_cast<int>(sizeof(Element))) == 0) &&
                     ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
 #pragma unroll 1
-  for (int column = 0; column < kColumns; column += 16) {
+  for (int column = 0; column < columns; column += 16) {
     if (feature0 + column >= features) break;      // uniform over the warp
     float acc[16];
     tmem_load16(lane_address + column, acc);
     if (EPI == EPI_SWIGLU) {
       float up[16];
-      tmem_load16(lane_address + BM + column, up);
+      tmem_load16(lane_address + columns + column, up);
       if (gate_bias != nullptr || up_bias != nullptr) {
         // this thread's 16 features: their biases (the same for every token of the tile)
 #pragma unroll
@@ -551,8 +561,8 @@ __device__ __forceinline__ void write_row(void* out, int ldo, int features, uint
 // The rotary/append epilogue for this thread's token: the same arithmetic as the separate
 // kernel (hx_rope_append) applied to the product rounded to bfloat16, as the plain store
 // would have rounded it: rotation in float32 from the cos/sin table, one more rounding.
-__device__ __forceinline__ void write_row_rope(const PersistentArgs& a, uint32_t lane_address,
-                                               int token, int feature0) {
+__device__ __forceinline__ void write_row_rope(int columns, const PersistentArgs& a,
+                                               uint32_t lane_address, int token, int feature0) {
   const RopeArgs& r = a.rope;
   const bool live = token < a.tokens;
   const int half = r.rotary_dim / 2;
@@ -582,7 +592,7 @@ __device__ __forceinline__ void write_row_rope(const PersistentArgs& a, uint32_t
                           ((reinterpret_cast<uintptr_t>(r.cos_table) |
                             reinterpret_cast<uintptr_t>(r.sin_table)) & 15) == 0;
 #pragma unroll 1
-  for (int column = 0; column < 2 * BM; column += 16) {
+  for (int column = 0; column < columns; column += 16) {
     const int feature = feature0 + column;
     if (feature >= a.features) break;      // uniform over the warp
     float x[16];
@@ -841,7 +851,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       }
       tc_fence_after();
       if constexpr (EPI == EPI_ROPE_APPEND) {
-        write_row_rope(args, lane_base + buffer * Config::kBufferColumns,
+        write_row_rope(FEATURES, args, lane_base + buffer * Config::kBufferColumns,
                        unit.token_tile * BM + quarter * 32 + lane, unit.feature_tile * FEATURES);
       } else if (EPI == EPI_ADD_F32 && unit.partial) {
         add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features,
@@ -850,13 +860,13 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
                            unit.feature_tile * FEATURES);
       } else if (EPI == EPI_STORE_BF16 && args.heads > 1) {
         const int head = unit.feature_tile / args.head_tiles;
-        write_row<EPI>(static_cast<__nv_bfloat16*>(args.out) + static_cast<size_t>(head) * args.head_out,
+        write_row<EPI>(FEATURES, static_cast<__nv_bfloat16*>(args.out) + static_cast<size_t>(head) * args.head_out,
                        args.ldo, args.features, lane_base + buffer * Config::kBufferColumns,
                        unit.token_tile * BM + quarter * 32 + lane, args.tokens,
                        (unit.feature_tile - head * args.head_tiles) * FEATURES, args.activation,
                        args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
       } else if (args.tile_group == nullptr || args.tile_group[unit.token_tile] >= 0) {
-        write_row<EPI>(args.out, args.ldo, args.features,
+        write_row<EPI>(FEATURES, args.out, args.ldo, args.features,
                        lane_base + buffer * Config::kBufferColumns,
                        unit.token_tile * BM + quarter * 32 + lane, args.tokens,
                        unit.feature_tile * FEATURES, args.activation, args.gate_limit,
@@ -890,7 +900,8 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
 // the weight rows (for SwiGLU: the gate rows, and the up rows), and tcgen05.mma.cta_group::2 reads
 // both halves: 32 KB a k-block and CTA, so six stages instead of four.  The leader (the even CTA)
 // issues the products for both; either CTA's accumulators hold its own 128 tokens, so the epilogues
-// are those of the kernel above.
+// are those of the kernel above.  Where the last round has few tiles and the epilogue does not add,
+// they are cut into two or four pieces of columns, a pair each.
 // Measured (2,048 tokens, alone, one CTA a tile and pairs): [12,288 x 4,096] 155.8 -> 139.6 us (1,476
 // TFLOP/s), sums by [4,096 x 4,096] 71.3 -> 55.7, gate and up [22,016 x 4,096] 270.3 -> 256.5, sums by
 // [4,096 x 11,008] 173.2 -> 167.9; 512 tokens 54.8 -> 48.2, 25.4 -> 24.6, 90.2 -> 79.9, 66.7 -> 54.5.
@@ -904,8 +915,8 @@ struct PairConfig {
 
 template <int EPI>
 __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pair_kernel(
-    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
-    const PersistentArgs args) {
+    const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_w_piece,
+    const __grid_constant__ CUtensorMap map_x, const PersistentArgs args) {
   using Config = PairConfig;
   constexpr int STAGES = Config::kStages;
   constexpr int FEATURES = EPI == EPI_SWIGLU ? BM : 2 * BM;
@@ -954,11 +965,22 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       uint32_t fill = 0;      // stages filled so far, over all units
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
-        const int feature0 = unit.feature_tile * FEATURES;
+        const int rows = BM / unit.pieces;      // this CTA's half of the tile's (or piece's) rows
+        int feature0 = unit.feature_tile * FEATURES + unit.piece * (FEATURES / unit.pieces);
+        int kb_end = unit.kb_end;
+        if (args.tile_group != nullptr) {
+          const int group = args.tile_group[unit.token_tile];
+          if (group < 0) kb_end = unit.kb_begin;
+          else feature0 += group * args.group_rows;
+        }
         const int weight_row = rank == 0 ? feature0
-                               : EPI == EPI_SWIGLU ? args.up_row_offset + feature0 : feature0 + BM;
+                               : EPI == EPI_SWIGLU ? args.up_row_offset + feature0 : feature0 + rows;
+        const CUtensorMap* map = unit.pieces > 1 ? &map_w_piece : &map_w;
+        const uint32_t bytes = Config::kBytesA + static_cast<uint32_t>(rows) * BK * 2;
+        // tiled weights: a piece lies inside one stored tile
+        const int tile_row = args.k_tiles > 0 ? (weight_row / BM) * args.k_tiles * BM + weight_row % BM : 0;
         const int token0 = unit.token_tile * 2 * BM + rank * BM;
-        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++fill) {
+        for (int kb = unit.kb_begin; kb < kb_end; ++kb, ++fill) {
           const int s = fill % STAGES;
           if (!mbar_wait(&empty_bar[s], ((fill / STAGES) & 1u) ^ 1u)) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
@@ -966,14 +988,13 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
             break;
           }
           uint8_t* stage = smem + s * Config::kStageBytes;
-          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * Config::kStageBytes);
+          if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * bytes);
           const uint32_t bar = cluster_address(&full_bar[s], 0);
           tma_load_2d_pair(stage, &map_x, bar, kb * BK, token0);
           if (args.k_tiles > 0)
-            tma_load_2d_pair(stage + Config::kBytesA, &map_w, bar, 0,
-                             ((weight_row / BM) * args.k_tiles + kb) * BM);
+            tma_load_2d_pair(stage + Config::kBytesA, map, bar, 0, tile_row + kb * BM);
           else
-            tma_load_2d_pair(stage + Config::kBytesA, &map_w, bar, kb * BK, weight_row);
+            tma_load_2d_pair(stage + Config::kBytesA, map, bar, kb * BK, weight_row);
         }
       }
       // the leader's last arrivals at this CTA's barriers, before the CTA may end
@@ -986,7 +1007,6 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
     if (rank == 0 && elect_one()) {
-      constexpr uint32_t idesc = make_idesc(2 * BM, 2 * BM);
       uint32_t drained = 0;
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
@@ -1000,7 +1020,9 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
         }
         tc_fence_after();
         const uint32_t accumulator = tmem_base + buffer * kBufferColumns;
-        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++drained) {
+        const uint32_t idesc = make_idesc(2 * BM, 2 * BM / unit.pieces);
+        const bool skipped = args.tile_group != nullptr && args.tile_group[unit.token_tile] < 0;
+        for (int kb = unit.kb_begin; kb < (skipped ? unit.kb_begin : unit.kb_end); ++kb, ++drained) {
           const int s = drained % STAGES;
           if (!mbar_wait_cluster(&full_bar[s], (drained / STAGES) & 1u)) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
@@ -1061,14 +1083,16 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       }
       tc_fence_after();
       const uint32_t accumulator = lane_base + buffer * kBufferColumns;
-      const int token = unit.token_tile * 2 * BM + row, feature0 = unit.feature_tile * FEATURES;
+      const int columns = FEATURES / unit.pieces;
+      const int token = unit.token_tile * 2 * BM + row;
+      const int feature0 = unit.feature_tile * FEATURES + unit.piece * columns;
       if constexpr (EPI == EPI_ROPE_APPEND) {
-        write_row_rope(args, accumulator, token, feature0);
+        write_row_rope(columns, args, accumulator, token, feature0);
       } else if (EPI == EPI_ADD_F32 && unit.partial) {
         add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
                            args.tokens, feature0);
-      } else {
-        write_row<EPI>(args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
+      } else if (args.tile_group == nullptr || args.tile_group[unit.token_tile] >= 0) {
+        write_row<EPI>(columns, args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
                        args.activation, args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
       }
       if (EPI == EPI_ADD_F32) prepare(iteration + 2);
@@ -1087,85 +1111,10 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
 
 // ----------------------------------------------------------------- host side
 
-using EncodeTiled = CUresult (*)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*,
-                                 const cuuint64_t*, const cuuint64_t*, const cuuint32_t*,
-                                 const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
-                                 CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-
-EncodeTiled encode_tiled() {
-  static EncodeTiled fn = [] {
-    void* symbol = nullptr;
-    cudaDriverEntryPointQueryResult result;
-    if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &symbol, cudaEnableDefault, &result) !=
-            cudaSuccess ||
-        result != cudaDriverEntryPointSuccess) {
-      return static_cast<EncodeTiled>(nullptr);
-    }
-    return reinterpret_cast<EncodeTiled>(symbol);
-  }();
-  return fn;
-}
-
-struct MapKey {
-  const void* base;
-  uint64_t rows;
-  uint64_t depth;
-  uint64_t ld;
-  uint32_t box_rows;
-  bool operator==(const MapKey& o) const {
-    return base == o.base && rows == o.rows && depth == o.depth && ld == o.ld &&
-           box_rows == o.box_rows;
-  }
-};
-struct MapKeyHash {
-  size_t operator()(const MapKey& k) const {
-    size_t h = reinterpret_cast<size_t>(k.base);
-    h = h * 1315423911u ^ k.rows;
-    h = h * 1315423911u ^ k.depth;
-    h = h * 1315423911u ^ k.ld;
-    h = h * 1315423911u ^ k.box_rows;
-    return h;
-  }
-};
-
-// Tensor maps are pure functions of (address, shape, box); encoding one costs a few
-// microseconds, so they are cached for the life of the process.
+// The map of a matrix of bfloat16 whose boxes are `box_rows` rows of one k-block.
 int get_tensor_map(const void* base, uint64_t rows, uint64_t depth, uint64_t ld, uint32_t box_rows,
                    CUtensorMap* out) {
-  static std::mutex mutex;
-  static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{base, rows, depth, ld, box_rows};
-  std::lock_guard<std::mutex> lock(mutex);
-  auto found = cache.find(key);
-  if (found != cache.end()) {
-    *out = found->second;
-    return HX_OK;
-  }
-  EncodeTiled encode = encode_tiled();
-  if (encode == nullptr) {
-    hx_set_error("hx_gemm_tc: the driver does not export cuTensorMapEncodeTiled");
-    return HX_ERR_UNSUPPORTED;
-  }
-  const cuuint64_t dims[2] = {depth, rows};
-  const cuuint64_t strides[1] = {ld * 2};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(BK), box_rows};
-  const cuuint32_t element_strides[2] = {1, 1};
-  CUtensorMap map;
-  const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
-                             dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
-                             CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (rc != CUDA_SUCCESS) {
-    hx_set_error("hx_gemm_tc: cuTensorMapEncodeTiled failed with %d (base %p rows %llu depth %llu "
-                 "ld %llu box %u)", static_cast<int>(rc), base,
-                 static_cast<unsigned long long>(rows), static_cast<unsigned long long>(depth),
-                 static_cast<unsigned long long>(ld), box_rows);
-    return HX_ERR_ARGUMENT;
-  }
-  if (cache.size() > 4096) cache.clear();
-  cache.emplace(key, map);
-  *out = map;
-  return HX_OK;
+  return hx_tensor_map("hx_gemm_tc", base, rows, depth, ld, box_rows, BK, true, out);
 }
 
 template <int BN, int EPI>
@@ -1210,12 +1159,25 @@ int launch_epilogue(int epilogue, const CUtensorMap& map_w, const CUtensorMap& m
 // out gains nothing, with 512 tokens (64 tiles, less than half the grid) it takes 20 % off.
 // 1,900 tokens by [5,120 x 13,824] leave 4 of 300 tiles: 261 us as a whole round, 195 shared out
 // among 80 CTAs.
-double plan_rounds(long long units, int workers, int k_blocks, bool add, int& whole_rounds,
-                   int& tail_workers) {
+//
+// Otherwise (pairs only, `most_pieces` > 1) the tiles of a last round may be cut into pieces of
+// columns: half a tile takes 0.55 of a tile's time, a quarter 0.35 (its tokens are loaded as for a
+// whole one).  256 tokens by [22,016 x 4,096], 86 tiles on 74 pairs: 63.6 -> 47.9 us; 2,048 by
+// [12,288 x 4,096], 384: 142 -> 132 us in place.
+double plan_rounds(long long units, int workers, int k_blocks, bool add, int most_pieces,
+                   int& whole_rounds, int& tail_workers, int& pieces) {
   const int rest = static_cast<int>(units % workers);
   const long long rounds = units / workers;
   whole_rounds = -1;
   tail_workers = 0;
+  pieces = 1;
+  if (!add && rest > 0) {
+    while (2 * pieces <= most_pieces && 2 * pieces * rest <= workers) pieces *= 2;
+    if (pieces > 1) {
+      whole_rounds = static_cast<int>(rounds);
+      return k_blocks * (static_cast<double>(rounds) + (pieces == 2 ? 0.55 : 0.35));
+    }
+  }
   if (add && HX_GEMM_STREAM_K && rest > 0 && rest * 2 <= workers) {
     const double blocks = static_cast<double>(rest) * k_blocks;
     int share = static_cast<int>(sqrt(blocks * workers / 15.0));
@@ -1243,9 +1205,25 @@ bool reserve_shared(Kernel kernel, int bytes) {
 #define HX_GEMM_PAIRS 1      // 0: every tile is one CTA's
 #endif
 
+// What the tensor map of the weights is made from; tiled ones (k_tiles > 0) are rows of 64 elements,
+// tile behind tile.
+struct WeightBoxes {
+  const void* base;
+  uint64_t rows, depth, ld;
+};
+WeightBoxes weight_boxes(const void* w, int weight_rows, int depth, int ldw, int k_tiles) {
+  if (k_tiles > 0)
+    return {w, static_cast<uint64_t>((weight_rows + BM - 1) / BM) * k_tiles * BM, BK, BK};
+  return {w, static_cast<uint64_t>(weight_rows), static_cast<uint64_t>(depth), static_cast<uint64_t>(ldw)};
+}
+
+#ifndef HX_GEMM_PIECES
+#define HX_GEMM_PIECES 4     // at most, of a tile of the last round
+#endif
+
 template <int EPI>
 int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
-                      cudaStream_t stream) {
+                      const WeightBoxes& boxes, cudaStream_t stream) {
   static bool configured = false;
   const int sms = hx_device_sm_count();
   if (sms <= 0) return HX_ERR_LAUNCH;
@@ -1262,9 +1240,9 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   const long long tiles = static_cast<long long>(args.token_tiles) * feature_tiles;
   HX_REQUIRE(tiles < (1ll << 30), "hx_gemm_tc: too many tiles");
   args.units = static_cast<int>(tiles);
-  int whole_rounds = -1, tail = 0;
-  const double alone = plan_rounds(tiles, sms, args.k_blocks, EPI == EPI_ADD_F32, args.whole_rounds,
-                                   args.tail_ctas);
+  int whole_rounds = -1, tail = 0, pieces = 1;
+  const double alone = plan_rounds(tiles, sms, args.k_blocks, EPI == EPI_ADD_F32, 1,
+                                   args.whole_rounds, args.tail_ctas, pieces);
   // Pairs, unless their tiles of 256 tokens make the rounds longer by more than the twentieth that a
   // round is shorter at least (1,900 tokens by [27,648 x 5,120]: 12 rounds against 11, 380 against 375
   // us); short sums that are all pieces have nothing to win (129 tokens by [4,096 x 4,096]: 18.8
@@ -1272,17 +1250,25 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   const int pair_tiles = (args.tokens + 2 * BM - 1) / (2 * BM), pairs = sms / 2;
   const long long pair_units = static_cast<long long>(pair_tiles) * feature_tiles;
   if (HX_GEMM_PAIRS && args.heads == 1 && args.tile_group == nullptr && args.tokens > BM && pairs > 0) {
-    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, whole_rounds,
-                                      tail);
-    const double penalty = whole_rounds == 0 && args.k_blocks < 96 ? 4.0 : 0.0;
+    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, HX_GEMM_PIECES,
+                                      whole_rounds, tail, pieces);
+    const double penalty = EPI == EPI_ADD_F32 && whole_rounds == 0 && args.k_blocks < 96 ? 4.0 : 0.0;
     if (0.95 * paired + penalty <= alone) {
       args.token_tiles = pair_tiles;
       args.units = static_cast<int>(pair_units);
       args.whole_rounds = whole_rounds;
       args.tail_ctas = tail;
-      const int used = whole_rounds == 0 ? tail : pair_units < pairs ? static_cast<int>(pair_units) : pairs;
-      hx_launch(gemm_tc_pair_kernel<EPI>, 2 * used, THREADS, PairConfig::kSmemBytes, stream, map_w, map_x,
-                args);
+      args.tail_pieces = pieces;
+      CUtensorMap map_piece = map_w;
+      if (pieces > 1) {
+        const int rc = get_tensor_map(boxes.base, boxes.rows, boxes.depth, boxes.ld, BM / pieces, &map_piece);
+        if (rc != HX_OK) return rc;
+      }
+      const long long work = pieces > 1 && whole_rounds == 0 ? pair_units * pieces
+                             : whole_rounds == 0             ? tail
+                                                             : pair_units;
+      hx_launch(gemm_tc_pair_kernel<EPI>, 2 * static_cast<int>(work < pairs ? work : pairs), THREADS,
+                PairConfig::kSmemBytes, stream, map_w, map_piece, map_x, args);
       return HX_OK;
     }
   }
@@ -1292,14 +1278,38 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   return HX_OK;
 }
 
+// The grouped product with tiles of 256 tokens: a pair's two CTAs read the same group's weights (1,024
+// tokens with 4 of 16 experts of [5,632 x 4,096] and [4,096 x 2,816]: 547 -> 511 us for the layer).
+template <int EPI>
+int launch_grouped_pairs(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
+                         cudaStream_t stream) {
+  static bool configured = false;
+  const int sms = hx_device_sm_count();
+  if (sms <= 0) return HX_ERR_LAUNCH;
+  if (!configured) {
+    if (!reserve_shared(gemm_tc_pair_kernel<EPI>, PairConfig::kSmemBytes)) return HX_ERR_LAUNCH;
+    configured = true;
+  }
+  constexpr int kFeatures = EPI == EPI_SWIGLU ? BM : 2 * BM;
+  args.token_tiles = (args.tokens + 2 * BM - 1) / (2 * BM);
+  const long long units = static_cast<long long>(args.token_tiles) * ((args.features + kFeatures - 1) / kFeatures);
+  HX_REQUIRE(units < (1ll << 30), "hx_gemm_tc_grouped: too many tiles");
+  args.units = static_cast<int>(units);
+  const int pairs = sms / 2 < args.units ? sms / 2 : args.units;
+  hx_launch(gemm_tc_pair_kernel<EPI>, 2 * pairs, THREADS, PairConfig::kSmemBytes, stream, map_w, map_w, map_x,
+            args);
+  return HX_OK;
+}
+
 int launch_persistent_epilogue(int epilogue, const CUtensorMap& map_w, const CUtensorMap& map_x,
-                               const PersistentArgs& args, cudaStream_t stream) {
+                               const PersistentArgs& args, const WeightBoxes& boxes,
+                               cudaStream_t stream) {
   switch (epilogue) {
-    case EPI_STORE_BF16: return launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, stream);
-    case EPI_STORE_F32: return launch_persistent<EPI_STORE_F32>(map_w, map_x, args, stream);
-    case EPI_ADD_F32: return launch_persistent<EPI_ADD_F32>(map_w, map_x, args, stream);
-    case EPI_SWIGLU: return launch_persistent<EPI_SWIGLU>(map_w, map_x, args, stream);
-    case EPI_ROPE_APPEND: return launch_persistent<EPI_ROPE_APPEND>(map_w, map_x, args, stream);
+    case EPI_STORE_BF16: return launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, boxes, stream);
+    case EPI_STORE_F32: return launch_persistent<EPI_STORE_F32>(map_w, map_x, args, boxes, stream);
+    case EPI_ADD_F32: return launch_persistent<EPI_ADD_F32>(map_w, map_x, args, boxes, stream);
+    case EPI_SWIGLU: return launch_persistent<EPI_SWIGLU>(map_w, map_x, args, boxes, stream);
+    case EPI_ROPE_APPEND: return launch_persistent<EPI_ROPE_APPEND>(map_w, map_x, args, boxes, stream);
     default:
       hx_set_error("hx_gemm_tc: unknown epilogue %d", epilogue);
       return HX_ERR_ARGUMENT;
@@ -1370,10 +1380,8 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
   CUtensorMap map_w, map_x;
   const int total_k_blocks = (depth + BK - 1) / BK;
   const int k_tiles = weight_tiles ? total_k_blocks : 0;
-  int rc = weight_tiles
-               ? get_tensor_map(w, static_cast<uint64_t>((weight_rows + BM - 1) / BM) * k_tiles * BM,
-                                BK, BK, BM, &map_w)
-               : get_tensor_map(w, weight_rows, depth, ldw, BM, &map_w);
+  const WeightBoxes boxes = weight_boxes(w, weight_rows, depth, ldw, k_tiles);
+  int rc = get_tensor_map(boxes.base, boxes.rows, boxes.depth, boxes.ld, BM, &map_w);
   if (rc != HX_OK) return rc;
   rc = get_tensor_map(x, x_capacity_rows, depth, ldx, persistent ? BM : bn, &map_x);
   if (rc != HX_OK) return rc;
@@ -1382,7 +1390,7 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
     PersistentArgs args{out, ldo, tokens, features, depth, up_row_offset, k_tiles, 0, 0,
                         total_k_blocks, status, RopeArgs{}, -1, activation, nullptr, 0,
                         gate_limit, gate_bias, up_bias, softcap};
-    rc = launch_persistent_epilogue(epilogue, map_w, map_x, args, stream);
+    rc = launch_persistent_epilogue(epilogue, map_w, map_x, args, boxes, stream);
     if (rc != HX_OK) return rc;
     HX_CHECK_LAUNCH("hx_gemm_tc");
     return HX_OK;
@@ -1484,15 +1492,26 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
   CUtensorMap map_w, map_x;
   int rc = get_tensor_map(w, static_cast<uint64_t>(groups) * group_rows, depth, ldw, BM, &map_w);
   if (rc != HX_OK) return rc;
-  rc = get_tensor_map(x, x_capacity_rows, depth, ldx, token_tile, &map_x);
+  rc = get_tensor_map(x, x_capacity_rows, depth, ldx, token_tile > BM ? BM : token_tile, &map_x);
   if (rc != HX_OK) return rc;
   const int total_k_blocks = (depth + BK - 1) / BK;
+  if (token_tile == 2 * BM) {
+    PersistentArgs pairs{out, ldo, tokens, features, depth, up_row_offset, 0, 0, 0,
+                         total_k_blocks, status, RopeArgs{}, -1, activation, tile_group,
+                         group_rows, gate_limit};
+    rc = epilogue == EPI_STORE_BF16  ? launch_grouped_pairs<EPI_STORE_BF16>(map_w, map_x, pairs, stream)
+         : epilogue == EPI_STORE_F32 ? launch_grouped_pairs<EPI_STORE_F32>(map_w, map_x, pairs, stream)
+                                     : launch_grouped_pairs<EPI_SWIGLU>(map_w, map_x, pairs, stream);
+    if (rc != HX_OK) return rc;
+    HX_CHECK_LAUNCH("hx_gemm_tc_grouped");
+    return HX_OK;
+  }
   if (token_tile == BM) {
     // tiles of 128 tokens: the persistent kernel, as for prompt portions of a plain product
     PersistentArgs persistent{out, ldo, tokens, features, depth, up_row_offset, 0, 0, 0,
                               total_k_blocks, status, RopeArgs{}, -1, activation, tile_group,
                               group_rows, gate_limit};
-    rc = launch_persistent_epilogue(epilogue, map_w, map_x, persistent, stream);
+    rc = launch_persistent_epilogue(epilogue, map_w, map_x, persistent, WeightBoxes{}, stream);
     if (rc != HX_OK) return rc;
     HX_CHECK_LAUNCH("hx_gemm_tc_grouped");
     return HX_OK;
@@ -1504,9 +1523,7 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
   switch (token_tile) {
     case 16: rc = launch_epilogue<16>(epilogue, map_w, map_x, args, grid, stream); break;
     case 32: rc = launch_epilogue<32>(epilogue, map_w, map_x, args, grid, stream); break;
-    case 64: rc = launch_epilogue<64>(epilogue, map_w, map_x, args, grid, stream); break;
-    case 128: rc = launch_epilogue<128>(epilogue, map_w, map_x, args, grid, stream); break;
-    default: rc = launch_epilogue<256>(epilogue, map_w, map_x, args, grid, stream); break;
+    default: rc = launch_epilogue<64>(epilogue, map_w, map_x, args, grid, stream); break;
   }
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_tc_grouped");
@@ -1575,7 +1592,7 @@ HX_API int hx_gemm_tc_heads(const void* x, int ldx, int x_capacity_rows, int x_s
   args.heads = heads;
   args.head_x = x_stride;
   args.head_out = out_stride;
-  rc = launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, stream);
+  rc = launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, WeightBoxes{}, stream);
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_tc_heads");
   return HX_OK;
@@ -1643,10 +1660,8 @@ HX_API int hx_gemm_tc_rope_append_shared(const void* x, int ldx, int x_capacity_
   CUtensorMap map_w, map_x;
   const int total_k_blocks = (depth + BK - 1) / BK;
   const int k_tiles = weight_tiles ? total_k_blocks : 0;
-  int rc = weight_tiles
-               ? get_tensor_map(w, static_cast<uint64_t>((weight_rows + BM - 1) / BM) * k_tiles * BM,
-                                BK, BK, BM, &map_w)
-               : get_tensor_map(w, weight_rows, depth, ldw, BM, &map_w);
+  const WeightBoxes boxes = weight_boxes(w, weight_rows, depth, ldw, k_tiles);
+  int rc = get_tensor_map(boxes.base, boxes.rows, boxes.depth, boxes.ld, BM, &map_w);
   if (rc != HX_OK) return rc;
   rc = get_tensor_map(x, x_capacity_rows, depth, ldx, BM, &map_x);
   if (rc != HX_OK) return rc;
@@ -1656,7 +1671,7 @@ HX_API int hx_gemm_tc_rope_append_shared(const void* x, int ldx, int x_capacity_
                                static_cast<__nv_bfloat16*>(v_cache), cos_table, sin_table,
                                table_positions, heads, kv_heads, head_dim, rotary_dim, page_size,
                                num_pages, shared_values}};
-  rc = launch_persistent_epilogue(EPI_ROPE_APPEND, map_w, map_x, args, stream);
+  rc = launch_persistent_epilogue(EPI_ROPE_APPEND, map_w, map_x, args, boxes, stream);
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_tc_rope_append");
   return HX_OK;

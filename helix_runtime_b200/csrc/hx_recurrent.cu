@@ -936,7 +936,7 @@ void linear_state_scan_kernel(const LinearStateArgs<T> a) {
 // (v = y silu(g); out = v / rms(v) * w); 1: after it (out = y / rms(y) * w * silu(g)).
 // A warp a group, four values a load, the group's values in registers between the sum and the
 // store: bfloat16 groups of up to 128 PIECES channels, in fours (1,725 tokens of 32 groups of 128: 59 us
-// with a CTA of 128 threads a group, HX_MEASURED_NORM now).
+// with a CTA of 128 threads a group, 18 now).
 template <int PIECES>
 __global__ __launch_bounds__(256) void gated_group_norm_pieces_kernel(
     const float* __restrict__ y, int ld_y, const __nv_bfloat16* __restrict__ gate, int ld_gate,

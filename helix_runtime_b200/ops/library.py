@@ -1699,7 +1699,7 @@ def expert_down(act: torch.Tensor, down: torch.Tensor, chosen: torch.Tensor,
                                 dtype_code(act.dtype), tokens, top, ff, width, experts, _stream()))
 
 
-GROUPED_TILES = (16, 32, 64, 128)
+GROUPED_TILES = (16, 32, 64, 128, 256)
 
 
 def expert_tile(pairs: int, experts: int) -> int:
