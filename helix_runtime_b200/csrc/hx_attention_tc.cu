@@ -3,43 +3,36 @@
 // a [heads, T, T] score tensor for it, src/attention/cuda.cu:31-77), with both products as
 // tcgen05.mma and the scores, the probabilities and the output in tensor memory.
 //
-// One CTA takes 256 consecutive query tokens of one request and one head, as two lanes of 128
-// rows (the M of a product), and walks the request's keys in tiles of 64, anchored at key 0.
-// The lanes share the keys and values in shared memory and nothing else: each has its own
-// thread issuing score products, its own four softmax warps, its own thread issuing output
-// products and its own accumulators in tensor memory.  The second lane's rows see up to two
-// key tiles more than the first's; a short request may leave it empty.  Warp roles:
-//   warps 0, 1  one lane of each asks for the pages of each tile, warp 0 for the keys and
-//               warp 1 for the values: the keys of a (page, head) are one contiguous block of
-//               the cache and so are its values, so a tile is a handful of bulk copies
-//               (cp.async.bulk counted on an mbarrier) into a ring of stages;
-//   warp 2      rewrites the keys of a landed tile piece-major over all 64 keys (see below);
-//   warps 3, 4  one lane each issues S_l = Q_l K^T for lane l into one of the lane's two score
-//               buffers in tensor memory, a tile ahead of the softmax;
-//   warps 5, 6  one lane each issues O_l += P_l V;
-//   warp 7      idles (the softmax groups start at a multiple of four warps, which is what
-//               selects their rows of tensor memory);
-//   warps 8-11, 12-15  softmax of lane 0 / lane 1: thread r owns query row r of its lane.  It
-//               reads its row of S from tensor memory, keeps the running maximum and sum in
-//               float32 registers and writes the probabilities back over the scores it has
-//               read, as TWO bfloat16 terms (P = hi + lo, so the softmax stays a float32
-//               quantity as far as the result can tell).  P is the A operand of O += P V
-//               straight from tensor memory, and O stays in tensor memory over all tiles.  The
-//               maximum a row's exponentials are taken against is only raised when a tile
-//               exceeds it by more than 2^8 (any fixed reference gives the same quotient;
-//               float32 has the range), so the pass over O that a new maximum costs is rare.
+// One CTA takes 128 consecutive query tokens of one request and one head (the M of a product), and
+// walks the request's keys in tiles of 64, anchored at key 0.  Warp roles:
+//   warp 0      one lane asks for the pages of each tile, its values behind the keys of the next
+//               one: the keys of a (page, head) are one contiguous block of the cache and so are
+//               its values, so a tile is a handful of bulk copies (cp.async.bulk counted on an
+//               mbarrier) into a ring of stages;
+//   warp 1      one lane issues S = Q K^T into one of two score buffers in tensor memory;
+//   warp 2      one lane issues O += P V;
+//   warp 3      (pages of 32 and 64 keys) rewrites the keys of a landed tile piece-major over all 64
+//               keys (see below);
+//   warps 4-7   softmax: thread r owns query row r.  It reads its row of S from tensor memory,
+//               keeps the running maximum and sum in float32 registers and writes the
+//               probabilities back over the scores it has read, as TWO bfloat16 terms (P = hi + lo,
+//               so the softmax stays a float32 quantity as far as the result can tell).  P is the
+//               A operand of O += P V straight from tensor memory, and O stays in tensor memory
+//               over all tiles.  The maximum a row's exponentials are taken against is only raised
+//               when a tile exceeds it by more than 2^8 (any fixed reference gives the same
+//               quotient; float32 has the range), so the pass over O that a new maximum costs is
+//               rare;
+//   warps 8-11  (the same, heads wider than 128) three more to rewrite keys.
 //
-// Why two lanes and four issuing threads: one softmax group alone leaves its four schedulers
-// waiting on the latencies of tensor-memory loads and stores and on the exponential unit, and two
-// groups need products issued for both; and what a CTA spends before its first and after its last
-// tile (about 12 us: some 3 us until its first loads from global memory are back, queries and
-// page table alike, then first pages, rewrite, the chain of first products; at the end the last
-// product and the output) is spent once for 256 rows, and every key tile is fetched and rewritten
-// once for them.  The issuing threads are picked by elect.sync: behind `lane == 0` a thread
-// needed 55 ns to issue a product of any size.  Measured (2,048 tokens, 32 heads of 128, in place): 129
-// us a layer, 108 with elect.sync, 87 with the softmax's arithmetic in pairs (its instructions are
-// what bounds the kernel).  Wide heads (2,048 tokens, 32 heads of 256 over one cached row, window
-// 1,024): 610 us on mma.sync, 133 here.
+// Heads of up to 128: two CTAs share an SM.  A tile's way through a CTA is a chain (products,
+// softmax, products), and what a CTA spends before its first and after its last tile is several
+// microseconds more; two CTAs fill each other's gaps, in the middle and at their ends.  The issuing
+// threads are picked by elect.sync (behind `lane == 0` a thread needs 55 ns to issue a product of any
+// size).
+// Measured (2,048 tokens, 32 heads of 128, in place): 129 us a layer with two lanes of 128 rows in one
+// CTA and four issuing threads, 108 with elect.sync, 87 with the softmax's arithmetic in pairs, 91
+// with two CTAs and 66 with their keys gathered.  Wide heads (2,048 tokens, 32 heads of 256 over
+// one cached row, window 1,024): 610 us on mma.sync, 127 here.
 //
 // Operand layouts.  Nothing is swizzled: every operand is made of "core matrices" of 8 rows
 // x 16 bytes (128 contiguous bytes), which is exactly what a page block of the cache is made
@@ -47,7 +40,8 @@
 // O = P V a page block is used as it lies: 16 keys are the K dimension of an MN-major operand
 // (a row of a core matrix is 8 consecutive coordinates of one key, its 8 rows are 8 keys).
 // For S = Q K^T the keys are the N operand (K-major), and one product should cover all 64
-// keys of the tile, which needs one stride from 8 keys to the next across pages: a warp
+// keys of the tile, which needs one stride from 8 keys to the next across pages: with pages of 16
+// keys a gathering copy (tile::gather4) brings one piece of the four pages at a time, otherwise a warp
 // rewrites the tile as [piece][64 keys][16 bytes] (products of one page each are four times
 // as many).  Q is written to shared memory by the CTA itself in the same core-matrix form.
 //
@@ -56,14 +50,15 @@
 // hx_paged_attention.  Every wait is bounded; a wait that runs out sets a status bit, and
 // the CTA frees its tensor memory and returns.
 #include "hx_tcgen05.cuh"
+#include "hx_tensor_map.cuh"
 
 namespace {
 
-constexpr int BLOCK_M = 128;   // query rows per lane (the MMA's M)
+constexpr int BLOCK_M = 128;   // query rows per CTA (the MMA's M)
 constexpr int BLOCK_N = 64;    // keys per tile
-constexpr int S_BUFFERS = 2;   // score tiles in tensor memory per lane
-constexpr int WARP_KEYS = 0, WARP_VALUES = 1, WARP_REWRITE = 2, WARP_SCORES = 3, WARP_OUTPUT = 5,
-              WARP_SOFTMAX = 8;
+constexpr int S_BUFFERS = 2;   // score tiles in tensor memory
+constexpr int WARP_PAGES = 0, WARP_SCORES = 1, WARP_OUTPUT = 2, WARP_REWRITE = 3, WARP_SOFTMAX = 4,
+              WARP_MORE = 8;
 constexpr int GROUP_STRIDE = 128;             // bytes from one 8-row core matrix to the next row group
 constexpr int CHUNK_STRIDE = BLOCK_M * 16;    // bytes from one 16-byte column of Q to the next
 constexpr float RAISE_MAXIMUM_BY = 8.0f;      // log2 units a tile must exceed a row's reference by
@@ -101,27 +96,29 @@ struct TcPrefillArgs {
                           // a tile's rows, token by token; the grid's x counts key/value heads
 };
 
-// Heads of up to 128: two lanes.  Wider ones: tensor memory holds the output of one lane, shared
-// memory its queries and fewer tiles, and four warps share the rewriting of a tile, which is
-// twice as large for half the rows.
-template <int D>
+// Shared memory holds the queries, key tiles as they land (where they are rewritten), key tiles as
+// they are used and value tiles (held until multiplied): 112 KB for a head of 128, so that two CTAs
+// fit.
+//
+// GATHER (pages of 16 keys): a gathering TMA copy brings one 16-byte piece of all 64 keys of a tile
+// from its four pages, which is the order the score product wants; the keys land where they are
+// used.  Other pages land as they are and are rewritten.
+template <int D, bool GATHER>
 struct TcConfig {
-  static constexpr int kLanes = D <= 128 ? 2 : 1;
-  static constexpr int kKeyStages = D <= 128 ? 2 : 1;      // key tiles in shared memory as they land
-  static constexpr int kValueStages = D <= 128 ? 4 : 2;    // value tiles, held until multiplied
-  static constexpr int kKeyBuffers = D <= 128 ? 3 : 2;     // rewritten key tiles
-  static constexpr int kRewriters = D <= 128 ? 1 : 4;
-  static constexpr int kThreads = 256 + 128 * kLanes;
-  static constexpr int kQBytes = BLOCK_M * D * 2;              // per lane
+  static constexpr int kCtas = D <= 128 ? 2 : 1;
+  static constexpr int kKeyStages = GATHER ? 0 : 2, kValueStages = 2, kKeyBuffers = GATHER ? 3 : 1;
+  static constexpr int kRewriters = GATHER ? 0 : D <= 128 ? 1 : 4;
+  static constexpr int kThreads = kRewriters <= 1 ? 256 : 384;
+  static constexpr int kQBytes = BLOCK_M * D * 2;
   static constexpr int kHalfBytes = BLOCK_N * D * 2;          // keys (or values) of a tile
-  static constexpr int kSmemBytes =
-      kLanes * kQBytes + (kKeyStages + kValueStages + kKeyBuffers) * kHalfBytes + 1024 + 512;
+  static constexpr int kSmemBytes = kQBytes + (kKeyStages + kValueStages + kKeyBuffers) * kHalfBytes +
+                                    128 /*alignment*/ + 256 /*barriers*/;
   static constexpr int kScoreColumns = BLOCK_N;               // per score buffer
   static constexpr int kLowTermColumn = BLOCK_N / 2;          // P: hi in columns [0, 32), lo after
-  static constexpr int kOutputColumn = kLanes * S_BUFFERS * BLOCK_N;  // lane 0's O; lane 1's follows
-  static constexpr int kTmemColumns = 512;
-  static_assert(kLanes * (S_BUFFERS * BLOCK_N + D) <= 512, "tensor memory has 512 columns");
-  static_assert(kSmemBytes <= 227 * 1024, "a CTA has 227 KB of shared memory");
+  static constexpr int kOutputColumn = S_BUFFERS * BLOCK_N;
+  static constexpr int kTmemColumns = D <= 128 ? 256 : 512;
+  static_assert(S_BUFFERS * BLOCK_N + D <= kTmemColumns, "tensor memory of a CTA");
+  static_assert(kCtas * (kSmemBytes + 1024) <= 228 * 1024, "an SM has 228 KB of shared memory");
 };
 
 __device__ __forceinline__ float fast_exp2(float x) {
@@ -169,47 +166,58 @@ __device__ __forceinline__ void bulk_copy(uint32_t dst, const void* src, uint32_
       : "memory");
 }
 
-template <int D, bool PACKED>
-__global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc_kernel(
-    TcPrefillArgs a) {
-  using Config = TcConfig<D>;
-  constexpr int LANES = Config::kLanes, THREADS = Config::kThreads;
+// Four rows of a matrix, the same columns of each, one behind the other into shared memory.
+__device__ __forceinline__ void tma_gather_rows(uint32_t dst, const CUtensorMap* map, uint64_t* bar,
+                                                int column, const int (&rows)[4]) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.shared::cluster.global.tile::gather4.mbarrier::complete_tx::bytes "
+      "[%0], [%1, {%3, %4, %5, %6, %7}], [%2];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(smem_u32(bar)), "r"(column), "r"(rows[0]), "r"(rows[1]),
+      "r"(rows[2]), "r"(rows[3])
+      : "memory");
+}
+
+template <int D, bool PACKED, bool GATHER>
+__global__ __launch_bounds__(TcConfig<D, GATHER>::kThreads, TcConfig<D, GATHER>::kCtas) void
+prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const TcPrefillArgs a) {
+  using Config = TcConfig<D, GATHER>;
+  constexpr int THREADS = Config::kThreads;
   constexpr int K_STAGES = Config::kKeyStages, V_STAGES = Config::kValueStages;
   constexpr int KEY_BUFFERS = Config::kKeyBuffers, REWRITERS = Config::kRewriters;
   constexpr int kDSteps = D / 16;      // k-steps of Q K^T
   hx_pdl_trigger();
 
-  // which request and which 256-row tile of it is this CTA?  The last rows of a request see
+  // which request and which 128-row tile of it is this CTA?  The last rows of a request see
   // the most keys: their CTAs are started first (the grid is walked heads first, then tiles),
   // so the short ones fill the gaps at the end.
   // A row is a token of one head, or with PACKED one of the `pack` heads of a token.
   const int pack = PACKED ? a.pack : 1;
   auto token_of = [&](int row) { return PACKED ? row / pack : row; };
-  const int tile_tokens = token_of(LANES * BLOCK_M);
+  const int tile_tokens = token_of(BLOCK_M);
   int tile_in_request = 0, tiles_of_request = 0;
   const int request = hx_find_query_tile(a.request_start, a.requests, a.min_query_len,
-                                         tile_tokens, blockIdx.y, tile_in_request,
-                                         tiles_of_request);
+                                         tile_tokens, blockIdx.z * gridDim.y + blockIdx.y,
+                                         tile_in_request, tiles_of_request);
   tile_in_request = tiles_of_request - 1 - tile_in_request;
   if (request < 0) return;      // before any barrier or allocation: the whole CTA leaves
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>(
-      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+      (reinterpret_cast<uintptr_t>(smem_raw) + 127) & ~static_cast<uintptr_t>(127));
   uint8_t* q_tile = smem;
-  uint8_t* k_stages = q_tile + LANES * Config::kQBytes;
+  uint8_t* k_stages = q_tile + Config::kQBytes;
   uint8_t* v_stages = k_stages + K_STAGES * Config::kHalfBytes;
   uint8_t* keys_by_piece = v_stages + V_STAGES * Config::kHalfBytes;      // [KEY_BUFFERS]
   uint64_t* k_full = reinterpret_cast<uint64_t*>(keys_by_piece + KEY_BUFFERS * Config::kHalfBytes);
   uint64_t* k_empty = k_full + K_STAGES;
   uint64_t* v_full = k_empty + K_STAGES;
-  uint64_t* v_empty = v_full + V_STAGES;              // [LANES][V_STAGES]: a lane's product has read it
-  uint64_t* s_full = v_empty + LANES * V_STAGES;      // [LANES][S_BUFFERS] scores of tile t in buffer t % 2
-  uint64_t* p_full = s_full + LANES * S_BUFFERS;      // [LANES][S_BUFFERS] its probabilities are in place
-  uint64_t* o_full = p_full + LANES * S_BUFFERS;      // [LANES][S_BUFFERS] its output product is done
-  uint64_t* k_ready = o_full + LANES * S_BUFFERS;     // [KEY_BUFFERS] the tile's keys are rewritten
-  uint64_t* k_done = k_ready + KEY_BUFFERS;           // [LANES][KEY_BUFFERS] a lane's scores have read them
-  uint64_t* q_ready = k_done + LANES * KEY_BUFFERS;   // the query tiles are in shared memory
+  uint64_t* v_empty = v_full + V_STAGES;       // the product has read it
+  uint64_t* s_full = v_empty + V_STAGES;       // [S_BUFFERS] scores of tile t in buffer t % 2
+  uint64_t* p_full = s_full + S_BUFFERS;       // [S_BUFFERS] its probabilities are in place
+  uint64_t* o_full = p_full + S_BUFFERS;       // [S_BUFFERS] its output product is done
+  uint64_t* k_ready = o_full + S_BUFFERS;      // [KEY_BUFFERS] the tile's keys are rewritten
+  uint64_t* k_done = k_ready + KEY_BUFFERS;    // [KEY_BUFFERS] its scores have read them
+  uint64_t* q_ready = k_done + KEY_BUFFERS;    // the query tile is in shared memory
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(q_ready + 1);
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_holder + 1);
 
@@ -236,14 +244,8 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       a.window > 0 ? min((a.keep_first + BLOCK_N - 1) / BLOCK_N, first_needed / BLOCK_N) : 0;
   const int skipped = first_needed / BLOCK_N - kept_tiles;
   auto tile_at = [&](int turn) { return turn < kept_tiles ? turn : turn + skipped; };
-  const int n_tiles = last_key / BLOCK_N + 1 - skipped;       // turns somebody here takes
-  // lane l has rows [128 l, ...) of the CTA's and takes the turns before lane_tiles(l); lane 1 may be empty
-  auto lane_rows = [&](int l) { return max(0, min(BLOCK_M, rows_here - l * BLOCK_M)); };
-  auto lane_tiles = [&](int l) {
-    const int rows = lane_rows(l);
-    return rows > 0 ? (context + token0 + token_of(l * BLOCK_M + rows - 1)) / BLOCK_N + 1 - skipped : 0;
-  };
-  const int page_size = a.page_size;
+  const int n_tiles = last_key / BLOCK_N + 1 - skipped;
+  const int page_size = GATHER ? BLOCK_N / 4 : a.page_size;
   const int pages_per_tile = BLOCK_N / page_size;
   const uint32_t page_bytes = static_cast<uint32_t>(page_size) * D * 2;
   const uint32_t piece_stride = static_cast<uint32_t>(page_size) * 16;   // next 16-byte piece of a key
@@ -253,15 +255,19 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       mbar_init(&k_full[s], 1);
       mbar_init(&k_empty[s], REWRITERS);
     }
-    for (int s = 0; s < V_STAGES; ++s) mbar_init(&v_full[s], 1);
-    for (int s = 0; s < LANES * V_STAGES; ++s) mbar_init(&v_empty[s], 1);
-    for (int b = 0; b < LANES * S_BUFFERS; ++b) {
+    for (int s = 0; s < V_STAGES; ++s) {
+      mbar_init(&v_full[s], 1);
+      mbar_init(&v_empty[s], 1);
+    }
+    for (int b = 0; b < S_BUFFERS; ++b) {
       mbar_init(&s_full[b], 1);
-      mbar_init(&p_full[b], 4);   // one arrival per softmax warp of the lane
+      mbar_init(&p_full[b], 4);   // one arrival per softmax warp
       mbar_init(&o_full[b], 1);
     }
-    for (int b = 0; b < KEY_BUFFERS; ++b) mbar_init(&k_ready[b], REWRITERS);
-    for (int b = 0; b < LANES * KEY_BUFFERS; ++b) mbar_init(&k_done[b], 1);
+    for (int b = 0; b < KEY_BUFFERS; ++b) {
+      mbar_init(&k_ready[b], GATHER ? 1 : REWRITERS);      // the copies, or the warps that rewrite
+      mbar_init(&k_done[b], 1);
+    }
     mbar_init(q_ready, THREADS / 32 - WARP_SCORES);      // one arrival per warp that loads queries
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -275,19 +281,19 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
   tc_fence_after();
   const uint32_t tmem_base = *tmem_holder;
 
-  // ---- the query tiles: per lane [D / 8 pieces][16 row groups][8 rows][16 bytes], written by
-  // the warps from WARP_SCORES on while the first pages are on their way.  All of a thread's
-  // loads are in flight together (one after the other they cost the CTA 6 us).
+  // ---- the query tile: [D / 8 pieces][16 row groups][8 rows][16 bytes], written by the warps from
+  // WARP_SCORES on while the first pages are on their way.  All of a thread's loads are in flight
+  // together (one after the other they cost the CTA 6 us).
   if (warp >= WARP_SCORES) {
     constexpr int kLoaders = THREADS - WARP_SCORES * 32;
-    constexpr int kPieces = LANES * BLOCK_M * (D / 8);
+    constexpr int kPieces = BLOCK_M * (D / 8);
     constexpr int kPerThread = (kPieces + kLoaders - 1) / kLoaders;
     const int loader = threadIdx.x - WARP_SCORES * 32;
     uint4 values[kPerThread];
 #pragma unroll
     for (int i = 0; i < kPerThread; ++i) {
       const int index = loader + i * kLoaders;
-      const int row = index / (D / 8);      // among the CTA's 256
+      const int row = index / (D / 8);
       const int piece = index - row * (D / 8);
       values[i] = make_uint4(0u, 0u, 0u, 0u);
       if (index < kPieces && row < rows_here) {
@@ -302,27 +308,18 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       const int index = loader + i * kLoaders;
       const int row = index / (D / 8);
       const int piece = index - row * (D / 8);
-      const int in_lane = row & (BLOCK_M - 1);
       if (index < kPieces)
-        *reinterpret_cast<uint4*>(q_tile + (row / BLOCK_M) * Config::kQBytes + piece * CHUNK_STRIDE +
-                                  (in_lane >> 3) * GROUP_STRIDE + (in_lane & 7) * 16) = values[i];
+        *reinterpret_cast<uint4*>(q_tile + piece * CHUNK_STRIDE + (row >> 3) * GROUP_STRIDE +
+                                  (row & 7) * 16) = values[i];
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
     if (lane == 0) mbar_arrive(q_ready);
   }
 
-  if (warp == WARP_KEYS || warp == WARP_VALUES) {
+  if (warp == WARP_PAGES) {
     // ------------------------------------------------------------ page requests
-    // Each as far ahead as its own ring allows: the keys of a tile are wanted well before
-    // its values (they are rewritten, then multiplied, then the softmax runs), and one ring
-    // must not hold up the other.
     if (elect_one()) {
-      const bool values = warp == WARP_VALUES;
-      const int stages = values ? V_STAGES : K_STAGES;
-      uint64_t* full = values ? v_full : k_full;
-      uint8_t* ring = values ? v_stages : k_stages;
-      const uint8_t* cache = reinterpret_cast<const uint8_t*>(values ? a.v_cache : a.k_cache);
       const int* table = a.block_tables +
                          static_cast<size_t>(a.request_table_row[request]) * a.table_stride;
       const int last_page = last_key / page_size;
@@ -333,56 +330,88 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
           // a page that holds no kept key and ends before the first key needed is not read
           const bool wanted = index * page_size < a.keep_first ||
                               (index + 1) * page_size > first_needed;
-          pages[p] = (p < pages_per_tile && index <= last_page && wanted) ? table[index]
-                                                                          : -2;   // -2: none
+          int page = -2;                                             // -2: none
+          if (p < pages_per_tile && index <= last_page && wanted) {
+            page = table[index];
+            if (page < 0 || page >= a.num_pages) page = -1;          // reported where it is asked for
+          }
+          pages[p] = page;
         }
       };
-      int pages[4], next_pages[4];
+      // the copies of a tile's page blocks into a stage that is free
+      auto request_tile = [&](const __nv_bfloat16* cache, uint8_t* stage, uint64_t* full,
+                              const int (&pages)[4]) {
+        uint32_t expected = 0;
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          if (pages[p] == -1) atomicOr(a.status, HX_FLAG_BAD_PAGE);
+          if (pages[p] >= 0) expected += page_bytes;
+        }
+        mbar_expect_tx(full, expected);
+        const uint32_t base = smem_u32(stage);
+#pragma unroll
+        for (int p = 0; p < 4; ++p) {
+          if (pages[p] >= 0) {
+            const size_t block = (static_cast<size_t>(pages[p]) * a.kv_heads + kv_head) * page_bytes;
+            bulk_copy(base + p * page_bytes, reinterpret_cast<const uint8_t*>(cache) + block, page_bytes,
+                      full);
+          }
+        }
+      };
+      int pages[4], value_pages[4];
       pages_of(0, pages);
-      for (int tile = 0; tile < n_tiles && !*failed; ++tile) {
-        if (tile + 1 < n_tiles) pages_of(tile + 1, next_pages);      // in flight during the wait
-        const int stage = tile % stages;
+      // turn t asks for the keys of tile t and for the values of tile t - 1, which are wanted
+      // later: their keys are rewritten and multiplied, and the softmax runs, in between
+      for (int tile = 0; tile <= n_tiles && !*failed; ++tile) {
+        int next_pages[4];
+        if (tile + 1 < n_tiles) pages_of(tile + 1, next_pages);      // in flight during the waits
         bool free = true;
-        if (!values) {
-          free = mbar_wait(&k_empty[stage], (static_cast<uint32_t>(tile / stages) & 1u) ^ 1u);
-        } else if (tile >= V_STAGES) {
-          // the stage held tile - V_STAGES: every lane that saw that tile has multiplied by it
-          const int before = tile - V_STAGES;
-          for (int l = 0; l < LANES && free; ++l)
-            if (before < lane_tiles(l))
-              free = mbar_wait(&v_empty[l * V_STAGES + stage],
-                               static_cast<uint32_t>(before / V_STAGES) & 1u);
+        if (tile < n_tiles) {
+          if constexpr (GATHER) {
+            const int buffer = tile % KEY_BUFFERS;
+            free = mbar_wait(&k_done[buffer], (static_cast<uint32_t>(tile / KEY_BUFFERS) & 1u) ^ 1u);
+            if (free) {
+              // no page: any row will do, no key of it is seen
+              int rows[4];
+#pragma unroll
+              for (int p = 0; p < 4; ++p) {
+                if (pages[p] == -1) atomicOr(a.status, HX_FLAG_BAD_PAGE);
+                rows[p] = max(pages[p], 0) * a.kv_heads + kv_head;
+              }
+              mbar_expect_tx(&k_ready[buffer], Config::kHalfBytes);
+              const uint32_t target = smem_u32(keys_by_piece + buffer * Config::kHalfBytes);
+#pragma unroll 4
+              for (int piece = 0; piece < D / 8; ++piece)
+                tma_gather_rows(target + piece * (BLOCK_N * 16), &key_pages, &k_ready[buffer],
+                                piece * (BLOCK_N / 4) * 8, rows);
+            }
+          } else {
+            const int stage = tile % K_STAGES;
+            free = mbar_wait(&k_empty[stage], (static_cast<uint32_t>(tile / K_STAGES) & 1u) ^ 1u);
+            if (free)
+              request_tile(a.k_cache, k_stages + stage * Config::kHalfBytes, &k_full[stage], pages);
+          }
+        }
+        if (free && tile > 0) {
+          const int before = tile - 1, stage = before % V_STAGES;
+          free = mbar_wait(&v_empty[stage], (static_cast<uint32_t>(before / V_STAGES) & 1u) ^ 1u);
+          if (free)
+            request_tile(a.v_cache, v_stages + stage * Config::kHalfBytes, &v_full[stage], value_pages);
         }
         if (!free) {
           atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
           break;
         }
-        uint32_t expected = 0;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
-          if (pages[p] >= a.num_pages || pages[p] == -1) {
-            atomicOr(a.status, HX_FLAG_BAD_PAGE);
-            pages[p] = -2;
-          }
-          if (pages[p] >= 0) expected += page_bytes;
+          value_pages[p] = pages[p];
+          pages[p] = next_pages[p];
         }
-        mbar_expect_tx(&full[stage], expected);
-        const uint32_t base = smem_u32(ring + stage * Config::kHalfBytes);
-#pragma unroll
-        for (int p = 0; p < 4; ++p) {
-          if (pages[p] >= 0) {
-            const size_t block = (static_cast<size_t>(pages[p]) * a.kv_heads + kv_head) * page_bytes;
-            bulk_copy(base + p * page_bytes, cache + block, page_bytes, &full[stage]);
-          }
-        }
-#pragma unroll
-        for (int p = 0; p < 4; ++p) pages[p] = next_pages[p];
       }
     }
-  } else if (warp == WARP_REWRITE ||
-             (REWRITERS == 4 && (warp == WARP_SCORES + 1 || warp == WARP_OUTPUT + 1 ||
-                                 warp == WARP_SOFTMAX - 1))) {
+  } else if (!GATHER && (warp == WARP_REWRITE || (warp >= WARP_MORE && warp < WARP_MORE + REWRITERS - 1))) {
+    if constexpr (!GATHER) {
     // ------------------------------------------------------ keys, piece by piece
     // The score product wants all 64 keys of the tile at one stride, but every page block
     // holds its own keys piece-major: this warp rewrites a landed tile as
@@ -390,10 +419,7 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
     bool ok = true;
     // this warp's share of the pieces
     constexpr int kShare = D / 8 / REWRITERS;
-    const int first_piece = REWRITERS == 1 || warp == WARP_REWRITE ? 0
-                            : warp == WARP_SCORES + 1              ? kShare
-                            : warp == WARP_OUTPUT + 1              ? 2 * kShare
-                                                                   : 3 * kShare;
+    const int first_piece = warp == WARP_REWRITE ? 0 : (warp - WARP_MORE + 1) * kShare;
     // where keys `lane` and `lane + 32` of a tile sit inside the landed page blocks
     const uint32_t source_low = (lane / page_size) * page_bytes + (lane % page_size) * 16;
     const uint32_t source_high =
@@ -401,16 +427,11 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
     for (int tile = 0; tile < n_tiles && ok && !*failed; ++tile) {
       if (lane == 0) {
         ok = mbar_wait(&k_full[tile % K_STAGES], static_cast<uint32_t>(tile / K_STAGES) & 1u);
-        // the score products that read this buffer KEY_BUFFERS tiles ago are done (one per
-        // lane that saw that tile; a barrier of its own per lane and buffer, whose next phase
-        // needs this very rewrite, so that no phase can be mistaken for another)
-        if (tile >= KEY_BUFFERS) {
-          const int before = tile - KEY_BUFFERS;
-          for (int l = 0; l < LANES && ok; ++l)
-            if (before < lane_tiles(l))
-              ok = mbar_wait(&k_done[l * KEY_BUFFERS + tile % KEY_BUFFERS],
-                             static_cast<uint32_t>(before / KEY_BUFFERS) & 1u);
-        }
+        // the score products that read this buffer KEY_BUFFERS tiles ago are done (the barrier's
+        // next phase needs this very rewrite, so no phase can be mistaken for another)
+        if (ok && tile >= KEY_BUFFERS)
+          ok = mbar_wait(&k_done[tile % KEY_BUFFERS],
+                         static_cast<uint32_t>((tile - KEY_BUFFERS) / KEY_BUFFERS) & 1u);
         if (!ok) {
           atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
@@ -455,29 +476,27 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
         mbar_arrive(&k_empty[tile % K_STAGES]);      // the landed copy may be overwritten
       }
     }
-  } else if (warp >= WARP_SCORES && warp < WARP_SCORES + LANES) {
+    }
+  } else if (warp == WARP_SCORES) {
     // ------------------------------------------------------------ score products
     if (elect_one()) {
       constexpr uint32_t idesc_scores = make_idesc(BLOCK_M, BLOCK_N);
       // Descriptors differ from product to product only in their start address (the low 14
       // bits, in units of 16 bytes): build one of each kind and add offsets.
-      const uint64_t desc_q0 = make_smem_desc_plain(smem_u32(q_tile), CHUNK_STRIDE, GROUP_STRIDE);
+      const uint64_t desc_q = make_smem_desc_plain(smem_u32(q_tile), CHUNK_STRIDE, GROUP_STRIDE);
       const uint64_t desc_k0 =
           make_smem_desc_plain(smem_u32(keys_by_piece), BLOCK_N * 16, GROUP_STRIDE);
       constexpr uint32_t kKeyBufferStep = Config::kHalfBytes >> 4;
       constexpr uint32_t kChunkPairStep = (2 * CHUNK_STRIDE) >> 4;      // 16 coordinates of Q on
       constexpr uint32_t kKeyPiecePairStep = (2 * BLOCK_N * 16) >> 4;   // 16 coordinates of the keys on
-      // S_l[tile % 2] = Q_l K_tile^T: one product of 64 keys per 16 coordinates.  The buffer
-      // held the probabilities of tile - 2, which the lane's output product must have read.
-      const int l = warp - WARP_SCORES;
-      const int my_tiles = lane_tiles(l);
-      const uint64_t desc_q = desc_q0 + l * (Config::kQBytes >> 4);
       if (!mbar_wait(q_ready, 0)) {
         atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
         *failed = 1;
       }
-      for (int tile = 0; tile < my_tiles && !*failed; ++tile) {
-        const int b = l * S_BUFFERS + tile % S_BUFFERS;
+      // S[tile % 2] = Q K_tile^T: one product of 64 keys per 16 coordinates.  The buffer held the
+      // probabilities of tile - 2, which the output product must have read.
+      for (int tile = 0; tile < n_tiles && !*failed; ++tile) {
+        const int b = tile % S_BUFFERS;
         if (!mbar_wait(&k_ready[tile % KEY_BUFFERS], static_cast<uint32_t>(tile / KEY_BUFFERS) & 1u) ||
             (tile >= S_BUFFERS &&
              !mbar_wait(&o_full[b], static_cast<uint32_t>((tile - S_BUFFERS) / S_BUFFERS) & 1u))) {
@@ -493,14 +512,12 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
           umma_bf16(target, desc_q + k * kChunkPairStep, desc_k + k * kKeyPiecePairStep,
                     idesc_scores, k > 0 ? 1u : 0u);
         umma_commit(&s_full[b]);
-        umma_commit(&k_done[l * KEY_BUFFERS + tile % KEY_BUFFERS]);
+        umma_commit(&k_done[tile % KEY_BUFFERS]);
       }
     }
-  } else if (warp >= WARP_OUTPUT && warp < WARP_OUTPUT + LANES) {
+  } else if (warp == WARP_OUTPUT) {
     // ----------------------------------------------------------- output products
     if (elect_one()) {
-      const int l = warp - WARP_OUTPUT;
-      const int my_tiles = lane_tiles(l);
       constexpr uint32_t idesc_output = make_idesc_b_mn_major(BLOCK_M, D);
       // values: MN-major, the next 8 keys are 128 bytes on, the next 8 coordinates one piece on
       const uint64_t desc_v0 = make_smem_desc_plain(smem_u32(v_stages), GROUP_STRIDE, piece_stride);
@@ -512,11 +529,10 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
         const int key = g * 16;
         value_step[g] = ((key / page_size) * page_bytes + (key % page_size) * 16) >> 4;
       }
-      const uint32_t target = tmem_base + Config::kOutputColumn + l * D;
-      for (int tile = 0; tile < my_tiles && !*failed; ++tile) {
+      const uint32_t target = tmem_base + Config::kOutputColumn;
+      for (int tile = 0; tile < n_tiles && !*failed; ++tile) {
         // the probabilities of this tile lie where its scores were
-        const int s = tile % V_STAGES;
-        const int b = l * S_BUFFERS + tile % S_BUFFERS;
+        const int b = tile % S_BUFFERS, s = tile % V_STAGES;
         if (!mbar_wait(&p_full[b], static_cast<uint32_t>(tile / S_BUFFERS) & 1u) ||
             !mbar_wait(&v_full[s], static_cast<uint32_t>(tile / V_STAGES) & 1u)) {
           atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
@@ -527,29 +543,25 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
         const uint64_t desc_v = desc_v0 + s * kStageStep;
         const uint32_t p_hi = tmem_base + b * Config::kScoreColumns;
         const uint32_t p_lo = p_hi + Config::kLowTermColumn;
-        // O_l += P V_tile: 16 keys (8 columns of P) per product, the hi and the lo term of P
+        // O += P V_tile: 16 keys (8 columns of P) per product, the hi and the lo term of P
 #pragma unroll
         for (int g = 0; g < BLOCK_N / 16; ++g) {
           umma_bf16_a_tmem(target, p_hi + g * 8, desc_v + value_step[g], idesc_output,
                            (tile > 0 || g > 0) ? 1u : 0u);
           umma_bf16_a_tmem(target, p_lo + g * 8, desc_v + value_step[g], idesc_output, 1u);
         }
-        umma_commit(&v_empty[l * V_STAGES + s]);     // this lane is done with the stage
+        umma_commit(&v_empty[s]);
         umma_commit(&o_full[b]);                     // O holds this tile; its P has been read
       }
     }
-  } else if (warp >= WARP_SOFTMAX) {
+  } else if (warp >= WARP_SOFTMAX && warp < WARP_MORE) {
     // ------------------------------------------------------------------ softmax
-    const int l = (warp - WARP_SOFTMAX) >> 2;      // the lane this group serves
-    const int my_tiles = lane_tiles(l);
-    const int my_rows = lane_rows(l);
     const int quarter = warp & 3;      // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
     const int row = quarter * 32 + lane;
-    const int group_thread = threadIdx.x - (WARP_SOFTMAX + 4 * l) * 32;      // 0..127
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-    const uint32_t output_base = lane_base + Config::kOutputColumn + l * D;
-    const int my_token = token_of(l * BLOCK_M + row);
-    const int head = min(head_of(l * BLOCK_M + row, my_token), a.heads - 1);
+    const uint32_t output_base = lane_base + Config::kOutputColumn;
+    const int my_token = token_of(row);
+    const int head = min(head_of(row, my_token), a.heads - 1);
     const int q_position = context + token0 + my_token;             // the last key this row sees
     float row_max = -INFINITY;      // the reference of this row's exponentials, in log2 units
     float row_sum = 0.0f;
@@ -575,8 +587,8 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       return state == 0;
     };
 
-    for (int tile = 0; tile < my_tiles && ok; ++tile) {
-      const int b = l * S_BUFFERS + tile % S_BUFFERS;
+    for (int tile = 0; tile < n_tiles && ok; ++tile) {
+      const int b = tile % S_BUFFERS;
       ok = wait_for(&s_full[b], static_cast<uint32_t>(tile / S_BUFFERS) & 1u);
       if (!ok) break;
       tc_fence_after();
@@ -638,12 +650,12 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
         // ---- a new reference: what O and the sum hold was taken against the old one.  The
         // product of the previous tile must have landed; the product of this tile waits for
         // this warp's arrival below.  (o_full[b] completes a phase for every other tile; its
-        // previous phase was complete before the scores of this tile were started.)
+        // previous phase was complete before the scores of the previous tile were.)
         const float new_max = fmaxf(row_max, tile_max);
         const float correction = row_max == -INFINITY ? 0.0f : fast_exp2(row_max - new_max);
         row_max = new_max;
         row_sum *= correction;
-        ok = wait_for(&o_full[l * S_BUFFERS + (tile - 1) % S_BUFFERS],
+        ok = wait_for(&o_full[(tile - 1) % S_BUFFERS],
                       static_cast<uint32_t>((tile - 1) / S_BUFFERS) & 1u);
         if (!ok) break;
         tc_fence_after();
@@ -702,9 +714,7 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       tmem_store_wait();
 
       // ---- value rows behind the last key hold whatever the pages (or an earlier tile)
-      // left there; a NaN would survive a zero probability, so they are cleared (by the group
-      // that is first to need the tile: the other waits for its own arrival barrier only, but
-      // the tile with the last key is seen by the last lane alone, or by lane 0 alone)
+      // left there; a NaN would survive a zero probability, so they are cleared.
       // The same goes for the keys between the kept ones and the first key needed, whose pages
       // were not read.
       const int first_stale = last_key + 1 - key0;
@@ -716,7 +726,7 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
         ok = wait_for(&v_full[tile % V_STAGES], static_cast<uint32_t>(tile / V_STAGES) & 1u);
         if (!ok) break;
         uint8_t* v_half = v_stages + (tile % V_STAGES) * Config::kHalfBytes;
-        for (int index = group_thread; index < BLOCK_N * (D / 8); index += 128) {
+        for (int index = row; index < BLOCK_N * (D / 8); index += 128) {
           const int key = index / (D / 8);
           const int piece = index - key * (D / 8);
           if (key >= first_stale || (has_unseen && key >= unseen_from && key < unseen_to))
@@ -731,11 +741,11 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
       if (lane == 0) mbar_arrive(&p_full[b]);
     }
 
-    // ---- a commit covers every product its thread issued before it: the lane's last tile
-    // says all of them are done
-    if (ok && my_tiles > 0) {
-      ok = wait_for(&o_full[l * S_BUFFERS + (my_tiles - 1) % S_BUFFERS],
-                    static_cast<uint32_t>((my_tiles - 1) / S_BUFFERS) & 1u);
+    // ---- a commit covers every product its thread issued before it: the last tile says all of
+    // them are done
+    if (ok) {
+      ok = wait_for(&o_full[(n_tiles - 1) % S_BUFFERS],
+                    static_cast<uint32_t>((n_tiles - 1) / S_BUFFERS) & 1u);
       if (ok) {
         tc_fence_after();
         float inverse = 1.0f / row_sum;
@@ -757,7 +767,7 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
           tmem_load16_issue(output_base + d0, r[0]);
           if (both) tmem_load16_issue(output_base + d0 + 16, r[1]);
           tmem_load_wait();
-          if (row < my_rows) {
+          if (row < rows_here) {
 #pragma unroll
             for (int h = 0; h < (both ? 2 : 1); ++h)
 #pragma unroll
@@ -784,12 +794,12 @@ __global__ __launch_bounds__(TcConfig<D>::kThreads, 1) void prefill_attention_tc
   }
 }
 
-template <int D, bool PACKED = false>
-int launch(const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
-  using Config = TcConfig<D>;
+template <int D, bool PACKED, bool GATHER>
+int launch_with(const CUtensorMap& key_pages, const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
+  using Config = TcConfig<D, GATHER>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(prefill_attention_tc_kernel<D, PACKED>,
+    if (cudaFuncSetAttribute(prefill_attention_tc_kernel<D, PACKED, GATHER>,
                              cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Config::kSmemBytes) != cudaSuccess) {
       cudaGetLastError();
@@ -799,9 +809,24 @@ int launch(const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
     }
     configured = true;
   }
-  hx_launch(prefill_attention_tc_kernel<D, PACKED>, dim3(PACKED ? a.heads / a.pack : a.heads, tiles),
-            Config::kThreads, Config::kSmemBytes, stream, a);
+  // `tiles` bounds tiles of 256 tokens, or exactly the packed ones
+  const dim3 grid(PACKED ? a.heads / a.pack : a.heads, tiles, PACKED ? 1 : 256 / BLOCK_M);
+  hx_launch(prefill_attention_tc_kernel<D, PACKED, GATHER>, grid, Config::kThreads, Config::kSmemBytes,
+            stream, key_pages, a);
   return HX_OK;
+}
+
+template <int D, bool PACKED = false>
+int launch(const TcPrefillArgs& a, int tiles, cudaStream_t stream) {
+  CUtensorMap key_pages{};
+  if (a.page_size != BLOCK_N / 4) return launch_with<D, PACKED, false>(key_pages, a, tiles, stream);
+  // a row of the map is the block of a page and key/value head
+  const uint64_t row = static_cast<uint64_t>(a.page_size) * D;
+  const int rc = hx_tensor_map("hx_prefill_attention_tc", a.k_cache,
+                               static_cast<uint64_t>(a.num_pages) * a.kv_heads, row, row, 1,
+                               8 * a.page_size, false, &key_pages);
+  if (rc != HX_OK) return rc;
+  return launch_with<D, PACKED, true>(key_pages, a, tiles, stream);
 }
 
 }  // namespace
@@ -836,7 +861,9 @@ HX_API int hx_prefill_attention_tc_biased(const void* q, int ldq, const void* k_
   HX_REQUIRE(requests >= 0 && tile_bound >= 0 && heads > 0 && kv_heads > 0 && heads % kv_heads == 0,
              "hx_prefill_attention_tc: bad sizes");
   HX_REQUIRE(tile_bound <= 65535, "hx_prefill_attention_tc: too many query tiles");
-  HX_REQUIRE(num_pages > 0 && table_stride > 0, "hx_prefill_attention_tc: bad cache geometry");
+  HX_REQUIRE(num_pages > 0 && table_stride > 0 &&
+                 static_cast<long long>(num_pages) * kv_heads < (1ll << 31),
+             "hx_prefill_attention_tc: bad cache geometry");
   HX_REQUIRE(status != nullptr, "hx_prefill_attention_tc: status word missing");
   HX_REQUIRE(ldq % 8 == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 &&
@@ -926,7 +953,9 @@ HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_
              heads, head_dim, kv_heads, page_size);
   HX_REQUIRE(requests >= 0 && tile_bound >= 0, "hx_prefill_attention_tc_packed: bad sizes");
   HX_REQUIRE(tile_bound <= 65535, "hx_prefill_attention_tc_packed: too many query tiles");
-  HX_REQUIRE(num_pages > 0 && table_stride > 0, "hx_prefill_attention_tc_packed: bad cache geometry");
+  HX_REQUIRE(num_pages > 0 && table_stride > 0 &&
+                 static_cast<long long>(num_pages) * kv_heads < (1ll << 31),
+             "hx_prefill_attention_tc_packed: bad cache geometry");
   HX_REQUIRE(status != nullptr, "hx_prefill_attention_tc_packed: status word missing");
   HX_REQUIRE(ldq % 8 == 0 && ldo % 8 == 0 && (reinterpret_cast<uintptr_t>(q) & 15) == 0 &&
                  (reinterpret_cast<uintptr_t>(k_cache) & 15) == 0 &&
