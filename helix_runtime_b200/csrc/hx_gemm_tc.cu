@@ -1592,7 +1592,8 @@ HX_API int hx_gemm_tc_heads(const void* x, int ldx, int x_capacity_rows, int x_s
   args.heads = heads;
   args.head_x = x_stride;
   args.head_out = out_stride;
-  rc = launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, WeightBoxes{}, stream);
+  rc = launch_persistent<EPI_STORE_BF16>(
+      map_w, map_x, args, weight_boxes(w, heads * out_dim, in_dim, in_dim, 0), stream);
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_tc_heads");
   return HX_OK;

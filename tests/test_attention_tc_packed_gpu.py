@@ -106,6 +106,7 @@ def test_wide_heads_against_the_formula(head_dim, heads, kv_heads, page, lengths
 @pytest.mark.parametrize("tokens,heads,in_dim,out_dim,x_stride,out_stride", [
     (33, 3, 64, 40, 72, 40), (129, 2, 192, 128, 256, 128), (300, 5, 128, 300, 128, 304),
     (1100, 40, 64, 256, 64, 256),      # more tiles than SMs
+    (257, 1, 64, 500, 72, 512),        # one head: pairs of CTAs, tiles in pieces
 ])
 def test_products_per_head_on_the_tensor_cores(tokens, heads, in_dim, out_dim, x_stride, out_stride):
     from helix_runtime_b200.ops import library as ops
