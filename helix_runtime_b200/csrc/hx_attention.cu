@@ -811,7 +811,7 @@ void paged_attention_stream_kernel(
     }
     unreadable = (unreadable & ~(0xfu << (4 * slot))) | (bits << (4 * slot));
     any_unreadable = any_unreadable || faulty;
-    if (lane == 0) {
+    if (hx_elect_one()) {
       asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
                        hx_shared_address(bar)), "r"(expected) : "memory");
 #pragma unroll

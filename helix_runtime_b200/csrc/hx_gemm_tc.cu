@@ -209,7 +209,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   if (n_k_blocks > 0) {
     if (warp == 0) {
       // ------------------------------------------------------------ TMA producer
-      if (elect_one()) {
+      if (hx_elect_one()) {
         // The weight tiles do not depend on the kernel before this one: the first STAGES of
         // them are requested at once, before the dependency wait, so that weights stream
         // across the kernel boundary.  The token tiles follow after the wait.
@@ -247,7 +247,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       }
     } else if (warp == 1) {
       // -------------------------------------------------------------- MMA issuer
-      if (elect_one()) {
+      if (hx_elect_one()) {
         constexpr uint32_t idesc = make_idesc(BM, BN);
         bool ok = true;
         for (int i = 0; i < n_k_blocks && ok; ++i) {
@@ -735,7 +735,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
 
   if (warp == 0) {
     // -------------------------------------------------------------- TMA producer
-    if (elect_one()) {
+    if (hx_elect_one()) {
       uint32_t fill = 0;      // stages filled so far, over all units
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
@@ -772,7 +772,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (elect_one()) {
+    if (hx_elect_one()) {
       constexpr uint32_t idesc = make_idesc(BM, Config::kRowsB);
       uint32_t drained = 0;      // stages consumed so far, over all units
       Unit unit;
@@ -961,7 +961,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
 
   if (warp == 0) {
     // -------------------------------------------------------------- TMA producer
-    if (elect_one()) {
+    if (hx_elect_one()) {
       uint32_t fill = 0;      // stages filled so far, over all units
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
@@ -1006,7 +1006,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
     }
   } else if (warp == 1) {
     // ---------------------------------------------------------------- MMA issuer
-    if (rank == 0 && elect_one()) {
+    if (rank == 0 && hx_elect_one()) {
       uint32_t drained = 0;
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {

@@ -17,20 +17,6 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
   return static_cast<uint32_t>(__cvta_generic_to_shared(p));
 }
 
-// One lane of a converged warp.  Where a branch is taken by elect.sync the compiler knows that a
-// single thread runs it: the operands of tcgen05.mma and TMA instructions, which the hardware
-// takes from uniform registers, then need no loop over the threads that might be there
-// (a prompt of 2,048 tokens in four layers of the Llama-2-7B sizes: 3,741 -> 3,637 us).
-__device__ __forceinline__ bool elect_one() {
-  uint32_t elected;
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "elect.sync _|p, 0xffffffff;\n\t"
-      "selp.u32 %0, 1, 0, p;\n\t}"
-      : "=r"(elected));
-  return elected != 0;
-}
-
 __device__ __forceinline__ void mbar_init(uint64_t* bar, uint32_t count) {
   asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(smem_u32(bar)), "r"(count));
 }
