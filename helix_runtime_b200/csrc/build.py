@@ -38,6 +38,7 @@ SOURCES = (
     "hx_latent.cu",
     "hx_gemm_simt.cu",
     "hx_gemm_tc.cu",
+    "hx_gemm_tc_runs.cu",
     "hx_attention.cu",
     "hx_attention_mma.cu",
     "hx_attention_tc.cu",

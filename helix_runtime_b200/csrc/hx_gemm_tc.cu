@@ -966,13 +966,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       Unit unit;
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
         const int rows = BM / unit.pieces;      // this CTA's half of the tile's (or piece's) rows
-        int feature0 = unit.feature_tile * FEATURES + unit.piece * (FEATURES / unit.pieces);
-        int kb_end = unit.kb_end;
-        if (args.tile_group != nullptr) {
-          const int group = args.tile_group[unit.token_tile];
-          if (group < 0) kb_end = unit.kb_begin;
-          else feature0 += group * args.group_rows;
-        }
+        const int feature0 = unit.feature_tile * FEATURES + unit.piece * (FEATURES / unit.pieces);
         const int weight_row = rank == 0 ? feature0
                                : EPI == EPI_SWIGLU ? args.up_row_offset + feature0 : feature0 + rows;
         const CUtensorMap* map = unit.pieces > 1 ? &map_w_piece : &map_w;
@@ -980,7 +974,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
         // tiled weights: a piece lies inside one stored tile
         const int tile_row = args.k_tiles > 0 ? (weight_row / BM) * args.k_tiles * BM + weight_row % BM : 0;
         const int token0 = unit.token_tile * 2 * BM + rank * BM;
-        for (int kb = unit.kb_begin; kb < kb_end; ++kb, ++fill) {
+        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++fill) {
           const int s = fill % STAGES;
           if (!mbar_wait(&empty_bar[s], ((fill / STAGES) & 1u) ^ 1u)) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
@@ -1021,8 +1015,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
         tc_fence_after();
         const uint32_t accumulator = tmem_base + buffer * kBufferColumns;
         const uint32_t idesc = make_idesc(2 * BM, 2 * BM / unit.pieces);
-        const bool skipped = args.tile_group != nullptr && args.tile_group[unit.token_tile] < 0;
-        for (int kb = unit.kb_begin; kb < (skipped ? unit.kb_begin : unit.kb_end); ++kb, ++drained) {
+        for (int kb = unit.kb_begin; kb < unit.kb_end; ++kb, ++drained) {
           const int s = drained % STAGES;
           if (!mbar_wait_cluster(&full_bar[s], (drained / STAGES) & 1u)) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
@@ -1091,7 +1084,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       } else if (EPI == EPI_ADD_F32 && unit.partial) {
         add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
                            args.tokens, feature0);
-      } else if (args.tile_group == nullptr || args.tile_group[unit.token_tile] >= 0) {
+      } else {
         write_row<EPI>(columns, args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
                        args.activation, args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
       }
@@ -1275,29 +1268,6 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   const int ctas = args.whole_rounds == 0 ? args.tail_ctas : args.units < sms ? args.units : sms;
   hx_launch(gemm_tc_persistent_kernel<EPI>, ctas, THREADS, PersistentConfig::kSmemBytes, stream, map_w,
             map_x, args);
-  return HX_OK;
-}
-
-// The grouped product with tiles of 256 tokens: a pair's two CTAs read the same group's weights (1,024
-// tokens with 4 of 16 experts of [5,632 x 4,096] and [4,096 x 2,816]: 547 -> 511 us for the layer).
-template <int EPI>
-int launch_grouped_pairs(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
-                         cudaStream_t stream) {
-  static bool configured = false;
-  const int sms = hx_device_sm_count();
-  if (sms <= 0) return HX_ERR_LAUNCH;
-  if (!configured) {
-    if (!reserve_shared(gemm_tc_pair_kernel<EPI>, PairConfig::kSmemBytes)) return HX_ERR_LAUNCH;
-    configured = true;
-  }
-  constexpr int kFeatures = EPI == EPI_SWIGLU ? BM : 2 * BM;
-  args.token_tiles = (args.tokens + 2 * BM - 1) / (2 * BM);
-  const long long units = static_cast<long long>(args.token_tiles) * ((args.features + kFeatures - 1) / kFeatures);
-  HX_REQUIRE(units < (1ll << 30), "hx_gemm_tc_grouped: too many tiles");
-  args.units = static_cast<int>(units);
-  const int pairs = sms / 2 < args.units ? sms / 2 : args.units;
-  hx_launch(gemm_tc_pair_kernel<EPI>, 2 * pairs, THREADS, PairConfig::kSmemBytes, stream, map_w, map_w, map_x,
-            args);
   return HX_OK;
 }
 
@@ -1486,26 +1456,14 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
                                     : features <= group_rows,
              "hx_gemm_tc_grouped: features exceed a group's rows");
   HX_REQUIRE(ldo >= features, "hx_gemm_tc_grouped: output stride too small");
-  HX_REQUIRE(token_tile == 16 || token_tile == 32 || token_tile == 64 || token_tile == 128 ||
-                 token_tile == 256,
+  HX_REQUIRE(token_tile == 16 || token_tile == 32 || token_tile == 64 || token_tile == 128,
              "hx_gemm_tc_grouped: token tile %d", token_tile);
   CUtensorMap map_w, map_x;
   int rc = get_tensor_map(w, static_cast<uint64_t>(groups) * group_rows, depth, ldw, BM, &map_w);
   if (rc != HX_OK) return rc;
-  rc = get_tensor_map(x, x_capacity_rows, depth, ldx, token_tile > BM ? BM : token_tile, &map_x);
+  rc = get_tensor_map(x, x_capacity_rows, depth, ldx, token_tile, &map_x);
   if (rc != HX_OK) return rc;
   const int total_k_blocks = (depth + BK - 1) / BK;
-  if (token_tile == 2 * BM) {
-    PersistentArgs pairs{out, ldo, tokens, features, depth, up_row_offset, 0, 0, 0,
-                         total_k_blocks, status, RopeArgs{}, -1, activation, tile_group,
-                         group_rows, gate_limit};
-    rc = epilogue == EPI_STORE_BF16  ? launch_grouped_pairs<EPI_STORE_BF16>(map_w, map_x, pairs, stream)
-         : epilogue == EPI_STORE_F32 ? launch_grouped_pairs<EPI_STORE_F32>(map_w, map_x, pairs, stream)
-                                     : launch_grouped_pairs<EPI_SWIGLU>(map_w, map_x, pairs, stream);
-    if (rc != HX_OK) return rc;
-    HX_CHECK_LAUNCH("hx_gemm_tc_grouped");
-    return HX_OK;
-  }
   if (token_tile == BM) {
     // tiles of 128 tokens: the persistent kernel, as for prompt portions of a plain product
     PersistentArgs persistent{out, ldo, tokens, features, depth, up_row_offset, 0, 0, 0,

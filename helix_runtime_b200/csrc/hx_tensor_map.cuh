@@ -37,9 +37,11 @@ struct MapKey {
   uint32_t box_rows;
   uint32_t box_columns;
   bool swizzled;
+  uint64_t up_rows;      // > 0: boxes of interleaved rows
   bool operator==(const MapKey& o) const {
     return base == o.base && rows == o.rows && depth == o.depth && ld == o.ld &&
-           box_rows == o.box_rows && box_columns == o.box_columns && swizzled == o.swizzled;
+           box_rows == o.box_rows && box_columns == o.box_columns && swizzled == o.swizzled &&
+           up_rows == o.up_rows;
   }
 };
 struct MapKeyHash {
@@ -50,19 +52,16 @@ struct MapKeyHash {
     h = h * 1315423911u ^ k.ld;
     h = h * 1315423911u ^ k.box_rows;
     h = h * 1315423911u ^ (2 * k.box_columns + (k.swizzled ? 1 : 0));
+    h = h * 1315423911u ^ k.up_rows;
     return h;
   }
 };
 
-// The map of a [rows, depth] matrix of bfloat16 with row stride ld, for boxes of box_rows rows by
-// box_columns columns, laid out in shared memory with the 128-byte swizzle or row behind row.  Maps
-// are pure functions of (address, shape, box); encoding one costs a few microseconds, so they are
+// Maps are pure functions of (address, shape, box); encoding one costs a few microseconds, so they are
 // cached for the life of the process.
-int hx_tensor_map(const char* caller, const void* base, uint64_t rows, uint64_t depth, uint64_t ld,
-                  uint32_t box_rows, uint32_t box_columns, bool swizzled, CUtensorMap* out) {
+int cached_tensor_map(const char* caller, const MapKey& key, CUtensorMap* out) {
   static std::mutex mutex;
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
-  const MapKey key{base, rows, depth, ld, box_rows, box_columns, swizzled};
   std::lock_guard<std::mutex> lock(mutex);
   auto found = cache.find(key);
   if (found != cache.end()) {
@@ -74,26 +73,49 @@ int hx_tensor_map(const char* caller, const void* base, uint64_t rows, uint64_t 
     hx_set_error("%s: the driver does not export cuTensorMapEncodeTiled", caller);
     return HX_ERR_UNSUPPORTED;
   }
-  const cuuint64_t dims[2] = {depth, rows};
-  const cuuint64_t strides[1] = {ld * 2};
-  const cuuint32_t box[2] = {box_columns, box_rows};
-  const cuuint32_t element_strides[2] = {1, 1};
+  const bool interleaved = key.up_rows > 0;
+  const cuuint64_t plain_dims[2] = {key.depth, key.rows};
+  const cuuint64_t plain_strides[1] = {key.ld * 2};
+  const cuuint32_t plain_box[2] = {key.box_columns, key.box_rows};
+  const cuuint64_t turns_dims[4] = {key.depth, 16, 2, (key.rows - key.up_rows) / 16};
+  const cuuint64_t turns_strides[3] = {key.ld * 2, key.up_rows * key.ld * 2, 16 * key.ld * 2};
+  const cuuint32_t turns_box[4] = {key.box_columns, 16, 2, key.box_rows / 32};
+  const cuuint32_t element_strides[4] = {1, 1, 1, 1};
   CUtensorMap map;
-  const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(base),
-                             dims, strides, box, element_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
-                             swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
+  const CUresult rc = encode(&map, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, interleaved ? 4 : 2,
+                             const_cast<void*>(key.base), interleaved ? turns_dims : plain_dims,
+                             interleaved ? turns_strides : plain_strides,
+                             interleaved ? turns_box : plain_box, element_strides,
+                             CU_TENSOR_MAP_INTERLEAVE_NONE,
+                             key.swizzled ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_NONE,
                              CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (rc != CUDA_SUCCESS) {
     hx_set_error("%s: cuTensorMapEncodeTiled failed with %d (base %p rows %llu depth %llu ld %llu box "
-                 "%u x %u)", caller, static_cast<int>(rc), base,
-                 static_cast<unsigned long long>(rows), static_cast<unsigned long long>(depth),
-                 static_cast<unsigned long long>(ld), box_rows, box_columns);
+                 "%u x %u)", caller, static_cast<int>(rc), key.base,
+                 static_cast<unsigned long long>(key.rows), static_cast<unsigned long long>(key.depth),
+                 static_cast<unsigned long long>(key.ld), key.box_rows, key.box_columns);
     return HX_ERR_ARGUMENT;
   }
   if (cache.size() > 4096) cache.clear();
   cache.emplace(key, map);
   *out = map;
   return HX_OK;
+}
+
+// The map of a [rows, depth] matrix of bfloat16 with row stride ld, for boxes of box_rows rows by
+// box_columns columns, laid out in shared memory with the 128-byte swizzle or row behind row.
+int hx_tensor_map(const char* caller, const void* base, uint64_t rows, uint64_t depth, uint64_t ld,
+                  uint32_t box_rows, uint32_t box_columns, bool swizzled, CUtensorMap* out) {
+  return cached_tensor_map(caller, MapKey{base, rows, depth, ld, box_rows, box_columns, swizzled, 0}, out);
+}
+
+// The map of the same matrix, whole rows, for boxes of box_rows rows (swizzled) that hold 16 rows, the 16
+// that lie up_rows behind them, the next 16, and so on.  Coordinates: column, 0, 0, first row / 16; up_rows
+// and rows are multiples of 16, so that nothing behind the matrix is read.
+[[maybe_unused]] int hx_tensor_map_interleaved(const char* caller, const void* base, uint64_t rows,
+                                               uint64_t depth, uint64_t up_rows, uint32_t box_rows,
+                                               uint32_t box_columns, CUtensorMap* out) {
+  return cached_tensor_map(caller, MapKey{base, rows, depth, depth, box_rows, box_columns, true, up_rows}, out);
 }
 
 }  // namespace

@@ -315,6 +315,11 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_float, _c_ptr, _c_ptr,
         _c_ptr, _c_int, _c_int, _c_float, _c_float, _c_ptr, _c_float, _c_ptr, _c_longlong, _c_ptr,
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
+    library.hx_gemm_tc_runs_supports.argtypes = [_c_int] * 6
+    library.hx_gemm_tc_runs.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int,
+                                        _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_ptr, _c_ptr,
+                                        _c_ptr]
+    library.hx_gemm_tc_runs_supports.restype = library.hx_gemm_tc_runs.restype = _c_int
     library.hx_gemm_tc_heads_supports.argtypes = [_c_int, _c_int, _c_int]
     library.hx_gemm_tc_heads_supports.restype = _c_int
     library.hx_gemm_tc_heads.argtypes = [_c_ptr, _c_int, _c_int, _c_int, _c_ptr, _c_ptr, _c_int,
@@ -1699,7 +1704,7 @@ def expert_down(act: torch.Tensor, down: torch.Tensor, chosen: torch.Tensor,
                                 dtype_code(act.dtype), tokens, top, ff, width, experts, _stream()))
 
 
-GROUPED_TILES = (16, 32, 64, 128, 256)
+GROUPED_TILES = (16, 32, 64, 128)
 
 
 def expert_tile(pairs: int, experts: int) -> int:
@@ -1773,6 +1778,38 @@ def gemm_tc_grouped(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: i
                                     group_rows, groups, out.data_ptr(), out.stride(0), rows,
                                     features, depth, epilogue, up_row_offset, token_tile,
                                     tile_group.data_ptr(), status.data_ptr(), _stream()))
+
+
+# Rows that an expert's rows are padded to for gemm_tc_runs, and the average share of the pairs from
+# which its experts take that road.  Measured, tiles of 64 against runs (both products): 16 experts of
+# 2,816 in 4,096 at shares of 48 and 64: 231 / 239 and 254 / 237 us; 64 experts of 1,408 in 2,048: 243 /
+# 242 and 279 / 237; at 32 tiles of 32: 232 / 231.
+RUN_STEP = 32
+RUNS_FROM_SHARE = 56
+
+
+def gemm_tc_runs_supports(rows: int, w: torch.Tensor, up_row_offset: int) -> bool:
+    groups, group_rows, depth = w.shape
+    return bool(lib().hx_gemm_tc_runs_supports(rows, groups, group_rows, up_row_offset, depth, depth))
+
+
+def gemm_tc_runs(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, rows: int, features: int,
+                 tile_group: torch.Tensor, status: torch.Tensor, up_row_offset: int = 0,
+                 gate_activation: int = 0, gate_limit: float = 0.0) -> None:
+    """:func:`gemm_tc_grouped` for many tokens, tiles of 32 rows in the list: the rows of equal
+    entries that follow one another are multiplied in as few equal tiles as hold them.
+    ``up_row_offset`` > 0: ``out`` is bfloat16, the gated activation; 0: float32 sums."""
+    _need(x, torch.bfloat16, "x")
+    _need(w, torch.bfloat16, "w")
+    _need(out, torch.bfloat16 if up_row_offset else torch.float32, "out")
+    _need(tile_group, torch.int32, "tile_group")
+    assert w.is_contiguous() and x.stride(-1) == 1 and out.stride(-1) == 1
+    assert tile_group.numel() * RUN_STEP >= rows and out.shape[0] >= rows
+    groups, group_rows, depth = w.shape
+    _check(lib().hx_gemm_tc_runs(x.data_ptr(), x.stride(0), x.shape[0], w.data_ptr(), group_rows, groups,
+                                 out.data_ptr(), out.stride(0), rows, features, depth,
+                                 int(gate_activation), float(gate_limit), up_row_offset,
+                                 tile_group.data_ptr(), status.data_ptr(), _stream()))
 
 
 # ---------------------------------------------------------- attention over a cached latent

@@ -302,6 +302,13 @@ class RoutedExperts(FeedForward):
         pairs = n * self.top
         tile = ops.expert_tile(pairs, self.experts)
         tiles = ops.expert_tile_bound(pairs, self.experts, tile)
+        runs = False
+        if pairs >= ops.RUNS_FROM_SHARE * self.experts:
+            steps = ops.expert_tile_bound(pairs, self.experts, ops.RUN_STEP)
+            runs = (ops.gemm_tc_runs_supports(steps * ops.RUN_STEP, self.w_gate_up, self.intermediate)
+                    and ops.gemm_tc_runs_supports(steps * ops.RUN_STEP, self.w_down, 0))
+            if runs:
+                tile, tiles = ops.RUN_STEP, steps
         # buffers are made once for the largest step: the widest tile pads the most rows
         most = max(ops.expert_tile_bound(ctx.capacity * self.top, self.experts, t) * t
                    for t in ops.GROUPED_TILES)
@@ -315,6 +322,13 @@ class RoutedExperts(FeedForward):
                        torch.float32)
         ops.expert_rows(chosen, pair_row, tile_group, pairs, self.experts, tile, tiles)
         ops.expert_gather(x, pair_row, rows_in, n, self.top)
+        if runs:
+            ops.gemm_tc_runs(rows_in, self.w_gate_up, rows_act, tiles * tile, self.intermediate,
+                             tile_group, ctx.status, self.intermediate, self.activation, self.limit)
+            ops.gemm_tc_runs(rows_act, self.w_down, rows_out, tiles * tile, self.hidden_size,
+                             tile_group, ctx.status)
+            ops.expert_combine(rows_out, pair_row, weights, residual, n, self.top, self.hidden_size)
+            return
         ops.gemm_tc_grouped(rows_in, self.w_gate_up, rows_act, tiles * tile, self.intermediate,
                             ops.EPI_SWIGLU, self.intermediate, tile, tile_group, ctx.status,
                             gate_activation=self.activation, gate_limit=self.limit)

@@ -530,13 +530,20 @@ int hx_gemm_tc_gated(const void* x, int ldx, int x_capacity_rows, const void* w,
                      int weight_rows, void* out, int ldo, int tokens, int features, int depth,
                      int activation, float gate_limit, const float* gate_bias, const float* up_bias,
                      int up_row_offset, int weight_tiles, int* status, cudaStream_t stream);
-/* grouped product: rows of x come in tiles of token_tile (16..256), tile t multiplies with
+/* grouped product: rows of x come in tiles of token_tile (16..128), tile t multiplies with
  * group tile_group[t] of w (`groups` matrices of group_rows rows one below the other); a
  * negative entry skips the tile; tile_group is device memory, written on the stream before */
 int hx_gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,
                        int group_rows, int groups, void* out, int ldo, int tokens, int features,
                        int depth, int epilogue, int up_row_offset, int token_tile,
                        const int* tile_group, int* status, cudaStream_t stream);
+/* the same for many tokens: a group's rows are padded to a multiple of 32 and tile_group has an entry for
+ * every 32 rows; up_row_offset > 0: bfloat16 gated activation, 0: float32 sums */
+int hx_gemm_tc_runs_supports(int rows, int groups, int group_rows, int up_row_offset, int depth, int ldx);
+int hx_gemm_tc_runs(const void* x, int ldx, int x_capacity_rows, const void* w, int group_rows,
+                    int groups, void* out, int ldo, int rows, int features, int depth,
+                    int activation, float gate_limit, int up_row_offset, const int* tile_group,
+                    int* status, cudaStream_t stream);
 /* the grouped product with the gated epilogue for every gate activation (see
  * hx_biased_gated_activation); gate_limit: the clamped form's limit */
 int hx_gemm_tc_grouped_gated(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,

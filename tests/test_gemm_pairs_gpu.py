@@ -56,36 +56,3 @@ def test_every_epilogue(tokens, features, depth, tiled):
             <= (2.0 ** -8 + 2.0 ** -18) * act.abs() + 2 * slack + 1e-6).all()
     assert (out[tokens:] == 7.0).all()
     assert int(status.item()) == 0
-
-
-@pytest.mark.parametrize("tile_groups,rows,features,depth", [
-    ([2, 0, 0, 1, -1], 300, 150, 200),       # a group of two tiles, one without tokens at the end
-    ([0], 256, 128, 64),
-    ([3, 1, 1, 0, 2, 2, 2, -1, -1, -1, -1], 2100, 1000, 72),      # more tiles than pairs
-])
-def test_groups_of_whole_tiles(tile_groups, rows, features, depth):
-    from helix_runtime_b200.ops import library as ops
-    torch.manual_seed(rows)
-    tokens, groups = 256 * len(tile_groups), 4
-    x = (torch.randn(tokens, depth) * 0.5).bfloat16().cuda()
-    w = (torch.randn(groups, 2 * rows, depth) * 0.1).bfloat16().cuda()
-    status = torch.zeros(1, dtype=torch.int32, device="cuda")
-    listed = torch.tensor(tile_groups, dtype=torch.int32).cuda()
-    out = torch.full((tokens, features), 7.0, device="cuda")
-    act = torch.full((tokens, features), 7.0, dtype=torch.bfloat16, device="cuda")
-    ops.gemm_tc_grouped(x, w, out, tokens, features, ops.EPI_STORE_F32, 0, 256, listed, status)
-    ops.gemm_tc_grouped(x, w, act, tokens, features, ops.EPI_SWIGLU, rows, 256, listed, status)
-    assert int(status.item()) == 0
-    for tile, group in enumerate(tile_groups):
-        part = slice(256 * tile, 256 * tile + 256)
-        if group < 0:
-            assert (out[part] == 7.0).all() and (act[part] == 7.0).all()
-            continue
-        gate = x[part].double() @ w[group, :features].double().T
-        up = x[part].double() @ w[group, rows:rows + features].double().T
-        size = x[part].double().abs() @ w[group].double().abs().max(0)[0][:, None]
-        bound = (depth + 2) * 2.0 ** -24 * size
-        assert ((out[part] - gate).abs() <= bound).all()
-        want = torch.nn.functional.silu(gate) * up
-        assert ((act[part].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -18) * want.abs()
-                + 2 * bound * (1.1 * up.abs() + gate.abs() + 1e-3) + 1e-6).all()
