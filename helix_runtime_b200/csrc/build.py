@@ -37,6 +37,7 @@ SOURCES = (
     "hx_routed_experts.cu",
     "hx_latent.cu",
     "hx_gemm_simt.cu",
+    "hx_gemm_split.cu",
     "hx_gemm_tc.cu",
     "hx_gemm_tc_runs.cu",
     "hx_attention.cu",

@@ -1,7 +1,8 @@
 // Matrix product on the CUDA cores: out[t, o] (+)= sum_k x[t, k] * w[o, k].
 //
 // This is the true 32-bit path (float32 storage, float32 fused multiply-adds, no
-// reduced-precision matrix mode) and also the bfloat16 path for shapes the tensor
+// reduced-precision matrix mode; many tokens take hx_gemm_split.cu, whose sums are closer
+// still) and also the bfloat16 path for shapes the tensor
 // core kernel refuses.  Each output element is one sequential sum over k in
 // ascending order, so its value never depends on how many rows the call has or on
 // which tile it falls into.  The reference's counterpart is its 16x16 tiled kernel

@@ -315,6 +315,12 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_ptr, _c_float, _c_ptr, _c_ptr,
         _c_ptr, _c_int, _c_int, _c_float, _c_float, _c_ptr, _c_float, _c_ptr, _c_longlong, _c_ptr,
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
+    library.hx_gemm_split_supports.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int]
+    library.hx_gemm_split_pays.argtypes = [_c_int, _c_int]
+    library.hx_gemm_split.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int,
+                                      _c_int, _c_int, _c_float, _c_ptr, _c_ptr]
+    for name in ("hx_gemm_split_supports", "hx_gemm_split_pays", "hx_gemm_split"):
+        getattr(library, name).restype = _c_int
     library.hx_gemm_tc_runs_supports.argtypes = [_c_int] * 6
     library.hx_gemm_tc_runs.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int,
                                         _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_ptr, _c_ptr,
@@ -621,6 +627,28 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, 
     _check(lib().hx_gemm_simt_softcapped(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
                                          out.data_ptr(), out.stride(0), dtype_code(x.dtype), tokens,
                                          features, depth, epilogue, float(softcap), _stream()))
+
+
+def gemm_split_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int) -> bool:
+    """Whether a float32 product runs, and is faster, as :func:`gemm_split`."""
+    return (x.dtype == w.dtype == out.dtype == torch.float32
+            and bool(lib().hx_gemm_split_pays(tokens, w.shape[0]))
+            and bool(lib().hx_gemm_split_supports(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
+                                                  w.shape[0], w.shape[1])))
+
+
+def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, epilogue: int,
+               status: torch.Tensor, softcap: float = 0.0) -> None:
+    """:func:`gemm_simt` for many float32 tokens, on the tensor cores: both operands as three
+    bfloat16 terms, 24 bits, sums of 64 products added in float32.  Closer to the sum of 64 bits than
+    the chain of multiply-adds; like that one, the same from call to call."""
+    for tensor, name in ((x, "x"), (w, "w"), (out, "out")):
+        _need(tensor, torch.float32, name)
+    assert x.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1
+    features, depth = w.shape
+    _check(lib().hx_gemm_split(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
+                               out.stride(0), tokens, features, depth, epilogue, float(softcap),
+                               status.data_ptr(), _stream()))
 
 
 WEIGHT_TILE_ROWS, WEIGHT_TILE_DEPTH = 128, 64

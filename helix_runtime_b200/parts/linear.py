@@ -75,13 +75,16 @@ def _gemm_tc(x, w: Weight, out, tokens, features, epilogue, status, **options) -
         ops.gemm_tc(x, w.matrix, out, tokens, features, epilogue, status, **options)
 
 
-def _gemm_simt(x, w: Weight, out, tokens, epilogue, softcap: float = 0.0,
+def _gemm_simt(x, w: Weight, out, tokens, epilogue, status, softcap: float = 0.0,
                features: Optional[int] = None) -> None:
     if w.matrix is None:
         raise RuntimeError("this product needs the CUDA-core kernel, but the weight is held as "
                            "tiles for the tensor cores")
-    ops.gemm_simt(x, w.matrix if features is None else w.matrix[:features], out, tokens, epilogue,
-                  softcap)
+    matrix = w.matrix if features is None else w.matrix[:features]
+    if ops.gemm_split_takes(x, matrix, out, tokens):
+        ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap)
+    else:
+        ops.gemm_simt(x, matrix, out, tokens, epilogue, softcap)
 
 
 def is_weight_stream(x: torch.Tensor, w: Weight, tokens: int) -> bool:
@@ -123,7 +126,7 @@ def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue
         _gemm_tc(x, w, out, tokens, features or w.rows, epilogue, status, k_splits=splits,
                  softcap=softcap)
     else:
-        _gemm_simt(x, w, out, tokens, epilogue, softcap, features)
+        _gemm_simt(x, w, out, tokens, epilogue, status, softcap, features)
 
 
 def project_into_accumulator(x: torch.Tensor, w: Weight, accumulator: torch.Tensor,
@@ -158,7 +161,7 @@ def project_swiglu(x: torch.Tensor, w_gate_up: Weight, intermediate: int, act: t
     else:
         scratch = workspace.get(f"mlp.gate_up/{intermediate}", (capacity, 2 * intermediate),
                                 torch.float32)
-        _gemm_simt(x, w_gate_up, scratch, tokens, ops.EPI_STORE_F32)
+        _gemm_simt(x, w_gate_up, scratch, tokens, ops.EPI_STORE_F32, status)
         ops.swiglu(scratch[:tokens], act[:tokens], activation=activation)
 
 

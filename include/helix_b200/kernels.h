@@ -493,6 +493,13 @@ int hx_gemm_tc_softcapped(const void* x, int ldx, int x_capacity_rows, const voi
                           int weight_rows, float* out, int ldo, int tokens, int features,
                           int depth, float softcap, int weight_tiles, int* status,
                           cudaStream_t stream);
+/* the float32 product on the tensor cores: operands as three bfloat16 terms (24 bits), sums of 64 k added
+ * in float32 registers; rows of a multiple of four that begin on 16 bytes */
+int hx_gemm_split_supports(const void* x, int ldx, const void* w, int ldw, int features, int depth);
+int hx_gemm_split_pays(int tokens, int features);
+int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
+                  int features, int depth, int epilogue, float softcap, int* status,
+                  cudaStream_t stream);
 /* tcgen05 tensor cores, bfloat16 operands, float32 accumulate in tensor memory.
  * weight_tiles != 0: w holds the matrix as [ceil(rows / 128)][ceil(depth / 64)] tiles of
  * [128][64] elements, zero padded, each tile 16 contiguous kilobytes (ldw is ignored). */

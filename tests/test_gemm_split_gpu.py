@@ -1,0 +1,88 @@
+"""The float32 product on the tensor cores, at the edges of its tiles, with operands of all sizes and with
+ones that are not finite, against double and against the CUDA-core product."""
+from __future__ import annotations
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("tokens,features,depth,pad", [
+    (1, 3, 4, 0), (128, 128, 64, 0), (129, 130, 68, 4), (17, 257, 60, 0), (300, 63, 1000, 8),
+    (200, 2500, 132, 0),      # columns of an output row that is no multiple of 16 bytes below
+])
+def test_every_epilogue(tokens, features, depth, pad):
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(tokens + features)
+    x = torch.randn(tokens + 2, depth + pad, device="cuda")[:, :depth]
+    w = torch.randn(features, depth + pad, device="cuda")[:, :depth]
+    x[1::3] *= 1e30
+    x[2::3] *= 1e-30
+    x[tokens:] = float("nan")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    want = x[:tokens].double() @ w.double().T
+    size = x[:tokens].double().abs() @ w.double().abs().T
+    # left out: x1 w2, x2 w1, x2 w2, below 2^-24 of a product together; the 24 sums of a block do not
+    # round to nearest (2^-23 each at most), those of the blocks do
+    bound = (2.0 ** -24 + 25 * 2.0 ** -23 + (depth // 64 + 1) * 2.0 ** -24) * size
+    for width in (features, features + 1):
+        out = torch.full((tokens + 2, width), 7.0, device="cuda")
+        ops.gemm_split(x, w, out, tokens, ops.EPI_STORE_F32, status)
+        assert ((out[:tokens, :features] - want).abs() <= bound).all()
+        assert (out[tokens:] == 7.0).all() and (out[:, features:] == 7.0).all()
+        again = torch.zeros((tokens, width), device="cuda")
+        ops.gemm_split(x, w, again, tokens, ops.EPI_STORE, status)
+        assert torch.equal(again[:, :features], out[:tokens, :features])
+        added = torch.full((tokens + 2, width), 0.5, device="cuda")
+        ops.gemm_split(x, w, added, tokens, ops.EPI_ADD_F32, status)
+        assert torch.equal(added[:tokens, :features], out[:tokens, :features] + 0.5)
+        assert (added[tokens:] == 0.5).all() and (added[:, features:] == 0.5).all()
+    ops.gemm_split(x, w, out, tokens, ops.EPI_STORE_F32, status, softcap=3.0)
+    assert ((out[:tokens, :features] - 3.0 * torch.tanh(want / 3.0)).abs() <= bound.clamp(max=6.0) + 1e-6).all()
+    assert int(status.item()) == 0
+
+
+def test_closer_to_64_bits_than_the_chain():
+    from helix_runtime_b200.ops import library as ops
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for seed, depth in enumerate((256, 3200, 8640)):
+        torch.manual_seed(seed)
+        for signs in (torch.randn, torch.rand):
+            x, w = signs(130, depth, device="cuda"), signs(200, depth, device="cuda") * 0.02
+            out, chain = torch.zeros(130, 200, device="cuda"), torch.zeros(130, 200, device="cuda")
+            ops.gemm_split(x, w, out, 130, ops.EPI_STORE_F32, status)
+            ops.gemm_simt(x, w, chain, 130, ops.EPI_STORE_F32)
+            want = x.double() @ w.double().T
+            assert (out - want).norm() <= (chain - want).norm()
+
+
+def test_what_is_not_finite_is_what_the_chain_says():
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(0)
+    x, w = torch.randn(140, 200, device="cuda"), torch.randn(150, 200, device="cuda")
+    inf, nan, huge = float("inf"), float("nan"), 3.4e38
+    x[3, 7], x[130, 1], x[20, 150], x[21, 0], x[21, 1], x[50] = inf, -inf, nan, inf, -inf, huge
+    w[9, 7], w[149, 199], w[30], w[77, 70] = 0.0, inf, 1e-39, -huge
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, chain = torch.zeros(140, 150, device="cuda"), torch.zeros(140, 150, device="cuda")
+    ops.gemm_split(x, w, out, 140, ops.EPI_STORE_F32, status)
+    ops.gemm_simt(x, w, chain, 140, ops.EPI_STORE_F32)
+    assert int(status.item()) == 0
+    assert torch.equal(out.isnan(), chain.isnan())
+    odd = ~chain.isfinite() & ~chain.isnan()
+    assert odd.any() and torch.equal(out[odd], chain[odd])
+    plain = chain.isfinite()
+    size = x.double().abs().nan_to_num(0, 0, 0) @ w.double().abs().nan_to_num(0, 0, 0).T
+    assert ((out - chain).abs()[plain] <= (201 * 2.0 ** -24 + 26 * 2.0 ** -23) * size[plain] + 1e-38).all()
+
+
+def test_which_products_take_it():
+    from helix_runtime_b200.ops import library as ops
+    x, out = torch.zeros(64, 132, device="cuda"), torch.zeros(64, 20000, device="cuda")
+    w = torch.zeros(20000, 132, device="cuda")
+    assert ops.gemm_split_takes(x, w, out, 64) and not ops.gemm_split_takes(x, w, out, 16)
+    assert not ops.gemm_split_takes(x, w[:64], out, 64)
+    assert not ops.gemm_split_takes(x[:, 1:129], w[:, 1:129], out, 64)
+    assert not ops.gemm_split_takes(x[:, :130], w[:, :130], out, 64)
+    assert not ops.gemm_split_takes(x.bfloat16(), w.bfloat16(), out, 64)
