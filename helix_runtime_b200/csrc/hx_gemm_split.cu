@@ -12,10 +12,12 @@
 // A sum that is not finite (an operand is not, or is so large that its first term is infinite) is taken
 // again as that chain, which says what it is.
 //
-// What bounds it: shared memory.  A block of 64 k of a tile of 128 x 128 writes 96 KB of terms and the 24
-// products read 192 KB of them, about 2,300 cycles where the products alone take 1,600 and the conversion
-// (8 warps, 16 loads of 16 bytes a thread, the next operand's on their way meanwhile) 1,300.
-// Measured (us, tiles of multiply-adds before): 512 tokens by [17,280 x 3,200] 1,581 -> 464, by [3,200 x 8,640] 947 ->
+// What bounds it: the conversion.  A block of 64 k of a tile of 128 x 128 takes about 4,000 cycles; with one
+// of the six products it takes as long, without the loads 3,300 (ncu: issue slots 54 % busy, tensor pipe 38 %):
+// eight warps that load, cut and store 16 pieces of four numbers each a block, two warps a scheduler.
+// Slower: sixteen such warps (too few registers for loads in flight: 463 -> 502 us), all warps converting
+// and summing in turn (539), the weights' lines asked for ahead (4 % faster alone, 3 % slower in place).
+// Measured (us, tiles of multiply-adds before): 512 tokens by [17,280 x 3,200] 1,581 -> 463, by [3,200 x 8,640] 947 ->
 // 317, by [4,096 x 4,096] 522 -> 157; 33 by the first 248 -> 117.
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets a status bit, the CTA skips its

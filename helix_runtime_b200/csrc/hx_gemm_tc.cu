@@ -1194,10 +1194,6 @@ bool reserve_shared(Kernel kernel, int bytes) {
   return false;
 }
 
-#ifndef HX_GEMM_PAIRS
-#define HX_GEMM_PAIRS 1      // 0: every tile is one CTA's
-#endif
-
 // What the tensor map of the weights is made from; tiled ones (k_tiles > 0) are rows of 64 elements,
 // tile behind tile.
 struct WeightBoxes {
@@ -1210,9 +1206,7 @@ WeightBoxes weight_boxes(const void* w, int weight_rows, int depth, int ldw, int
   return {w, static_cast<uint64_t>(weight_rows), static_cast<uint64_t>(depth), static_cast<uint64_t>(ldw)};
 }
 
-#ifndef HX_GEMM_PIECES
-#define HX_GEMM_PIECES 4     // at most, of a tile of the last round
-#endif
+constexpr int MOST_PIECES = 4;      // of a tile of the last round
 
 template <int EPI>
 int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
@@ -1242,8 +1236,8 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   // against 17.0 us).
   const int pair_tiles = (args.tokens + 2 * BM - 1) / (2 * BM), pairs = sms / 2;
   const long long pair_units = static_cast<long long>(pair_tiles) * feature_tiles;
-  if (HX_GEMM_PAIRS && args.heads == 1 && args.tile_group == nullptr && args.tokens > BM && pairs > 0) {
-    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, HX_GEMM_PIECES,
+  if (args.heads == 1 && args.tile_group == nullptr && args.tokens > BM && pairs > 0) {
+    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, MOST_PIECES,
                                       whole_rounds, tail, pieces);
     const double penalty = EPI == EPI_ADD_F32 && whole_rounds == 0 && args.k_blocks < 96 ? 4.0 : 0.0;
     if (0.95 * paired + penalty <= alone) {
@@ -1425,7 +1419,7 @@ HX_API int hx_gemm_tc_gated(const void* x, int ldx, int x_capacity_rows, const v
                  weight_tiles, status, stream);
 }
 
-// The grouped product: rows of x come in tiles of `token_tile` (16, 32, 64, 128 or 256), and
+// The grouped product: rows of x come in tiles of `token_tile` (16, 32, 64 or 128), and
 // tile t multiplies with group tile_group[t] of w, which holds `groups` matrices of
 // `group_rows` rows one below the other (row-major, row stride ldw); a negative entry skips the
 // tile.  tile_group (device memory, ceil(tokens / token_tile) entries) may be written by the
