@@ -17,8 +17,9 @@
 // eight warps that load, cut and store 16 pieces of four numbers each a block, two warps a scheduler.
 // Slower: sixteen such warps (too few registers for loads in flight: 463 -> 502 us), all warps converting
 // and summing in turn (539), the weights' lines asked for ahead (4 % faster alone, 3 % slower in place).
-// Measured (us, tiles of multiply-adds before): 512 tokens by [17,280 x 3,200] 1,581 -> 463, by [3,200 x 8,640] 947 ->
-// 317, by [4,096 x 4,096] 522 -> 157; 33 by the first 248 -> 117.
+// Measured (us, tiles of multiply-adds before): 512 tokens by [17,280 x 3,200] 1,581 -> 434, by [3,200 x 8,640] 947 ->
+// 287, by [4,096 x 4,096] 522 -> 157; 33 by the first 248 -> 117.  (With the next block's tokens asked for in front
+// of the proxy fence, which waits for loads too: 459 and 311.)
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets a status bit, the CTA skips its
 // remaining work, frees its tensor memory and returns.
@@ -191,11 +192,12 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
       }
       uint8_t* stage = smem + s * STAGE_BYTES;
       store(stage, xv);
-      if (kb + 1 < blocks) load(xv, x, a.ldx, x_rows, kb + 1);
       store(stage + 3 * TERM_BYTES, wv);
       asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&full_bar[s]);
+      // (not in front of the fence, which waits for loads too)
+      if (kb + 1 < blocks) load(xv, x, a.ldx, x_rows, kb + 1);
     }
   } else {
     // ------------------------------------- products, sums of the blocks, and the epilogue
