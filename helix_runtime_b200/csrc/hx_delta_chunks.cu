@@ -24,6 +24,10 @@
 // float32 sums.  The products of the small terms are summed before those of the large ones,
 // which are then the only ones whose rounding counts.
 //
+// The weights of tokens that come later are zeros, and zero times a number that is not finite is
+// none: such a number, wherever it comes in, shows in the chunk's outputs.  A warp that finds one
+// there takes the chunk again token by token, from the state that it still holds.
+//
 // The scan walks a token in 0.6 us whatever the chip could do beside it (a chain of two dot
 // products over the state); a chunk is a chain of about 800 products a warp, which is what bounds
 // it now.  Measured (one B200, 32 heads of 128 by 128): a portion of 1,000 tokens 1,030 -> 198 us,
@@ -31,6 +35,8 @@
 // (state) where the scan has 2.3e-7 and 2.2e-7, and the layer's outputs are 0.0031 off either way.
 #include "hx_mma.cuh"
 #include "hx_scan.cuh"
+
+#include <cfloat>
 
 namespace {
 
@@ -391,6 +397,77 @@ __device__ __forceinline__ void triangular_product(float (&sums)[8][4], const fl
   }
 }
 
+// The chunk's tokens one after the other, as the recurrence is written, for chunks with numbers that
+// are not finite.  S, queries, keys, values: as delta_states_kernel holds them; `first`: the chunk's
+// first token, `column`: the first of the lane's two columns (8 apart).  (Not inlined: its caller
+// has no register to spare.)
+template <int TILES>
+__device__ __noinline__ void tokens_in_turn(const DeltaArgs& a, float (*S)[4], const __nv_bfloat16* queries,
+                                            const __nv_bfloat16* keys, int stride,
+                                            const __nv_bfloat16* values, int value_stride, int first,
+                                            int live, int head, int column) {
+  const int pair = 2 * (threadIdx.x & 3);
+  const float rate = a.decay_in != nullptr ? expf(a.a_log[head]) : 0.0f;
+  // over the four lanes that share the columns
+  auto summed = [](float x) {
+    x += __shfl_xor_sync(0xffffffffu, x, 1);
+    return x + __shfl_xor_sync(0xffffffffu, x, 2);
+  };
+#pragma unroll 1
+  for (int t = 0; t < live; ++t) {
+    const size_t gate = static_cast<size_t>(first + t) * a.ld_gates + head;
+    const float decay = a.decay_in != nullptr
+                            ? expf(-rate * softplus(__bfloat162float(a.decay_in[gate]) + a.dt_bias[head]))
+                            : 1.0f + a.fixed_decay_m1[head];
+    const float beta = hx_sigmoid(__bfloat162float(a.beta_in[gate]));
+    const __nv_bfloat16* q = queries + t * stride + pair;
+    const __nv_bfloat16* k = keys + t * stride + pair;
+    float fq = a.q_scale, fk = a.k_scale;
+    if (a.unit_norm) {
+      float sq = 0.0f, sk = 0.0f;
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) {
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q + 8 * n));
+        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(k + 8 * n));
+        sq = fmaf(x.x, x.x, fmaf(x.y, x.y, sq));
+        sk = fmaf(y.x, y.x, fmaf(y.y, y.y, sk));
+      }
+      fq /= sqrtf(summed(sq) + a.unit_eps);
+      fk /= sqrtf(summed(sk) + a.unit_eps);
+    }
+    float u[2], o[2] = {0.0f, 0.0f};
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      float held = 0.0f;
+#pragma unroll
+      for (int n = 0; n < TILES; ++n) {
+        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(k + 8 * n));
+        held = fmaf(S[n][2 * c], fk * y.x, fmaf(S[n][2 * c + 1], fk * y.y, held));
+      }
+      u[c] = beta * (__bfloat162float(values[t * value_stride + 8 * c]) - decay * summed(held));
+    }
+#pragma unroll
+    for (int n = 0; n < TILES; ++n) {
+      if (8 * n < a.dim) {      // (the dimension is a multiple of 8; what lies behind it stays zero)
+        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(q + 8 * n));
+        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(k + 8 * n));
+#pragma unroll
+        for (int c = 0; c < 2; ++c) {
+          S[n][2 * c] = fmaf(decay, S[n][2 * c], fk * y.x * u[c]);
+          S[n][2 * c + 1] = fmaf(decay, S[n][2 * c + 1], fk * y.y * u[c]);
+          o[c] = fmaf(S[n][2 * c], fq * x.x, fmaf(S[n][2 * c + 1], fq * x.y, o[c]));
+        }
+      }
+    }
+#pragma unroll
+    for (int c = 0; c < 2; ++c) {
+      const float sum = summed(o[c]);
+      if (pair == 0 && column + 8 * c < a.vdim)
+        a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + column + 8 * c] = sum;
+    }
+  }
+}
+
 // grid (requests, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
 template <int STEPS>
 __global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a) {
@@ -545,27 +622,46 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a)
     float u[8][4];
     triangular_product(u, rest, weights + weight_lane);
     triangular_product(rest, u, weights + weight_lane + 2 * TERMS * CHUNK);
-    {
-      const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
+    const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
+    bool finite = true;
 #pragma unroll
-      for (int n = 0; n < 8; ++n)
+    for (int n = 0; n < 8; ++n)
 #pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const int t = 8 * n + pair + (j & 1), c = my_column + 8 * (j >> 1);
-          if (t < live && c < a.vdim)
-            a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j] + rest[n][j];
-        }
+      for (int j = 0; j < 4; ++j) {
+        out[n][j] += rest[n][j];
+        u[n][j] *= factors[8 * n + pair + (j & 1)].w;
+        finite = finite && fabsf(out[n][j]) <= FLT_MAX && fabsf(u[n][j]) <= FLT_MAX;
+      }
+    if (__any_sync(0xffffffffu, !finite)) {
+      const __nv_bfloat16* staged = queries_of(stage);
+      float held[2 * STEPS][4];
+#pragma unroll
+      for (int n = 0; n < 2 * STEPS; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) held[n][j] = S[n][j];
+      tokens_in_turn<2 * STEPS>(a, held, staged, staged + CHUNK * STRIDE, STRIDE,
+                                staged + CHUNK * (2 * STRIDE + WEIGHT_STRIDE) + 16 * warp + row, value_stride,
+                                first, live, head, my_column);
+#pragma unroll
+      for (int n = 0; n < 2 * STEPS; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[n][j] = held[n][j];
+      continue;
     }
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int t = 8 * n + pair + (j & 1), c = my_column + 8 * (j >> 1);
+        if (t < live && c < a.vdim)
+          a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j];
+      }
     // the state behind the chunk
     const float total = factors[CHUNK].x;
 #pragma unroll
     for (int n = 0; n < 2 * STEPS; ++n)
 #pragma unroll
       for (int j = 0; j < 4; ++j) S[n][j] *= total;
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) u[n][j] *= factors[8 * n + pair + (j & 1)].w;
 #pragma unroll
     for (int step = 0; step < CHUNK / 16; ++step) {
       uint32_t u0[4], u1[4], u2[4];

@@ -104,6 +104,87 @@ def test_chunks_against_the_recurrence(heads, qk_heads, dim, vdim, lengths, unit
     assert (got_state[untouched] == 7.0).all()
 
 
+def chunks_and_recurrence(q, k, v, gates, before, starts, qk_heads, a_log=None, dt_bias=None,
+                          fixed=None):
+    """What the chunks and what the recurrence in double make of one step of the delta rule on unit
+    vectors: outputs ``[T, H, V]`` and states ``[R, H, D, V]`` of both.  ``fixed``: constant decays."""
+    from helix_runtime_b200.ops import library as ops
+    requests, heads, dim, vdim = before.shape
+    tokens = q.shape[0]
+    per_head = ops.scan_state_floats(vdim, dim)
+    state = torch.tensor(np.stack([packed_state(row, per_head).reshape(-1) for row in before]),
+                         dtype=torch.float32).cuda()
+    o = torch.full((tokens, heads * vdim), 7.0, device="cuda")
+    scratch = torch.full((ops.delta_chunks_scratch(heads, tokens) // 4 + 1,), float("nan"),
+                         device="cuda")
+    decays = dict(decay_in=gates[:, heads:], a_log=torch.tensor(a_log).cuda(),
+                  dt_bias=torch.tensor(dt_bias).cuda()) if fixed is None else \
+        dict(fixed_decay_m1=torch.tensor(fixed - 1.0, dtype=torch.float32).cuda())
+    ops.delta_chunks(q, k, v, state, o, scratch, torch.tensor(starts, dtype=torch.int32).cuda(),
+                     torch.arange(requests, dtype=torch.int32).cuda(), requests, tokens,
+                     ops.recurrence_tiles(np.diff(starts).tolist()), heads, qk_heads, dim, vdim,
+                     beta_in=gates[:, :heads], unit_norm=True, unit_eps=1e-6, **decays)
+    qd, kd, vd, gd = (t.double().cpu().numpy() for t in (q, k, v, gates))
+    with np.errstate(all="ignore"):
+        qd, kd = (np.repeat(x / np.sqrt((x * x).sum(-1, keepdims=True) + 1e-6), heads // qk_heads, 1)
+                  for x in (qd.reshape(tokens, qk_heads, dim), kd.reshape(tokens, qk_heads, dim)))
+        beta = 1.0 / (1.0 + np.exp(-gd[:, :heads]))
+        decay = np.broadcast_to(fixed, (tokens, heads)) if fixed is not None else \
+            np.exp(-np.exp(a_log.astype(np.float64)) * np.logaddexp(0.0, gd[:, heads:] + dt_bias))
+        want, after = np.zeros((tokens, heads, vdim)), before.astype(np.float64)
+        for r in range(requests):
+            for t in range(starts[r], starts[r + 1]):
+                held = after[r] * decay[t][:, None, None]
+                u = beta[t][:, None] * (vd.reshape(tokens, heads, vdim)[t] -
+                                        (held * kd[t][:, :, None]).sum(1))
+                after[r] = held + kd[t][:, :, None] * u[:, None]
+                want[t] = (after[r] * qd[t][:, :, None]).sum(1)
+    got_state = state.cpu().numpy().reshape(requests, heads, 16, vdim, -1).transpose(0, 1, 4, 2, 3)
+    return o.cpu().numpy().reshape(want.shape), want, \
+        got_state.reshape(requests, heads, -1, vdim)[:, :, :dim], after
+
+
+def alike(got, want):
+    """Not finite in the same places and alike there; elsewhere as near as the rest of this file asks."""
+    assert np.array_equal(np.isnan(got), np.isnan(want))
+    odd, plain_ones = np.isinf(want), np.isfinite(want)
+    assert np.array_equal(got[odd], want[odd])
+    error = np.linalg.norm(got[plain_ones] - want[plain_ones])
+    assert error <= 8 * 128 ** 0.5 * 2.0 ** -24 * np.linalg.norm(want[plain_ones])
+
+
+def inputs(rng, heads, qk_heads, dim, vdim, lengths):
+    tokens = sum(lengths)
+    q, k = (rounded(rng.normal(size=(tokens, qk_heads * dim))) for _ in range(2))
+    v = rounded(rng.normal(size=(tokens, heads * vdim)))
+    gates = rounded(rng.normal(size=(tokens, 2 * heads)))
+    before = rng.normal(size=(len(lengths), heads, dim, vdim)).astype(np.float32)
+    return q, k, v, gates, before, np.concatenate([[0], np.cumsum(lengths)])
+
+
+@pytest.mark.parametrize("at", [37, 69])
+@pytest.mark.parametrize("where", ["v inf", "v nan", "k nan", "q inf", "beta nan", "decay nan", "state inf"])
+def test_what_is_not_finite_stays_behind_its_token(where, at):
+    """Tokens in front of one that is not finite are what they are without it, in its chunk too; from
+    it on the recurrence says what is what."""
+    rng = np.random.default_rng(at)
+    heads, qk_heads, dim, vdim = 4, 2, 48, 40
+    q, k, v, gates, before, starts = inputs(rng, heads, qk_heads, dim, vdim, (70, 5))
+    name, number = where.split()
+    if name == "state":
+        before[0, 1, 5, 7] = float(number)
+    else:
+        rows, column = {"v": (v, vdim + 3), "k": (k, 11), "q": (q, dim + 2), "beta": (gates, 1),
+                        "decay": (gates, heads + 2)}[name]
+        rows[at, column] = float(number)
+    got, want, got_state, after = chunks_and_recurrence(
+        q, k, v, gates, before, starts, qk_heads, np.linspace(-1.0, 0.5, heads).astype(np.float32),
+        np.full(heads, -2.0, dtype=np.float32))
+    assert not np.isfinite(want).all()
+    alike(got, want)
+    alike(got_state, after)
+
+
 def test_refusals():
     from helix_runtime_b200.ops import library as ops
     assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
