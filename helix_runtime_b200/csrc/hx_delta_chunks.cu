@@ -10,7 +10,10 @@
 //     o_t  = e^(L_t) S_0' q_t + sum_(s <= t) P_ts u_s,   P_ts = (q_t . k_s) e^(L_t - L_s)
 //     S_64 = e^(L_64) S_0 + sum_s e^(L_64 - L_s) k_s u_s'
 //
-// Every exponent is a difference of decays between two tokens of the chunk, never positive.
+// Every exponent is a difference of decays between two tokens of the chunk, never positive (decays
+// of at most one).  A decay so small that float32 has only zero for it counts as e^-256, zero too,
+// whose logarithm can be summed; a negative one has no logarithm and takes the road of numbers that
+// are not finite (below).
 //
 //   * delta_weights_kernel, all chunks at once: T = (1 + A)^-1 by forward substitution in float32,
 //     P, and the factors of a token.
@@ -45,6 +48,7 @@ constexpr int ROW_PAD = 8;             // elements behind a staged row: rows sta
 constexpr int TERMS = 3;
 constexpr int WEIGHT_COLUMNS = 2 * TERMS * CHUNK;      // a token's row of T, then of P, three terms each
 constexpr int WEIGHT_STRIDE = WEIGHT_COLUMNS + ROW_PAD;
+constexpr float NO_DECAY_LEFT = -256.0f;      // e^this is zero in float32 (from -104 on)
 
 struct DeltaArgs {
   const __nv_bfloat16* q;    // [tokens, ld_q], already offset; qk_heads * dim columns
@@ -178,6 +182,7 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
         d[i] = a.decay_in != nullptr
                    ? -expf(a.a_log[head]) * softplus(__bfloat162float(a.decay_in[gate]) + a.dt_bias[head])
                    : log1pf(a.fixed_decay_m1[head]);
+        if (d[i] < NO_DECAY_LEFT) d[i] = NO_DECAY_LEFT;      // (a NaN stays one)
         beta = hx_sigmoid(__bfloat162float(a.beta_in[gate]));
       }
       write[t] = beta;

@@ -367,12 +367,19 @@ class LinearState(Mixer):
     # requests they win earlier (16 portions of 32: 149 us against 258).
     CHUNKS_FROM_TOKENS = 32
 
+    @staticmethod
+    def decays_suit_chunks(decays: Optional[List[float]]) -> bool:
+        """Learned decays (None) lie between zero and one.  A chunk of a negative one is taken token
+        by token, and powers of one above one leave float32's range inside a chunk."""
+        return decays is None or all(0.0 <= decay <= 1.0 for decay in decays)
+
     def runs_in_chunks(self, ctx: StepContext, qkv: torch.Tensor) -> bool:
         """Whether the recurrence takes this step 64 tokens at a time on the tensor cores: the
         delta rule in bfloat16 without a rotation (turned queries and keys are float32 numbers
         that no stored row holds), for a step with a prompt portion in it."""
         return (self.rule == "delta" and not self.rotary_dims and ctx.dtype == torch.bfloat16
                 and ctx.max_query_len >= self.CHUNKS_FROM_TOKENS and qkv.stride(0) % 8 == 0
+                and self.decays_suit_chunks(self.fixed_decay)
                 and ops.delta_chunks_supports(self.head_dim, self.value_dim))
 
     def weight_bytes(self) -> int:

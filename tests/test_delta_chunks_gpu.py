@@ -185,6 +185,33 @@ def test_what_is_not_finite_stays_behind_its_token(where, at):
     alike(got_state, after)
 
 
+@pytest.mark.parametrize("learned", [False, True])
+def test_decays_that_leave_nothing_and_negative_ones(learned):
+    """Constant decays of zero and below are only factors to the recurrence; a learned one leaves
+    nothing where its rate or its input is large."""
+    rng = np.random.default_rng(5)
+    heads, qk_heads, dim, vdim = 4, 2, 40, 24
+    q, k, v, gates, before, starts = inputs(rng, heads, qk_heads, dim, vdim, (70, 5))
+    if learned:
+        gates[20, heads] = float("inf")
+        gates[30:33, heads + 1] = 3e30
+        decays = dict(a_log=np.array([0.0, 1.0, 60.0, 90.0], dtype=np.float32),
+                      dt_bias=np.full(heads, -2.0, dtype=np.float32))
+    else:
+        decays = dict(fixed=np.array([0.0, -0.5, -1.0, 0.9]))
+    got, want, got_state, after = chunks_and_recurrence(q, k, v, gates, before, starts, qk_heads, **decays)
+    assert np.isfinite(want).all()
+    alike(got, want)
+    alike(got_state, after)
+
+
+def test_constant_decays_outside_zero_to_one_take_the_scan():
+    from helix_runtime_b200.parts.recurrent import LinearState
+    assert LinearState.decays_suit_chunks(None) and LinearState.decays_suit_chunks([1.0, 0.5, 0.0])
+    for other in (-0.25, 1.0 + 2.0 ** -23, float("nan")):
+        assert not LinearState.decays_suit_chunks([0.5, other])
+
+
 def test_refusals():
     from helix_runtime_b200.ops import library as ops
     assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
