@@ -1,7 +1,9 @@
 // float32 products of many tokens on the tensor cores: out[t, o] (+)= sum_k x[t, k] * w[o, k].
 //
-// Every operand goes in as three bfloat16 terms, x = x0 + x1 + x2, each the nearest to what the ones
-// before it leave: 24 bits, all that a float32 holds.  Of the nine products the three below 2^-25 of the
+// Every operand goes in as three bfloat16 terms, 2^16 x = x0 + x1 + x2, each the nearest to what the ones
+// before it leave: 24 bits, all that a float32 holds.  (Times 2^16 because bfloat16 ends at 2^-133: the last
+// bit of every float32, 2^-149 at least, is then one of a term.  Blocks of sums are divided by 2^32 as they
+// are added.)  Of the nine products the three below 2^-25 of the
 // whole (x1 w2, x2 w1, x2 w2) are left out.  The tensor cores add in float32 but do not round to nearest,
 // so a sum stays in tensor memory for one block of 64 k only, the products of the small terms first, and
 // the blocks are added in registers.  The sums are closer to those of 64 bits than a chain of float32
@@ -9,8 +11,8 @@
 // 256 8.8e-8 and 2.9e-7, 3,200 1.5e-7 and 1.0e-6, 8,640 2.2e-7 and 1.7e-6; positive operands alike.  (Where a few
 // products are the whole sum, operands e^(4 n): 1.8e-8 and 1.7e-8, 1.3e-7 and 1.1e-7 at the last two.)
 //
-// A sum that is not finite (an operand is not, or is so large that its first term is infinite) is taken
-// again as that chain, which says what it is.
+// A sum that is not finite (an operand is not, or 2^16 times it leaves float32, or 2^32 times a block's
+// sum does: operands from 2^112 and sums from 2^96 on) is taken again as that chain, which says what it is.
 //
 // What bounds it: the conversion.  A block of 64 k of a tile of 128 x 128 takes about 4,000 cycles; with one
 // of the six products it takes as long, without the loads 3,300 (ncu: issue slots 54 % busy, tensor pipe 38 %):
@@ -44,7 +46,13 @@ constexpr int COPY_THREADS = 32 * COPY_WARPS;
 constexpr int PASS_ROWS = COPY_THREADS / (BK / 4);      // rows that the copying threads take at a time
 constexpr int PASSES = TILE / PASS_ROWS;
 constexpr int COLUMNS = TILE / 2;   // of a summing thread
+// A thread's registers: 128 at launch, of which the summing warps need fewer and the others, with 64
+// loaded numbers on their way, more.
+constexpr int SUM_REGISTERS = 104, COPY_REGISTERS = 152;
+static_assert(SUM_WARPS * SUM_REGISTERS + COPY_WARPS * COPY_REGISTERS <= 128 * (SUM_WARPS + COPY_WARPS),
+              "what one side takes the other has given back");
 constexpr int TMEM_COLUMNS = 2 * TILE;
+constexpr float OPERAND_SCALE = 65536.0f, SUM_SCALE = 1.0f / (OPERAND_SCALE * OPERAND_SCALE);
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
 
 struct SplitArgs {
@@ -71,6 +79,12 @@ __device__ __forceinline__ void leave(uint32_t terms, float& a, float& b) {
 
 // The terms of four numbers, 8 bytes each, to `at` in the three matrices of terms.
 __device__ __forceinline__ void store_terms(uint8_t* at, float4 v) {
+  asm("{\n\t.reg .b64 s, p, q;\n\t"
+      "mov.b64 s, {%4, %4};\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\t"
+      "mul.rn.f32x2 p, p, s;\n\tmul.rn.f32x2 q, q, s;\n\t"
+      "mov.b64 {%0, %1}, p;\n\tmov.b64 {%2, %3}, q;\n\t}"
+      : "+f"(v.x), "+f"(v.y), "+f"(v.z), "+f"(v.w)
+      : "f"(OPERAND_SCALE));
 #pragma unroll
   for (int term = 0; term < 3; ++term) {
     const uint2 packed = make_uint2(two_terms(v.x, v.y), two_terms(v.z, v.w));
@@ -156,6 +170,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
 
   if (warp >= SUM_WARPS) {
     // ------------------------------------------- operands: loaded, cut into terms, stored swizzled
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(COPY_REGISTERS));
     const int thread = threadIdx.x - 32 * SUM_WARPS;
     const int piece = thread % (BK / 4), row0 = thread / (BK / 4);      // four k of rows row0 + PASS_ROWS p
     const float* x = a.x + static_cast<size_t>(token0) * a.ldx + 4 * piece;
@@ -201,6 +216,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
     }
   } else {
     // ------------------------------------- products, sums of the blocks, and the epilogue
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(SUM_REGISTERS));
     const int quarter = warp & 3, half = warp >> 2;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * COLUMNS;
     float sum[COLUMNS];
@@ -230,7 +246,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
         float v[16];
         tmem_load16(lane_base + buffer * TILE + column, v);
 #pragma unroll
-        for (int j = 0; j < 16; ++j) sum[column + j] += v[j];
+        for (int j = 0; j < 16; ++j) sum[column + j] = fmaf(v[j], SUM_SCALE, sum[column + j]);
       }
       tc_fence_before();
       __syncwarp();

@@ -74,7 +74,27 @@ def test_what_is_not_finite_is_what_the_chain_says():
     assert odd.any() and torch.equal(out[odd], chain[odd])
     plain = chain.isfinite()
     size = x.double().abs().nan_to_num(0, 0, 0) @ w.double().abs().nan_to_num(0, 0, 0).T
-    assert ((out - chain).abs()[plain] <= (201 * 2.0 ** -24 + 26 * 2.0 ** -23) * size[plain] + 1e-38).all()
+    assert ((out - chain).abs()[plain] <= (201 * 2.0 ** -24 + 26 * 2.0 ** -23) * size[plain]).all()
+
+
+@pytest.mark.parametrize("small", [1e-34, 1e-36, 1e-38, 1e-39, 3e-44])
+def test_small_operands_keep_their_bits(small):
+    """The smallest numbers of float32, those without a full mantissa too, beside ones that make ordinary
+    sums of them: what float32 holds of an operand all reaches the sum."""
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(1)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for swapped in (False, True):
+        x, w = torch.randn(140, 68, device="cuda") * small, torch.randn(130, 68, device="cuda") * 1e25
+        if swapped:
+            x, w = w, x
+        tokens, features = x.shape[0], w.shape[0]
+        out = torch.zeros(tokens, features, device="cuda")
+        ops.gemm_split(x, w, out, tokens, ops.EPI_STORE_F32, status)
+        want, size = x.double() @ w.double().T, x.double().abs() @ w.double().abs().T
+        # the bound of the other operands (see test_every_epilogue)
+        assert ((out - want).abs() <= (2.0 ** -24 + 25 * 2.0 ** -23 + 2.0 ** -23) * size).all()
+    assert int(status.item()) == 0
 
 
 def test_which_products_take_it():
