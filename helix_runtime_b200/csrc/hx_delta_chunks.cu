@@ -33,9 +33,10 @@
 //
 // The scan walks a token in 0.6 us whatever the chip could do beside it (a chain of two dot
 // products over the state); a chunk is a chain of about 800 products a warp, which is what bounds
-// it now.  Measured (one B200, 32 heads of 128 by 128): a portion of 1,000 tokens 1,030 -> 198 us,
-// eight of 256 1,092 -> 225, one of 64 73 -> 42; errors against 64 bits 2.7e-7 (outputs) and 2.6e-7
-// (state) where the scan has 2.3e-7 and 2.2e-7, and the layer's outputs are 0.0031 off either way.
+// it now.  Measured (one B200, 32 heads of 128 by 128, against the scan): a portion of 1,000 tokens
+// 979 -> 215 us, eight of 256 1,065 -> 215, one of 64 71 -> 44; errors against 64 bits, 1,024 tokens, 2.0e-7
+// (outputs) and 1.3e-7 (state) where the scan has 2.3e-7 and 2.2e-7 (2.6e-7 and 2.5e-7 with a chunk's
+// products added onto the state itself).
 #include "hx_mma.cuh"
 #include "hx_scan.cuh"
 
@@ -661,27 +662,46 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a)
         if (t < live && c < a.vdim)
           a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j];
       }
-    // the state behind the chunk
+    // The state behind the chunk.  What the chunk adds is summed by itself and meets the state in one
+    // multiply-add: the tensor cores cut off what a sum of theirs cannot hold, and onto the state itself
+    // they would do so a dozen times a chunk.
     const float total = factors[CHUNK].x;
+    uint32_t u0[CHUNK / 16][4], u1[CHUNK / 16][4], u2[CHUNK / 16][4];
 #pragma unroll
-    for (int n = 0; n < 2 * STEPS; ++n)
+    for (int step = 0; step < CHUNK / 16; ++step) operand_terms(u, step, u0[step], u1[step], u2[step]);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) S[n][j] *= total;
+    for (int n0 = 0; n0 < STEPS; n0 += 2) {
+      float added[4][4];
 #pragma unroll
-    for (int step = 0; step < CHUNK / 16; ++step) {
-      uint32_t u0[4], u1[4], u2[4];
-      operand_terms(u, step, u0, u1, u2);
+      for (int n = 0; n < 4; ++n)
 #pragma unroll
-      for (int n = 0; n < STEPS; ++n) {
-        uint32_t b[4];
-        hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * n));
-        hx_mma_bf16(S[2 * n], u2, b[0], b[1]);
-        hx_mma_bf16(S[2 * n + 1], u2, b[2], b[3]);
-        hx_mma_bf16(S[2 * n], u1, b[0], b[1]);
-        hx_mma_bf16(S[2 * n + 1], u1, b[2], b[3]);
-        hx_mma_bf16(S[2 * n], u0, b[0], b[1]);
-        hx_mma_bf16(S[2 * n + 1], u0, b[2], b[3]);
+        for (int j = 0; j < 4; ++j) added[n][j] = 0.0f;
+#pragma unroll
+      for (int step = 0; step < CHUNK / 16; ++step) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          uint32_t b[4];
+          hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * (n0 + n)));
+          hx_mma_bf16(added[2 * n], u2[step], b[0], b[1]);
+          hx_mma_bf16(added[2 * n + 1], u2[step], b[2], b[3]);
+          hx_mma_bf16(added[2 * n], u1[step], b[0], b[1]);
+          hx_mma_bf16(added[2 * n + 1], u1[step], b[2], b[3]);
+        }
       }
+#pragma unroll
+      for (int step = 0; step < CHUNK / 16; ++step) {
+#pragma unroll
+        for (int n = 0; n < 2; ++n) {
+          uint32_t b[4];
+          hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * (n0 + n)));
+          hx_mma_bf16(added[2 * n], u0[step], b[0], b[1]);
+          hx_mma_bf16(added[2 * n + 1], u0[step], b[2], b[3]);
+        }
+      }
+#pragma unroll
+      for (int n = 0; n < 4; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) S[2 * n0 + n][j] = fmaf(total, S[2 * n0 + n][j], added[n][j]);
     }
   }
 #pragma unroll

@@ -212,6 +212,28 @@ def test_constant_decays_outside_zero_to_one_take_the_scan():
         assert not LinearState.decays_suit_chunks([0.5, other])
 
 
+def test_no_further_from_64_bits_than_the_scan():
+    from helix_runtime_b200.ops import library as ops
+    rng = np.random.default_rng(2)
+    heads, qk_heads, dim, vdim, lengths = 4, 2, 128, 128, (512, 130)
+    q, k, v, gates, before, starts = inputs(rng, heads, qk_heads, dim, vdim, lengths)
+    a_log = np.linspace(-2.77, 0.0, heads).astype(np.float32)
+    dt_bias = np.full(heads, -2.25, dtype=np.float32)
+    got, want, got_state, after = chunks_and_recurrence(q, k, v, gates, before, starts, qk_heads, a_log, dt_bias)
+    per_head = ops.scan_state_floats(vdim, dim)
+    state = torch.tensor(np.stack([packed_state(row, per_head).reshape(-1) for row in before]),
+                         dtype=torch.float32).cuda()
+    o = torch.empty((sum(lengths), heads * vdim), device="cuda")
+    ops.linear_state_scan(q, k, v, state, o, torch.tensor(starts, dtype=torch.int32).cuda(),
+                          torch.arange(2, dtype=torch.int32).cuda(), 2, heads, qk_heads, dim, vdim, delta=True,
+                          decay_in=gates[:, heads:], beta_in=gates[:, :heads], a_log=torch.tensor(a_log).cuda(),
+                          dt_bias=torch.tensor(dt_bias).cuda(), unit_norm=True, unit_eps=1e-6)
+    scanned = state.cpu().numpy().reshape(2, heads, 16, vdim, -1).transpose(0, 1, 4, 2, 3).reshape(after.shape)
+    scan_error = np.linalg.norm(o.cpu().numpy().reshape(want.shape) - want)
+    assert np.linalg.norm(got - want) <= scan_error
+    assert np.linalg.norm(got_state - after) <= np.linalg.norm(scanned - after)
+
+
 def test_refusals():
     from helix_runtime_b200.ops import library as ops
     assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
