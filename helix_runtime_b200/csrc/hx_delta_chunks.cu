@@ -75,6 +75,8 @@ struct DeltaArgs {
   const int* request_start;
   const int* request_slot;
   int requests, heads, qk_heads, dim, vdim, parts, column_warps;
+  int min_query_len;         // requests with fewer tokens are left alone;
+  int portions;              // so many have as many
 };
 
 // two neighbouring values in three bfloat16 terms, a word each
@@ -151,7 +153,7 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
   __shared__ float level_hi[CHUNK], level_lo[CHUNK], q_length[CHUNK], k_length[CHUNK], write[CHUNK];
   hx_pdl_prologue();
   int chunk, chunks;
-  const int request = hx_find_query_tile(a.request_start, a.requests, 1, CHUNK, blockIdx.x, chunk, chunks);
+  const int request = hx_find_query_tile(a.request_start, a.requests, a.min_query_len, CHUNK, blockIdx.x, chunk, chunks);
   if (request < 0) return;
   const int head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
   const int first = a.request_start[request] + chunk * CHUNK;
@@ -474,16 +476,22 @@ __device__ __noinline__ void tokens_in_turn(const DeltaArgs& a, float (*S)[4], c
   }
 }
 
-// grid (requests, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
+// grid (portions, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
 template <int STEPS>
 __global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a) {
   constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
   extern __shared__ uint4 shared_pieces[];
   hx_pdl_prologue();
-  const int request = blockIdx.x, head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
+  const int head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
+  int request = blockIdx.x;
+  if (a.portions < a.requests) {
+    int only, of_one;      // a portion is one tile of as many tokens as there can be
+    request = hx_find_query_tile(a.request_start, a.requests, a.min_query_len, 1 << 30, blockIdx.x, only, of_one);
+    if (request < 0) return;
+  }
   const int start = a.request_start[request];
   const int count = a.request_start[request + 1] - start;
-  if (count <= 0) return;
+  if (count < a.min_query_len) return;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int row = lane >> 2, pair = 2 * (lane & 3);
   const int matrix = lane >> 3, in_matrix = lane & 7;
@@ -727,7 +735,7 @@ int launch_delta(const DeltaArgs& a, int tiles, cudaStream_t stream) {
   }
   hx_launch(delta_weights_kernel<STEPS>, dim3(tiles, a.heads), 128, first, stream, a);
   const int block_columns = 16 * a.column_warps;
-  hx_launch(delta_states_kernel<STEPS>, dim3(a.requests, a.heads, (a.vdim + block_columns - 1) / block_columns),
+  hx_launch(delta_states_kernel<STEPS>, dim3(a.portions, a.heads, (a.vdim + block_columns - 1) / block_columns),
             32 * a.column_warps, shared, stream, a);
   return HX_OK;
 }
@@ -749,17 +757,20 @@ HX_API long long hx_delta_chunks_scratch(int heads, int tokens) {
 // as for hx_linear_state_scan with its delta rule and without a rotation.  scratch:
 // hx_delta_chunks_scratch bytes on 16 bytes.  tiles: at least the chunks of 64 tokens in the step,
 // counted request by request.
-HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
-                           const void* decay_in, const void* beta_in, int ld_gates,
-                           const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
-                           int unit_norm, float unit_eps, float q_scale, float k_scale,
-                           void* scratch, float* state, long long state_stride, int head_stride,
-                           float* o, const int* request_start, const int* request_slot,
-                           int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
-                           int vdim, cudaStream_t stream) {
+// Requests that bring fewer than min_query_len tokens are left alone (hx_linear_state_scan_below takes
+// them); portions: how many bring as many, tiles: the chunks of those.
+HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                                const void* decay_in, const void* beta_in, int ld_gates,
+                                const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
+                                int unit_norm, float unit_eps, float q_scale, float k_scale,
+                                void* scratch, float* state, long long state_stride, int head_stride,
+                                float* o, const int* request_start, const int* request_slot,
+                                int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
+                                int vdim, int min_query_len, int portions, cudaStream_t stream) {
   HX_REQUIRE(hx_delta_chunks_supports(dim, vdim), "hx_delta_chunks: heads of %d by %d are not supported",
              dim, vdim);
-  HX_REQUIRE(requests >= 0 && tokens >= requests && tiles >= requests && heads > 0 && heads <= 65535 &&
+  HX_REQUIRE(requests >= 0 && tokens >= requests && min_query_len > 0 && portions >= 0 &&
+                 portions <= requests && tiles >= portions && heads > 0 && heads <= 65535 &&
                  qk_heads > 0 && heads % qk_heads == 0,
              "hx_delta_chunks: bad sizes");
   HX_REQUIRE(ld_q % 8 == 0 && ld_k % 8 == 0 && ld_v % 8 == 0 && ld_q >= qk_heads * dim &&
@@ -773,12 +784,12 @@ HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, con
              "hx_delta_chunks: gates missing");
   HX_REQUIRE(head_stride >= state_floats(vdim, dim), "hx_delta_chunks: a head's state takes %d floats, not %d",
              state_floats(vdim, dim), head_stride);
-  if (requests == 0) return HX_OK;
+  if (portions == 0) return HX_OK;
   // four warps of 16 columns a CTA, one for each quarter of an SM (the staged chunks leave room for
   // one CTA); eight where there are more CTAs than SMs, so that a chunk is staged for twice as many
   const int sms = hx_device_sm_count();
   if (sms <= 0) return HX_ERR_LAUNCH;
-  const long long ctas = static_cast<long long>(requests) * heads * ((vdim + 63) / 64);
+  const long long ctas = static_cast<long long>(portions) * heads * ((vdim + 63) / 64);
   const int column_warps = vdim > 64 && ctas > sms ? 8 : vdim > 32 ? 4 : (vdim + 15) / 16;
   const size_t rows = static_cast<size_t>(heads) * tokens;
   float4* factors = static_cast<float4*>(scratch);
@@ -789,7 +800,8 @@ HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, con
                     static_cast<const __nv_bfloat16*>(decay_in), static_cast<const __nv_bfloat16*>(beta_in),
                     ld_gates, a_log, dt_bias, fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, weights,
                     factors, total, tokens, state, state_stride, head_stride, o, request_start, request_slot,
-                    requests, heads, qk_heads, dim, vdim, parts_for(dim), column_warps};
+                    requests, heads, qk_heads, dim, vdim, parts_for(dim), column_warps, min_query_len,
+                    portions};
   int rc;
   switch ((dim + 15) / 16) {
     case 1: case 2: rc = launch_delta<2>(a, tiles, stream); break;
@@ -801,4 +813,19 @@ HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, con
   hx_count_launches(1);
   HX_CHECK_LAUNCH("hx_delta_chunks");
   return HX_OK;
+}
+
+// Every request of the step.
+HX_API int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                           const void* decay_in, const void* beta_in, int ld_gates,
+                           const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
+                           int unit_norm, float unit_eps, float q_scale, float k_scale,
+                           void* scratch, float* state, long long state_stride, int head_stride,
+                           float* o, const int* request_start, const int* request_slot,
+                           int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
+                           int vdim, cudaStream_t stream) {
+  return hx_delta_chunks_from(q, ld_q, k, ld_k, v, ld_v, decay_in, beta_in, ld_gates, a_log, dt_bias, fixed_decay_m1,
+                              unit_norm, unit_eps, q_scale, k_scale, scratch, state, state_stride, head_stride, o,
+                              request_start, request_slot, requests, tokens, tiles, heads, qk_heads, dim, vdim, 1,
+                              requests, stream);
 }

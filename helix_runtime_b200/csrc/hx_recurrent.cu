@@ -727,6 +727,7 @@ struct LinearStateArgs {
   const int* request_slot;
   int heads, qk_heads, dim, vdim;
   int parts, block_lanes, tile, per_token;
+  int below;                // > 0: requests of so many tokens and more are another kernel's
 };
 
 template <typename T, bool DELTA, bool ONE_TOKEN>
@@ -742,6 +743,10 @@ void linear_state_scan_kernel(const LinearStateArgs<T> a) {
   const int head = blockIdx.y;
   const int qk_head = head / (a.heads / a.qk_heads);
   const int start = a.request_start[request];
+  if (a.below > 0) {
+    const int length = a.request_start[request + 1] - start;
+    if (length == 0 || length >= a.below) return;      // before any barrier: the whole CTA leaves
+  }
   const int count = ONE_TOKEN ? 1 : a.request_start[request + 1] - start;
   const int parts = a.parts;
   const int dim = a.dim;
@@ -1245,17 +1250,17 @@ void launch_linear_state(const LinearStateArgs<T>& a, bool delta, bool one_token
 // `fixed_decay_m1` [heads] give the head's constant decay and the same minus one);
 // delta != 0 needs `beta_in`.  Rotation: `positions` with `freq` (and `freq_exact` in the
 // float32 engine), or null.  o [tokens, heads * vdim] float32.
-HX_API int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k, const void* v,
-                                int ld_v, int dtype, int delta, const void* decay_in,
-                                const void* beta_in, int ld_gates, const float* a_log,
-                                const float* dt_bias, const float* fixed_decay,
-                                const float* fixed_decay_m1, const int* positions,
-                                const float* freq, const double* freq_exact, int rotary_dim,
-                                int rotary_layout, int unit_norm, float unit_eps, float q_scale,
-                                float k_scale, float* state, long long state_stride,
-                                int head_stride, float* o, const int* request_start,
-                                const int* request_slot, int requests, int tokens, int heads,
-                                int qk_heads, int dim, int vdim, cudaStream_t stream) {
+static int linear_state_scan(const void* q, int ld_q, const void* k, int ld_k, const void* v,
+                             int ld_v, int dtype, int delta, const void* decay_in,
+                             const void* beta_in, int ld_gates, const float* a_log,
+                             const float* dt_bias, const float* fixed_decay,
+                             const float* fixed_decay_m1, const int* positions,
+                             const float* freq, const double* freq_exact, int rotary_dim,
+                             int rotary_layout, int unit_norm, float unit_eps, float q_scale,
+                             float k_scale, float* state, long long state_stride,
+                             int head_stride, float* o, const int* request_start,
+                             const int* request_slot, int requests, int tokens, int heads,
+                             int qk_heads, int dim, int vdim, int below, int longest, cudaStream_t stream) {
   HX_REQUIRE(requests >= 0 && heads > 0 && qk_heads > 0 && dim > 0 && vdim > 0,
              "hx_linear_state_scan: bad sizes");
   HX_REQUIRE(heads % qk_heads == 0,
@@ -1282,7 +1287,7 @@ HX_API int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k
   if (requests == 0) return HX_OK;
   const dim3 grid(requests, heads, column_blocks);
   const size_t shared_bytes = static_cast<size_t>(tile) * per_token * sizeof(float);
-  const bool one_token = tokens == requests;
+  const bool one_token = below > 0 ? longest == 1 : tokens == requests;
   const size_t one_bytes = static_cast<size_t>(per_token) * sizeof(float);
   if (dtype == HX_F32) {
     LinearStateArgs<float> a{static_cast<const float*>(q), static_cast<const float*>(k),
@@ -1292,7 +1297,7 @@ HX_API int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k
                              freq_exact, rotary_dim, rotary_layout, unit_norm, unit_eps, q_scale,
                              k_scale, state, state_stride, head_stride, o, request_start,
                              request_slot, heads, qk_heads, dim, vdim, parts, block_lanes, tile,
-                             per_token};
+                             per_token, below};
     launch_linear_state(a, delta != 0, one_token, grid, threads, shared_bytes, one_bytes, stream);
   } else if (dtype == HX_BF16) {
     LinearStateArgs<__nv_bfloat16> a{
@@ -1302,13 +1307,55 @@ HX_API int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k
         ld_gates, a_log, dt_bias, fixed_decay, fixed_decay_m1, positions, freq, freq_exact,
         rotary_dim, rotary_layout, unit_norm, unit_eps, q_scale, k_scale, state, state_stride,
         head_stride, o, request_start, request_slot, heads, qk_heads, dim, vdim, parts,
-        block_lanes, tile, per_token};
+        block_lanes, tile, per_token, below};
     launch_linear_state(a, delta != 0, one_token, grid, threads, shared_bytes, one_bytes, stream);
   } else {
     HX_REQUIRE(false, "hx_linear_state_scan: unknown dtype %d", dtype);
   }
   HX_CHECK_LAUNCH("hx_linear_state_scan");
   return HX_OK;
+}
+
+HX_API int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k, const void* v,
+                                int ld_v, int dtype, int delta, const void* decay_in,
+                                const void* beta_in, int ld_gates, const float* a_log,
+                                const float* dt_bias, const float* fixed_decay,
+                                const float* fixed_decay_m1, const int* positions,
+                                const float* freq, const double* freq_exact, int rotary_dim,
+                                int rotary_layout, int unit_norm, float unit_eps, float q_scale,
+                                float k_scale, float* state, long long state_stride,
+                                int head_stride, float* o, const int* request_start,
+                                const int* request_slot, int requests, int tokens, int heads,
+                                int qk_heads, int dim, int vdim, cudaStream_t stream) {
+  return linear_state_scan(q, ld_q, k, ld_k, v, ld_v, dtype, delta, decay_in, beta_in, ld_gates, a_log, dt_bias,
+                           fixed_decay, fixed_decay_m1, positions, freq, freq_exact, rotary_dim, rotary_layout,
+                           unit_norm, unit_eps, q_scale, k_scale, state, state_stride, head_stride, o,
+                           request_start, request_slot, requests, tokens, heads, qk_heads, dim, vdim, 0, 0,
+                           stream);
+}
+
+// The same for the requests that bring fewer than `below` tokens to the step, whose longest brings
+// `longest`; the others (hx_delta_chunks_from takes them) are left alone.
+HX_API int hx_linear_state_scan_below(const void* q, int ld_q, const void* k, int ld_k, const void* v,
+                                      int ld_v, int dtype, int delta, const void* decay_in,
+                                      const void* beta_in, int ld_gates, const float* a_log,
+                                      const float* dt_bias, const float* fixed_decay,
+                                      const float* fixed_decay_m1, const int* positions,
+                                      const float* freq, const double* freq_exact, int rotary_dim,
+                                      int rotary_layout, int unit_norm, float unit_eps, float q_scale,
+                                      float k_scale, float* state, long long state_stride,
+                                      int head_stride, float* o, const int* request_start,
+                                      const int* request_slot, int requests, int tokens, int heads,
+                                      int qk_heads, int dim, int vdim, int below,
+                                      int longest, cudaStream_t stream) {
+  HX_REQUIRE(below > 0 && longest >= 0 && longest < below, "hx_linear_state_scan_below: %d tokens of %d", longest,
+             below);
+  if (longest == 0) return HX_OK;
+  return linear_state_scan(q, ld_q, k, ld_k, v, ld_v, dtype, delta, decay_in, beta_in, ld_gates, a_log, dt_bias,
+                           fixed_decay, fixed_decay_m1, positions, freq, freq_exact, rotary_dim, rotary_layout,
+                           unit_norm, unit_eps, q_scale, k_scale, state, state_stride, head_stride, o,
+                           request_start, request_slot, requests, tokens, heads, qk_heads, dim, vdim, below,
+                           longest, stream);
 }
 
 HX_API int hx_gated_group_norm(const float* y, int ld_y, const void* gate, int ld_gate, int dtype,

@@ -343,7 +343,12 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr,
         _c_ptr, _c_int, _c_float, _c_float, _c_float, _c_ptr, _c_ptr, _c_longlong, _c_int, _c_ptr,
         _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
-    library.hx_delta_chunks.restype = _c_int
+    library.hx_delta_chunks_from.argtypes = \
+        library.hx_delta_chunks.argtypes[:-1] + [_c_int, _c_int, _c_ptr]
+    library.hx_delta_chunks.restype = library.hx_delta_chunks_from.restype = _c_int
+    library.hx_linear_state_scan_below.argtypes = \
+        library.hx_linear_state_scan.argtypes[:-1] + [_c_int, _c_int, _c_ptr]
+    library.hx_linear_state_scan_below.restype = _c_int
     library.hx_state_chunks_supports.argtypes = [_c_int, _c_int]
     library.hx_state_chunks_scratch.argtypes = [_c_int, _c_int]
     library.hx_state_chunks_scratch.restype = _c_longlong
@@ -1307,7 +1312,7 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
                       freq_exact: Optional[torch.Tensor] = None, rotary_dim: int = 0,
                       rotary_layout: int = 1, unit_norm: bool = False, unit_eps: float = 0.0,
                       q_scale: float = 1.0, k_scale: float = 1.0,
-                      tokens: Optional[int] = None) -> None:
+                      tokens: Optional[int] = None, below: int = 0, longest: int = 0) -> None:
     """Linear attention with one ``[dim, vdim]`` matrix per head, token by token along each
     request: ``S <- g S + k v'`` (plain) or ``S <- g S; u = beta (v - S' k); S <- S + k u'``
     (``delta``), then ``o = S' q``.  ``q, k`` ``[tokens, qk_heads * dim]`` and ``v``
@@ -1318,7 +1323,8 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
     head (``unit_norm``: ``x / sqrt(sum x^2 + unit_eps)``) or rotated over their first
     ``rotary_dim`` coordinates by ``positions * freq`` (layout as ``ROTARY_LAYOUTS``), then
     times ``q_scale`` / ``k_scale``.  ``state`` ``[slots, >= heads * scan_state_floats(vdim,
-    dim)]`` and ``o`` ``[tokens, heads * vdim]`` float32."""
+    dim)]`` and ``o`` ``[tokens, heads * vdim]`` float32.  ``below`` > 0: only requests with fewer
+    tokens, the longest of which has ``longest``."""
     _need(state, torch.float32, "state")
     _need(o, torch.float32, "o")
     assert q.dtype == k.dtype == v.dtype and q.stride(-1) == k.stride(-1) == v.stride(-1) == 1
@@ -1337,14 +1343,18 @@ def linear_state_scan(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: 
             _need(tensor, torch.float32, name)
     if freq_exact is not None:
         _need(freq_exact, torch.float64, "freq_exact")
-    _check(lib().hx_linear_state_scan(
+    arguments = (
         q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
         dtype_code(q.dtype), 1 if delta else 0, _ptr(decay_in), _ptr(beta_in), ld_gates,
         _ptr(a_log), _ptr(dt_bias), _ptr(fixed_decay), _ptr(fixed_decay_m1), _ptr(positions),
         _ptr(freq), _ptr(freq_exact), rotary_dim, rotary_layout, 1 if unit_norm else 0,
         float(unit_eps), float(q_scale), float(k_scale), state.data_ptr(), state.stride(0),
         head_stride, o.data_ptr(), request_start.data_ptr(), request_slot.data_ptr(), requests,
-        q.shape[0] if tokens is None else tokens, heads, qk_heads, dim, vdim, _stream()))
+        q.shape[0] if tokens is None else tokens, heads, qk_heads, dim, vdim)
+    if below > 0:
+        _check(lib().hx_linear_state_scan_below(*arguments, below, longest, _stream()))
+    else:
+        _check(lib().hx_linear_state_scan(*arguments, _stream()))
 
 
 def delta_chunks_supports(dim: int, vdim: int) -> bool:
@@ -1364,10 +1374,12 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
                  decay_in: Optional[torch.Tensor] = None, a_log: Optional[torch.Tensor] = None,
                  dt_bias: Optional[torch.Tensor] = None,
                  fixed_decay_m1: Optional[torch.Tensor] = None, unit_norm: bool = False,
-                 unit_eps: float = 0.0, q_scale: float = 1.0, k_scale: float = 1.0) -> None:
+                 unit_eps: float = 0.0, q_scale: float = 1.0, k_scale: float = 1.0,
+                 min_query_len: int = 1, portions: Optional[int] = None) -> None:
     """The ``delta`` rule of :func:`linear_state_scan` without a rotation, 64 tokens at a time on
     the tensor cores (bfloat16 rows on 16 bytes); arguments as there.  ``scratch``:
-    :func:`delta_chunks_scratch` bytes; ``tiles``: :func:`recurrence_tiles` of the step."""
+    :func:`delta_chunks_scratch` bytes; ``tiles``: :func:`recurrence_tiles` of the step.
+    ``min_query_len`` > 1: only the ``portions`` requests with as many tokens, ``tiles`` are theirs."""
     _need(state, torch.float32, "state")
     _need(o, torch.float32, "o")
     for tensor in (q, k, v, beta_in):
@@ -1383,13 +1395,14 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
         if tensor is not None:
             _need(tensor, torch.float32, name)
     assert scratch.numel() * scratch.element_size() >= delta_chunks_scratch(heads, tokens)
-    _check(lib().hx_delta_chunks(
+    _check(lib().hx_delta_chunks_from(
         q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
         _ptr(decay_in), beta_in.data_ptr(), beta_in.stride(0), _ptr(a_log), _ptr(dt_bias),
         _ptr(fixed_decay_m1), 1 if unit_norm else 0, float(unit_eps), float(q_scale),
         float(k_scale), scratch.data_ptr(), state.data_ptr(), state.stride(0), head_stride,
         o.data_ptr(), request_start.data_ptr(), request_slot.data_ptr(), requests, tokens, tiles,
-        heads, qk_heads, dim, vdim, _stream()))
+        heads, qk_heads, dim, vdim, min_query_len, requests if portions is None else portions,
+        _stream()))
 
 
 # ------------------------------------------------------------- gated residual connection

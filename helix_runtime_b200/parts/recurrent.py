@@ -362,10 +362,18 @@ class LinearState(Mixer):
             self.rotary_dims = dims
             self.rotary_layout = ops.ROTARY_LAYOUTS[self.rotary.get("layout", "halves")]
 
-    # The chunks' two kernels take about as long for one portion of up to 64 tokens as the scan
-    # for 35 (32 heads of 128 by 128: 43 us against 39 for 32 tokens, 73 for 64); with more
-    # requests they win earlier (16 portions of 32: 149 us against 258).
+    # What the recurrence takes, alone (us, 32 heads of 128 by 128): one portion of 32 / 64 / 128
+    # tokens 42 / 43 / 53 in chunks and 42 / 76 / 144 by the scan; a decoding request in chunks costs a
+    # whole one, 75 for 8 of them and 456 for 64, where the scan takes 18 and 99.  So a step without
+    # decoding requests goes in chunks from 32 tokens on.  Beside decoding requests the portions
+    # (SHORT_TOKENS and more) go in chunks and the others by the scan, one behind the other: 18 + 43 for
+    # 8 and a portion of 64, 99 + 42 for 64 and one of 32 (by the scan alone 79 and 236).  With few
+    # decoding requests and a portion of fewer than 64 tokens the scan takes both in the time of the
+    # portion.
     CHUNKS_FROM_TOKENS = 32
+    SHORT_TOKENS = 16
+    MIXED_CHUNKS_FROM_TOKENS = 64
+    MIXED_CHUNKS_FROM_HEADS = 512      # requests times heads
 
     @staticmethod
     def decays_suit_chunks(decays: Optional[List[float]]) -> bool:
@@ -373,14 +381,21 @@ class LinearState(Mixer):
         by token, and powers of one above one leave float32's range inside a chunk."""
         return decays is None or all(0.0 <= decay <= 1.0 for decay in decays)
 
-    def runs_in_chunks(self, ctx: StepContext, qkv: torch.Tensor) -> bool:
-        """Whether the recurrence takes this step 64 tokens at a time on the tensor cores: the
-        delta rule in bfloat16 without a rotation (turned queries and keys are float32 numbers
-        that no stored row holds), for a step with a prompt portion in it."""
-        return (self.rule == "delta" and not self.rotary_dims and ctx.dtype == torch.bfloat16
-                and ctx.max_query_len >= self.CHUNKS_FROM_TOKENS and qkv.stride(0) % 8 == 0
-                and self.decays_suit_chunks(self.fixed_decay)
-                and ops.delta_chunks_supports(self.head_dim, self.value_dim))
+    def chunks_from(self, ctx: StepContext, qkv: torch.Tensor) -> int:
+        """The tokens from which a request of this step takes the recurrence 64 tokens at a time on
+        the tensor cores (0: none does): the delta rule in bfloat16 without a rotation (turned
+        queries and keys are float32 numbers that no stored row holds)."""
+        if (self.rule != "delta" or self.rotary_dims or ctx.dtype != torch.bfloat16
+                or ctx.max_query_len < self.CHUNKS_FROM_TOKENS or qkv.stride(0) % 8 != 0
+                or not self.decays_suit_chunks(self.fixed_decay)
+                or not ops.delta_chunks_supports(self.head_dim, self.value_dim)):
+            return 0
+        if ctx.min_query_len >= self.SHORT_TOKENS:
+            return 1
+        if (ctx.max_query_len >= self.MIXED_CHUNKS_FROM_TOKENS
+                or ctx.n_requests * self.heads >= self.MIXED_CHUNKS_FROM_HEADS):
+            return self.SHORT_TOKENS
+        return 0
 
     def weight_bytes(self) -> int:
         return self.w_in.nbytes() + self.w_o.nbytes()
@@ -414,20 +429,26 @@ class LinearState(Mixer):
             a_log=self.a_log, dt_bias=self.dt_bias, fixed_decay_m1=self.decay_m1,
             unit_norm=self.unit_norm, unit_eps=self.unit_eps, q_scale=self.q_scale,
             k_scale=self.k_scale)
-        if self.runs_in_chunks(ctx, qkv):
+        chunks_from = self.chunks_from(ctx, qkv)
+        if chunks_from > 0:
+            portions = [length for length in ctx.host_query_lengths if length >= chunks_from]
             scratch = ctx.workspace.get(
                 f"linear_state.chunks/{self.heads}",
                 (ops.delta_chunks_scratch(self.heads, ctx.capacity),), torch.uint8)
             ops.delta_chunks(q, k, v, state, o, scratch, ctx.request_start, ctx.request_slot,
-                             ctx.n_requests, n, ops.recurrence_tiles(ctx.host_query_lengths),
-                             self.heads, self.qk_heads, self.head_dim, self.value_dim, **gates)
-        else:
+                             ctx.n_requests, n, ops.recurrence_tiles(portions), self.heads,
+                             self.qk_heads, self.head_dim, self.value_dim,
+                             min_query_len=chunks_from, portions=len(portions), **gates)
+        if chunks_from != 1:
+            longest = max((length for length in ctx.host_query_lengths if length < chunks_from),
+                          default=0) if chunks_from > 0 else 0
             ops.linear_state_scan(
                 q, k, v, state, o, ctx.request_start, ctx.request_slot, ctx.n_requests, self.heads,
                 self.qk_heads, self.head_dim, self.value_dim, delta=self.rule == "delta",
                 fixed_decay=self.decay, positions=ctx.positions if self.rotary_dims else None,
                 freq=self.freq, freq_exact=self.freq_exact, rotary_dim=self.rotary_dims,
-                rotary_layout=self.rotary_layout, tokens=n, **gates)
+                rotary_layout=self.rotary_layout, tokens=n, below=chunks_from, longest=longest,
+                **gates)
         ops.gated_group_norm(o, rows[:, self.gate_at:self.gate_at + self.v_width], self.norm, gated,
                              n, self.heads, self.eps, gate_after=True)
         project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)

@@ -244,6 +244,19 @@ int hx_linear_state_scan(const void* q, int ld_q, const void* k, int ld_k, const
                          const int* request_start, const int* request_slot, int requests,
                          int tokens, int heads, int qk_heads, int dim, int vdim,
                          cudaStream_t stream);
+/* the same for the requests that bring fewer than `below` tokens, the longest of which brings
+ * `longest`; the others are left alone */
+int hx_linear_state_scan_below(const void* q, int ld_q, const void* k, int ld_k, const void* v,
+                               int ld_v, int dtype, int delta, const void* decay_in,
+                               const void* beta_in, int ld_gates, const float* a_log,
+                               const float* dt_bias, const float* fixed_decay,
+                               const float* fixed_decay_m1, const int* positions, const float* freq,
+                               const double* freq_exact, int rotary_dim, int rotary_layout,
+                               int unit_norm, float unit_eps, float q_scale, float k_scale,
+                               float* state, long long state_stride, int head_stride, float* o,
+                               const int* request_start, const int* request_slot, int requests,
+                               int tokens, int heads, int qk_heads, int dim, int vdim,
+                               int below, int longest, cudaStream_t stream);
 /* channels in `groups` equal parts, each over its root mean square, times weight; the gate
  * silu(gate) multiplies before the norm (gate_after 0) or after it (1) */
 int hx_gated_group_norm(const float* y, int ld_y, const void* gate, int ld_gate, int dtype,
@@ -414,6 +427,16 @@ int hx_delta_chunks(const void* q, int ld_q, const void* k, int ld_k, const void
                     long long state_stride, int head_stride, float* o, const int* request_start,
                     const int* request_slot, int requests, int tokens, int tiles, int heads,
                     int qk_heads, int dim, int vdim, cudaStream_t stream);
+/* the same for the requests that bring at least min_query_len tokens, `portions` of them with `tiles`
+ * chunks; the others are left alone */
+int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                         const void* decay_in, const void* beta_in, int ld_gates, const float* a_log,
+                         const float* dt_bias, const float* fixed_decay_m1, int unit_norm,
+                         float unit_eps, float q_scale, float k_scale, void* scratch, float* state,
+                         long long state_stride, int head_stride, float* o, const int* request_start,
+                         const int* request_slot, int requests, int tokens, int tiles, int heads,
+                         int qk_heads, int dim, int vdim, int min_query_len,
+                         int portions, cudaStream_t stream);
 
 /* ---- attention over a cached latent ----------------------------------------------------- */
 /* down [tokens][q_rank + kv_rank + rot] float32: both latents RMS-normed with a weight; the

@@ -234,6 +234,97 @@ def test_no_further_from_64_bits_than_the_scan():
     assert np.linalg.norm(got_state - after) <= np.linalg.norm(scanned - after)
 
 
+@pytest.mark.parametrize("lengths", [(1, 70, 1, 1, 129), (1, 64), (3, 1, 100, 15, 16, 1), (2, 1)])
+def test_portions_in_chunks_beside_the_scan_of_the_others(lengths):
+    """Portions of 16 tokens and more in chunks, the other requests by the scan, to the last bit as
+    if they were alone; neither touches what is the other's."""
+    from helix_runtime_b200.ops import library as ops
+    rng = np.random.default_rng(len(lengths))
+    heads, qk_heads, dim, vdim, short = 4, 2, 48, 40, 16
+    q, k, v, gates, before, starts = inputs(rng, heads, qk_heads, dim, vdim, lengths)
+    tokens, requests = sum(lengths), len(lengths)
+    per_head = ops.scan_state_floats(vdim, dim)
+    held = torch.tensor(np.stack([packed_state(row, per_head).reshape(-1) for row in before]),
+                        dtype=torch.float32).cuda()
+    start = torch.tensor(starts, dtype=torch.int32).cuda()
+    slots = torch.arange(requests, dtype=torch.int32).cuda()
+    options = dict(decay_in=gates[:, heads:], beta_in=gates[:, :heads], unit_norm=True, unit_eps=1e-6,
+                   a_log=torch.linspace(-1.0, 0.5, heads).cuda(), dt_bias=torch.full((heads,), -2.0).cuda())
+    sizes = (requests, heads, qk_heads, dim, vdim)
+    scanned, o_scanned = held.clone(), torch.full((tokens, heads * vdim), 7.0, device="cuda")
+    ops.linear_state_scan(q, k, v, scanned, o_scanned, start, slots, *sizes, delta=True, tokens=tokens, **options)
+    state, o = held.clone(), torch.full((tokens, heads * vdim), 7.0, device="cuda")
+    scratch = torch.empty((ops.delta_chunks_scratch(heads, tokens),), dtype=torch.uint8, device="cuda")
+    portions = [length for length in lengths if length >= short]
+    ops.delta_chunks(q, k, v, state, o, scratch, start, slots, requests, tokens,
+                     ops.recurrence_tiles(portions), heads, qk_heads, dim, vdim, min_query_len=short,
+                     portions=len(portions), **options)
+    for r, length in enumerate(lengths):
+        rows = slice(starts[r], starts[r + 1])
+        if length < short:
+            assert (o[rows] == 7.0).all() and torch.equal(state[r], held[r])
+            continue
+        for got, want in ((o[rows], o_scanned[rows]), (state[r], scanned[r])):
+            # both are within this of the recurrence in double (see above)
+            assert (got - want).norm() <= 16 * 128 ** 0.5 * 2.0 ** -24 * want.norm()
+    after_chunks, o_after_chunks = state.clone(), o.clone()
+    ops.linear_state_scan(q, k, v, state, o, start, slots, *sizes, delta=True, tokens=tokens, below=short,
+                          longest=max(length for length in lengths if length < short), **options)
+    for r, length in enumerate(lengths):
+        rows = slice(starts[r], starts[r + 1])
+        same, o_same = (scanned, o_scanned) if length < short else (after_chunks, o_after_chunks)
+        assert torch.equal(state[r], same[r]) and torch.equal(o[rows], o_same[rows])
+
+
+@pytest.mark.parametrize("lengths,chunks_from", [
+    ((1,) * 8, 0), ((31,), 0), ((32,), 1), ((16, 33), 1),
+    ((1,) * 15 + (40,), 0),                # the scan takes all of it in the portion's time
+    ((1,) * 15 + (64,), 16), ((1,) * 150 + (32,), 16), ((1, 20, 500), 16),
+])
+def test_a_decoding_request_does_not_take_the_chunks(lengths, chunks_from, monkeypatch):
+    """What a step's requests bring decides their road: a chunk costs a decoding request as much as 64
+    tokens, so portions alone go in chunks."""
+    from helix_runtime_b200 import StepEntry, StepFunction
+    from helix_runtime_b200.cache.manager import CacheManager
+    from helix_runtime_b200.config.medolorn import DeltaMixerConfig, MedolornConfig, MedolornLayerConfig
+    from helix_runtime_b200.config.registry import architecture_for
+    from helix_runtime_b200.models.decoder import DecoderModel
+    from helix_runtime_b200.parts import recurrent
+    mixer = DeltaMixerConfig(heads=4, kv_heads=2, dim=16, vdim=16, conv=4)
+    config = MedolornConfig(vocab=64, width=64, norm_eps=1e-5, canon_taps=4, max_positions=1024,
+                            layers=(MedolornLayerConfig("delta", mixer, None),))
+    model = DecoderModel(architecture_for(config.to_dict()).build_spec(config))
+    torch.manual_seed(0)
+    model.bind({request.name: torch.randn(request.shape, device="cuda").mul_(0.1).to(
+        torch.float32 if request.role == "scale" else torch.bfloat16)
+        for request in model.tensor_requests()}, torch.bfloat16, torch.device("cuda:0"))
+    kv, state = model.cache_needs()
+    cache = CacheManager(kv, state, 16, 64, len(lengths), model.max_positions, model.dtype, model.device)
+    step = StepFunction(model, cache, max_tokens=sum(lengths), max_requests=len(lengths))
+    for request in range(len(lengths)):
+        cache.admit(request)
+    routes = {}
+    chunks, scan = recurrent.ops.delta_chunks, recurrent.ops.linear_state_scan
+
+    def watched_chunks(*args, **options):
+        routes["chunks"] = (options.get("min_query_len", 1), options.get("portions", args[8]))
+        return chunks(*args, **options)
+
+    def watched_scan(*args, **options):
+        routes["scan"] = (options.get("below", 0), options.get("longest", 0))
+        return scan(*args, **options)
+    monkeypatch.setattr(recurrent.ops, "delta_chunks", watched_chunks)
+    monkeypatch.setattr(recurrent.ops, "linear_state_scan", watched_scan)
+    step.run([StepEntry(request, [1] * length, [length - 1]) for request, length in enumerate(lengths)])
+    want = {}
+    if chunks_from:
+        want["chunks"] = (chunks_from, sum(length >= chunks_from for length in lengths))
+    if chunks_from != 1:
+        below = [length for length in lengths if length < chunks_from]
+        want["scan"] = (chunks_from, max(below, default=0))
+    assert routes == want
+
+
 def test_refusals():
     from helix_runtime_b200.ops import library as ops
     assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
