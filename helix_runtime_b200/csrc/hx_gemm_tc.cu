@@ -1157,7 +1157,8 @@ int launch_epilogue(int epilogue, const CUtensorMap& map_w, const CUtensorMap& m
 // columns: half a tile takes 0.55 of a tile's time, a quarter 0.35 (its tokens are loaded as for a
 // whole one).  256 tokens by [22,016 x 4,096], 86 tiles on 74 pairs: 63.6 -> 47.9 us; 2,048 by
 // [12,288 x 4,096], 384: 142 -> 132 us in place.
-double plan_rounds(long long units, int workers, int k_blocks, bool add, int most_pieces,
+// `ordered`: every sum has one writer, so nothing is shared out.
+double plan_rounds(long long units, int workers, int k_blocks, bool add, bool ordered, int most_pieces,
                    int& whole_rounds, int& tail_workers, int& pieces) {
   const int rest = static_cast<int>(units % workers);
   const long long rounds = units / workers;
@@ -1171,7 +1172,7 @@ double plan_rounds(long long units, int workers, int k_blocks, bool add, int mos
       return k_blocks * (static_cast<double>(rounds) + (pieces == 2 ? 0.55 : 0.35));
     }
   }
-  if (add && HX_GEMM_STREAM_K && rest > 0 && rest * 2 <= workers) {
+  if (add && !ordered && HX_GEMM_STREAM_K && rest > 0 && rest * 2 <= workers) {
     const double blocks = static_cast<double>(rest) * k_blocks;
     int share = static_cast<int>(sqrt(blocks * workers / 15.0));
     share = share < rest ? rest : share > workers ? workers : share;
@@ -1210,7 +1211,7 @@ constexpr int MOST_PIECES = 4;      // of a tile of the last round
 
 template <int EPI>
 int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, PersistentArgs args,
-                      const WeightBoxes& boxes, cudaStream_t stream) {
+                      const WeightBoxes& boxes, cudaStream_t stream, bool ordered = false) {
   static bool configured = false;
   const int sms = hx_device_sm_count();
   if (sms <= 0) return HX_ERR_LAUNCH;
@@ -1228,7 +1229,7 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   HX_REQUIRE(tiles < (1ll << 30), "hx_gemm_tc: too many tiles");
   args.units = static_cast<int>(tiles);
   int whole_rounds = -1, tail = 0, pieces = 1;
-  const double alone = plan_rounds(tiles, sms, args.k_blocks, EPI == EPI_ADD_F32, 1,
+  const double alone = plan_rounds(tiles, sms, args.k_blocks, EPI == EPI_ADD_F32, ordered, 1,
                                    args.whole_rounds, args.tail_ctas, pieces);
   // Pairs, unless their tiles of 256 tokens make the rounds longer by more than the twentieth that a
   // round is shorter at least (1,900 tokens by [27,648 x 5,120]: 12 rounds against 11, 380 against 375
@@ -1237,8 +1238,8 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
   const int pair_tiles = (args.tokens + 2 * BM - 1) / (2 * BM), pairs = sms / 2;
   const long long pair_units = static_cast<long long>(pair_tiles) * feature_tiles;
   if (args.heads == 1 && args.tile_group == nullptr && args.tokens > BM && pairs > 0) {
-    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, MOST_PIECES,
-                                      whole_rounds, tail, pieces);
+    const double paired = plan_rounds(pair_units, pairs, args.k_blocks, EPI == EPI_ADD_F32, ordered,
+                                      MOST_PIECES, whole_rounds, tail, pieces);
     const double penalty = EPI == EPI_ADD_F32 && whole_rounds == 0 && args.k_blocks < 96 ? 4.0 : 0.0;
     if (0.95 * paired + penalty <= alone) {
       args.token_tiles = pair_tiles;
@@ -1267,11 +1268,11 @@ int launch_persistent(const CUtensorMap& map_w, const CUtensorMap& map_x, Persis
 
 int launch_persistent_epilogue(int epilogue, const CUtensorMap& map_w, const CUtensorMap& map_x,
                                const PersistentArgs& args, const WeightBoxes& boxes,
-                               cudaStream_t stream) {
+                               cudaStream_t stream, bool ordered = false) {
   switch (epilogue) {
     case EPI_STORE_BF16: return launch_persistent<EPI_STORE_BF16>(map_w, map_x, args, boxes, stream);
     case EPI_STORE_F32: return launch_persistent<EPI_STORE_F32>(map_w, map_x, args, boxes, stream);
-    case EPI_ADD_F32: return launch_persistent<EPI_ADD_F32>(map_w, map_x, args, boxes, stream);
+    case EPI_ADD_F32: return launch_persistent<EPI_ADD_F32>(map_w, map_x, args, boxes, stream, ordered);
     case EPI_SWIGLU: return launch_persistent<EPI_SWIGLU>(map_w, map_x, args, boxes, stream);
     case EPI_ROPE_APPEND: return launch_persistent<EPI_ROPE_APPEND>(map_w, map_x, args, boxes, stream);
     default:
@@ -1310,7 +1311,7 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
                    int weight_rows, void* out, int ldo, int tokens, int features, int depth,
                    int epilogue, int activation, float gate_limit, const float* gate_bias,
                    const float* up_bias, int up_row_offset, int k_splits, int weight_tiles,
-                   int* status, cudaStream_t stream, float softcap = 0.0f) {
+                   int* status, cudaStream_t stream, float softcap = 0.0f, bool ordered = false) {
   if (weight_tiles) ldw = 8;      // not a stride of anything here
   HX_REQUIRE(softcap >= 0.0f && (softcap == 0.0f || epilogue == EPI_STORE_F32),
              "hx_gemm_tc: a softcap belongs to a float32 store");
@@ -1354,7 +1355,7 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
     PersistentArgs args{out, ldo, tokens, features, depth, up_row_offset, k_tiles, 0, 0,
                         total_k_blocks, status, RopeArgs{}, -1, activation, nullptr, 0,
                         gate_limit, gate_bias, up_bias, softcap};
-    rc = launch_persistent_epilogue(epilogue, map_w, map_x, args, boxes, stream);
+    rc = launch_persistent_epilogue(epilogue, map_w, map_x, args, boxes, stream, ordered);
     if (rc != HX_OK) return rc;
     HX_CHECK_LAUNCH("hx_gemm_tc");
     return HX_OK;
@@ -1392,6 +1393,17 @@ HX_API int hx_gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w
   return gemm_tc(x, ldx, x_capacity_rows, w, ldw, weight_rows, out, ldo, tokens, features, depth,
                  epilogue, activation, 0.0f, nullptr, nullptr, up_row_offset, k_splits,
                  weight_tiles, status, stream);
+}
+
+// The product added to a float32 output by one writer per sum, for any number of tokens: the same call
+// gives the same bits.  (hx_gemm_tc shares a short last round of sums out by atomic adds: 512 tokens by
+// [4,096 x 4,096] 24.6 us.)
+HX_API int hx_gemm_tc_ordered(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,
+                              int weight_rows, float* out, int ldo, int tokens, int features,
+                              int depth, int weight_tiles, int* status, cudaStream_t stream) {
+  return gemm_tc(x, ldx, x_capacity_rows, w, ldw, weight_rows, out, ldo, tokens, features, depth,
+                 EPI_ADD_F32, HX_GATE_SILU, 0.0f, nullptr, nullptr, 0, 1, weight_tiles, status, stream,
+                 0.0f, true);
 }
 
 // The product with a float32 store whose sums run into a level: out = cap * tanh(x w^T / cap).

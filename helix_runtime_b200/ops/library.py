@@ -321,6 +321,9 @@ def _declare(library: ctypes.CDLL) -> None:
                                       _c_int, _c_int, _c_float, _c_ptr, _c_ptr]
     for name in ("hx_gemm_split_supports", "hx_gemm_split_pays", "hx_gemm_split"):
         getattr(library, name).restype = _c_int
+    library.hx_gemm_tc_ordered.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr,
+                                           _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr]
+    library.hx_gemm_tc_ordered.restype = _c_int
     library.hx_gemm_tc_runs_supports.argtypes = [_c_int] * 6
     library.hx_gemm_tc_runs.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int,
                                         _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_ptr, _c_ptr,
@@ -676,13 +679,15 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, fe
             epilogue: int, status: torch.Tensor, up_row_offset: int = 0, k_splits: int = 1,
             weight_shape: Optional[Tuple[int, int]] = None, gate_activation: Optional[int] = None,
             gate_limit: float = 0.0, gate_bias: Optional[torch.Tensor] = None,
-            up_bias: Optional[torch.Tensor] = None, softcap: float = 0.0) -> None:
+            up_bias: Optional[torch.Tensor] = None, softcap: float = 0.0,
+            ordered: bool = False) -> None:
     """out[:tokens, :features] (op)= x[:tokens] @ w.T on the tensor cores (bfloat16).  ``w``
     is the matrix ``[rows, depth]`` or its tiles from :func:`tile_weights` (then
     ``weight_shape`` gives rows and depth).  With ``gate_activation`` (any of GATE_ACTIVATIONS)
     the epilogue is that gated activation of ``[gate; up]`` whatever ``epilogue`` says, with the
     optional float32 biases ``gate_bias`` and ``up_bias`` ``[features]`` added first.
-    ``softcap`` > 0 with ``EPI_STORE_F32``: softcap * tanh(product / softcap) is stored."""
+    ``softcap`` > 0 with ``EPI_STORE_F32``: softcap * tanh(product / softcap) is stored.
+    ``ordered`` with ``EPI_ADD_F32``: one writer per sum, so that a call repeats bit for bit."""
     _need(x, torch.bfloat16, "x")
     _need(w, torch.bfloat16, "w")
     tiled = w.dim() == 4
@@ -715,6 +720,14 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, fe
                                            rows, out.data_ptr(), out.stride(0), tokens, features,
                                            depth, float(softcap), 1 if tiled else 0,
                                            status.data_ptr(), _stream()))
+        return
+    if ordered and epilogue == EPI_ADD_F32:
+        if k_splits != 1:
+            raise ValueError("an ordered sum is not cut along the reduction")
+        _need(out, torch.float32, "out")
+        _check(lib().hx_gemm_tc_ordered(x.data_ptr(), x.stride(0), x.shape[0], w.data_ptr(), ldw, rows,
+                                        out.data_ptr(), out.stride(0), tokens, features, depth,
+                                        1 if tiled else 0, status.data_ptr(), _stream()))
         return
     _check(lib().hx_gemm_tc(x.data_ptr(), x.stride(0), x.shape[0], w.data_ptr(), ldw, rows,
                             out.data_ptr(), out.stride(0), tokens, features, depth, epilogue,

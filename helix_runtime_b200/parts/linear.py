@@ -116,7 +116,8 @@ def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue
             status: torch.Tensor, ordered: bool = False, softcap: float = 0.0,
             features: Optional[int] = None) -> None:
     """``out[:tokens] (op)= x[:tokens] @ w.T``; epilogue is one of ops.EPI_STORE,
-    ops.EPI_STORE_F32, ops.EPI_ADD_F32.  ``features``: only the first so many rows of ``w``.  ``ordered``: no split-K (see ``split_k_for``).
+    ops.EPI_STORE_F32, ops.EPI_ADD_F32.  ``features``: only the first so many rows of ``w``.
+    ``ordered``: one writer per sum, no split-K (see ``split_k_for``) and no shared last round.
     ``softcap`` > 0 (ops.EPI_STORE_F32 only): ``softcap * tanh(product / softcap)``."""
     if tokens == 0:
         return
@@ -124,7 +125,7 @@ def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue
         splits = split_k_for(tokens, w.rows, w.depth, ordered) \
             if epilogue == ops.EPI_ADD_F32 else 1
         _gemm_tc(x, w, out, tokens, features or w.rows, epilogue, status, k_splits=splits,
-                 softcap=softcap)
+                 softcap=softcap, ordered=ordered)
     else:
         _gemm_simt(x, w, out, tokens, epilogue, status, softcap, features)
 
@@ -134,7 +135,8 @@ def project_into_accumulator(x: torch.Tensor, w: Weight, accumulator: torch.Tens
     """``accumulator[:tokens] += x[:tokens] @ w.T`` as a split-K weight stream (float32; the
     accumulator is clear on entry and its reader clears it again)."""
     splits = split_k_for(tokens, w.rows, w.depth, ordered)
-    _gemm_tc(x, w, accumulator, tokens, w.rows, ops.EPI_ADD_F32, status, k_splits=splits)
+    _gemm_tc(x, w, accumulator, tokens, w.rows, ops.EPI_ADD_F32, status, k_splits=splits,
+             ordered=ordered)
 
 
 def project_swiglu(x: torch.Tensor, w_gate_up: Weight, intermediate: int, act: torch.Tensor,

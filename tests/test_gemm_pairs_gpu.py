@@ -56,3 +56,26 @@ def test_every_epilogue(tokens, features, depth, tiled):
             <= (2.0 ** -8 + 2.0 ** -18) * act.abs() + 2 * slack + 1e-6).all()
     assert (out[tokens:] == 7.0).all()
     assert int(status.item()) == 0
+
+
+def test_an_ordered_sum_repeats_bit_for_bit():
+    """Sizes whose last round of tiles is shared out by atomic adds unless the caller wants an order."""
+    from helix_runtime_b200.ops import library as ops
+    from helix_runtime_b200.parts.linear import Weight, project
+    torch.manual_seed(3)
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for tokens, features, depth in ((512, 4096, 4096), (1200, 4096, 4096), (300, 2050, 11008)):
+        x = torch.randn(tokens, depth, device="cuda").bfloat16()
+        matrix = torch.randn(features, depth, device="cuda").bfloat16()
+        before = torch.randn(tokens, features, device="cuda")
+        want = before.double() + x.double() @ matrix.double().T
+        for weight in (Weight(matrix), Weight(matrix, tile=False)):
+            first = None
+            for _ in range(40):
+                out = before.clone()
+                project(x, weight, out, tokens, ops.EPI_ADD_F32, status, True)
+                first = out if first is None else first
+                assert torch.equal(out, first)
+            size = before.double().abs() + x.double().abs() @ matrix.double().abs().T
+            assert ((first - want).abs() <= (depth + 2) * 2.0 ** -24 * size).all()
+    assert int(status.item()) == 0
