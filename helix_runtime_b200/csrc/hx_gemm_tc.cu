@@ -1431,7 +1431,7 @@ HX_API int hx_gemm_tc_gated(const void* x, int ldx, int x_capacity_rows, const v
                  weight_tiles, status, stream);
 }
 
-// The grouped product: rows of x come in tiles of `token_tile` (16, 32, 64 or 128), and
+// The grouped product: rows of x come in tiles of `token_tile` (16, 32, 64, 128 or 256), and
 // tile t multiplies with group tile_group[t] of w, which holds `groups` matrices of
 // `group_rows` rows one below the other (row-major, row stride ldw); a negative entry skips the
 // tile.  tile_group (device memory, ceil(tokens / token_tile) entries) may be written by the
@@ -1462,7 +1462,8 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
                                     : features <= group_rows,
              "hx_gemm_tc_grouped: features exceed a group's rows");
   HX_REQUIRE(ldo >= features, "hx_gemm_tc_grouped: output stride too small");
-  HX_REQUIRE(token_tile == 16 || token_tile == 32 || token_tile == 64 || token_tile == 128,
+  HX_REQUIRE(token_tile == 16 || token_tile == 32 || token_tile == 64 || token_tile == 128 ||
+                 token_tile == 256,
              "hx_gemm_tc_grouped: token tile %d", token_tile);
   CUtensorMap map_w, map_x;
   int rc = get_tensor_map(w, static_cast<uint64_t>(groups) * group_rows, depth, ldw, BM, &map_w);
@@ -1487,7 +1488,8 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
   switch (token_tile) {
     case 16: rc = launch_epilogue<16>(epilogue, map_w, map_x, args, grid, stream); break;
     case 32: rc = launch_epilogue<32>(epilogue, map_w, map_x, args, grid, stream); break;
-    default: rc = launch_epilogue<64>(epilogue, map_w, map_x, args, grid, stream); break;
+    case 64: rc = launch_epilogue<64>(epilogue, map_w, map_x, args, grid, stream); break;
+    default: rc = launch_epilogue<256>(epilogue, map_w, map_x, args, grid, stream); break;
   }
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_tc_grouped");

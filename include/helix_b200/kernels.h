@@ -564,7 +564,7 @@ int hx_gemm_tc_gated(const void* x, int ldx, int x_capacity_rows, const void* w,
                      int weight_rows, void* out, int ldo, int tokens, int features, int depth,
                      int activation, float gate_limit, const float* gate_bias, const float* up_bias,
                      int up_row_offset, int weight_tiles, int* status, cudaStream_t stream);
-/* grouped product: rows of x come in tiles of token_tile (16..128), tile t multiplies with
+/* grouped product: rows of x come in tiles of token_tile (16, 32, 64, 128 or 256), tile t multiplies with
  * group tile_group[t] of w (`groups` matrices of group_rows rows one below the other); a
  * negative entry skips the tile; tile_group is device memory, written on the stream before */
 int hx_gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,

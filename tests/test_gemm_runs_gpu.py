@@ -50,6 +50,36 @@ def test_runs_of_every_length(runs, rows, features, depth):
                 + 2 * bound * (1.1 * up.abs() + gate.abs() + 1e-3) + 1e-6).all()
 
 
+@pytest.mark.parametrize("token_tile", [16, 32, 64, 128, 256])
+def test_tiles_of_every_size_the_grouped_product_takes(token_tile):
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(token_tile)
+    listed, rows, features, depth = [2, -1, 0], 144, 136, 200
+    tokens = token_tile * len(listed)
+    x = (torch.randn(tokens, depth) * 0.5).bfloat16().cuda()
+    w = (torch.randn(3, 2 * rows, depth) * 0.1).bfloat16().cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    tile_group = torch.tensor(listed, dtype=torch.int32).cuda()
+    out = torch.full((tokens, features), 7.0, device="cuda")
+    act = torch.full((tokens, features), 7.0, dtype=torch.bfloat16, device="cuda")
+    ops.gemm_tc_grouped(x, w, out, tokens, features, ops.EPI_STORE_F32, 0, token_tile, tile_group, status)
+    ops.gemm_tc_grouped(x, w, act, tokens, features, ops.EPI_SWIGLU, rows, token_tile, tile_group, status)
+    assert int(status.item()) == 0
+    for tile, group in enumerate(listed):
+        part = slice(token_tile * tile, token_tile * (tile + 1))
+        if group < 0:
+            assert (out[part] == 7.0).all() and (act[part] == 7.0).all()
+            continue
+        gate = x[part].double() @ w[group, :features].double().T
+        up = x[part].double() @ w[group, rows:rows + features].double().T
+        # as in test_runs_of_every_length
+        bound = (depth + 2) * 2.0 ** -24 * (x[part].double().abs() @ w[group].double().abs().max(0)[0][:, None])
+        assert ((out[part] - gate).abs() <= bound).all()
+        want = torch.nn.functional.silu(gate) * up
+        assert ((act[part].double() - want).abs() <= (2.0 ** -8 + 2.0 ** -18) * want.abs()
+                + 2 * bound * (1.1 * up.abs() + gate.abs() + 1e-3) + 1e-6).all()
+
+
 def test_sizes_that_take_another_road():
     from helix_runtime_b200.ops import library as ops
     supports = ops.lib().hx_gemm_tc_runs_supports
