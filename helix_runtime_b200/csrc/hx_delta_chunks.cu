@@ -34,13 +34,12 @@
 // The scan walks a token in 0.6 us whatever the chip could do beside it (a chain of two dot
 // products over the state); a chunk is a chain of about 800 products a warp, which is what bounds
 // it now.  Measured (one B200, 32 heads of 128 by 128, against the scan): a portion of 1,000 tokens
-// 979 -> 215 us, eight of 256 1,065 -> 215, one of 64 71 -> 44; errors against 64 bits, 1,024 tokens, 2.0e-7
+// 957 -> 201 us, eight of 256 1,064 -> 222, one of 64 71 -> 46 (the numbers that are not finite found by
+// comparing instead: spills, 215, 215, 44); errors against 64 bits, 1,024 tokens, 2.0e-7
 // (outputs) and 1.3e-7 (state) where the scan has 2.3e-7 and 2.2e-7 (2.6e-7 and 2.5e-7 with a chunk's
 // products added onto the state itself).
 #include "hx_mma.cuh"
 #include "hx_scan.cuh"
-
-#include <cfloat>
 
 namespace {
 
@@ -478,7 +477,7 @@ __device__ __noinline__ void tokens_in_turn(const DeltaArgs& a, float (*S)[4], c
 
 // grid (portions, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
 template <int STEPS>
-__global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a) {
+__global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_constant__ DeltaArgs a) {
   constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
   extern __shared__ uint4 shared_pieces[];
   hx_pdl_prologue();
@@ -637,16 +636,16 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const DeltaArgs a)
     triangular_product(u, rest, weights + weight_lane);
     triangular_product(rest, u, weights + weight_lane + 2 * TERMS * CHUNK);
     const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
-    bool finite = true;
+    float odd = 0.0f;      // NaN with any number that is not finite (zero times it is)
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         out[n][j] += rest[n][j];
         u[n][j] *= factors[8 * n + pair + (j & 1)].w;
-        finite = finite && fabsf(out[n][j]) <= FLT_MAX && fabsf(u[n][j]) <= FLT_MAX;
+        odd = fmaf(out[n][j], 0.0f, fmaf(u[n][j], 0.0f, odd));
       }
-    if (__any_sync(0xffffffffu, !finite)) {
+    if (__any_sync(0xffffffffu, odd != 0.0f)) {
       const __nv_bfloat16* staged = queries_of(stage);
       float held[2 * STEPS][4];
 #pragma unroll

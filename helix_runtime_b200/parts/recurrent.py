@@ -363,14 +363,16 @@ class LinearState(Mixer):
             self.rotary_layout = ops.ROTARY_LAYOUTS[self.rotary.get("layout", "halves")]
 
     # What the recurrence takes, alone (us, 32 heads of 128 by 128): one portion of 32 / 64 / 128
-    # tokens 42 / 43 / 53 in chunks and 42 / 76 / 144 by the scan; a decoding request in chunks costs a
-    # whole one, 75 for 8 of them and 456 for 64, where the scan takes 18 and 99.  So a step without
-    # decoding requests goes in chunks from 32 tokens on.  Beside decoding requests the portions
-    # (SHORT_TOKENS and more) go in chunks and the others by the scan, one behind the other: 18 + 43 for
-    # 8 and a portion of 64, 99 + 42 for 64 and one of 32 (by the scan alone 79 and 236).  With few
-    # decoding requests and a portion of fewer than 64 tokens the scan takes both in the time of the
-    # portion.
-    CHUNKS_FROM_TOKENS = 32
+    # tokens 45 / 46 / 56 in chunks (two launches) and 42 / 76 / 144 by the scan, 16 portions of 32 152
+    # and 272; a decoding request in chunks costs a whole one, 82 for 8 of them and 473 for 64, where
+    # the scan takes 19 and 100.  So a step without decoding requests goes in chunks from a portion of
+    # 32 tokens and 48 tokens in all on.  Beside decoding requests the portions (SHORT_TOKENS and
+    # more) go in chunks and the others by the scan, one behind the other.  With few decoding requests
+    # and a portion of fewer than 64 tokens the scan takes both in the time of the portion.  A layer:
+    # 64 decoding requests and a portion of 32 / 128 / 512 tokens 567 / 599 / 733 all in chunks, 319 /
+    # 461 / 937 all by the scan, 241 / 266 / 352 so; 8 and 32 / 64 / 512 158 / 163 / 336, 129 / 169 /
+    # 726, 125 / 149 / 261.
+    CHUNKS_FROM_TOKENS, CHUNKS_FROM_TOKENS_IN_ALL = 32, 48
     SHORT_TOKENS = 16
     MIXED_CHUNKS_FROM_TOKENS = 64
     MIXED_CHUNKS_FROM_HEADS = 512      # requests times heads
@@ -391,7 +393,7 @@ class LinearState(Mixer):
                 or not ops.delta_chunks_supports(self.head_dim, self.value_dim)):
             return 0
         if ctx.min_query_len >= self.SHORT_TOKENS:
-            return 1
+            return 1 if ctx.n_tokens >= self.CHUNKS_FROM_TOKENS_IN_ALL else 0
         if (ctx.max_query_len >= self.MIXED_CHUNKS_FROM_TOKENS
                 or ctx.n_requests * self.heads >= self.MIXED_CHUNKS_FROM_HEADS):
             return self.SHORT_TOKENS

@@ -277,7 +277,7 @@ def test_portions_in_chunks_beside_the_scan_of_the_others(lengths):
 
 
 @pytest.mark.parametrize("lengths,chunks_from", [
-    ((1,) * 8, 0), ((31,), 0), ((32,), 1), ((16, 33), 1),
+    ((1,) * 8, 0), ((31, 31), 0), ((47,), 0), ((48,), 1), ((16, 32), 1),
     ((1,) * 15 + (40,), 0),                # the scan takes all of it in the portion's time
     ((1,) * 15 + (64,), 16), ((1,) * 150 + (32,), 16), ((1, 20, 500), 16),
 ])
