@@ -142,8 +142,8 @@ class EngineConfig:
     cuda_graphs: bool = True                  # replay decode-only steps as CUDA graphs
     lookahead: bool = True                    # queue the next decode step before this one's
                                               # tokens have been read (needs cuda_graphs)
-    ordered_sums: bool = False                # decode products sum in a fixed order (no split-K
-                                              # atomics): logits repeat bit for bit from run to
+    ordered_sums: bool = False                # products sum in a fixed order (one writer per sum,
+                                              # no atomics): logits repeat bit for bit from run to
                                               # run, at the price of slower weight streams
 
 
