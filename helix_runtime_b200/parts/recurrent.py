@@ -5,7 +5,7 @@ exponential gates, and mixers that wrap or run others.
 All of them keep per-request state in ONE float32 row per schedule entry (``StateNeed`` of a flat
 shape); a mixer cuts its row into the pieces it needs.  A step brings a portion of each
 request's tokens (cut anywhere, one token when decoding); the kernels carry the state from
-portion to portion, so the result does not depend on the cut.
+portion to portion, so the result does not depend on the cut (but for float32 rounding).
 
 :class:`StateSpaceMixer` (``state_space``).  Parameters ``heads``, ``head_width`` (``P``),
 ``state_size`` (``N``), ``groups`` (``G``), ``filter_taps``, ``norm_groups``, ``eps``.  With
@@ -361,6 +361,10 @@ class LinearState(Mixer):
             self.freq = exact.to(torch.float32).to(device).contiguous()
             self.rotary_dims = dims
             self.rotary_layout = ops.ROTARY_LAYOUTS[self.rotary.get("layout", "halves")]
+        self.chunkable = (self.rule == "delta" and not self.rotary_dims and dtype == torch.bfloat16
+                          and torch.device(device).type == "cuda"
+                          and self.decays_suit_chunks(self.fixed_decay)
+                          and ops.delta_chunks_supports(self.head_dim, self.value_dim))
 
     # What the recurrence takes, alone (us, 32 heads of 128 by 128): one portion of 32 / 64 / 128
     # tokens 45 / 46 / 56 in chunks (two launches) and 42 / 76 / 144 by the scan, 16 portions of 32 152
@@ -387,10 +391,8 @@ class LinearState(Mixer):
         """The tokens from which a request of this step takes the recurrence 64 tokens at a time on
         the tensor cores (0: none does): the delta rule in bfloat16 without a rotation (turned
         queries and keys are float32 numbers that no stored row holds)."""
-        if (self.rule != "delta" or self.rotary_dims or ctx.dtype != torch.bfloat16
-                or ctx.max_query_len < self.CHUNKS_FROM_TOKENS or qkv.stride(0) % 8 != 0
-                or not self.decays_suit_chunks(self.fixed_decay)
-                or not ops.delta_chunks_supports(self.head_dim, self.value_dim)):
+        if (not self.chunkable or ctx.max_query_len < self.CHUNKS_FROM_TOKENS
+                or qkv.stride(0) % 8 != 0):
             return 0
         if ctx.min_query_len >= self.SHORT_TOKENS:
             return 1 if ctx.n_tokens >= self.CHUNKS_FROM_TOKENS_IN_ALL else 0
@@ -421,9 +423,8 @@ class LinearState(Mixer):
                               n, True,
                               ctx.token_request, ctx.request_slot, ctx.request_start)
         learned = self.fixed_decay is None
-        q, k, v = (qkv[:, begin:end] for begin, end in
-                   ((0, self.qk_width), (self.qk_width, 2 * self.qk_width),
-                    (2 * self.qk_width, self.filtered)))
+        q, k = qkv[:, :self.qk_width], qkv[:, self.qk_width:2 * self.qk_width]
+        v = qkv[:, 2 * self.qk_width:self.filtered]
         state = _state_piece(cache, self.filter_state, self.matrix_state)
         gates = dict(
             decay_in=rows[:, self.decay_at:self.decay_at + self.heads] if learned else None,
