@@ -772,7 +772,7 @@ void paged_attention_stream_kernel(
   bool any_unreadable = false;
 
   // request the copies of the chunk at `ahead` into ring slot `slot`; every lane follows,
-  // lane 0 issues
+  // the elected one issues
   auto request_chunk = [&](int slot) {
     const int first = ahead.block() * pages_per_chunk;
     // keys below this one are outside the row's window or chunk; their pages, unless they hold

@@ -41,6 +41,8 @@
 #include "hx_mma.cuh"
 #include "hx_scan.cuh"
 
+#include <mutex>
+
 namespace {
 
 constexpr int CHUNK = 64;
@@ -724,11 +726,16 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_const
 template <int STEPS>
 int launch_delta(const DeltaArgs& a, int tiles, cudaStream_t stream) {
   const int shared = DeltaLayout(16 * STEPS, a.column_warps).bytes, first = weights_shared(16 * STEPS);
-  if (cudaFuncSetAttribute(delta_weights_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           first) != cudaSuccess ||
-      cudaFuncSetAttribute(delta_states_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           227 * 1024) != cudaSuccess) {
-    cudaGetLastError();
+  static std::once_flag once;
+  static bool configured = false;
+  std::call_once(once, [first] {
+    configured = cudaFuncSetAttribute(delta_weights_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      first) == cudaSuccess &&
+                 cudaFuncSetAttribute(delta_states_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      227 * 1024) == cudaSuccess;
+    if (!configured) cudaGetLastError();
+  });
+  if (!configured) {
     hx_set_error("hx_delta_chunks: the device refuses %d bytes of shared memory", shared);
     return HX_ERR_LAUNCH;
   }

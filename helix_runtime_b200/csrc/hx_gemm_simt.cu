@@ -4,8 +4,9 @@
 // reduced-precision matrix mode; many tokens take hx_gemm_split.cu, whose sums are closer
 // still) and also the bfloat16 path for shapes the tensor
 // core kernel refuses.  Each output element is one sequential sum over k in
-// ascending order, so its value never depends on how many rows the call has or on
-// which tile it falls into.  The reference's counterpart is its 16x16 tiled kernel
+// ascending order, so in this kernel its value never depends on how many rows the call has or
+// on which tile it falls into (a product that hx_gemm_split.cu takes for its many rows is another
+// order of the same sums).  The reference's counterpart is its 16x16 tiled kernel
 // (src/kernels/cuda/matmul.cu:36-71).
 //
 // Prompt portions are bound by the multiply-adds and by the 16-byte loads from shared memory

@@ -28,6 +28,7 @@
 #include "hx_tcgen05.cuh"
 
 #include <cfloat>
+#include <mutex>
 
 namespace {
 
@@ -301,15 +302,16 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
 
 template <int EPI>
 int launch_split(const SplitArgs& a, cudaStream_t stream) {
+  static std::once_flag once;
   static bool configured = false;
+  std::call_once(once, [] {
+    configured = cudaFuncSetAttribute(gemm_split_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      SMEM_BYTES) == cudaSuccess;
+    if (!configured) cudaGetLastError();
+  });
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_split_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_BYTES) !=
-        cudaSuccess) {
-      cudaGetLastError();
-      hx_set_error("hx_gemm_split: cannot reserve %d bytes of shared memory", SMEM_BYTES);
-      return HX_ERR_LAUNCH;
-    }
-    configured = true;
+    hx_set_error("hx_gemm_split: cannot reserve %d bytes of shared memory", SMEM_BYTES);
+    return HX_ERR_LAUNCH;
   }
   const dim3 grid((a.tokens + TILE - 1) / TILE, (a.features + TILE - 1) / TILE);
   hx_launch(gemm_split_kernel<EPI>, grid, THREADS, SMEM_BYTES, stream, a);

@@ -362,17 +362,18 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_run
 
 template <bool GATED>
 int launch_runs(const CUtensorMap& map_w, const TokenMaps& map_x, const RunsArgs& args, cudaStream_t stream) {
+  static std::once_flag once;
   static bool configured = false;
   const int sms = hx_device_sm_count();
   if (sms <= 0) return HX_ERR_LAUNCH;
+  std::call_once(once, [] {
+    configured = cudaFuncSetAttribute(gemm_tc_runs_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      SMEM_BYTES) == cudaSuccess;
+    if (!configured) cudaGetLastError();
+  });
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_runs_kernel<GATED>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                             SMEM_BYTES) != cudaSuccess) {
-      hx_set_error("hx_gemm_tc_runs: cannot reserve %d bytes of shared memory", SMEM_BYTES);
-      cudaGetLastError();
-      return HX_ERR_LAUNCH;
-    }
-    configured = true;
+    hx_set_error("hx_gemm_tc_runs: cannot reserve %d bytes of shared memory", SMEM_BYTES);
+    return HX_ERR_LAUNCH;
   }
   hx_launch(gemm_tc_runs_kernel<GATED>, 2 * (sms / 2), THREADS, SMEM_BYTES, stream, map_w, map_x, args);
   return HX_OK;
