@@ -26,6 +26,7 @@
 // Every wait on an mbarrier is bounded; a wait that runs out sets a status bit, the CTA skips its
 // remaining work, frees its tensor memory and returns.
 #include "hx_tcgen05.cuh"
+#include "hx_tensor_map.cuh"
 
 #include <cfloat>
 #include <mutex>
@@ -56,6 +57,9 @@ constexpr int TMEM_COLUMNS = 2 * TILE;
 constexpr float OPERAND_SCALE = 65536.0f, SUM_SCALE = 1.0f / (OPERAND_SCALE * OPERAND_SCALE);
 constexpr int SMEM_BYTES = STAGES * STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
 
+// The products of a block, term of x and term of w: the smallest first.
+__device__ constexpr int TERM_OF_X[6] = {2, 0, 1, 1, 0, 0}, TERM_OF_W[6] = {0, 2, 1, 0, 1, 0};
+
 struct SplitArgs {
   const float* x;
   int ldx;
@@ -78,8 +82,8 @@ __device__ __forceinline__ void leave(uint32_t terms, float& a, float& b) {
   b -= __uint_as_float(terms & 0xffff0000u);
 }
 
-// The terms of four numbers, 8 bytes each, to `at` in the three matrices of terms.
-__device__ __forceinline__ void store_terms(uint8_t* at, float4 v) {
+// The terms of four numbers, 8 bytes each, to `at` in the three matrices of terms, term_bytes apart.
+__device__ __forceinline__ void store_terms(uint8_t* at, float4 v, size_t term_bytes = TERM_BYTES) {
   asm("{\n\t.reg .b64 s, p, q;\n\t"
       "mov.b64 s, {%4, %4};\n\tmov.b64 p, {%0, %1};\n\tmov.b64 q, {%2, %3};\n\t"
       "mul.rn.f32x2 p, p, s;\n\tmul.rn.f32x2 q, q, s;\n\t"
@@ -89,7 +93,7 @@ __device__ __forceinline__ void store_terms(uint8_t* at, float4 v) {
 #pragma unroll
   for (int term = 0; term < 3; ++term) {
     const uint2 packed = make_uint2(two_terms(v.x, v.y), two_terms(v.z, v.w));
-    *reinterpret_cast<uint2*>(at + term * TERM_BYTES) = packed;
+    *reinterpret_cast<uint2*>(at + term * term_bytes) = packed;
     leave(packed.x, v.x, v.y);
     leave(packed.y, v.z, v.w);
   }
@@ -100,6 +104,46 @@ __device__ __noinline__ float chained_sum(const float* x, const float* w, int de
   float sum = 0.0f;
   for (int k = 0; k < depth && !isnan(sum); ++k) sum = fmaf(x[k], w[k], sum);
   return sum;
+}
+
+// A summing thread's columns to the output (or added to it).
+template <int EPI>
+__device__ __forceinline__ void write_sums(const SplitArgs& a, float (&sum)[COLUMNS], int token, int column0) {
+  const int live = min(COLUMNS, a.features - column0);
+  if (token >= a.tokens || live <= 0) return;
+  float* out = a.out + static_cast<size_t>(token) * a.ldo + column0;
+  const bool wide = a.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && live == COLUMNS;
+#pragma unroll
+  for (int j = 0; j < COLUMNS; ++j)
+    if (!(fabsf(sum[j]) <= FLT_MAX) && j < live)
+      sum[j] = chained_sum(a.x + static_cast<size_t>(token) * a.ldx,
+                           a.w + static_cast<size_t>(column0 + j) * a.ldw, a.depth);
+  if (EPI == EPI_STORE_F32 && a.softcap > 0.0f) {
+#pragma unroll
+    for (int j = 0; j < COLUMNS; ++j) sum[j] = a.softcap * tanhf(sum[j] / a.softcap);
+  }
+  if (wide) {
+#pragma unroll
+    for (int j = 0; j < COLUMNS; j += 4) {
+      float4 v = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
+      if (EPI == EPI_ADD_F32) {
+        const float4 old = *reinterpret_cast<const float4*>(out + j);
+        v.x += old.x;
+        v.y += old.y;
+        v.z += old.z;
+        v.w += old.w;
+      }
+      *reinterpret_cast<float4*>(out + j) = v;
+    }
+  } else {
+#pragma unroll
+    for (int j = 0; j < COLUMNS; ++j) {
+      if (j < live) {
+        if (EPI == EPI_ADD_F32) out[j] += sum[j];
+        else out[j] = sum[j];
+      }
+    }
+  }
 }
 
 template <int EPI>
@@ -153,12 +197,10 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
     constexpr uint32_t idesc = make_idesc(TILE, TILE);
     const uint32_t stage = smem_u32(smem + s * STAGE_BYTES);
     const uint32_t sums = tmem_base + buffer * TILE;
-    // term of x, term of w: the smallest products first
-    constexpr int X[6] = {2, 0, 1, 1, 0, 0}, W[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
     for (int i = 0; i < 6; ++i) {
-      const uint64_t desc_x = make_smem_desc(stage + X[i] * TERM_BYTES);
-      const uint64_t desc_w = make_smem_desc(stage + (3 + W[i]) * TERM_BYTES);
+      const uint64_t desc_x = make_smem_desc(stage + TERM_OF_X[i] * TERM_BYTES);
+      const uint64_t desc_w = make_smem_desc(stage + (3 + TERM_OF_W[i]) * TERM_BYTES);
 #pragma unroll
       for (int k = 0; k < BK / UMMA_K; ++k) {
         const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
@@ -253,43 +295,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
       __syncwarp();
       if (lane == 0) mbar_arrive(&sum_empty_bar[buffer]);
     }
-    const int token = token0 + quarter * 32 + lane, column0 = feature0 + half * COLUMNS;
-    const int live = min(COLUMNS, a.features - column0);
-    if (ok && token < a.tokens && live > 0) {
-      float* out = a.out + static_cast<size_t>(token) * a.ldo + column0;
-      const bool wide = a.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(a.out) & 15) == 0 && live == COLUMNS;
-#pragma unroll
-      for (int j = 0; j < COLUMNS; ++j)
-        if (!(fabsf(sum[j]) <= FLT_MAX) && j < live)
-          sum[j] = chained_sum(a.x + static_cast<size_t>(token) * a.ldx,
-                               a.w + static_cast<size_t>(column0 + j) * a.ldw, a.depth);
-      if (EPI == EPI_STORE_F32 && a.softcap > 0.0f) {
-#pragma unroll
-        for (int j = 0; j < COLUMNS; ++j) sum[j] = a.softcap * tanhf(sum[j] / a.softcap);
-      }
-      if (wide) {
-#pragma unroll
-        for (int j = 0; j < COLUMNS; j += 4) {
-          float4 v = make_float4(sum[j], sum[j + 1], sum[j + 2], sum[j + 3]);
-          if (EPI == EPI_ADD_F32) {
-            const float4 old = *reinterpret_cast<const float4*>(out + j);
-            v.x += old.x;
-            v.y += old.y;
-            v.z += old.z;
-            v.w += old.w;
-          }
-          *reinterpret_cast<float4*>(out + j) = v;
-        }
-      } else {
-#pragma unroll
-        for (int j = 0; j < COLUMNS; ++j) {
-          if (j < live) {
-            if (EPI == EPI_ADD_F32) out[j] += sum[j];
-            else out[j] = sum[j];
-          }
-        }
-      }
-    }
+    if (ok) write_sums<EPI>(a, sum, token0 + quarter * 32 + lane, feature0 + half * COLUMNS);
   }
 
   tc_fence_before();
@@ -300,18 +306,294 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
   }
 }
 
+// ------------------------------------------------------------------ many tokens: pairs of CTAs
+//
+// Above, every tile cuts its tokens again, for each of its 128 features once: with 512 tokens by [17,280 x
+// 3,200] the conversion of the tokens is done 135 times.  Here split_cut_kernel cuts the tokens once (6 bytes a
+// number to scratch, which the copy engine brings in swizzled), and two CTAs share a tile of 256 tokens by 128
+// features (tcgen05.mma.cta_group::2): each cuts 64 of the weight rows a block, a quarter of the numbers that a
+// CTA above cuts for as many products.  Two groups of four warps cut alternate blocks, so a group's loads
+// have two blocks' time to arrive.  Persistent: the ring of stages runs on from tile to tile, and the next
+// tile's first products run while this one's sums are stored.  Sums of four blocks lie in tensor memory, so
+// that the summing warps' round trip is hidden.  The sums are those of the kernel above, bit for bit.
+//
+// Measured (us, that kernel and this one with its cut): 512 tokens by [17,280 x 3,200] 434 -> 251, by [3,200 x
+// 8,640] 287 -> 156.  A block takes 2,300 cycles, its products 1,540 of them; with one product of six 2,000: the
+// ring of three stages (72 KB each) hardly covers the tokens' way from the L2, 48 KB a block and CTA.
+// Slower: arrivals at the leader's barriers that release all memory (349 us, see mbar_arrive_pair), two
+// blocks of weights on their way in registers (318), all eight warps on one block (296), terms kept in registers
+// until their stage is free (255 to 282), sums of two blocks (257).
+constexpr int PAIR_TOKENS = 2 * TILE;
+constexpr int PAIR_ROWS = TILE / 2;                     // weight rows of a CTA
+constexpr int PAIR_X_BYTES = TILE * BK * 2, PAIR_W_BYTES = PAIR_ROWS * BK * 2;      // a term
+constexpr int PAIR_STAGE_BYTES = 3 * (PAIR_X_BYTES + PAIR_W_BYTES);
+constexpr int PAIR_STAGES = 3;
+#ifndef GROUPS
+#define GROUPS 2
+#endif
+constexpr int PAIR_BUFFERS = 4;                         // of a block's sums
+constexpr int PAIR_TMEM_COLUMNS = PAIR_BUFFERS * TILE;
+constexpr int PAIR_GROUPS = GROUPS, PAIR_GROUP_WARPS = 8 / PAIR_GROUPS;
+constexpr int PAIR_TMA_WARP = SUM_WARPS + PAIR_GROUPS * PAIR_GROUP_WARPS, PAIR_MMA_WARP = PAIR_TMA_WARP + 1;
+constexpr int PAIR_THREADS = 32 * (PAIR_TMA_WARP + 4);      // whole warpgroups, whose registers are dealt anew
+// At launch 96 a thread; those that issue copies and products need few, the others take what they leave.
+constexpr int PAIR_REGISTERS = 96, PAIR_WORK_REGISTERS = 112, PAIR_ISSUE_REGISTERS = 32;
+static_assert((PAIR_THREADS / 128 - 1) * PAIR_WORK_REGISTERS + PAIR_ISSUE_REGISTERS <=
+                  PAIR_THREADS / 128 * PAIR_REGISTERS,
+              "what one side takes the other has given back");
+constexpr int PAIR_PASS_ROWS = 32 * PAIR_GROUP_WARPS / (BK / 4), PAIR_PASSES = PAIR_ROWS / PAIR_PASS_ROWS;
+constexpr int PAIR_SMEM_BYTES = PAIR_STAGES * PAIR_STAGE_BYTES + 1024 /*alignment*/ + 256 /*barriers*/;
+
+// x [tokens, depth] as three matrices of terms [tokens, ldt], zeros behind the depth.
+constexpr int CUT_THREADS = 256;
+__global__ __launch_bounds__(CUT_THREADS) void split_cut_kernel(const float* x, int ldx, __nv_bfloat16* terms,
+                                                                int ldt, int tokens, int depth) {
+  hx_pdl_prologue();
+  const int pieces = ldt / 4;
+  const size_t term_bytes = static_cast<size_t>(tokens) * ldt * 2;
+  for (int token = blockIdx.y; token < tokens; token += gridDim.y) {
+    const int piece = blockIdx.x * CUT_THREADS + threadIdx.x;
+    if (piece >= pieces) continue;
+    const float4 v = 4 * piece < depth
+                         ? *reinterpret_cast<const float4*>(x + static_cast<size_t>(token) * ldx + 4 * piece)
+                         : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    store_terms(reinterpret_cast<uint8_t*>(terms + static_cast<size_t>(token) * ldt + 4 * piece), v, term_bytes);
+  }
+}
+
 template <int EPI>
-int launch_split(const SplitArgs& a, cudaStream_t stream) {
+__global__ __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) void gemm_split_pair_kernel(
+    const __grid_constant__ CUtensorMap map_terms, const SplitArgs a) {
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>(
+      (reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~static_cast<uintptr_t>(1023));
+  uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + PAIR_STAGES * PAIR_STAGE_BYTES);      // leader's count
+  uint64_t* empty_bar = full_bar + PAIR_STAGES;
+  uint64_t* sum_full_bar = empty_bar + PAIR_STAGES;
+  uint64_t* sum_empty_bar = sum_full_bar + PAIR_BUFFERS;      // leader's count
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(sum_empty_bar + PAIR_BUFFERS);
+  volatile int* failed = reinterpret_cast<volatile int*>(tmem_holder + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(cluster_rank());
+  const int worker = blockIdx.x >> 1, workers = gridDim.x >> 1;
+  const int blocks = (a.depth + BK - 1) / BK;
+  const int token_tiles = (a.tokens + PAIR_TOKENS - 1) / PAIR_TOKENS;
+  const int units = token_tiles * ((a.features + TILE - 1) / TILE);
+  const int own_units = worker < units ? (units - worker - 1) / workers + 1 : 0;
+  const int fills = own_units * blocks;      // blocks of all its tiles
+  // the tile that the i-th of them is, the tokens of a feature tile one after the other
+  auto tile_at = [&](int i, int& token0, int& feature0) {
+    const int unit = worker + i * workers;
+    token0 = unit % token_tiles * PAIR_TOKENS + rank * TILE;
+    feature0 = unit / token_tiles * TILE;
+  };
+  hx_pdl_trigger();
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < PAIR_STAGES; ++s) {
+      mbar_init(&full_bar[s], 1 + 2 * PAIR_GROUP_WARPS);
+      mbar_init(&empty_bar[s], 1);
+    }
+    for (int b = 0; b < PAIR_BUFFERS; ++b) {
+      mbar_init(&sum_full_bar[b], 1);
+      mbar_init(&sum_empty_bar[b], 2 * SUM_WARPS);
+    }
+    *failed = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  if (warp == PAIR_MMA_WARP) tmem_alloc_pair(tmem_holder, PAIR_TMEM_COLUMNS);
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // nothing arrives at the other CTA's barriers before they are there
+  tc_fence_after();
+  const uint32_t tmem_base = *tmem_holder;
+  auto give_up = [&]() {
+    atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
+    *failed = 1;
+  };
+
+  if (warp < SUM_WARPS) {
+    // ------------------------------------------------------- sums of the blocks, and the epilogue
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PAIR_WORK_REGISTERS));
+    hx_pdl_wait();
+    const int quarter = warp & 3, half = warp >> 2;
+    const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + half * COLUMNS;
+    uint32_t block = 0;
+    bool ok = true;
+    for (int i = 0; i < own_units && ok; ++i) {
+      float sum[COLUMNS];
+#pragma unroll
+      for (int j = 0; j < COLUMNS; ++j) sum[j] = 0.0f;
+      for (int kb = 0; kb < blocks; ++kb, ++block) {
+        const int buffer = block % PAIR_BUFFERS;
+        if (lane == 0) ok = !*failed && mbar_wait(&sum_full_bar[buffer], (block / PAIR_BUFFERS) & 1u);
+        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+        if (!ok) {
+          if (lane == 0) give_up();
+          break;
+        }
+        tc_fence_after();
+#pragma unroll
+        for (int column = 0; column < COLUMNS; column += 32) {
+          uint32_t v[2][16];
+          tmem_load16_issue(lane_base + buffer * TILE + column, v[0]);
+          tmem_load16_issue(lane_base + buffer * TILE + column + 16, v[1]);
+          tmem_load_wait();
+#pragma unroll
+          for (int j = 0; j < 32; ++j)
+            sum[column + j] = fmaf(__uint_as_float(v[j / 16][j % 16]), SUM_SCALE, sum[column + j]);
+        }
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive_pair(cluster_address(&sum_empty_bar[buffer], 0));
+      }
+      int token0, feature0;
+      tile_at(i, token0, feature0);
+      if (ok) write_sums<EPI>(a, sum, token0 + quarter * 32 + lane, feature0 + half * COLUMNS);
+    }
+  } else if (warp < PAIR_TMA_WARP) {
+    // -------------------------------- weights (no kernel of a step writes them: no wait for the one before)
+    asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(PAIR_WORK_REGISTERS));
+    const int thread = (threadIdx.x - 32 * SUM_WARPS) % (32 * PAIR_GROUP_WARPS);
+    const int piece = thread % (BK / 4), row0 = thread / (BK / 4);
+    float4 v[PAIR_PASSES];
+    auto load = [&](int fill) {
+      int token0, feature0;
+      tile_at(fill / blocks, token0, feature0);
+      const int first = feature0 + rank * PAIR_ROWS, k = fill % blocks * BK + 4 * piece;
+      const float* from = a.w + static_cast<size_t>(first) * a.ldw + k;
+#pragma unroll
+      for (int p = 0; p < PAIR_PASSES; ++p) {
+        const int row = row0 + PAIR_PASS_ROWS * p;
+        v[p] = k < a.depth && first + row < a.features      // the depth is a multiple of four
+                   ? *reinterpret_cast<const float4*>(from + static_cast<size_t>(row) * a.ldw)
+                   : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+      }
+    };
+    int fill = (warp - SUM_WARPS) / PAIR_GROUP_WARPS;
+    if (fill < fills) load(fill);
+    for (; fill < fills; fill += PAIR_GROUPS) {
+      const int s = fill % PAIR_STAGES;
+      bool ok = true;
+      if (lane == 0) ok = !*failed && mbar_wait(&empty_bar[s], ((fill / PAIR_STAGES) & 1u) ^ 1u);
+      ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+      if (!ok) {
+        if (lane == 0) give_up();
+        break;
+      }
+      uint8_t* terms = smem + s * PAIR_STAGE_BYTES + 3 * PAIR_X_BYTES;
+#pragma unroll
+      for (int p = 0; p < PAIR_PASSES; ++p) {
+        const int row = row0 + PAIR_PASS_ROWS * p;
+        store_terms(terms + row * (BK * 2) + (((piece >> 1) ^ (row & 7)) << 4) + ((piece & 1) << 3), v[p],
+                    PAIR_W_BYTES);
+      }
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) mbar_arrive_pair(cluster_address(&full_bar[s], 0));
+      if (fill + PAIR_GROUPS < fills) load(fill + PAIR_GROUPS);
+    }
+  } else {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(PAIR_ISSUE_REGISTERS));
+    if (warp == PAIR_TMA_WARP) {
+      // ------------------------------------------------------------------ the tokens' terms
+      hx_pdl_wait();
+      if (hx_elect_one()) {
+        int fill = 0;
+        for (int i = 0; i < own_units && !*failed; ++i) {
+          int token0, feature0;
+          tile_at(i, token0, feature0);
+          for (int kb = 0; kb < blocks; ++kb, ++fill) {
+            const int s = fill % PAIR_STAGES;
+            if (!mbar_wait(&empty_bar[s], ((fill / PAIR_STAGES) & 1u) ^ 1u)) {
+              give_up();
+              break;
+            }
+            if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * 3 * PAIR_X_BYTES);
+            const uint32_t bar = cluster_address(&full_bar[s], 0);
+  #pragma unroll
+            for (int term = 0; term < 3; ++term)
+              tma_load_2d_pair(smem + s * PAIR_STAGE_BYTES + term * PAIR_X_BYTES, &map_terms, bar, kb * BK,
+                               term * a.tokens + token0);
+          }
+        }
+        // the leader's last arrivals at this CTA's barriers, before the CTA may end
+        for (int last = fill > PAIR_STAGES ? fill - PAIR_STAGES : 0; last < fill && !*failed; ++last)
+          if (!mbar_wait(&empty_bar[last % PAIR_STAGES], (last / PAIR_STAGES) & 1u)) give_up();
+      }
+    } else if (warp == PAIR_MMA_WARP && rank == 0 && hx_elect_one()) {
+      // ---------------------------------------------------------------- products, for both CTAs
+      constexpr uint32_t idesc = make_idesc(PAIR_TOKENS, TILE);
+      for (int fill = 0; fill < fills && !*failed; ++fill) {
+        const int s = fill % PAIR_STAGES, buffer = fill % PAIR_BUFFERS;
+        if (!mbar_wait(&sum_empty_bar[buffer], ((fill / PAIR_BUFFERS) & 1u) ^ 1u) ||
+            !mbar_wait(&full_bar[s], (fill / PAIR_STAGES) & 1u)) {
+          give_up();
+          break;
+        }
+        tc_fence_after();
+        const uint32_t stage = smem_u32(smem + s * PAIR_STAGE_BYTES);
+        const uint32_t sums = tmem_base + buffer * TILE;
+  #pragma unroll
+        for (int i = 0; i < 6; ++i) {
+          const uint64_t desc_x = make_smem_desc(stage + TERM_OF_X[i] * PAIR_X_BYTES);
+          const uint64_t desc_w = make_smem_desc(stage + 3 * PAIR_X_BYTES + TERM_OF_W[i] * PAIR_W_BYTES);
+  #pragma unroll
+          for (int k = 0; k < BK / UMMA_K; ++k) {
+            const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
+            umma_bf16_pair(sums, desc_x + step, desc_w + step, idesc, i > 0 || k > 0 ? 1u : 0u);
+          }
+        }
+        umma_commit_pair(&empty_bar[s]);
+        umma_commit_pair(&sum_full_bar[buffer]);
+      }
+    }
+  }
+
+  tc_fence_before();
+  __syncthreads();
+  cluster_sync();      // neither CTA's memory is read or arrived at any more
+  if (warp == PAIR_MMA_WARP) {
+    tc_fence_after();
+    tmem_dealloc_pair(tmem_base, PAIR_TMEM_COLUMNS);
+  }
+}
+
+// Numbers of a row of terms: rows of a tensor map begin on 16 bytes.
+int terms_row(int depth) { return (depth + 7) / 8 * 8; }
+
+template <int EPI>
+int launch_split(const SplitArgs& a, __nv_bfloat16* terms, cudaStream_t stream) {
   static std::once_flag once;
   static bool configured = false;
   std::call_once(once, [] {
     configured = cudaFuncSetAttribute(gemm_split_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      SMEM_BYTES) == cudaSuccess;
+                                      SMEM_BYTES) == cudaSuccess &&
+                 cudaFuncSetAttribute(gemm_split_pair_kernel<EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                      PAIR_SMEM_BYTES) == cudaSuccess;
     if (!configured) cudaGetLastError();
   });
   if (!configured) {
     hx_set_error("hx_gemm_split: cannot reserve %d bytes of shared memory", SMEM_BYTES);
     return HX_ERR_LAUNCH;
+  }
+  const int pairs = hx_device_sm_count() / 2;
+  const long long units = static_cast<long long>((a.tokens + PAIR_TOKENS - 1) / PAIR_TOKENS) *
+                          ((a.features + TILE - 1) / TILE);
+  // (a pair counts its blocks in 32 bits, a tensor map the rows of all three terms)
+  if (terms != nullptr && (units / pairs + 1) * ((a.depth + BK - 1) / BK) < (1ll << 30) && a.tokens < (1 << 29)) {
+    const int ldt = terms_row(a.depth);
+    CUtensorMap map;
+    const int rc = hx_tensor_map("hx_gemm_split", terms, 3ull * a.tokens, ldt, ldt, TILE, BK, true, &map);
+    if (rc != HX_OK) return rc;
+    const int piece_blocks = (ldt / 4 + CUT_THREADS - 1) / CUT_THREADS;
+    hx_launch(split_cut_kernel, dim3(piece_blocks, a.tokens < 65535 ? a.tokens : 65535), CUT_THREADS, 0, stream,
+              a.x, a.ldx, terms, ldt, a.tokens, a.depth);
+    HX_CHECK_LAUNCH("hx_gemm_split (terms)");
+    hx_launch(gemm_split_pair_kernel<EPI>, 2 * static_cast<int>(units < pairs ? units : pairs), PAIR_THREADS,
+              PAIR_SMEM_BYTES, stream, map, a);
+    return HX_OK;
   }
   const dim3 grid((a.tokens + TILE - 1) / TILE, (a.features + TILE - 1) / TILE);
   hx_launch(gemm_split_kernel<EPI>, grid, THREADS, SMEM_BYTES, stream, a);
@@ -336,9 +618,17 @@ HX_API int hx_gemm_split_pays(int tokens, int features) {
   return tokens > 16 && small >= 2ll * hx_device_sm_count();
 }
 
+// Numbers of bfloat16 scratch (on 16 bytes) with which hx_gemm_split_scratch is the faster road, 0 where it has
+// no use for any: a tile of 128 tokens that are fewer is for the kernel that cuts its own.
+HX_API long long hx_gemm_split_terms(int tokens, int depth) {
+  return tokens > TILE && hx_device_sm_count() >= 2 ? 3ll * tokens * terms_row(depth) : 0;
+}
+
 // float32 x [tokens, ldx], w [features, ldw], out [tokens, ldo]; epilogues and softcap as hx_gemm_simt_softcapped.
-HX_API int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
-                         int features, int depth, int epilogue, float softcap, int* status, cudaStream_t stream) {
+// `terms`: scratch of hx_gemm_split_terms() numbers, or null.
+HX_API int hx_gemm_split_scratch(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
+                                 int features, int depth, int epilogue, float softcap, void* terms,
+                                 long long terms_size, int* status, cudaStream_t stream) {
   HX_REQUIRE(tokens >= 0 && features > 0 && depth > 0, "hx_gemm_split: bad sizes");
   HX_REQUIRE(softcap >= 0.0f && (softcap == 0.0f || epilogue == EPI_STORE_F32),
              "hx_gemm_split: a softcap belongs to a float32 store");
@@ -347,12 +637,19 @@ HX_API int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float
              "hx_gemm_split: rows of %d and %d for a depth of %d are not supported", ldx, ldw, depth);
   HX_REQUIRE(status != nullptr, "hx_gemm_split: status word missing");
   if (tokens == 0) return HX_OK;
+  __nv_bfloat16* cut = nullptr;
+  const long long needed = hx_gemm_split_terms(tokens, depth);
+  if (terms != nullptr && needed > 0) {
+    HX_REQUIRE(terms_size >= needed && (reinterpret_cast<uintptr_t>(terms) & 15) == 0,
+               "hx_gemm_split: scratch of %lld numbers for %lld, or not on 16 bytes", terms_size, needed);
+    cut = static_cast<__nv_bfloat16*>(terms);
+  }
   const SplitArgs a{x, ldx, w, ldw, out, ldo, tokens, features, depth, softcap, status};
   int rc;
   switch (epilogue) {
-    case EPI_STORE: rc = launch_split<EPI_STORE>(a, stream); break;
-    case EPI_STORE_F32: rc = launch_split<EPI_STORE_F32>(a, stream); break;
-    case EPI_ADD_F32: rc = launch_split<EPI_ADD_F32>(a, stream); break;
+    case EPI_STORE: rc = launch_split<EPI_STORE>(a, cut, stream); break;
+    case EPI_STORE_F32: rc = launch_split<EPI_STORE_F32>(a, cut, stream); break;
+    case EPI_ADD_F32: rc = launch_split<EPI_ADD_F32>(a, cut, stream); break;
     default:
       hx_set_error("hx_gemm_split: unknown epilogue %d", epilogue);
       return HX_ERR_ARGUMENT;
@@ -360,4 +657,10 @@ HX_API int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_gemm_split");
   return HX_OK;
+}
+
+HX_API int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
+                         int features, int depth, int epilogue, float softcap, int* status, cudaStream_t stream) {
+  return hx_gemm_split_scratch(x, ldx, w, ldw, out, ldo, tokens, features, depth, epilogue, softcap, nullptr, 0,
+                               status, stream);
 }

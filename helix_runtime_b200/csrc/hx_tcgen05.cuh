@@ -129,6 +129,14 @@ __device__ __forceinline__ void mbar_arrive_cluster(uint32_t bar) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
 }
 
+// An arrival that orders no more than this CTA's own shared memory (or tensor memory, behind its fence) before
+// it: what the products of a pair read, each SM from its own.  The one above waits for all memory that
+// the thread has written or read, about a microsecond (float32 products of 512 tokens by [17,280 x 3,200],
+// three such arrivals a block: 349 us against 284).
+__device__ __forceinline__ void mbar_arrive_pair(uint32_t bar) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(bar) : "memory");
+}
+
 // mbar_wait for a barrier that threads of the other CTA arrive at.
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity) {
   const uint32_t addr = smem_u32(bar);

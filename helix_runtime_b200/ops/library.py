@@ -319,7 +319,13 @@ def _declare(library: ctypes.CDLL) -> None:
     library.hx_gemm_split_pays.argtypes = [_c_int, _c_int]
     library.hx_gemm_split.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int,
                                       _c_int, _c_int, _c_float, _c_ptr, _c_ptr]
-    for name in ("hx_gemm_split_supports", "hx_gemm_split_pays", "hx_gemm_split"):
+    library.hx_gemm_split_scratch.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int,
+                                              _c_int, _c_int, _c_int, _c_float, _c_ptr, _c_longlong,
+                                              _c_ptr, _c_ptr]
+    library.hx_gemm_split_terms.argtypes = [_c_int, _c_int]
+    library.hx_gemm_split_terms.restype = _c_longlong
+    for name in ("hx_gemm_split_supports", "hx_gemm_split_pays", "hx_gemm_split",
+                 "hx_gemm_split_scratch"):
         getattr(library, name).restype = _c_int
     library.hx_gemm_tc_ordered.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr,
                                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr]
@@ -645,18 +651,31 @@ def gemm_split_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens
                                                   w.shape[0], w.shape[1])))
 
 
+def gemm_split_terms(tokens: int, depth: int) -> int:
+    """bfloat16 numbers of scratch that :func:`gemm_split` has a use for."""
+    return int(lib().hx_gemm_split_terms(tokens, depth))
+
+
 def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, epilogue: int,
-               status: torch.Tensor, softcap: float = 0.0) -> None:
+               status: torch.Tensor, softcap: float = 0.0,
+               terms: Optional[torch.Tensor] = None) -> None:
     """:func:`gemm_simt` for many float32 tokens, on the tensor cores: both operands as three
     bfloat16 terms, 24 bits, sums of 64 products added in float32.  Closer to the sum of 64 bits than
-    the chain of multiply-adds; like that one, the same from call to call."""
+    the chain of multiply-adds; like that one, the same from call to call.  ``terms``: contiguous
+    scratch of :func:`gemm_split_terms` numbers (allocated here if there is none)."""
     for tensor, name in ((x, "x"), (w, "w"), (out, "out")):
         _need(tensor, torch.float32, name)
     assert x.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1
     features, depth = w.shape
-    _check(lib().hx_gemm_split(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
-                               out.stride(0), tokens, features, depth, epilogue, float(softcap),
-                               status.data_ptr(), _stream()))
+    if terms is None:
+        size = gemm_split_terms(tokens, depth)
+        terms = torch.empty(size, dtype=torch.bfloat16, device=x.device) if size > 0 else None
+    else:
+        _need(terms, torch.bfloat16, "terms")
+    _check(lib().hx_gemm_split_scratch(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
+                                       out.data_ptr(), out.stride(0), tokens, features, depth, epilogue,
+                                       float(softcap), _ptr(terms), 0 if terms is None else terms.numel(),
+                                       status.data_ptr(), _stream()))
 
 
 WEIGHT_TILE_ROWS, WEIGHT_TILE_DEPTH = 128, 64

@@ -319,7 +319,7 @@ class PagedAttention(Mixer):
         else:
             raw = ctx.workspace.get(f"attention.projected/{self.projected_size}",
                                     (ctx.capacity, self.projected_size), ctx.dtype)
-            project(x, self.w_qkv, raw, n, ops.EPI_STORE, ctx.status)
+            project(x, self.w_qkv, raw, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
         ops.short_conv_append(raw, accumulator, qkv, self.conv_filter, cache.state, ctx.positions,
                               ctx.token_request, ctx.request_slot, ctx.request_start,
                               cache.block_tables if appends else None,
@@ -431,7 +431,7 @@ class PagedAttention(Mixer):
             self.position.apply(ctx, cache, qkv, self.heads, self.kv_heads, accum=accumulator)
         elif not self.position.project_and_apply(ctx, cache, x, self.w_qkv, qkv, self.heads,
                                                  self.kv_heads):
-            project(x, self.w_qkv, qkv, n, ops.EPI_STORE, ctx.status)
+            project(x, self.w_qkv, qkv, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
             self.position.apply(ctx, cache, qkv, self.heads, self.kv_heads)
 
         self.attend(ctx, cache, qkv, context)
@@ -444,11 +444,12 @@ class PagedAttention(Mixer):
             else:
                 gate = ctx.workspace.get(f"attention.gate/{self.q_size}",
                                          (ctx.capacity, self.q_size), ctx.dtype)
-                project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status)
+                project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
             ops.sigmoid_gate(context, gate, n, self.q_size, clear=uncleared)
         elif uncleared is not None:
             uncleared[:n].zero_()
-        project(context, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(context, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class NormedProjectionAttention(PagedAttention):
@@ -589,7 +590,8 @@ class NormedProjectionAttention(PagedAttention):
         else:
             projected = get(f"attention.projected_sums/{self.projected_size}",
                             (ctx.capacity, self.projected_size), torch.float32)
-            project(x, self.w_proj, projected, n, ops.EPI_STORE_F32, ctx.status)
+            project(x, self.w_proj, projected, n, ops.EPI_STORE_F32, ctx.status,
+                    workspace=ctx.workspace)
             clear = False
         ops.biased_normed_rows(projected, clear, qkv, n, self.heads, self.kv_heads, self.head_dim,
                                self.value_dim, self.row_dim, ctx.positions, q_bias=self.q_bias,
@@ -608,7 +610,8 @@ class NormedProjectionAttention(PagedAttention):
         self.attend(ctx, cache, qkv, context)
         if self.head_gated:
             ops.head_gate(context, gates, n, self.heads, self.row_dim)
-        project(context, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(context, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class LatentAttention(PagedAttention):
@@ -756,12 +759,12 @@ class LatentAttention(PagedAttention):
         rows = get(f"latent.rows/{self.rows_size}", (ctx.capacity, self.rows_size), ctx.dtype)
         context = get(f"attention.context/{self.q_size}", (ctx.capacity, self.q_size), ctx.dtype)
         heads_out = get(f"latent.heads/{self.o_columns}", (ctx.capacity, self.o_columns), ctx.dtype)
-        project(x, self.w_down, down, n, ops.EPI_STORE_F32, ctx.status)
+        project(x, self.w_down, down, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
         ops.latent_prepare(down, self.q_norm, self.kv_norm, self.eps, ctx.positions, self.freq,
                            self.freq_exact, self.rotary_dims, self.rotary_layout, latent, rows,
                            self.q_size, n, self.q_rank, self.kv_rank, self.rotated_dim,
                            self.row_dim, amplitude=self.amplitude)
-        project(latent, self.w_q_up, q, n, ops.EPI_STORE, ctx.status)
+        project(latent, self.w_q_up, q, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
         # [Uk_h' q_h | rot(qr_h) | 0] per head
         ops.head_products(q, self.plain_dim, self.w_k_up, rows, self.row_dim, n, ctx.status)
         ops.latent_queries(q, self.heads * self.plain_dim, rows, ctx.positions, self.freq,
@@ -779,9 +782,10 @@ class LatentAttention(PagedAttention):
                           ctx.status)
         if self.gated:
             gate = get(f"attention.gate/{self.o_columns}", (ctx.capacity, self.o_columns), ctx.dtype)
-            project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status)
+            project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
             ops.sigmoid_gate(heads_out, gate, n, self.o_columns)
-        project(heads_out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(heads_out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class DifferentialAttention(PagedAttention):
@@ -940,7 +944,8 @@ class DifferentialAttention(PagedAttention):
         else:
             size = -(-self.projected_size // 8) * 8
             projected = get(f"attention.projected/{size}", (ctx.capacity, size), ctx.dtype)
-            project(x, self.w_proj, projected, n, ops.EPI_STORE, ctx.status)
+            project(x, self.w_proj, projected, n, ops.EPI_STORE, ctx.status,
+                    workspace=ctx.workspace)
         table = self.table
         write = not self.shared_cache
         ops.filtered_heads(projected, sums, rows, self.taps_weight, self.biases,
@@ -960,7 +965,8 @@ class DifferentialAttention(PagedAttention):
                            clear=used if sums else None)
         if self.o_bias is not None and not bias_in_place:
             ops.add_bias(residual, self.o_bias, n)
-        project(heads_out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(heads_out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 register_part("mixer", "paged_attention", PagedAttention)

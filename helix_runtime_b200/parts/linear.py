@@ -76,13 +76,15 @@ def _gemm_tc(x, w: Weight, out, tokens, features, epilogue, status, **options) -
 
 
 def _gemm_simt(x, w: Weight, out, tokens, epilogue, status, softcap: float = 0.0,
-               features: Optional[int] = None) -> None:
+               features: Optional[int] = None, workspace=None) -> None:
     if w.matrix is None:
         raise RuntimeError("this product needs the CUDA-core kernel, but the weight is held as "
                            "tiles for the tensor cores")
     matrix = w.matrix if features is None else w.matrix[:features]
     if ops.gemm_split_takes(x, matrix, out, tokens):
-        ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap)
+        size = ops.gemm_split_terms(tokens, w.depth) if workspace is not None else 0
+        terms = workspace.at_least("split.terms", size, torch.bfloat16) if size > 0 else None
+        ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap, terms)
     else:
         ops.gemm_simt(x, matrix, out, tokens, epilogue, softcap)
 
@@ -114,11 +116,12 @@ def split_k_for(tokens: int, features: int, depth: int, ordered: bool = False) -
 
 def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue: int,
             status: torch.Tensor, ordered: bool = False, softcap: float = 0.0,
-            features: Optional[int] = None) -> None:
+            features: Optional[int] = None, workspace=None) -> None:
     """``out[:tokens] (op)= x[:tokens] @ w.T``; epilogue is one of ops.EPI_STORE,
     ops.EPI_STORE_F32, ops.EPI_ADD_F32.  ``features``: only the first so many rows of ``w``.
     ``ordered``: one writer per sum, no split-K (see ``split_k_for``) and no shared last round.
-    ``softcap`` > 0 (ops.EPI_STORE_F32 only): ``softcap * tanh(product / softcap)``."""
+    ``softcap`` > 0 (ops.EPI_STORE_F32 only): ``softcap * tanh(product / softcap)``.
+    ``workspace``: where a product that wants scratch takes it from (else it allocates)."""
     if tokens == 0:
         return
     if uses_tensor_cores(x, w, tokens):
@@ -127,7 +130,7 @@ def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue
         _gemm_tc(x, w, out, tokens, features or w.rows, epilogue, status, k_splits=splits,
                  softcap=softcap, ordered=ordered)
     else:
-        _gemm_simt(x, w, out, tokens, epilogue, status, softcap, features)
+        _gemm_simt(x, w, out, tokens, epilogue, status, softcap, features, workspace)
 
 
 def project_into_accumulator(x: torch.Tensor, w: Weight, accumulator: torch.Tensor,
@@ -163,7 +166,7 @@ def project_swiglu(x: torch.Tensor, w_gate_up: Weight, intermediate: int, act: t
     else:
         scratch = workspace.get(f"mlp.gate_up/{intermediate}", (capacity, 2 * intermediate),
                                 torch.float32)
-        _gemm_simt(x, w_gate_up, scratch, tokens, ops.EPI_STORE_F32, status)
+        _gemm_simt(x, w_gate_up, scratch, tokens, ops.EPI_STORE_F32, status, workspace=workspace)
         ops.swiglu(scratch[:tokens], act[:tokens], activation=activation)
 
 
@@ -191,7 +194,7 @@ def project_gated(x: torch.Tensor, w_gate_up: Weight, intermediate: int, act: to
     else:
         sums = workspace.get(f"mlp.gate_up/{intermediate}", (capacity, 2 * intermediate),
                              torch.float32)
-        project(x, w_gate_up, sums, tokens, ops.EPI_STORE_F32, status)
+        project(x, w_gate_up, sums, tokens, ops.EPI_STORE_F32, status, workspace=workspace)
         clear = False
     ops.swiglu(sums[:tokens], act[:tokens], zero_input=clear, activation=activation,
                gate_bias=gate_bias, up_bias=up_bias, limit=limit)

@@ -150,7 +150,7 @@ class StateSpaceMixer(Mixer):
                               torch.float32)
         gated = ctx.workspace.get(f"state_space.gated/{self.inner}", (ctx.capacity, self.inner),
                                   ctx.dtype)
-        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status)
+        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
         inner, bc = self.inner, self.groups * self.state_size
         ops.causal_filter(rows[:, inner:inner + self.filtered], filtered, self.filter,
                           self.filter_bias,
@@ -165,7 +165,8 @@ class StateSpaceMixer(Mixer):
                              self.head_width, self.state_size, self.groups, tokens=n)
         ops.gated_group_norm(y, rows[:, :inner], self.norm, gated, n, self.norm_groups, self.eps,
                              gate_after=False)
-        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 MIXES = ("r", "k", "v", "g", "w")
@@ -225,12 +226,14 @@ class TimeMix(Mixer):
         ops.token_shift(x, self.mu, mixes, _state_piece(cache, 0, h), n, ctx.token_request,
                         ctx.request_slot, ctx.request_start)
         for index, role in enumerate(("r", "k", "v", "g")):
-            project(mixes[index], self.weights[role], projected[index], n, ops.EPI_STORE, ctx.status)
-        project(mixes[4], self.weights["w1"], low_sums, n, ops.EPI_STORE_F32, ctx.status)
+            project(mixes[index], self.weights[role], projected[index], n, ops.EPI_STORE, ctx.status,
+                    workspace=ctx.workspace)
+        project(mixes[4], self.weights["w1"], low_sums, n, ops.EPI_STORE_F32, ctx.status,
+                workspace=ctx.workspace)
         ops.biased_activation(low_sums[:, :self.decay_rank], None, low[:, :self.decay_rank], n,
                               ops.ACT_TANH)
         project(low[:, :self.decay_rank], self.weights["w2"], decay_log, n, ops.EPI_STORE_F32,
-                ctx.status)
+                ctx.status, workspace=ctx.workspace)
         ops.outer_product_scan(projected[0], projected[1], projected[2], decay_log, self.w0,
                                self.bonus, _state_piece(cache, h, self.matrix_state), o,
                                ctx.request_start, ctx.request_slot, ctx.n_requests, self.heads,
@@ -238,7 +241,7 @@ class TimeMix(Mixer):
         ops.gated_group_norm(o, projected[3], self.norm, normed, n, self.heads, self.eps,
                              gate_after=True)
         project(normed, self.weights["o"], residual, n, ops.EPI_ADD_F32, ctx.status,
-                ctx.ordered_sums)
+                ctx.ordered_sums, workspace=ctx.workspace)
 
 
 def _flat_state(mixer: Mixer) -> int:
@@ -413,7 +416,7 @@ class LinearState(Mixer):
                               torch.float32)
         gated = ctx.workspace.get(f"linear_state.gated/{self.v_width}",
                                   (ctx.capacity, self.v_width), ctx.dtype)
-        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status)
+        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
         qkv = rows
         if self.taps is not None:
             qkv = ctx.workspace.get(f"linear_state.filtered/{self.filtered}",
@@ -454,7 +457,8 @@ class LinearState(Mixer):
                 **gates)
         ops.gated_group_norm(o, rows[:, self.gate_at:self.gate_at + self.v_width], self.norm, gated,
                              n, self.heads, self.eps, gate_after=True)
-        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class GatedRecurrence(Mixer):
@@ -527,7 +531,7 @@ class GatedRecurrence(Mixer):
             project_into_accumulator(x, self.w_in, rows, n, ctx.status, ctx.ordered_sums)
         else:
             rows = get(f"gated_recurrence.rows/{w}", (ctx.capacity, -(-2 * w // 8) * 8), ctx.dtype)
-            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status)
+            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
         # rows of a width that keeps them 16-byte aligned
         wide = -(-w // 8) * 8
         u = get(f"gated_recurrence.filtered/{w}", (ctx.capacity, wide), ctx.dtype)
@@ -558,7 +562,8 @@ class GatedRecurrence(Mixer):
             else:
                 ops.block_gates(*gates, n)
                 ops.gated_scan(decay, push, rows, self.y_bias, state, gated, *batch, sums=sums)
-        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(gated, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class MatrixLstm(Mixer):
@@ -639,10 +644,12 @@ class MatrixLstm(Mixer):
         else:
             size = -(-self.rows_size // 8) * 8
             rows = get(f"matrix_lstm.rows/{size}", (ctx.capacity, size), ctx.dtype)
-            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, features=self.rows_size)
+            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, features=self.rows_size,
+                    workspace=ctx.workspace)
             width = -(-2 * heads // 4) * 4
             gate_sums = get(f"matrix_lstm.gate_sums/{width}", (ctx.capacity, width), torch.float32)
-            project(x, self.w_gates, gate_sums, n, ops.EPI_STORE_F32, ctx.status)
+            project(x, self.w_gates, gate_sums, n, ops.EPI_STORE_F32, ctx.status,
+                    workspace=ctx.workspace)
         batch = (ctx.request_start, ctx.request_slot, ctx.n_requests, n, heads, self.head_dim,
                  self.value_dim)
         decay, push, level, weight, total = arrays
@@ -663,7 +670,8 @@ class MatrixLstm(Mixer):
                         None if one_token else (decay, push, level),
                         gate_sums if one_token else None, self.q_scale, self.floor, self.norm, self.eps,
                         cache.state, o, weight, out, ctx.token_request, *batch, scan=not chunked)
-        project(out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums)
+        project(out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
 
 
 class InputFilter(Mixer):

@@ -527,6 +527,12 @@ int hx_gemm_split_pays(int tokens, int features);
 int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
                   int features, int depth, int epilogue, float softcap, int* status,
                   cudaStream_t stream);
+/* the same with scratch for the terms of x (hx_gemm_split_terms() bfloat16 numbers on 16 bytes; 0: none are
+ * wanted; null: the product does without) */
+long long hx_gemm_split_terms(int tokens, int depth);
+int hx_gemm_split_scratch(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
+                          int features, int depth, int epilogue, float softcap, void* terms,
+                          long long terms_size, int* status, cudaStream_t stream);
 /* tcgen05 tensor cores, bfloat16 operands, float32 accumulate in tensor memory.
  * weight_tiles != 0: w holds the matrix as [ceil(rows / 128)][ceil(depth / 64)] tiles of
  * [128][64] elements, zero padded, each tile 16 contiguous kilobytes (ldw is ignored). */

@@ -106,3 +106,27 @@ def test_which_products_take_it():
     assert not ops.gemm_split_takes(x[:, 1:129], w[:, 1:129], out, 64)
     assert not ops.gemm_split_takes(x[:, :130], w[:, :130], out, 64)
     assert not ops.gemm_split_takes(x.bfloat16(), w.bfloat16(), out, 64)
+
+
+@pytest.mark.parametrize("tokens,features,depth", [
+    (129, 129, 68), (256, 128, 64), (257, 300, 132), (300, 63, 4), (520, 9700, 196), (130, 40, 1000),
+])
+def test_pairs_have_the_sums_of_single_tiles(tokens, features, depth):
+    """More tokens than a tile, with scratch for their terms and without: the same order of the same sums.
+    (9,700 by 520: more tiles than pairs of CTAs.)"""
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(tokens)
+    x, w = torch.randn(tokens, depth + 4, device="cuda")[:, :depth], torch.randn(features, depth, device="cuda")
+    x[7, 3], w[5, 1] = float("inf"), float("nan")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    size = ops.gemm_split_terms(tokens, depth)
+    assert size >= 3 * tokens * depth and ops.gemm_split_terms(128, depth) == 0
+    terms = torch.full((size + 64,), float("nan"), dtype=torch.bfloat16, device="cuda")
+    for epilogue in (ops.EPI_STORE_F32, ops.EPI_ADD_F32):
+        out, plain = torch.full((2, tokens + 1, features + 3), 2.0, device="cuda")
+        ops.gemm_split(x, w, out, tokens, epilogue, status, terms=terms[:size])
+        parts = [slice(begin, min(begin + 100, tokens)) for begin in range(0, tokens, 100)]
+        for part in parts:
+            ops.gemm_split(x[part], w, plain[part], part.stop - part.start, epilogue, status)
+        torch.testing.assert_close(out, plain, rtol=0, atol=0, equal_nan=True)
+    assert terms[size:].isnan().all() and int(status.item()) == 0
