@@ -17,10 +17,10 @@
 //
 //   * delta_weights_kernel, all chunks at once: T = (1 + A)^-1 by forward substitution in float32,
 //     P, and the factors of a token.
-//   * delta_states_kernel, one CTA per (request, head, block of columns), chunk after chunk: a
-//     warp keeps S' for 16 columns in registers as accumulators of mma.sync, whose layout is also
-//     that of an A operand, so S' goes into S' K' and S' Q', R' into R' T', U' into U' P' and
-//     U' K without leaving the registers.  The next chunk's rows are on their way meanwhile.
+//   * delta_states_kernel, one CTA per (request, head, 64 columns), chunk after chunk: two warps keep
+//     S' for 16 columns in registers, half of the key coordinates each, as accumulators of mma.sync,
+//     whose layout is also that of an A operand, so S' goes into S' K' and S' Q', R' into R' T', U'
+//     into U' P' and U' K from registers.  A warpgroup copies the next chunk's rows meanwhile.
 //
 // Queries, keys and values go in as they are stored; what the scan holds in float32 (S, R, U, T,
 // P) goes into the products as three bfloat16 terms, 24 bits; lengths and decays multiply the
@@ -28,18 +28,18 @@
 // which are then the only ones whose rounding counts.
 //
 // The weights of tokens that come later are zeros, and zero times a number that is not finite is
-// none: such a number, wherever it comes in, shows in the chunk's outputs.  A warp that finds one
-// there takes the chunk again token by token, from the state that it still holds.
+// none: such a number, wherever it comes in, shows in the chunk's outputs.  Warps that find one
+// there take the chunk again token by token, from the state that they still hold.
 //
 // The scan walks a token in 0.6 us whatever the chip could do beside it (a chain of two dot
-// products over the state); a chunk is a chain of about 800 products a warp, which is what bounds
-// it now.  Measured (one B200, 32 heads of 128 by 128, against the scan): a portion of 1,000 tokens
-// 957 -> 201 us, eight of 256 1,064 -> 222, one of 64 71 -> 46 (the numbers that are not finite found by
-// comparing instead: spills, 215, 215, 44); errors against 64 bits, 1,024 tokens, 2.0e-7
-// (outputs) and 1.3e-7 (state) where the scan has 2.3e-7 and 2.2e-7 (2.6e-7 and 2.5e-7 with a chunk's
-// products added onto the state itself).
+// products over the state); a chunk is a chain of about 800 products for 16 columns, in which the
+// instructions between the products count as much.  Measured (one B200, 32 heads of 128 by 128, against the
+// scan): a portion of 1,000 tokens 980 -> 142 us, eight of 256 1,064 -> 184, one of 128 134 -> 39; errors
+// against 64 bits, 1,024 tokens, 1.8e-7 (outputs) and 1.3e-7 (state) where the scan has 2.3e-7 and 2.2e-7
+// (2.6e-7 and 2.5e-7 with a chunk's products added onto the state itself).
 #include "hx_mma.cuh"
 #include "hx_scan.cuh"
+#include "hx_tcgen05.cuh"
 
 #include <mutex>
 
@@ -75,9 +75,10 @@ struct DeltaArgs {
   float* o;                  // [tokens, heads * vdim]
   const int* request_start;
   const int* request_slot;
-  int requests, heads, qk_heads, dim, vdim, parts, column_warps;
+  int requests, heads, qk_heads, dim, vdim, parts;
   int min_query_len;         // requests with fewer tokens are left alone;
   int portions;              // so many have as many
+  int* status;               // may be null
 };
 
 // two neighbouring values in three bfloat16 terms, a word each
@@ -141,12 +142,22 @@ __device__ __forceinline__ void clear_columns(__nv_bfloat16* dst, int stride, in
 
 constexpr int SOLVE_STRIDE = CHUNK + 4;
 
-// Shared memory of delta_weights_kernel: queries, keys, A transposed, T.
+constexpr int TERMS_STRIDE = TERMS * CHUNK + ROW_PAD;      // of a token's row of T or P
+
+// Shared memory of delta_weights_kernel: queries and keys (later the terms of P, then of T), A
+// transposed, T.
+__host__ __device__ constexpr int weights_rows(int padded) {
+  return 2 * (padded + ROW_PAD) > TERMS_STRIDE ? 2 * (padded + ROW_PAD) : TERMS_STRIDE;
+}
 int weights_shared(int padded) {
-  return 2 * 2 * CHUNK * (padded + ROW_PAD) + 2 * 4 * CHUNK * SOLVE_STRIDE;
+  return 2 * CHUNK * weights_rows(padded) + 2 * 4 * CHUNK * SOLVE_STRIDE;
 }
 
 // grid (chunks of the step, heads), 128 threads: a warp takes 16 of the chunk's tokens
+//
+// Bound by chains of latency, three CTAs an SM to fill them.  Measured, 27 chunks of 32 heads: 44 -> 34 us with
+// lengths a row a thread and P stored 16 bytes a thread beside the solution (of a CTA's 30,000 cycles 10,500
+// solve, 4,200 find the chunk, 3,600 make the gates).
 template <int STEPS>
 __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
   constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
@@ -161,7 +172,7 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
   const int live = min(CHUNK, a.request_start[request + 1] - first);
   __nv_bfloat16* queries = reinterpret_cast<__nv_bfloat16*>(shared_pieces);
   __nv_bfloat16* keys = queries + CHUNK * STRIDE;
-  float* system = reinterpret_cast<float*>(keys + CHUNK * STRIDE);      // [s][t]: A
+  float* system = reinterpret_cast<float*>(queries + CHUNK * weights_rows(PADDED));      // [s][t]: A
   float* solution = system + CHUNK * SOLVE_STRIDE;                      // [t][s]: T
   copy_rows<2 * STEPS>(queries, STRIDE, a.q + static_cast<size_t>(first) * a.ld_q + qk_head * a.dim, a.ld_q, a.dim, live);
   copy_rows<2 * STEPS>(keys, STRIDE, a.k + static_cast<size_t>(first) * a.ld_k + qk_head * a.dim, a.ld_k, a.dim, live);
@@ -172,7 +183,11 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
   }
   const size_t rows = static_cast<size_t>(head) * a.rows + first;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  // One warp makes what the gates make of the tokens while the others take the lengths and go on to their
+  // products (that warp's are the fewest).
+  hx_cp_async_wait<0>();
   if (warp == 0) {
+    asm volatile("bar.arrive 1, 128;" ::: "memory");
     // sums of the decays' logarithms, two neighbouring tokens a lane, in double: their
     // differences are what counts
     float d[2];
@@ -202,45 +217,41 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
     level_lo[2 * lane] = static_cast<float>(before - static_cast<double>(static_cast<float>(before)));
     level_hi[2 * lane + 1] = static_cast<float>(sum);
     level_lo[2 * lane + 1] = static_cast<float>(sum - static_cast<double>(static_cast<float>(sum)));
-  }
-  hx_cp_async_wait<0>();
-  __syncthreads();
-  // what lengths and scales make of a query and a key
-  for (int i = 0; i < 16; ++i) {
-    const int t = 16 * warp + i;
-    float fq = a.q_scale, fk = a.k_scale;
-    if (a.unit_norm) {
-      float sq = 0.0f, sk = 0.0f;
-      for (int e = 2 * lane; e < PADDED; e += 64) {
-        const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(queries + t * STRIDE + e));
-        const float2 y = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(keys + t * STRIDE + e));
-        sq = fmaf(x.x, x.x, fmaf(x.y, x.y, sq));
-        sk = fmaf(y.x, y.x, fmaf(y.y, y.y, sk));
-      }
+    asm volatile("bar.sync 2, 128;" ::: "memory");
+  } else {
+    asm volatile("bar.sync 1, 128;" ::: "memory");
+    // what lengths and scales make of a query and a key, a row a thread (neighbours' 16-byte pieces lie on
+    // different banks); one warp for 16 rows took 12,000 cycles of the kernel's 40,000
+    for (int i = threadIdx.x - 32; i < 2 * CHUNK; i += 96) {
+      const bool key = i >= CHUNK;
+      const int t = i & (CHUNK - 1);
+      float length = key ? a.k_scale : a.q_scale;
+      if (a.unit_norm) {
+        const __nv_bfloat16* x = (key ? keys : queries) + t * STRIDE;
+        float squares[16];
 #pragma unroll
-      for (int offset = 16; offset > 0; offset >>= 1) {
-        sq += __shfl_xor_sync(0xffffffffu, sq, offset);
-        sk += __shfl_xor_sync(0xffffffffu, sk, offset);
+        for (int j = 0; j < 16; ++j) squares[j] = 0.0f;
+#pragma unroll
+        for (int e = 0; e < PADDED; e += 8) {
+          const uint4 piece = *reinterpret_cast<const uint4*>(x + e);
+          const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&piece);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 v = __bfloat1622float2(pairs[j]);
+            float* sum = squares + (e & 8) + 2 * j;
+            sum[0] = fmaf(v.x, v.x, sum[0]);
+            sum[1] = fmaf(v.y, v.y, sum[1]);
+          }
+        }
+#pragma unroll
+        for (int offset = 8; offset > 0; offset >>= 1)
+#pragma unroll
+          for (int j = 0; j < offset; ++j) squares[j] += squares[j + offset];
+        length /= sqrtf(squares[0] + a.unit_eps);
       }
-      fq /= sqrtf(sq + a.unit_eps);
-      fk /= sqrtf(sk + a.unit_eps);
+      (key ? k_length : q_length)[t] = length;
     }
-    if (lane == 0) {
-      q_length[t] = fq;
-      k_length[t] = fk;
-    }
-  }
-  __syncthreads();
-  // e^(L_t - L_s)
-  auto faded = [&](int t, int s) {
-    return expf((level_hi[t] - level_hi[s]) + (level_lo[t] - level_lo[s]));
-  };
-  if (threadIdx.x < live) {
-    const int t = threadIdx.x;
-    const float level = expf(level_hi[t] + level_lo[t]);
-    a.factors[rows + t] = make_float4(q_length[t] * level, write[t] * k_length[t] * level, write[t],
-                                      k_length[t] * faded(CHUNK - 1, t));
-    if (t == 0) a.total[rows] = expf(level_hi[CHUNK - 1] + level_lo[CHUNK - 1]);
+    asm volatile("bar.arrive 2, 128;" ::: "memory");
   }
   // sums of tokens 16 warp .. + 15 against the tiles of 8 tokens that do not lie behind them
   float qk[8][4], kk[8][4];
@@ -270,11 +281,24 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
       }
     }
   }
+  __syncthreads();      // (queries and keys are read, too: the terms of T and P gather in their place)
+  // e^(L_t - L_s)
+  auto faded = [&](int t, int s) {
+    return expf((level_hi[t] - level_hi[s]) + (level_lo[t] - level_lo[s]));
+  };
+  if (threadIdx.x < live) {
+    const int t = threadIdx.x;
+    const float level = expf(level_hi[t] + level_lo[t]);
+    a.factors[rows + t] = make_float4(q_length[t] * level, write[t] * k_length[t] * level, write[t],
+                                      k_length[t] * faded(CHUNK - 1, t));
+    if (t == 0) a.total[rows] = expf(level_hi[CHUNK - 1] + level_lo[CHUNK - 1]);
+  }
   const int row = lane >> 2, column = 2 * (lane & 3);
+  __nv_bfloat16* terms = queries;
 #pragma unroll
   for (int half = 0; half < 2; ++half) {
     const int t = 16 * warp + row + 8 * half;
-    __nv_bfloat16* out = a.weights + (rows + min(t, live - 1)) * WEIGHT_COLUMNS + TERMS * CHUNK;
+    __nv_bfloat16* out = terms + t * TERMS_STRIDE;
 #pragma unroll
     for (int n = 0; n < 8; ++n) {
       const int s = 8 * n + column;
@@ -289,13 +313,11 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
         }
         system[(s + i) * SOLVE_STRIDE + t] = held;
       }
-      if (t < live) {
-        uint32_t t0, t1, t2;
-        split_terms(p[0], p[1], t0, t1, t2);
-        *reinterpret_cast<uint32_t*>(out + s) = t0;
-        *reinterpret_cast<uint32_t*>(out + CHUNK + s) = t1;
-        *reinterpret_cast<uint32_t*>(out + 2 * CHUNK + s) = t2;
-      }
+      uint32_t t0, t1, t2;
+      split_terms(p[0], p[1], t0, t1, t2);
+      *reinterpret_cast<uint32_t*>(out + s) = t0;
+      *reinterpret_cast<uint32_t*>(out + CHUNK + s) = t1;
+      *reinterpret_cast<uint32_t*>(out + 2 * CHUNK + s) = t2;
     }
   }
   __syncthreads();
@@ -309,7 +331,7 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
 #pragma unroll
       for (int r = 0; r < 16; ++r) x[r] = 16 * block + r == j ? 1.0f : 0.0f;
       if (16 * (block + 1) > (warp << 5)) {      // else all the warp's columns are zero here
-#pragma unroll 2
+#pragma unroll 4
         for (int s = warp << 5; s < 16 * block; ++s) {
           const float known = solution[s * SOLVE_STRIDE + j];
           const float4* held = reinterpret_cast<const float4*>(system + s * SOLVE_STRIDE + 16 * block);
@@ -324,41 +346,72 @@ __global__ __launch_bounds__(128) void delta_weights_kernel(const DeltaArgs a) {
         }
 #pragma unroll
         for (int s = 0; s < 15; ++s) {
-          const float* held = system + (16 * block + s) * SOLVE_STRIDE + 16 * block;
+          const float4* held = reinterpret_cast<const float4*>(system + (16 * block + s) * SOLVE_STRIDE + 16 * block);
 #pragma unroll
-          for (int r = s + 1; r < 16; ++r) x[r] = fmaf(-held[r], x[s], x[r]);
+          for (int r = (s + 1) / 4; r < 4; ++r) {
+            const float4 h = held[r];
+            if (4 * r > s) x[4 * r] = fmaf(-h.x, x[s], x[4 * r]);
+            if (4 * r + 1 > s) x[4 * r + 1] = fmaf(-h.y, x[s], x[4 * r + 1]);
+            if (4 * r + 2 > s) x[4 * r + 2] = fmaf(-h.z, x[s], x[4 * r + 2]);
+            if (4 * r + 3 > s) x[4 * r + 3] = fmaf(-h.w, x[s], x[4 * r + 3]);
+          }
         }
       }
 #pragma unroll
       for (int r = 0; r < 16; ++r) solution[(16 * block + r) * SOLVE_STRIDE + j] = x[r];
     }
   }
+  // The warps that do not solve store P meanwhile: whole 16-byte pieces, a row's one behind the other.
+  auto store = [&](int thread, int threads, int column) {
+    constexpr int PIECES = TERMS * CHUNK / 8;
+    for (int i = thread; i < live * PIECES; i += threads) {
+      const int t = i / PIECES, piece = i - t * PIECES;
+      *reinterpret_cast<uint4*>(a.weights + (rows + t) * WEIGHT_COLUMNS + column + 8 * piece) =
+          *reinterpret_cast<const uint4*>(terms + t * TERMS_STRIDE + 8 * piece);
+    }
+  };
+  if (threadIdx.x >= CHUNK) store(threadIdx.x - CHUNK, CHUNK, TERMS * CHUNK);
   __syncthreads();
-  for (int i = threadIdx.x; i < live * (CHUNK / 2); i += 128) {
+  for (int i = threadIdx.x; i < CHUNK * (CHUNK / 2); i += 128) {
     const int t = i / (CHUNK / 2), s = 2 * (i - t * (CHUNK / 2));
     const float2 x = *reinterpret_cast<const float2*>(solution + t * SOLVE_STRIDE + s);
-    __nv_bfloat16* out = a.weights + (rows + t) * WEIGHT_COLUMNS + s;
+    __nv_bfloat16* out = terms + t * TERMS_STRIDE + s;
     uint32_t t0, t1, t2;
     split_terms(x.x, x.y, t0, t1, t2);
     *reinterpret_cast<uint32_t*>(out) = t0;
     *reinterpret_cast<uint32_t*>(out + CHUNK) = t1;
     *reinterpret_cast<uint32_t*>(out + 2 * CHUNK) = t2;
   }
+  __syncthreads();
+  store(threadIdx.x, 128, 0);
 }
 
-// Shared memory of delta_states_kernel: two stages of [queries | keys | weights | values | factors |
-// total].
+// Shared memory of delta_states_kernel: two stages of [queries | keys | weights | values | factors], then
+// what the two warps of a block of 16 columns tell each other: two buffers of 32 numbers a lane, and a
+// word; then a barrier for each stage.
+constexpr int EXCHANGED = 32;
+constexpr int BLOCKS = 4, BLOCK_COLUMNS = 16 * BLOCKS;      // of a CTA: a block of 16 columns for each quarter of an SM
+constexpr int STATES_THREADS = 3 * 32 * BLOCKS;             // two warps a block, and a warpgroup that copies
+// At launch 168 a thread; the warps that copy need few, the others take what they leave.
+constexpr int WORK_REGISTERS = 224, COPY_REGISTERS = 56;
+static_assert(2 * WORK_REGISTERS + COPY_REGISTERS <= 3 * 168, "what one side takes the other has given back");
+template <int PADDED>
 struct DeltaLayout {
-  int rows_bytes, stage_bytes, bytes;
-  __host__ __device__ DeltaLayout(int padded, int column_warps) {
-    rows_bytes = 2 * CHUNK * (2 * (padded + ROW_PAD) + WEIGHT_STRIDE + 16 * column_warps + ROW_PAD);
-    stage_bytes = rows_bytes + 16 * (CHUNK + 1);
-    bytes = 2 * stage_bytes;
-  }
+  static constexpr int kValueStride = BLOCK_COLUMNS + ROW_PAD;
+  static constexpr int kRowsBytes = 2 * CHUNK * (2 * (PADDED + ROW_PAD) + WEIGHT_STRIDE + kValueStride);
+  static constexpr int kStageBytes = kRowsBytes + 16 * CHUNK;
+  static constexpr int kExchange = 2 * kStageBytes;
+  static constexpr int kOdd = kExchange + BLOCKS * 2 * EXCHANGED * 32 * 4;
+  static constexpr int kBars = kOdd + BLOCKS * 16;
+  static constexpr int kBytes = kBars + 16;
 };
 
-__device__ __forceinline__ void copy_4(uint32_t dst, const void* src) {
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"(dst), "l"(src) : "memory");
+// A row into shared memory, counted on a barrier; both ends and the size are multiples of 16 bytes.
+__device__ __forceinline__ void copy_row(void* dst, const void* src, int bytes, uint64_t* bar) {
+  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                   hx_shared_address(dst)),
+               "l"(src), "r"(bytes), "r"(hx_shared_address(bar))
+               : "memory");
 }
 
 // sums = x' w', with x' [16 columns x 64 tokens s] in accumulators and w [t][s] of three terms in
@@ -373,35 +426,44 @@ __device__ __forceinline__ void triangular_product(float (&sums)[8][4], const fl
   for (int step = 0; step < CHUNK / 16; ++step) {
     uint32_t x0[4], x1[4], x2[4];
     operand_terms(x, step, x0, x1, x2);
+    // up to four tiles of tokens side by side: a sum's products follow one another
 #pragma unroll
-    for (int n = 2 * step; n < 8; n += 2) {
-      uint32_t w0[4], w1[4], w2[4];
-      const uint32_t at = weights_at + 2 * (8 * n * WEIGHT_STRIDE + 16 * step);
-      hx_ldmatrix_x4(w0, at);
-      hx_ldmatrix_x4(w1, at + 2 * CHUNK);
-      hx_ldmatrix_x4(w2, at + 4 * CHUNK);
-      hx_mma_bf16(sums[n], x2, w0[0], w0[1]);
-      hx_mma_bf16(sums[n + 1], x2, w0[2], w0[3]);
-      hx_mma_bf16(sums[n], x0, w2[0], w2[1]);
-      hx_mma_bf16(sums[n + 1], x0, w2[2], w2[3]);
-      hx_mma_bf16(sums[n], x1, w1[0], w1[1]);
-      hx_mma_bf16(sums[n + 1], x1, w1[2], w1[3]);
-      hx_mma_bf16(sums[n], x1, w0[0], w0[1]);
-      hx_mma_bf16(sums[n + 1], x1, w0[2], w0[3]);
-      hx_mma_bf16(sums[n], x0, w1[0], w1[1]);
-      hx_mma_bf16(sums[n + 1], x0, w1[2], w1[3]);
+    for (int n0 = 2 * step; n0 < 8; n0 += 4) {
+      uint32_t w0[2][4], w1[2][4], w2[2][4];
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (n0 + 2 * i >= 8) continue;
+        const uint32_t at = weights_at + 2 * (8 * (n0 + 2 * i) * WEIGHT_STRIDE + 16 * step);
+        hx_ldmatrix_x4(w0[i], at);
+        hx_ldmatrix_x4(w2[i], at + 4 * CHUNK);
+        hx_ldmatrix_x4(w1[i], at + 2 * CHUNK);
+      }
+      auto products = [&](const uint32_t (&xt)[4], const uint32_t (&wt)[2][4]) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int n = n0 + 2 * i;
+          if (n >= 8) continue;
+          hx_mma_bf16(sums[n], xt, wt[i][0], wt[i][1]);
+          hx_mma_bf16(sums[n + 1], xt, wt[i][2], wt[i][3]);
+        }
+      };
+      products(x2, w0);
+      products(x0, w2);
+      products(x1, w1);
+      products(x1, w0);
+      products(x0, w1);
     }
   }
 #pragma unroll
   for (int step = 0; step < CHUNK / 16; ++step) {
-    uint32_t x0[4];
+    uint32_t x0[4], w0[4][4];
+#pragma unroll
+    for (int i = step; i < 4; ++i) hx_ldmatrix_x4(w0[i], weights_at + 2 * (16 * i * WEIGHT_STRIDE + 16 * step));
     operand_high(x, step, x0);
 #pragma unroll
-    for (int n = 2 * step; n < 8; n += 2) {
-      uint32_t w0[4];
-      hx_ldmatrix_x4(w0, weights_at + 2 * (8 * n * WEIGHT_STRIDE + 16 * step));
-      hx_mma_bf16(sums[n], x0, w0[0], w0[1]);
-      hx_mma_bf16(sums[n + 1], x0, w0[2], w0[3]);
+    for (int i = step; i < 4; ++i) {
+      hx_mma_bf16(sums[2 * i], x0, w0[i][0], w0[i][1]);
+      hx_mma_bf16(sums[2 * i + 1], x0, w0[i][2], w0[i][3]);
     }
   }
 }
@@ -477,10 +539,73 @@ __device__ __noinline__ void tokens_in_turn(const DeltaArgs& a, float (*S)[4], c
   }
 }
 
-// grid (portions, heads, blocks of columns); a warp keeps 16 columns.  STEPS: steps of 16 key coordinates
+// sums = S' x' over HALF steps of 16 key coordinates for all tokens of the chunk, [16 columns x 64
+// tokens]; x: staged rows of keys or queries.  The rows that half a step takes are asked for while the
+// products of the half before run.
+template <int HALF>
+__device__ __forceinline__ void state_product(float (&sums)[8][4], const float (&S)[2 * HALF][4], uint32_t rows_at,
+                                              int stride) {
+#pragma unroll
+  for (int n = 0; n < 8; ++n)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sums[n][j] = 0.0f;
+  uint32_t x[2][2][4];
+  auto fetch = [&](int half) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i)
+      hx_ldmatrix_x4(x[half & 1][i], rows_at + 2 * (8 * (4 * (half & 1) + 2 * i) * stride + 16 * (half >> 1)));
+  };
+  auto products = [&](int half, const uint32_t (&st)[4]) {
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int n = 4 * (half & 1) + 2 * i;
+      hx_mma_bf16(sums[n], st, x[half & 1][i][0], x[half & 1][i][1]);
+      hx_mma_bf16(sums[n + 1], st, x[half & 1][i][2], x[half & 1][i][3]);
+    }
+  };
+  fetch(0);
+#pragma unroll
+  for (int step = 0; step < HALF; ++step) {
+    uint32_t s0[4], s1[4], s2[4];
+    operand_terms(S, step, s0, s1, s2);
+#pragma unroll
+    for (int half = 2 * step; half < 2 * step + 2; ++half) {
+      fetch((half + 1) % (2 * HALF));
+      products(half, s2);
+      products(half, s1);
+    }
+  }
+#pragma unroll
+  for (int step = 0; step < HALF; ++step) {
+    uint32_t s0[4];
+    operand_high(S, step, s0);
+#pragma unroll
+    for (int half = 2 * step; half < 2 * step + 2; ++half) {
+      if (half + 1 < 2 * HALF) fetch(half + 1);
+      products(half, s0);
+    }
+  }
+}
+
+// grid (portions, heads, blocks of columns); two warps keep 16 columns, each one half of the key
+// coordinates.  STEPS: steps of 16 key coordinates
+//
+// What bounds a chunk is a chain of warp-wide products and of the instructions between them, so the work of
+// 16 columns is dealt to two warps of the same quarter of an SM, which fill each other's gaps: either
+// multiplies its half of S' and carries it on; the first makes R and U, the second the outputs meanwhile:
+//
+//     first:   S' k | + the other's | R, U = T R | S' q (its half)  | state
+//     second:  S' k |  S' q (its half)           | P U, + the first's S' q, outputs | state
+//
+// A third warpgroup copies (a row a bulk copy), because issuing them takes as long as a third of the chunk's
+// products.  Cycles a chunk of 11,800: S' k 2,600, R 750, U 1,900, S' q beside P U 2,300, terms 1,100, outputs and
+// state 2,600; the tensor pipe has 6,500 of work.  Measured, portions of 763 and 957 tokens, 32 heads of 128 by
+// 128: 156 -> 101 us.  (One warp for 16 columns, 19,000 cycles a chunk; its products in another order, four to
+// eight sums side by side, 156; two warps and their copies as cp.async 130, as bulk copies of the same warps 119.)
 template <int STEPS>
-__global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_constant__ DeltaArgs a) {
-  constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD;
+__global__ __launch_bounds__(STATES_THREADS, 1) void delta_states_kernel(const __grid_constant__ DeltaArgs a) {
+  constexpr int PADDED = 16 * STEPS, STRIDE = PADDED + ROW_PAD, HALF = STEPS / 2;
+  static_assert(8 * HALF <= EXCHANGED, "a half of the state passes through a buffer");
   extern __shared__ uint4 shared_pieces[];
   hx_pdl_prologue();
   const int head = blockIdx.y, qk_head = head / (a.heads / a.qk_heads);
@@ -493,16 +618,19 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_const
   const int start = a.request_start[request];
   const int count = a.request_start[request + 1] - start;
   if (count < a.min_query_len) return;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int lane = threadIdx.x & 31;
+  const int block = (threadIdx.x >> 5) % BLOCKS;      // of 16 columns
+  const bool second = (threadIdx.x >> 5) >= BLOCKS;
   const int row = lane >> 2, pair = 2 * (lane & 3);
   const int matrix = lane >> 3, in_matrix = lane & 7;
-  const int block_columns = 16 * a.column_warps;
-  const int column0 = blockIdx.z * block_columns;
-  const int copied = min(a.vdim - column0, block_columns);
-  const int value_stride = block_columns + ROW_PAD;
-  const DeltaLayout layout(PADDED, a.column_warps);
+  const int column0 = blockIdx.z * BLOCK_COLUMNS;
+  const int copied = min(a.vdim - column0, BLOCK_COLUMNS);
+  using Layout = DeltaLayout<PADDED>;
+  constexpr int value_stride = Layout::kValueStride;
   char* base = reinterpret_cast<char*>(shared_pieces);
-  auto queries_of = [&](int stage) { return reinterpret_cast<__nv_bfloat16*>(base + stage * layout.stage_bytes); };
+  auto queries_of = [&](int stage) { return reinterpret_cast<__nv_bfloat16*>(base + stage * Layout::kStageBytes); };
+  uint64_t* bars = reinterpret_cast<uint64_t*>(base + Layout::kBars);
+  // A chunk's rows, a copy each (of queries, keys, weights, values); rows behind the portion are zeros.
   auto fetch = [&](int chunk, int stage) {
     const size_t first = start + chunk * CHUNK;
     const int live = min(CHUNK, count - chunk * CHUNK);
@@ -511,27 +639,42 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_const
     __nv_bfloat16* keys = queries + CHUNK * STRIDE;
     __nv_bfloat16* weights = keys + CHUNK * STRIDE;
     __nv_bfloat16* values = weights + CHUNK * WEIGHT_STRIDE;
-    copy_rows<2 * STEPS>(queries, STRIDE, a.q + first * a.ld_q + qk_head * a.dim, a.ld_q, a.dim, live);
-    copy_rows<2 * STEPS>(keys, STRIDE, a.k + first * a.ld_k + qk_head * a.dim, a.ld_k, a.dim, live);
-    copy_rows<WEIGHT_COLUMNS / 8>(weights, WEIGHT_STRIDE, a.weights + rows * WEIGHT_COLUMNS, WEIGHT_COLUMNS,
-                                  WEIGHT_COLUMNS, live);
-    {
-      // a warp brings its own 16 columns of the values
-      const __nv_bfloat16* from = a.v + first * a.ld_v + head * a.vdim + column0;
-      const int column = 16 * warp + 8 * (lane & 1);
-      if (column < copied) {
-#pragma unroll
-        for (int t = lane >> 1; t < CHUNK; t += 16)
-          hx_cp_async_16(hx_shared_address(values + t * value_stride + column),
-                         t < live ? from + static_cast<size_t>(t) * a.ld_v + column : from, t < live ? 16 : 0);
+    char* factors = base + stage * Layout::kStageBytes + Layout::kRowsBytes;
+    uint64_t* bar = bars + stage;
+    const int thread = threadIdx.x - 2 * 32 * BLOCKS;
+    if (thread == 0) {
+      mbar_expect_tx(bar, 2 * live * (2 * a.dim + WEIGHT_COLUMNS + copied) + 16 * live);
+      copy_row(factors, a.factors + rows, 16 * live, bar);
+    }
+    for (int i = thread; i < 4 * CHUNK; i += 32 * BLOCKS) {
+      const int what = i / CHUNK, t = i % CHUNK;
+      __nv_bfloat16* to;
+      const __nv_bfloat16* from;
+      int size;
+      if (what == 0) {
+        to = queries + t * STRIDE, from = a.q + (first + t) * a.ld_q + qk_head * a.dim, size = a.dim;
+      } else if (what == 1) {
+        to = keys + t * STRIDE, from = a.k + (first + t) * a.ld_k + qk_head * a.dim, size = a.dim;
+      } else if (what == 2) {
+        to = weights + t * WEIGHT_STRIDE, from = a.weights + (rows + t) * WEIGHT_COLUMNS, size = WEIGHT_COLUMNS;
+      } else {
+        to = values + t * value_stride, from = a.v + (first + t) * a.ld_v + head * a.vdim + column0, size = copied;
+      }
+      if (t < live) {
+        copy_row(to, from, 2 * size, bar);
+      } else {
+        for (int e = 0; e < size; e += 8) *reinterpret_cast<uint4*>(to + e) = make_uint4(0u, 0u, 0u, 0u);
+        if (what == 3) *reinterpret_cast<float4*>(factors + 16 * t) = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
       }
     }
-    const uint32_t factors = hx_shared_address(base + stage * layout.stage_bytes + layout.rows_bytes);
-    for (int t = threadIdx.x; t < CHUNK; t += blockDim.x)
-      hx_cp_async_16(factors + 16 * t, a.factors + rows + (t < live ? t : 0), t < live ? 16 : 0);
-    if (threadIdx.x == 0) copy_4(factors + 16 * CHUNK, a.total + rows);
-    hx_cp_async_commit();
   };
+  if (threadIdx.x == 0) {
+    mbar_init(&bars[0], 1);
+    mbar_init(&bars[1], 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+  }
+  __syncthreads();
   // what the copies leave alone
   for (int stage = 0; stage < 2; ++stage) {
     __nv_bfloat16* queries = queries_of(stage);
@@ -539,185 +682,245 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_const
       clear_columns(queries, STRIDE, a.dim, PADDED);
       clear_columns(queries + CHUNK * STRIDE, STRIDE, a.dim, PADDED);
     }
-    if (copied < block_columns)
-      clear_columns(queries + CHUNK * (2 * STRIDE + WEIGHT_STRIDE), value_stride, copied, block_columns);
+    if (copied < BLOCK_COLUMNS)
+      clear_columns(queries + CHUNK * (2 * STRIDE + WEIGHT_STRIDE), value_stride, copied, BLOCK_COLUMNS);
   }
-  fetch(0, 0);
+  const int chunks = (count + CHUNK - 1) / CHUNK;
+  // Whether the chunk's rows are there; behind it nobody reads the other stage any more.
+  auto arrived = [&](int chunk) {
+    const bool there = mbar_wait(&bars[chunk & 1], (chunk >> 1) & 1u);
+    return __syncthreads_or(!there) == 0;
+  };
+  if (threadIdx.x >= 2 * 32 * BLOCKS) {
+    asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(COPY_REGISTERS));
+    fetch(0, 0);
+    for (int chunk = 0; chunk < chunks && arrived(chunk); ++chunk)
+      if (chunk + 1 < chunks) fetch(chunk + 1, (chunk + 1) & 1);
+    return;
+  }
+  asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WORK_REGISTERS));
 
-  // the warp's part of S': columns my_column (+ 8), key coordinates 8 n + pair (+ 1)
+  // what the two warps tell each other, a lane's numbers 32 floats apart
+  float* told = reinterpret_cast<float*>(base + Layout::kExchange) + block * (2 * EXCHANGED * 32) + lane;
+  float* told_too = told + EXCHANGED * 32;
+  int* any_odd = reinterpret_cast<int*>(base + Layout::kOdd) + 4 * block;
+  auto meet = [&]() { asm volatile("bar.sync %0, 64;" ::"r"(block + 1) : "memory"); };
+  auto tell = [&](float* to, const float (&x)[8][4]) {
+#pragma unroll
+    for (int n = 0; n < 8; ++n)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) to[32 * (4 * n + j)] = x[n][j];
+  };
+
+  // the warp's part of S': columns my_column (+ 8), key coordinates 8 n + pair (+ 1) of its half
   float* s_state = a.state + static_cast<size_t>(a.request_slot[request]) * a.state_stride +
                    static_cast<size_t>(head) * a.head_stride;
   const int lanes = a.vdim * a.parts;
-  const int my_column = column0 + 16 * warp + row;
-  float S[2 * STEPS][4];
+  const int my_column = column0 + 16 * block + row;
+  const int half_column = second ? 16 * HALF : 0;
+  float S[2 * HALF][4];
 #pragma unroll
-  for (int n = 0; n < 2 * STEPS; ++n)
+  for (int n = 0; n < 2 * HALF; ++n)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int c = my_column + 8 * (j >> 1), d = 8 * n + pair + (j & 1);
+      const int c = my_column + 8 * (j >> 1), d = half_column + 8 * n + pair + (j & 1);
       S[n][j] = c < a.vdim && d < a.dim
                     ? s_state[static_cast<size_t>(d & 15) * lanes + c * a.parts + (d >> 4)] : 0.0f;
     }
   // offsets of the lane's rows in the operands
-  const uint32_t row_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * STRIDE + (matrix & 1) * 8);
-  const uint32_t key_lane = 2 * (((matrix & 1) * 8 + in_matrix) * STRIDE + (matrix >> 1) * 8);
+  const uint32_t row_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * STRIDE + (matrix & 1) * 8 + half_column);
+  const uint32_t key_lane = 2 * (((matrix & 1) * 8 + in_matrix) * STRIDE + (matrix >> 1) * 8 + half_column);
   const uint32_t weight_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * WEIGHT_STRIDE + (matrix & 1) * 8);
-  const uint32_t value_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * value_stride + 16 * warp + (matrix & 1) * 8);
-  const int chunks = (count + CHUNK - 1) / CHUNK;
+  const uint32_t value_lane = 2 * (((matrix >> 1) * 8 + in_matrix) * value_stride + 16 * block + (matrix & 1) * 8);
   for (int chunk = 0; chunk < chunks; ++chunk) {
     const int stage = chunk & 1;
-    hx_cp_async_wait<0>();
-    __syncthreads();
-    if (chunk + 1 < chunks) fetch(chunk + 1, stage ^ 1);
+    if (!arrived(chunk)) {
+      if (threadIdx.x == 0 && a.status != nullptr) atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
+      for (int t = chunk * CHUNK + pair / 2; second && t < count; t += 4)
+        for (int c = my_column; c < min(a.vdim, my_column + 16); c += 8)
+          a.o[static_cast<size_t>(start + t) * (a.heads * a.vdim) + head * a.vdim + c] = __int_as_float(0x7fc00000);
+      return;
+    }
+    const float total = a.total[static_cast<size_t>(head) * a.rows + start + chunk * CHUNK];
     const uint32_t queries = hx_shared_address(queries_of(stage));
     const uint32_t keys = queries + 2 * CHUNK * STRIDE;
     const uint32_t weights = keys + 2 * CHUNK * STRIDE;
     const uint32_t values = weights + 2 * CHUNK * WEIGHT_STRIDE;
-    const float4* factors = reinterpret_cast<const float4*>(base + stage * layout.stage_bytes + layout.rows_bytes);
+    const float4* factors = reinterpret_cast<const float4*>(base + stage * Layout::kStageBytes + Layout::kRowsBytes);
+    const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
 
-    // S_0' q and S_0' k of all tokens, [16 columns x 64 tokens] each
-    float out[8][4], rest[8][4];
+    // S_0' k of all tokens, [16 columns x 64 tokens], over the warp's coordinates
+    float u[8][4];
+    {
+      float rest[8][4];
+      state_product<HALF>(rest, S, keys + row_lane, STRIDE);
+      if (second) tell(told, rest);
+      meet();
+      if (!second) {
+        // R: what the values leave to be written
 #pragma unroll
-    for (int n = 0; n < 8; ++n)
+        for (int step = 0; step < CHUNK / 16; ++step) {
+          uint32_t v[4];      // in the order of two neighbouring accumulator tiles
+          hx_ldmatrix_x4_trans(v, values + value_lane + 2 * (16 * step * value_stride));
 #pragma unroll
-      for (int j = 0; j < 4; ++j) out[n][j] = rest[n][j] = 0.0f;
+          for (int i = 0; i < 2; ++i) {
+            const int n = 2 * step + i;
+            const float4 f0 = factors[8 * n + pair], f1 = factors[8 * n + pair + 1];
 #pragma unroll
-    for (int step = 0; step < STEPS; ++step) {
-      uint32_t s0[4], s1[4], s2[4];
-      operand_terms(S, step, s0, s1, s2);
+            for (int j = 0; j < 4; ++j) rest[n][j] += told[32 * (4 * n + j)];
 #pragma unroll
-      for (int n = 0; n < 8; n += 2) {
-        uint32_t kf[4], qf[4];
-        hx_ldmatrix_x4(kf, keys + row_lane + 2 * (8 * n * STRIDE + 16 * step));
-        hx_ldmatrix_x4(qf, queries + row_lane + 2 * (8 * n * STRIDE + 16 * step));
-        hx_mma_bf16(rest[n], s2, kf[0], kf[1]);
-        hx_mma_bf16(rest[n + 1], s2, kf[2], kf[3]);
-        hx_mma_bf16(out[n], s2, qf[0], qf[1]);
-        hx_mma_bf16(out[n + 1], s2, qf[2], qf[3]);
-        hx_mma_bf16(rest[n], s1, kf[0], kf[1]);
-        hx_mma_bf16(rest[n + 1], s1, kf[2], kf[3]);
-        hx_mma_bf16(out[n], s1, qf[0], qf[1]);
-        hx_mma_bf16(out[n + 1], s1, qf[2], qf[3]);
+            for (int half = 0; half < 2; ++half) {
+              const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[2 * i + half]));
+              rest[n][2 * half] = fmaf(f0.z, x.x, -f0.y * rest[n][2 * half]);
+              rest[n][2 * half + 1] = fmaf(f1.z, x.y, -f1.y * rest[n][2 * half + 1]);
+            }
+          }
+        }
+        triangular_product(u, rest, weights + weight_lane);
+        tell(told, u);
+        meet();
+        state_product<HALF>(rest, S, queries + row_lane, STRIDE);
+        tell(told_too, rest);
+        meet();
       }
     }
+    float out[8][4];
+    bool odd_here = false;
+    if (second) {
+      state_product<HALF>(out, S, queries + row_lane, STRIDE);
+      meet();
 #pragma unroll
-    for (int step = 0; step < STEPS; ++step) {
-      uint32_t s0[4];
-      operand_high(S, step, s0);
+      for (int n = 0; n < 8; ++n)
 #pragma unroll
-      for (int n = 0; n < 8; n += 2) {
-        uint32_t kf[4], qf[4];
-        hx_ldmatrix_x4(kf, keys + row_lane + 2 * (8 * n * STRIDE + 16 * step));
-        hx_ldmatrix_x4(qf, queries + row_lane + 2 * (8 * n * STRIDE + 16 * step));
-        hx_mma_bf16(rest[n], s0, kf[0], kf[1]);
-        hx_mma_bf16(rest[n + 1], s0, kf[2], kf[3]);
-        hx_mma_bf16(out[n], s0, qf[0], qf[1]);
-        hx_mma_bf16(out[n + 1], s0, qf[2], qf[3]);
-      }
-    }
-    // R: what the values leave to be written
+        for (int j = 0; j < 4; ++j) u[n][j] = told[32 * (4 * n + j)];
+      float written[8][4];
+      triangular_product(written, u, weights + weight_lane + 2 * TERMS * CHUNK);
+      meet();
+      float odd = 0.0f;      // NaN with any number that is not finite (zero times it is)
 #pragma unroll
-    for (int step = 0; step < CHUNK / 16; ++step) {
-      uint32_t v[4];      // in the order of two neighbouring accumulator tiles
-      hx_ldmatrix_x4_trans(v, values + value_lane + 2 * (16 * step * value_stride));
+      for (int n = 0; n < 8; ++n) {
+        const float by[2] = {factors[8 * n + pair].x, factors[8 * n + pair + 1].x};
 #pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int n = 2 * step + i;
-        const float4 f0 = factors[8 * n + pair], f1 = factors[8 * n + pair + 1];
-#pragma unroll
-        for (int half = 0; half < 2; ++half) {
-          const float2 x = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&v[2 * i + half]));
-          rest[n][2 * half] = fmaf(f0.z, x.x, -f0.y * rest[n][2 * half]);
-          rest[n][2 * half + 1] = fmaf(f1.z, x.y, -f1.y * rest[n][2 * half + 1]);
-          out[n][2 * half] *= f0.x;
-          out[n][2 * half + 1] *= f1.x;
+        for (int j = 0; j < 4; ++j) {
+          out[n][j] = fmaf(out[n][j] + told_too[32 * (4 * n + j)], by[j & 1], written[n][j]);
+          odd = fmaf(out[n][j], 0.0f, odd);
         }
       }
+      odd_here = odd != 0.0f;
     }
-    float u[8][4];
-    triangular_product(u, rest, weights + weight_lane);
-    triangular_product(rest, u, weights + weight_lane + 2 * TERMS * CHUNK);
-    const int first = start + chunk * CHUNK, live = min(CHUNK, count - chunk * CHUNK);
-    float odd = 0.0f;      // NaN with any number that is not finite (zero times it is)
+    // what the chunk adds to the state, in terms
+    float odd = 0.0f;
 #pragma unroll
     for (int n = 0; n < 8; ++n)
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        out[n][j] += rest[n][j];
         u[n][j] *= factors[8 * n + pair + (j & 1)].w;
-        odd = fmaf(out[n][j], 0.0f, fmaf(u[n][j], 0.0f, odd));
+        odd = fmaf(u[n][j], 0.0f, odd);
       }
-    if (__any_sync(0xffffffffu, odd != 0.0f)) {
-      const __nv_bfloat16* staged = queries_of(stage);
-      float held[2 * STEPS][4];
-#pragma unroll
-      for (int n = 0; n < 2 * STEPS; ++n)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) held[n][j] = S[n][j];
-      tokens_in_turn<2 * STEPS>(a, held, staged, staged + CHUNK * STRIDE, STRIDE,
-                                staged + CHUNK * (2 * STRIDE + WEIGHT_STRIDE) + 16 * warp + row, value_stride,
-                                first, live, head, my_column);
-#pragma unroll
-      for (int n = 0; n < 2 * STEPS; ++n)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) S[n][j] = held[n][j];
-      continue;
+    if (second) {
+      odd_here = __any_sync(0xffffffffu, odd_here || odd != 0.0f);
+      if (lane == 0) *any_odd = odd_here ? 1 : 0;
     }
-#pragma unroll
-    for (int n = 0; n < 8; ++n)
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const int t = 8 * n + pair + (j & 1), c = my_column + 8 * (j >> 1);
-        if (t < live && c < a.vdim)
-          a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j];
-      }
-    // The state behind the chunk.  What the chunk adds is summed by itself and meets the state in one
-    // multiply-add: the tensor cores cut off what a sum of theirs cannot hold, and onto the state itself
-    // they would do so a dozen times a chunk.
-    const float total = factors[CHUNK].x;
     uint32_t u0[CHUNK / 16][4], u1[CHUNK / 16][4], u2[CHUNK / 16][4];
 #pragma unroll
     for (int step = 0; step < CHUNK / 16; ++step) operand_terms(u, step, u0[step], u1[step], u2[step]);
+    meet();
+    if (*any_odd != 0) {
+      // the first warp goes through the tokens with all of S'
+      if (second) {
 #pragma unroll
-    for (int n0 = 0; n0 < STEPS; n0 += 2) {
-      float added[4][4];
+        for (int n = 0; n < 2 * HALF; ++n)
 #pragma unroll
-      for (int n = 0; n < 4; ++n)
+          for (int j = 0; j < 4; ++j) told[32 * (4 * n + j)] = S[n][j];
+      }
+      meet();
+      if (!second) {
+        const __nv_bfloat16* staged = queries_of(stage);
+        float held[2 * STEPS][4];
+#pragma unroll
+        for (int n = 0; n < 2 * HALF; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            held[n][j] = S[n][j];
+            held[2 * HALF + n][j] = told[32 * (4 * n + j)];
+          }
+        tokens_in_turn<2 * STEPS>(a, held, staged, staged + CHUNK * STRIDE, STRIDE,
+                                  staged + CHUNK * (2 * STRIDE + WEIGHT_STRIDE) + 16 * block + row, value_stride,
+                                  first, live, head, my_column);
+#pragma unroll
+        for (int n = 0; n < 2 * HALF; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            S[n][j] = held[n][j];
+            told[32 * (4 * n + j)] = held[2 * HALF + n][j];
+          }
+      }
+      meet();
+      if (second) {
+#pragma unroll
+        for (int n = 0; n < 2 * HALF; ++n)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) S[n][j] = told[32 * (4 * n + j)];
+      }
+      continue;
+    }
+    if (second) {
+#pragma unroll
+      for (int n = 0; n < 8; ++n)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int t = 8 * n + pair + (j & 1), c = my_column + 8 * (j >> 1);
+          if (t < live && c < a.vdim)
+            a.o[static_cast<size_t>(first + t) * (a.heads * a.vdim) + head * a.vdim + c] = out[n][j];
+        }
+    }
+    // The state behind the chunk.  What the chunk adds is summed by itself and meets the state in one
+    // multiply-add: the tensor cores cut off what a sum of theirs cannot hold, and onto the state itself
+    // they would do so a dozen times a chunk.
+    constexpr int TURN = HALF % 2 == 0 ? 2 : 1;      // steps of key coordinates side by side
+#pragma unroll
+    for (int n0 = 0; n0 < HALF; n0 += TURN) {
+      float added[2 * TURN][4];
+#pragma unroll
+      for (int n = 0; n < 2 * TURN; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) added[n][j] = 0.0f;
+      uint32_t b[2][TURN][4];      // of a step of tokens, asked for while the products of the one before run
+      auto keys_of = [&](int step, int slot) {
+#pragma unroll
+        for (int n = 0; n < TURN; ++n)
+          hx_ldmatrix_x4_trans(b[slot][n], keys + key_lane + 2 * (16 * step * STRIDE + 16 * (n0 + n)));
+      };
+      auto added_by = [&](const uint32_t (&ut)[4], int slot) {
+#pragma unroll
+        for (int n = 0; n < TURN; ++n) {
+          hx_mma_bf16(added[2 * n], ut, b[slot][n][0], b[slot][n][1]);
+          hx_mma_bf16(added[2 * n + 1], ut, b[slot][n][2], b[slot][n][3]);
+        }
+      };
+      keys_of(0, 0);
 #pragma unroll
       for (int step = 0; step < CHUNK / 16; ++step) {
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          uint32_t b[4];
-          hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * (n0 + n)));
-          hx_mma_bf16(added[2 * n], u2[step], b[0], b[1]);
-          hx_mma_bf16(added[2 * n + 1], u2[step], b[2], b[3]);
-          hx_mma_bf16(added[2 * n], u1[step], b[0], b[1]);
-          hx_mma_bf16(added[2 * n + 1], u1[step], b[2], b[3]);
-        }
+        keys_of((step + 1) % (CHUNK / 16), (step + 1) & 1);
+        added_by(u2[step], step & 1);
+        added_by(u1[step], step & 1);
       }
 #pragma unroll
       for (int step = 0; step < CHUNK / 16; ++step) {
-#pragma unroll
-        for (int n = 0; n < 2; ++n) {
-          uint32_t b[4];
-          hx_ldmatrix_x4_trans(b, keys + key_lane + 2 * (16 * step * STRIDE + 16 * (n0 + n)));
-          hx_mma_bf16(added[2 * n], u0[step], b[0], b[1]);
-          hx_mma_bf16(added[2 * n + 1], u0[step], b[2], b[3]);
-        }
+        if (step + 1 < CHUNK / 16) keys_of(step + 1, (step + 1) & 1);
+        added_by(u0[step], step & 1);
       }
 #pragma unroll
-      for (int n = 0; n < 4; ++n)
+      for (int n = 0; n < 2 * TURN; ++n)
 #pragma unroll
         for (int j = 0; j < 4; ++j) S[2 * n0 + n][j] = fmaf(total, S[2 * n0 + n][j], added[n][j]);
     }
   }
 #pragma unroll
-  for (int n = 0; n < 2 * STEPS; ++n)
+  for (int n = 0; n < 2 * HALF; ++n)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const int c = my_column + 8 * (j >> 1), d = 8 * n + pair + (j & 1);
+      const int c = my_column + 8 * (j >> 1), d = half_column + 8 * n + pair + (j & 1);
       if (c < a.vdim && d < a.dim)
         s_state[static_cast<size_t>(d & 15) * lanes + c * a.parts + (d >> 4)] = S[n][j];
     }
@@ -725,14 +928,15 @@ __global__ __launch_bounds__(256, 1) void delta_states_kernel(const __grid_const
 
 template <int STEPS>
 int launch_delta(const DeltaArgs& a, int tiles, cudaStream_t stream) {
-  const int shared = DeltaLayout(16 * STEPS, a.column_warps).bytes, first = weights_shared(16 * STEPS);
+  constexpr int shared = DeltaLayout<16 * STEPS>::kBytes;
+  const int first = weights_shared(16 * STEPS);
   static std::once_flag once;
   static bool configured = false;
   std::call_once(once, [first] {
     configured = cudaFuncSetAttribute(delta_weights_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                       first) == cudaSuccess &&
                  cudaFuncSetAttribute(delta_states_kernel<STEPS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                      227 * 1024) == cudaSuccess;
+                                      shared) == cudaSuccess;
     if (!configured) cudaGetLastError();
   });
   if (!configured) {
@@ -740,9 +944,8 @@ int launch_delta(const DeltaArgs& a, int tiles, cudaStream_t stream) {
     return HX_ERR_LAUNCH;
   }
   hx_launch(delta_weights_kernel<STEPS>, dim3(tiles, a.heads), 128, first, stream, a);
-  const int block_columns = 16 * a.column_warps;
-  hx_launch(delta_states_kernel<STEPS>, dim3(a.portions, a.heads, (a.vdim + block_columns - 1) / block_columns),
-            32 * a.column_warps, shared, stream, a);
+  hx_launch(delta_states_kernel<STEPS>, dim3(a.portions, a.heads, (a.vdim + BLOCK_COLUMNS - 1) / BLOCK_COLUMNS),
+            STATES_THREADS, shared, stream, a);
   return HX_OK;
 }
 
@@ -764,15 +967,17 @@ HX_API long long hx_delta_chunks_scratch(int heads, int tokens) {
 // hx_delta_chunks_scratch bytes on 16 bytes.  tiles: at least the chunks of 64 tokens in the step,
 // counted request by request.
 // Requests that bring fewer than min_query_len tokens are left alone (hx_linear_state_scan_below takes
-// them); portions: how many bring as many, tiles: the chunks of those.
-HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+// them); portions: how many bring as many, tiles: the chunks of those.  status: the device status word, or
+// null; a wait that runs out leaves NaN in the outputs besides.
+HX_API int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
                                 const void* decay_in, const void* beta_in, int ld_gates,
                                 const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
                                 int unit_norm, float unit_eps, float q_scale, float k_scale,
                                 void* scratch, float* state, long long state_stride, int head_stride,
                                 float* o, const int* request_start, const int* request_slot,
                                 int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
-                                int vdim, int min_query_len, int portions, cudaStream_t stream) {
+                                int vdim, int min_query_len, int portions, int* status,
+                                cudaStream_t stream) {
   HX_REQUIRE(hx_delta_chunks_supports(dim, vdim), "hx_delta_chunks: heads of %d by %d are not supported",
              dim, vdim);
   HX_REQUIRE(requests >= 0 && tokens >= requests && min_query_len > 0 && portions >= 0 &&
@@ -791,12 +996,6 @@ HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k
   HX_REQUIRE(head_stride >= state_floats(vdim, dim), "hx_delta_chunks: a head's state takes %d floats, not %d",
              state_floats(vdim, dim), head_stride);
   if (portions == 0) return HX_OK;
-  // four warps of 16 columns a CTA, one for each quarter of an SM (the staged chunks leave room for
-  // one CTA); eight where there are more CTAs than SMs, so that a chunk is staged for twice as many
-  const int sms = hx_device_sm_count();
-  if (sms <= 0) return HX_ERR_LAUNCH;
-  const long long ctas = static_cast<long long>(portions) * heads * ((vdim + 63) / 64);
-  const int column_warps = vdim > 64 && ctas > sms ? 8 : vdim > 32 ? 4 : (vdim + 15) / 16;
   const size_t rows = static_cast<size_t>(heads) * tokens;
   float4* factors = static_cast<float4*>(scratch);
   __nv_bfloat16* weights = reinterpret_cast<__nv_bfloat16*>(factors + rows);
@@ -806,8 +1005,8 @@ HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k
                     static_cast<const __nv_bfloat16*>(decay_in), static_cast<const __nv_bfloat16*>(beta_in),
                     ld_gates, a_log, dt_bias, fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, weights,
                     factors, total, tokens, state, state_stride, head_stride, o, request_start, request_slot,
-                    requests, heads, qk_heads, dim, vdim, parts_for(dim), column_warps, min_query_len,
-                    portions};
+                    requests, heads, qk_heads, dim, vdim, parts_for(dim), min_query_len,
+                    portions, status};
   int rc;
   switch ((dim + 15) / 16) {
     case 1: case 2: rc = launch_delta<2>(a, tiles, stream); break;
@@ -819,6 +1018,20 @@ HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k
   hx_count_launches(1);
   HX_CHECK_LAUNCH("hx_delta_chunks");
   return HX_OK;
+}
+
+HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                                const void* decay_in, const void* beta_in, int ld_gates,
+                                const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
+                                int unit_norm, float unit_eps, float q_scale, float k_scale,
+                                void* scratch, float* state, long long state_stride, int head_stride,
+                                float* o, const int* request_start, const int* request_slot,
+                                int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
+                                int vdim, int min_query_len, int portions, cudaStream_t stream) {
+  return hx_delta_chunks_checked(q, ld_q, k, ld_k, v, ld_v, decay_in, beta_in, ld_gates, a_log, dt_bias,
+                                 fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, scratch, state, state_stride,
+                                 head_stride, o, request_start, request_slot, requests, tokens, tiles, heads,
+                                 qk_heads, dim, vdim, min_query_len, portions, nullptr, stream);
 }
 
 // Every request of the step.

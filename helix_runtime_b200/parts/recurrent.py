@@ -444,7 +444,8 @@ class LinearState(Mixer):
             ops.delta_chunks(q, k, v, state, o, scratch, ctx.request_start, ctx.request_slot,
                              ctx.n_requests, n, ops.recurrence_tiles(portions), self.heads,
                              self.qk_heads, self.head_dim, self.value_dim,
-                             min_query_len=chunks_from, portions=len(portions), **gates)
+                             min_query_len=chunks_from, portions=len(portions),
+                             status=ctx.status, **gates)
         if chunks_from != 1:
             longest = max((length for length in ctx.host_query_lengths if length < chunks_from),
                           default=0) if chunks_from > 0 else 0
