@@ -149,7 +149,23 @@ __device__ __forceinline__ void filter_input8(const FilterArgs<__nv_bfloat16>& a
   }
 }
 
-template <int TAPS, bool SUMS>
+__device__ __forceinline__ uint64_t float_pair(float low, float high) {
+  uint64_t pair;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(pair) : "f"(low), "f"(high));
+  return pair;
+}
+__device__ __forceinline__ void float_pair_halves(uint64_t pair, float& low, float& high) {
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(pair));
+}
+__device__ __forceinline__ uint64_t float_pair_fma(uint64_t x, uint64_t y, uint64_t z) {
+  uint64_t r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
+  return r;
+}
+
+// BIASED: inputs have a bias, which the state holds and the rows do not; the first tokens of a portion then
+// go a road of their own.
+template <int TAPS, bool SUMS, bool BIASED>
 __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const FilterArgs<__nv_bfloat16> a,
                                                                    int tokens, int run) {
   constexpr int REACH = TAPS - 1;
@@ -180,7 +196,7 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     b[i] = a.bias != nullptr ? a.bias[c + i] : 0.0f;
-    in_bias[i] = a.in_bias != nullptr ? a.in_bias[c + i] : 0.0f;
+    in_bias[i] = BIASED ? a.in_bias[c + i] : 0.0f;
   }
   int request = a.token_request[first];
   int start = a.request_start[request];
@@ -218,39 +234,30 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
       return packed;
     }
   };
-  auto tap = [&](const uint4& packed, int j, float (&y)[8]) {
-    const __nv_bfloat162* pairs = reinterpret_cast<const __nv_bfloat162*>(&packed);
+  // two channels an instruction, each rounded as its scalar form
+  uint64_t w2[TAPS][4], inside[4];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const float2 v = __bfloat1622float2(pairs[i]);
-      y[2 * i] = fmaf(w[j][2 * i], v.x, y[2 * i]);
-      y[2 * i + 1] = fmaf(w[j][2 * i + 1], v.y, y[2 * i + 1]);
+  for (int i = 0; i < 4; ++i) {
+    float sums[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      float sum = 0.0f;
+#pragma unroll
+      for (int j = 0; j < TAPS; ++j) sum += w[j][2 * i + k];
+      sums[k] = fmaf(sum, in_bias[2 * i + k], b[2 * i + k]);
     }
-  };
-  float inside[8];
+    inside[i] = float_pair(sums[0], sums[1]);
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    float sum = 0.0f;
-#pragma unroll
-    for (int j = 0; j < TAPS; ++j) sum += w[j][i];
-    inside[i] = fmaf(sum, in_bias[i], b[i]);
+    for (int j = 0; j < TAPS; ++j) w2[j][i] = float_pair(w[j][2 * i], w[j][2 * i + 1]);
   }
-  uint4 rows[TAPS];
+  auto unpack = [](const uint4& packed, uint64_t (&x)[4]) {
+    const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
 #pragma unroll
-  for (int j = 0; j < REACH; ++j)
-    rows[j] = first - REACH + j >= start ? packed_input(first - REACH + j) : make_uint4(0u, 0u, 0u, 0u);
-  // the next tokens' inputs are in flight while a token is worked on
-  constexpr int AHEAD = SUMS ? 1 : 4;
-  uint4 ahead[AHEAD];
-#pragma unroll
-  for (int k = 0; k < AHEAD; ++k)
-    ahead[k] = first + k < last ? packed_input(first + k) : make_uint4(0u, 0u, 0u, 0u);
-#pragma unroll 1
-  for (int token = first; token < last; ++token) {
-    rows[REACH] = ahead[0];
-#pragma unroll
-    for (int k = 0; k + 1 < AHEAD; ++k) ahead[k] = ahead[k + 1];
-    if (token + AHEAD < last) ahead[AHEAD - 1] = packed_input(token + AHEAD);
+    for (int i = 0; i < 4; ++i)
+      x[i] = float_pair(__uint_as_float(words[i] << 16), __uint_as_float(words[i] & 0xffff0000u));
+  };
+  int token = first;
+  while (token < last) {
     if (token >= end) {
       request = a.token_request[token];
       start = a.request_start[request];
@@ -258,16 +265,95 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
       slot = a.request_slot[request];
     }
     const int index = token - start;
-    if (index >= REACH) {
-      float y[8];
+    if (index >= REACH || (!BIASED && index == 0 && end - start > 1)) {
+      // RING tokens at a time: a row is unpacked once, and the rows of the RING tokens behind are on their way
+      // meanwhile.  The thread of a portion's first token begins with the state's rows, takes all the tokens
+      // that these reach, and writes the new state.
+      constexpr int RING = 4;
+      const bool from_state = !BIASED && REACH > 0 && index == 0;
+      const int stop = min(end, from_state ? max(last, start + REACH) : last);
+      uint4 ahead[RING];
+      uint64_t rows[REACH + RING][4];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) y[i] = inside[i];
+      for (int k = 0; k < RING; ++k) ahead[k] = packed_input(min(token + k, stop - 1));
+      if (from_state) {
+        const int count = end - start;
+        float* state = a.state + static_cast<size_t>(slot) * a.state_stride + c;
+        uint4 newest[REACH > 0 ? REACH : 1];
 #pragma unroll
-      for (int j = 0; j < TAPS; ++j) tap(rows[j], j, y);
-      emit(token, y);
-    } else if (index == 0) {
-      // the portion's first token: the tokens whose filter reaches behind the portion, then
-      // the new state (see the scalar kernel)
+        for (int r = 0; r < REACH; ++r) {
+          const float* source = state + static_cast<size_t>(r) * a.channels;
+          if (wide_state) {
+            const float4 lo = reinterpret_cast<const float4*>(source)[0], hi = reinterpret_cast<const float4*>(source)[1];
+            rows[r][0] = float_pair(lo.x, lo.y), rows[r][1] = float_pair(lo.z, lo.w);
+            rows[r][2] = float_pair(hi.x, hi.y), rows[r][3] = float_pair(hi.z, hi.w);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) rows[r][i] = float_pair(source[2 * i], source[2 * i + 1]);
+          }
+          newest[r] = packed_input(start + max(count - REACH + r, 0));
+        }
+#pragma unroll
+        for (int r = 0; r < REACH; ++r) {
+          // a portion shorter than the filter's reach: what it does not cover moves up from the old rows
+          uint64_t x[4];
+          unpack(newest[r], x);
+          float* target = state + static_cast<size_t>(r) * a.channels;
+          float y[8];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+#pragma unroll
+            for (int k = 2; k < REACH; ++k) x[i] = count + r == k ? rows[k][i] : x[i];
+            float_pair_halves(x[i], y[2 * i], y[2 * i + 1]);
+          }
+          if (wide_state) {
+            reinterpret_cast<float4*>(target)[0] = make_float4(y[0], y[1], y[2], y[3]);
+            reinterpret_cast<float4*>(target)[1] = make_float4(y[4], y[5], y[6], y[7]);
+          } else {
+#pragma unroll
+            for (int i = 0; i < 8; ++i) target[i] = y[i];
+          }
+        }
+      } else {
+        uint4 early[REACH > 0 ? REACH : 1];
+#pragma unroll
+        for (int j = 0; j < REACH; ++j) early[j] = packed_input(token - REACH + j);
+#pragma unroll
+        for (int j = 0; j < REACH; ++j) unpack(early[j], rows[j]);
+      }
+#pragma unroll 1
+      for (; token < stop; token += RING) {
+#pragma unroll
+        for (int k = 0; k < RING; ++k) unpack(ahead[k], rows[REACH + k]);
+        if (token + RING < stop) {
+#pragma unroll
+          for (int k = 0; k < RING; ++k) ahead[k] = packed_input(min(token + RING + k, stop - 1));
+        }
+#pragma unroll
+        for (int k = 0; k < RING; ++k) {
+          if (token + k < stop) {
+            float y[8];
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+              uint64_t sum = inside[i];
+#pragma unroll
+              for (int j = 0; j < TAPS; ++j) sum = float_pair_fma(w2[j][i], rows[k + j][i], sum);
+              float_pair_halves(sum, y[2 * i], y[2 * i + 1]);
+            }
+            emit(token + k, y);
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < REACH; ++j)
+#pragma unroll
+          for (int i = 0; i < 4; ++i) rows[j][i] = rows[RING + j][i];
+      }
+      token = stop;
+      continue;
+    }
+    if (index == 0 && (BIASED || end - start == 1)) {
+      // A portion of one token, or (BIASED) the first tokens of any portion: their filter reaches behind the
+      // portion.  Then the new state (see the scalar kernel).
       const int count = end - start;
       float* state = a.state + static_cast<size_t>(slot) * a.state_stride + c;
       // the input at a place of the portion, or in front of it the state's
@@ -285,7 +371,7 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
           for (int i = 0; i < 8; ++i) x[i] = state[static_cast<size_t>(place + REACH) * a.channels + i];
         }
       };
-      if (count == 1) {
+      if (!BIASED || count == 1) {
         // a decoded token: its filter reads the state and itself, and the state moves up by one
         float x[TAPS][8], y[8];
 #pragma unroll
@@ -333,8 +419,7 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
         }
       }
     }
-#pragma unroll
-    for (int j = 0; j < REACH; ++j) rows[j] = rows[j + 1];
+    token = min(start + REACH, end);      // (with index 1 .. REACH - 1: the first token's thread makes them)
   }
 }
 
@@ -349,11 +434,11 @@ bool filter_pieces_apply(const FilterArgs<__nv_bfloat16>& a) {
 template <int TAPS>
 void launch_filter_pieces(const FilterArgs<__nv_bfloat16>& a, dim3 grid, int block, int tokens, int run,
                           bool sums, cudaStream_t stream) {
-  if (sums) {
-    hx_launch(causal_filter_pieces_kernel<TAPS, true>, grid, block, 0, stream, a, tokens, run);
-  } else {
-    hx_launch(causal_filter_pieces_kernel<TAPS, false>, grid, block, 0, stream, a, tokens, run);
-  }
+  const bool biased = a.in_bias != nullptr;
+  auto kernel = sums ? (biased ? causal_filter_pieces_kernel<TAPS, true, true> : causal_filter_pieces_kernel<TAPS, true, false>)
+                     : (biased ? causal_filter_pieces_kernel<TAPS, false, true>
+                               : causal_filter_pieces_kernel<TAPS, false, false>);
+  hx_launch(kernel, grid, block, 0, stream, a, tokens, run);
 }
 
 int launch_filter(const FilterArgs<__nv_bfloat16>& a, int tokens, cudaStream_t stream) {
@@ -362,10 +447,18 @@ int launch_filter(const FilterArgs<__nv_bfloat16>& a, int tokens, cudaStream_t s
               stream, a);
     return HX_OK;
   }
-  const int run = tokens >= 1024 ? 8 : (tokens >= 256 ? 4 : 1);
   const int pieces = a.channels / 8;
   const int block = pieces >= 256 ? 256 : ((pieces + 31) / 32) * 32;
-  const dim3 grid((tokens + run - 1) / run, (pieces + block - 1) / block);
+  const int blocks = (pieces + block - 1) / block;
+  // As many tokens a thread (in fours, which it works on side by side, from three on) as let the CTAs, two an
+  // SM, run at once: a second round is a second chain of weights, request and rows.  Measured, with 8 tokens a thread
+  // from 1,024 tokens on, 4 from 256 on, and this (us, alone): two portions of 1,720 tokens in all of 8,192 channels
+  // 25.3 -> 16.7, 2,048 of 4,096 12.8 -> 7.0, 300 of 8,192 8.7 -> 6.5, two of 100 8.2 -> 4.5, 64 decoded tokens 4.7, 4.7.
+  const int sms = hx_device_sm_count();
+  if (sms <= 0) return HX_ERR_LAUNCH;
+  const long long share = (static_cast<long long>(tokens) * blocks + 2ll * sms - 1) / (2ll * sms);
+  const int run = static_cast<int>(share <= 2 ? (share < 1 ? 1 : share) : (share + 3) / 4 * 4);
+  const dim3 grid((tokens + run - 1) / run, blocks);
   const bool sums = a.accum != nullptr;
   switch (a.taps) {
     case 1: launch_filter_pieces<1>(a, grid, block, tokens, run, sums, stream); break;
@@ -941,7 +1034,8 @@ void linear_state_scan_kernel(const LinearStateArgs<T> a) {
 // (v = y silu(g); out = v / rms(v) * w); 1: after it (out = y / rms(y) * w * silu(g)).
 // A warp a group, four values a load, the group's values in registers between the sum and the
 // store: bfloat16 groups of up to 128 PIECES channels, in fours (1,725 tokens of 32 groups of 128: 59 us
-// with a CTA of 128 threads a group, 18 now).
+// with a CTA of 128 threads a group, 18 so; four groups
+// a warp, their loads in flight together, 28).
 template <int PIECES>
 __global__ __launch_bounds__(256) void gated_group_norm_pieces_kernel(
     const float* __restrict__ y, int ld_y, const __nv_bfloat16* __restrict__ gate, int ld_gate,
