@@ -116,13 +116,13 @@ __global__ __launch_bounds__(128) void latent_prepare_kernel(const LatentPrepare
 
 // One CTA a token: the angles' sines and cosines once, then every head.  q_rot [tokens, ld_q] holds
 // heads * rot rotated-part coordinates from column rot_offset on.  (2,048 tokens of 32 heads with 64
-// coordinates: 67 us with a CTA and its own angles for every head, 14 now.)
+// coordinates: 67 us with a CTA and its own angles for every head, 14 a coordinate a thread, 7 in pieces of eight.)
 template <typename T>
 __global__ __launch_bounds__(256) void latent_queries_kernel(
     const T* __restrict__ q, int ld_q, int rot_offset, T* __restrict__ rows, int ld_rows,
     const int* __restrict__ positions, const float* __restrict__ freq,
     const double* __restrict__ freq_exact, int rotary_dims, int layout, int heads, int kv_rank,
-    int rot, int row_dim, float amplitude) {
+    int rot, int row_dim, float amplitude, bool pieces) {
   constexpr bool EXACT = sizeof(T) == 4;
   extern __shared__ float2 turns[];      // [rotary_dims / 2]: cosine, sine
   hx_pdl_prologue();
@@ -137,6 +137,35 @@ __global__ __launch_bounds__(256) void latent_queries_kernel(
   const T* parts = q + static_cast<size_t>(token) * ld_q + rot_offset;
   T* row = rows + static_cast<size_t>(token) * ld_rows + kv_rank;
   const int extra = row_dim - kv_rank, half = rotary_dims >> 1;
+  if constexpr (!EXACT) {
+    if (pieces) {
+      for (int index = threadIdx.x; index < heads * (extra / 8); index += blockDim.x) {
+        const int head = index / (extra / 8), e = 8 * (index - head * (extra / 8));
+        const T* part = parts + head * rot;
+        uint4 packed = make_uint4(0u, 0u, 0u, 0u);
+        if (e < rot) packed = *reinterpret_cast<const uint4*>(part + e);
+        if (e < rotary_dims) {
+          const bool leads = e < half;
+          uint4 other = packed;
+          if (layout != 0) other = *reinterpret_cast<const uint4*>(part + (leads ? e + half : e - half));
+          T* x = reinterpret_cast<T*>(&packed);
+          const T* y = reinterpret_cast<const T*>(&other);
+          float turned[8];
+#pragma unroll
+          for (int i = 0; i < 8; ++i) {
+            const bool first = layout == 0 ? (i & 1) == 0 : leads;
+            const float2 turn = turns[layout == 0 ? (e + i) >> 1 : leads ? e + i : e + i - half];
+            const float v = hx_to_float<T>(x[i]), partner = hx_to_float<T>(y[layout == 0 ? i ^ 1 : i]);
+            turned[i] = first ? v * turn.x - partner * turn.y : v * turn.x + partner * turn.y;
+          }
+#pragma unroll
+          for (int i = 0; i < 8; ++i) x[i] = hx_from_float<T>(turned[i]);
+        }
+        *reinterpret_cast<uint4*>(row + static_cast<size_t>(head) * row_dim + e) = packed;
+      }
+      return;
+    }
+  }
   for (int index = threadIdx.x; index < heads * extra; index += blockDim.x) {
     const int head = index / extra, e = index - head * extra;
     const T* part = parts + head * rot;
@@ -209,12 +238,16 @@ HX_API int hx_latent_queries(const void* q, int ld_q, int rot_offset, void* rows
   if (dtype == HX_F32) {
     hx_launch(latent_queries_kernel<float>, tokens, 256, shared, stream, static_cast<const float*>(q),
               ld_q, rot_offset, static_cast<float*>(rows), ld_rows, positions, freq, freq_exact,
-              rotary_dims, layout, heads, kv_rank, rot, row_dim, amplitude);
+              rotary_dims, layout, heads, kv_rank, rot, row_dim, amplitude, false);
   } else if (dtype == HX_BF16) {
+    // eight coordinates a thread where they lie and turn in whole pieces of 16 bytes
+    const bool pieces = kv_rank % 8 == 0 && rot % 8 == 0 && row_dim % 8 == 0 && ld_q % 8 == 0 &&
+                        rot_offset % 8 == 0 && ld_rows % 8 == 0 && rotary_dims % (layout == 0 ? 8 : 16) == 0 &&
+                        ((reinterpret_cast<uintptr_t>(q) | reinterpret_cast<uintptr_t>(rows)) & 15) == 0;
     hx_launch(latent_queries_kernel<__nv_bfloat16>, tokens, 256, shared, stream,
               static_cast<const __nv_bfloat16*>(q), ld_q, rot_offset,
               static_cast<__nv_bfloat16*>(rows), ld_rows, positions, freq, freq_exact, rotary_dims,
-              layout, heads, kv_rank, rot, row_dim, amplitude);
+              layout, heads, kv_rank, rot, row_dim, amplitude, pieces);
   } else {
     HX_REQUIRE(false, "hx_latent_queries: unknown dtype %d", dtype);
   }
