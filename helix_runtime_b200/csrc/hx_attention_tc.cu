@@ -9,10 +9,10 @@
 //               one: the keys of a (page, head) are one contiguous block of the cache and so are
 //               its values, so a tile is a handful of bulk copies (cp.async.bulk counted on an
 //               mbarrier) into a ring of stages;
-//   warp 1      one lane issues S = Q K^T into one of two score buffers in tensor memory;
+//   warp 1      one lane issues S = Q K^T into one of two (four) score buffers in tensor memory;
 //   warp 2      one lane issues O += P V;
 //   warp 3      (pages of 32 and 64 keys) rewrites the keys of a landed tile piece-major over all 64
-//               keys (see below);
+//               keys (see below); (pages of 16, heads wider than 128) one lane asks for the values;
 //   warps 4-7   softmax: thread r owns query row r.  It reads its row of S from tensor memory,
 //               keeps the running maximum and sum in float32 registers and writes the
 //               probabilities back over the scores it has read, as TWO bfloat16 terms (P = hi + lo,
@@ -22,7 +22,7 @@
 //               when a tile exceeds it by more than 2^8 (any fixed reference gives the same
 //               quotient; float32 has the range), so the pass over O that a new maximum costs is
 //               rare;
-//   warps 8-11  (the same, heads wider than 128) three more to rewrite keys.
+//   warps 8-11  (heads wider than 128) three more to rewrite keys, or a second group of softmax warps.
 //
 // Heads of up to 128: two CTAs share an SM.  A tile's way through a CTA is a chain (products,
 // softmax, products), and what a CTA spends before its first and after its last tile is several
@@ -31,8 +31,17 @@
 // size).
 // Measured (2,048 tokens, 32 heads of 128, in place): 129 us a layer with two lanes of 128 rows in one
 // CTA and four issuing threads, 108 with elect.sync, 87 with the softmax's arithmetic in pairs, 91
-// with two CTAs and 66 with their keys gathered.  Wide heads (2,048 tokens, 32 heads of 256 over
-// one cached row, window 1,024): 610 us on mma.sync, 127 here.
+// with two CTAs and 66 with their keys gathered.
+//
+// Wider heads leave one CTA an SM (64 KB of queries, a page's values 8 KB).  There a tile of an even turn and
+// one of an odd turn go through two groups of softmax warps, with four score buffers, so that scores are
+// multiplied while the output products of earlier tiles still run; the reference of a row is told from
+// group to group.  Measured (2,048 tokens, 32 heads of 256 over one cached row, window 1,024): 610 us on
+// mma.sync, 126 with one group and two buffers (2,850 cycles a tile), 128 with two groups, 112 with four
+// buffers (2,330), 104 with queries loaded four pieces a row and values asked for by a thread of their own, 96
+// with the 192 coordinates of the values that are wanted (and queries asked for before the second tile).
+// Of a CTA's 43,000 cycles 13,000 bring queries and first tiles in and the output out, which a second CTA
+// would hide.
 //
 // Operand layouts.  Nothing is swizzled: every operand is made of "core matrices" of 8 rows
 // x 16 bytes (128 contiguous bytes), which is exactly what a page block of the cache is made
@@ -56,7 +65,6 @@ namespace {
 
 constexpr int BLOCK_M = 128;   // query rows per CTA (the MMA's M)
 constexpr int BLOCK_N = 64;    // keys per tile
-constexpr int S_BUFFERS = 2;   // score tiles in tensor memory
 constexpr int WARP_PAGES = 0, WARP_SCORES = 1, WARP_OUTPUT = 2, WARP_REWRITE = 3, WARP_SOFTMAX = 4,
               WARP_MORE = 8;
 constexpr int GROUP_STRIDE = 128;             // bytes from one 8-row core matrix to the next row group
@@ -94,6 +102,8 @@ struct TcPrefillArgs {
   float softcap = 0.0f;   // > 0: the scaled score s becomes softcap * tanh(s / softcap)
   int pack = 1;           // packed kernels: the query heads of a key/value head, side by side in
                           // a tile's rows, token by token; the grid's x counts key/value heads
+  int value_dim = 0;      // packed kernels: so many leading coordinates of the values are wanted (a multiple
+                          // of 16); the others of `out` are not written
 };
 
 // Shared memory holds the queries, key tiles as they land (where they are rewritten), key tiles as
@@ -108,16 +118,21 @@ struct TcConfig {
   static constexpr int kCtas = D <= 128 ? 2 : 1;
   static constexpr int kKeyStages = GATHER ? 0 : 2, kValueStages = 2, kKeyBuffers = GATHER ? 3 : 1;
   static constexpr int kRewriters = GATHER ? 0 : D <= 128 ? 1 : 4;
-  static constexpr int kThreads = kRewriters <= 1 ? 256 : 384;
+  // Softmax warps: four, a row a thread; where the CTA has an SM to itself and no warp rewrites keys a second
+  // four take every other tile.
+  static constexpr int kSoftmaxGroups = D > 128 && GATHER ? 2 : 1;
+  static constexpr int kScoreBuffers = 2 * kSoftmaxGroups;      // score tiles in tensor memory
+  static constexpr int kThreads = kRewriters <= 1 && kSoftmaxGroups == 1 ? 256 : 384;
   static constexpr int kQBytes = BLOCK_M * D * 2;
   static constexpr int kHalfBytes = BLOCK_N * D * 2;          // keys (or values) of a tile
   static constexpr int kSmemBytes = kQBytes + (kKeyStages + kValueStages + kKeyBuffers) * kHalfBytes +
-                                    128 /*alignment*/ + 256 /*barriers*/;
+                                    128 /*alignment*/ + 256 /*barriers*/ +
+                                    (kSoftmaxGroups > 1 ? 2 * kSoftmaxGroups * BLOCK_M * 4 : 0);
   static constexpr int kScoreColumns = BLOCK_N;               // per score buffer
   static constexpr int kLowTermColumn = BLOCK_N / 2;          // P: hi in columns [0, 32), lo after
-  static constexpr int kOutputColumn = S_BUFFERS * BLOCK_N;
+  static constexpr int kOutputColumn = kScoreBuffers * BLOCK_N;
   static constexpr int kTmemColumns = D <= 128 ? 256 : 512;
-  static_assert(S_BUFFERS * BLOCK_N + D <= kTmemColumns, "tensor memory of a CTA");
+  static_assert(kScoreBuffers * BLOCK_N + D <= kTmemColumns, "tensor memory of a CTA");
   static_assert(kCtas * (kSmemBytes + 1024) <= 228 * 1024, "an SM has 228 KB of shared memory");
 };
 
@@ -185,6 +200,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
   constexpr int K_STAGES = Config::kKeyStages, V_STAGES = Config::kValueStages;
   constexpr int KEY_BUFFERS = Config::kKeyBuffers, REWRITERS = Config::kRewriters;
   constexpr int kDSteps = D / 16;      // k-steps of Q K^T
+  constexpr int GROUPS = Config::kSoftmaxGroups, S_BUFFERS = Config::kScoreBuffers;
+  // (with two CTAs an SM a second thread that asks costs more than it gives: 68 -> 74 us)
+  constexpr bool SPLIT_REQUESTS = GATHER && GROUPS > 1;
   hx_pdl_trigger();
 
   // which request and which 128-row tile of it is this CTA?  The last rows of a request see
@@ -218,8 +236,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
   uint64_t* k_ready = o_full + S_BUFFERS;      // [KEY_BUFFERS] the tile's keys are rewritten
   uint64_t* k_done = k_ready + KEY_BUFFERS;    // [KEY_BUFFERS] its scores have read them
   uint64_t* q_ready = k_done + KEY_BUFFERS;    // the query tile is in shared memory
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(q_ready + 1);
+  uint64_t* told_bar = q_ready + 1;            // [GROUPS][4] a group's warp has told its reference
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(told_bar + (GROUPS > 1 ? 4 * GROUPS : 0));
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  // two groups of softmax warps: [GROUPS][BLOCK_M] references they tell each other, then their sums
+  float* told = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(k_full) + 256);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -268,6 +289,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       mbar_init(&k_ready[b], GATHER ? 1 : REWRITERS);      // the copies, or the warps that rewrite
       mbar_init(&k_done[b], 1);
     }
+    if (GROUPS > 1) {
+      for (int i = 0; i < 4 * GROUPS; ++i) mbar_init(&told_bar[i], 1);
+    }
     mbar_init(q_ready, THREADS / 32 - WARP_SCORES);      // one arrival per warp that loads queries
     *failed = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -283,20 +307,25 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
 
   // ---- the query tile: [D / 8 pieces][16 row groups][8 rows][16 bytes], written by the warps from
   // WARP_SCORES on while the first pages are on their way.  All of a thread's loads are in flight
-  // together (one after the other they cost the CTA 6 us).
+  // together (one after the other they cost the CTA 6 us); a warp takes four neighbouring pieces of eight
+  // rows, which it stores to different banks (32 pieces of a row, 2 KB apart, cost 4 us more).
   if (warp >= WARP_SCORES) {
-    constexpr int kLoaders = THREADS - WARP_SCORES * 32;
-    constexpr int kPieces = BLOCK_M * (D / 8);
-    constexpr int kPerThread = (kPieces + kLoaders - 1) / kLoaders;
-    const int loader = threadIdx.x - WARP_SCORES * 32;
-    uint4 values[kPerThread];
+    constexpr int kLoaders = THREADS / 32 - WARP_SCORES;      // warps
+    constexpr int kPieces = D / 8, kItems = BLOCK_M / 8 * kPieces;
+    constexpr int kTurns = (kItems + 4 * kLoaders - 1) / (4 * kLoaders);
+    uint4 values[kTurns];
+    auto place = [&](int turn, int& row, int& piece) {
+      const int item = (turn * kLoaders + warp - WARP_SCORES) * 4 + (lane >> 3);
+      const int row_group = item / kPieces;
+      piece = item - row_group * kPieces;
+      row = 8 * row_group + (lane & 7);
+      return item < kItems;
+    };
 #pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
-      const int index = loader + i * kLoaders;
-      const int row = index / (D / 8);
-      const int piece = index - row * (D / 8);
+    for (int i = 0; i < kTurns; ++i) {
+      int row, piece;
       values[i] = make_uint4(0u, 0u, 0u, 0u);
-      if (index < kPieces && row < rows_here) {
+      if (place(i, row, piece) && row < rows_here) {
         const int token = token_of(row);
         values[i] = *reinterpret_cast<const uint4*>(
             a.q + static_cast<size_t>(q_begin + token0 + token) * a.ldq +
@@ -304,11 +333,9 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       }
     }
 #pragma unroll
-    for (int i = 0; i < kPerThread; ++i) {
-      const int index = loader + i * kLoaders;
-      const int row = index / (D / 8);
-      const int piece = index - row * (D / 8);
-      if (index < kPieces)
+    for (int i = 0; i < kTurns; ++i) {
+      int row, piece;
+      if (place(i, row, piece))
         *reinterpret_cast<uint4*>(q_tile + piece * CHUNK_STRIDE + (row >> 3) * GROUP_STRIDE +
                                   (row & 7) * 16) = values[i];
     }
@@ -317,7 +344,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
     if (lane == 0) mbar_arrive(q_ready);
   }
 
-  if (warp == WARP_PAGES) {
+  if (warp == WARP_PAGES || (SPLIT_REQUESTS && warp == WARP_REWRITE)) {
     // ------------------------------------------------------------ page requests
     if (hx_elect_one()) {
       const int* table = a.block_tables +
@@ -340,64 +367,75 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       };
       // the copies of a tile's page blocks into a stage that is free
       auto request_tile = [&](const __nv_bfloat16* cache, uint8_t* stage, uint64_t* full,
-                              const int (&pages)[4]) {
+                              const int (&pages)[4], uint32_t bytes) {
         uint32_t expected = 0;
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           if (pages[p] == -1) atomicOr(a.status, HX_FLAG_BAD_PAGE);
           if (pages[p] >= 0) expected += page_bytes;
         }
+        if (PACKED) expected = expected / page_bytes * bytes;
         mbar_expect_tx(full, expected);
         const uint32_t base = smem_u32(stage);
 #pragma unroll
         for (int p = 0; p < 4; ++p) {
           if (pages[p] >= 0) {
             const size_t block = (static_cast<size_t>(pages[p]) * a.kv_heads + kv_head) * page_bytes;
-            bulk_copy(base + p * page_bytes, reinterpret_cast<const uint8_t*>(cache) + block, page_bytes,
-                      full);
+            bulk_copy(base + p * page_bytes, reinterpret_cast<const uint8_t*>(cache) + block,
+                      PACKED ? bytes : page_bytes, full);
           }
         }
       };
+      auto request_keys = [&](int tile, const int (&pages)[4]) {
+        if constexpr (GATHER) {
+          const int buffer = tile % KEY_BUFFERS;
+          if (!mbar_wait(&k_done[buffer], (static_cast<uint32_t>(tile / KEY_BUFFERS) & 1u) ^ 1u)) return false;
+          // no page: any row will do, no key of it is seen
+          int rows[4];
+#pragma unroll
+          for (int p = 0; p < 4; ++p) {
+            if (pages[p] == -1) atomicOr(a.status, HX_FLAG_BAD_PAGE);
+            rows[p] = max(pages[p], 0) * a.kv_heads + kv_head;
+          }
+          mbar_expect_tx(&k_ready[buffer], Config::kHalfBytes);
+          const uint32_t target = smem_u32(keys_by_piece + buffer * Config::kHalfBytes);
+#pragma unroll 4
+          for (int piece = 0; piece < D / 8; ++piece)
+            tma_gather_rows(target + piece * (BLOCK_N * 16), &key_pages, &k_ready[buffer],
+                            piece * (BLOCK_N / 4) * 8, rows);
+        } else {
+          const int stage = tile % K_STAGES;
+          if (!mbar_wait(&k_empty[stage], (static_cast<uint32_t>(tile / K_STAGES) & 1u) ^ 1u)) return false;
+          request_tile(a.k_cache, k_stages + stage * Config::kHalfBytes, &k_full[stage], pages, page_bytes);
+        }
+        return true;
+      };
+      auto request_values = [&](int tile, const int (&pages)[4]) {
+        const int stage = tile % V_STAGES;
+        if (!mbar_wait(&v_empty[stage], (static_cast<uint32_t>(tile / V_STAGES) & 1u) ^ 1u)) return false;
+        request_tile(a.v_cache, v_stages + stage * Config::kHalfBytes, &v_full[stage], pages,
+                     static_cast<uint32_t>(page_size) * a.value_dim * 2);
+        return true;
+      };
+      // Turn t asks for the keys of tile t and for the values of tile t - 1, which are wanted
+      // later: their keys are (rewritten and) multiplied, and the softmax runs, in between.  With two threads
+      // that ask, one asks for values alone, as soon as there is room.
+      const bool asks_keys = !SPLIT_REQUESTS || warp == WARP_PAGES;
+      const bool asks_values = !SPLIT_REQUESTS || warp != WARP_PAGES;
+      // (behind the first tile's keys and the queries, which the first products wait for)
+      bool waited = !SPLIT_REQUESTS;
       int pages[4], value_pages[4];
       pages_of(0, pages);
-      // turn t asks for the keys of tile t and for the values of tile t - 1, which are wanted
-      // later: their keys are rewritten and multiplied, and the softmax runs, in between
       for (int tile = 0; tile <= n_tiles && !*failed; ++tile) {
         int next_pages[4];
         if (tile + 1 < n_tiles) pages_of(tile + 1, next_pages);      // in flight during the waits
         bool free = true;
-        if (tile < n_tiles) {
-          if constexpr (GATHER) {
-            const int buffer = tile % KEY_BUFFERS;
-            free = mbar_wait(&k_done[buffer], (static_cast<uint32_t>(tile / KEY_BUFFERS) & 1u) ^ 1u);
-            if (free) {
-              // no page: any row will do, no key of it is seen
-              int rows[4];
-#pragma unroll
-              for (int p = 0; p < 4; ++p) {
-                if (pages[p] == -1) atomicOr(a.status, HX_FLAG_BAD_PAGE);
-                rows[p] = max(pages[p], 0) * a.kv_heads + kv_head;
-              }
-              mbar_expect_tx(&k_ready[buffer], Config::kHalfBytes);
-              const uint32_t target = smem_u32(keys_by_piece + buffer * Config::kHalfBytes);
-#pragma unroll 4
-              for (int piece = 0; piece < D / 8; ++piece)
-                tma_gather_rows(target + piece * (BLOCK_N * 16), &key_pages, &k_ready[buffer],
-                                piece * (BLOCK_N / 4) * 8, rows);
-            }
-          } else {
-            const int stage = tile % K_STAGES;
-            free = mbar_wait(&k_empty[stage], (static_cast<uint32_t>(tile / K_STAGES) & 1u) ^ 1u);
-            if (free)
-              request_tile(a.k_cache, k_stages + stage * Config::kHalfBytes, &k_full[stage], pages);
-          }
+        if (!waited && (tile > 0 || !asks_keys)) {
+          free = mbar_wait(q_ready, 0);
+          waited = true;
         }
-        if (free && tile > 0) {
-          const int before = tile - 1, stage = before % V_STAGES;
-          free = mbar_wait(&v_empty[stage], (static_cast<uint32_t>(before / V_STAGES) & 1u) ^ 1u);
-          if (free)
-            request_tile(a.v_cache, v_stages + stage * Config::kHalfBytes, &v_full[stage], value_pages);
-        }
+        if (free && asks_keys && tile < n_tiles) free = request_keys(tile, pages);
+        if (free && asks_values && tile > 0) free = request_values(tile - 1, value_pages);
         if (!free) {
           atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
@@ -518,7 +556,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
   } else if (warp == WARP_OUTPUT) {
     // ----------------------------------------------------------- output products
     if (hx_elect_one()) {
-      constexpr uint32_t idesc_output = make_idesc_b_mn_major(BLOCK_M, D);
+      const uint32_t idesc_output = make_idesc_b_mn_major(BLOCK_M, PACKED ? a.value_dim : D);
       // values: MN-major, the next 8 keys are 128 bytes on, the next 8 coordinates one piece on
       const uint64_t desc_v0 = make_smem_desc_plain(smem_u32(v_stages), GROUP_STRIDE, piece_stride);
       constexpr uint32_t kStageStep = Config::kHalfBytes >> 4;
@@ -554,8 +592,12 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
         umma_commit(&o_full[b]);                     // O holds this tile; its P has been read
       }
     }
-  } else if (warp >= WARP_SOFTMAX && warp < WARP_MORE) {
+  } else if (warp >= WARP_SOFTMAX && warp < WARP_SOFTMAX + 4 * GROUPS) {
     // ------------------------------------------------------------------ softmax
+    // With two groups a row has a thread in each: one takes the even tiles, the other the odd ones.  The
+    // reference goes from tile to tile through shared memory, told before the exponentials are taken; each
+    // keeps the sum of its own tiles.
+    const int softmax_group = GROUPS > 1 ? (warp - WARP_SOFTMAX) >> 2 : 0;
     const int quarter = warp & 3;      // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
     const int row = quarter * 32 + lane;
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
@@ -587,7 +629,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       return state == 0;
     };
 
-    for (int tile = 0; tile < n_tiles && ok; ++tile) {
+    for (int tile = softmax_group; tile < n_tiles && ok; tile += GROUPS) {
       const int b = tile % S_BUFFERS;
       ok = wait_for(&s_full[b], static_cast<uint32_t>(tile / S_BUFFERS) & 1u);
       if (!ok) break;
@@ -644,23 +686,37 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       // without a window key 0 is visible to every row and the reference is finite from the
       // first tile on; with one a row may see nothing of the CTA's first tiles and keeps
       // -inf as its reference (and zeros as its probabilities) until it does
-      if (tile == 0) {
-        row_max = tile_max;
-      } else if (__any_sync(0xffffffffu, tile_max > row_max + RAISE_MAXIMUM_BY)) {
-        // ---- a new reference: what O and the sum hold was taken against the old one.  The
+      const float own_max = row_max;      // what the sum is taken against
+      if (GROUPS > 1 && tile > 0) {
+        const int other = softmax_group ^ 1;
+        ok = wait_for(&told_bar[4 * other + quarter], static_cast<uint32_t>((tile - 1) / GROUPS) & 1u);
+        if (!ok) break;
+        row_max = told[other * BLOCK_M + row];
+      }
+      const float old_max = row_max;
+      const bool raised = tile > 0 && __any_sync(0xffffffffu, tile_max > old_max + RAISE_MAXIMUM_BY);
+      if (tile == 0) row_max = tile_max;
+      else if (raised) row_max = fmaxf(old_max, tile_max);
+      if (GROUPS > 1) {
+        told[softmax_group * BLOCK_M + row] = row_max;
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&told_bar[4 * softmax_group + quarter]);
+      }
+      if (GROUPS > 1 && row_max != own_max) row_sum *= own_max == -INFINITY ? 0.0f : fast_exp2(own_max - row_max);
+      if (raised) {
+        // ---- a new reference: what O holds was taken against the old one.  The
         // product of the previous tile must have landed; the product of this tile waits for
         // this warp's arrival below.  (o_full[b] completes a phase for every other tile; its
         // previous phase was complete before the scores of the previous tile were.)
-        const float new_max = fmaxf(row_max, tile_max);
-        const float correction = row_max == -INFINITY ? 0.0f : fast_exp2(row_max - new_max);
-        row_max = new_max;
-        row_sum *= correction;
+        const float correction = old_max == -INFINITY ? 0.0f : fast_exp2(old_max - row_max);
+        if (GROUPS == 1) row_sum *= correction;
         ok = wait_for(&o_full[(tile - 1) % S_BUFFERS],
                       static_cast<uint32_t>((tile - 1) / S_BUFFERS) & 1u);
         if (!ok) break;
         tc_fence_after();
 #pragma unroll
         for (int d0 = 0; d0 < D; d0 += 32) {
+          if (PACKED && d0 >= a.value_dim) break;
           const bool both = d0 + 16 < D;      // (compile time: D is a multiple of 16)
           uint32_t r0[16], r1[16];
           tmem_load16_issue(output_base + d0, r0);
@@ -741,6 +797,20 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       if (lane == 0) mbar_arrive(&p_full[b]);
     }
 
+    // ---- both groups' sums against the last reference, which is the largest (the barrier is met whatever went
+    // wrong: every wait in front of it ends)
+    if constexpr (GROUPS > 1) {
+      // (a reference that was told is read before the next is: no place is written too early)
+      float* sums = told + GROUPS * BLOCK_M;
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * GROUPS) : "memory");
+      told[softmax_group * BLOCK_M + row] = row_max;
+      sums[softmax_group * BLOCK_M + row] = row_sum;
+      asm volatile("bar.sync 1, %0;" ::"n"(128 * GROUPS) : "memory");
+      const float max0 = told[row], max1 = told[BLOCK_M + row];
+      row_max = fmaxf(max0, max1);
+      row_sum = (max0 == -INFINITY ? 0.0f : sums[row] * fast_exp2(max0 - row_max)) +
+                (max1 == -INFINITY ? 0.0f : sums[BLOCK_M + row] * fast_exp2(max1 - row_max));
+    }
     // ---- a commit covers every product its thread issued before it: the last tile says all of
     // them are done
     if (ok) {
@@ -757,29 +827,61 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
           const float keep = row_max == -INFINITY ? 0.0f : fast_exp2(row_max - top);
           inverse = keep / (row_sum * keep + fast_exp2(sink_log2 - top));
         }
-        __nv_bfloat16* out = a.out +
-                             static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
-                             static_cast<size_t>(head) * D;
+        // A group takes its share of the coordinates.  The rows gather in shared memory, where the queries and
+        // values were (every product is done), 16 bytes apart more than they are long, so that a warp's rows
+        // use different banks (a thread's own row, 16 bytes at a time, is half a sector a store).  With two CTAs
+        // an SM they leave with whole rows side by side, with one by a bulk copy each (the other way round: heads
+        // of 128 67 -> 70 us, heads of 256 96 -> 101).
+        constexpr int SHARE = D / GROUPS, ROW_BYTES = SHARE * 2 + 16;
+        static_assert(4 * GROUPS * 32 * ROW_BYTES <= Config::kQBytes + (K_STAGES + V_STAGES) * Config::kHalfBytes,
+                      "the rows' place");
+        uint8_t* gathered = q_tile + ((4 * softmax_group + quarter) * 32 + lane) * ROW_BYTES;
+        const int share = min(SHARE, a.value_dim - softmax_group * SHARE);      // coordinates that are wanted
 #pragma unroll
-        for (int d0 = 0; d0 < D; d0 += 32) {
-          const bool both = d0 + 16 < D;
+        for (int d0 = 0; d0 < SHARE; d0 += 32) {
+          if (d0 >= share) break;
+          const bool both = d0 + 16 < SHARE;
           uint32_t r[2][16];
-          tmem_load16_issue(output_base + d0, r[0]);
-          if (both) tmem_load16_issue(output_base + d0 + 16, r[1]);
+          tmem_load16_issue(output_base + softmax_group * SHARE + d0, r[0]);
+          if (both) tmem_load16_issue(output_base + softmax_group * SHARE + d0 + 16, r[1]);
           tmem_load_wait();
-          if (row < rows_here) {
 #pragma unroll
-            for (int h = 0; h < (both ? 2 : 1); ++h)
+          for (int h = 0; h < (both ? 2 : 1); ++h)
 #pragma unroll
-              for (int d = 0; d < 16; d += 8) {
-                uint4 packed;
-                __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&packed);
+            for (int d = 0; d < 16; d += 8) {
+              uint4 packed;
+              __nv_bfloat162* pairs = reinterpret_cast<__nv_bfloat162*>(&packed);
 #pragma unroll
-                for (int i = 0; i < 4; ++i)
-                  pairs[i] = __floats2bfloat162_rn(__uint_as_float(r[h][d + 2 * i]) * inverse,
-                                                   __uint_as_float(r[h][d + 2 * i + 1]) * inverse);
-                *reinterpret_cast<uint4*>(out + d0 + h * 16 + d) = packed;
-              }
+              for (int i = 0; i < 4; ++i)
+                pairs[i] = __floats2bfloat162_rn(__uint_as_float(r[h][d + 2 * i]) * inverse,
+                                                 __uint_as_float(r[h][d + 2 * i + 1]) * inverse);
+              *reinterpret_cast<uint4*>(gathered + (d0 + h * 16 + d) * 2) = packed;
+            }
+        }
+        if constexpr (GROUPS > 1) {
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+          if (row < rows_here && share > 0) {
+            __nv_bfloat16* out = a.out + static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
+                                 static_cast<size_t>(head) * D + softmax_group * SHARE;
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out),
+                         "r"(smem_u32(gathered)), "r"(2 * share)
+                         : "memory");
+            asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+            asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+          }
+        } else {
+          __syncwarp();
+          constexpr int PIECES = SHARE / 8;
+          const uint8_t* of_warp = q_tile + quarter * 32 * ROW_BYTES;
+#pragma unroll 4
+          for (int item = lane; item < 32 * PIECES; item += 32) {
+            const int r = item / PIECES, piece = item - r * PIECES, out_row = quarter * 32 + r;
+            if (out_row < rows_here && 8 * piece < share) {
+              const int token = token_of(out_row);
+              *reinterpret_cast<uint4*>(a.out + static_cast<size_t>(q_begin + token0 + token) * a.ldo +
+                                        static_cast<size_t>(head_of(out_row, token)) * D + piece * 8) =
+                  *reinterpret_cast<const uint4*>(of_warp + r * ROW_BYTES + piece * 16);
+            }
           }
         }
       }
@@ -876,7 +978,7 @@ HX_API int hx_prefill_attention_tc_biased(const void* q, int ldq, const void* k_
                   static_cast<const __nv_bfloat16*>(v_cache), request_start, request_context,
                   request_table_row, block_tables, table_stride, static_cast<__nv_bfloat16*>(out),
                   ldo, requests, heads, kv_heads, page_size, num_pages, scale, min_query_len, status,
-                  window, keep_first, sinks, slopes, chunk, softcap};
+                  window, keep_first, sinks, slopes, chunk, softcap, 1, head_dim};
   int rc;
   switch (head_dim) {
     case 64: rc = launch<64>(a, tile_bound, stream); break;
@@ -935,7 +1037,9 @@ HX_API int hx_prefill_attention_tc_packed_tokens(int heads, int kv_heads, int he
 // The arguments of hx_prefill_attention_tc_biased, for heads of 160 to 256 in steps of 32: a tile's
 // 128 rows are the query heads of a key/value head, side by side, of
 // hx_prefill_attention_tc_packed_tokens tokens; tile_bound bounds the number of such tiles.
-HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_cache,
+// value_dim: the leading coordinates of the values that are wanted, a multiple of 32; the others of a row of
+// `out` are not written.
+HX_API int hx_prefill_attention_tc_packed_values(const void* q, int ldq, const void* k_cache,
                                           const void* v_cache, const int* request_start,
                                           const int* request_context,
                                           const int* request_table_row, const int* block_tables,
@@ -944,7 +1048,8 @@ HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_
                                           int page_size, int num_pages, float scale,
                                           int min_query_len, int window, int keep_first,
                                           const float* sinks, const float* slopes, int chunk,
-                                          float softcap, int* status, cudaStream_t stream) {
+                                          float softcap, int value_dim, int* status,
+                                          cudaStream_t stream) {
   HX_REQUIRE(chunk >= 0 && softcap >= 0.0f, "hx_prefill_attention_tc_packed: bad chunk or softcap");
   HX_REQUIRE(window >= 0 && keep_first >= 0, "hx_prefill_attention_tc_packed: bad window");
   if (window == 0) keep_first = 0;
@@ -952,6 +1057,8 @@ HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_
              "hx_prefill_attention_tc_packed: %d heads of %d on %d with pages of %d are not supported",
              heads, head_dim, kv_heads, page_size);
   HX_REQUIRE(requests >= 0 && tile_bound >= 0, "hx_prefill_attention_tc_packed: bad sizes");
+  HX_REQUIRE(value_dim > 0 && value_dim <= head_dim && value_dim % 32 == 0,
+             "hx_prefill_attention_tc_packed: %d of %d coordinates of the values", value_dim, head_dim);
   HX_REQUIRE(tile_bound <= 65535, "hx_prefill_attention_tc_packed: too many query tiles");
   HX_REQUIRE(num_pages > 0 && table_stride > 0 &&
                  static_cast<long long>(num_pages) * kv_heads < (1ll << 31),
@@ -969,7 +1076,7 @@ HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_
                   static_cast<const __nv_bfloat16*>(v_cache), request_start, request_context,
                   request_table_row, block_tables, table_stride, static_cast<__nv_bfloat16*>(out),
                   ldo, requests, heads, kv_heads, page_size, num_pages, scale, min_query_len, status,
-                  window, keep_first, sinks, slopes, chunk, softcap, heads / kv_heads};
+                  window, keep_first, sinks, slopes, chunk, softcap, heads / kv_heads, value_dim};
   int rc;
   switch (head_dim) {
     case 160: rc = launch<160, true>(a, tile_bound, stream); break;
@@ -980,4 +1087,22 @@ HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_
   if (rc != HX_OK) return rc;
   HX_CHECK_LAUNCH("hx_prefill_attention_tc_packed");
   return HX_OK;
+}
+
+// All of them.
+HX_API int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_cache,
+                                          const void* v_cache, const int* request_start,
+                                          const int* request_context,
+                                          const int* request_table_row, const int* block_tables,
+                                          int table_stride, void* out, int ldo, int requests,
+                                          int tile_bound, int heads, int kv_heads, int head_dim,
+                                          int page_size, int num_pages, float scale,
+                                          int min_query_len, int window, int keep_first,
+                                          const float* sinks, const float* slopes, int chunk,
+                                          float softcap, int* status, cudaStream_t stream) {
+  return hx_prefill_attention_tc_packed_values(q, ldq, k_cache, v_cache, request_start, request_context,
+                                               request_table_row, block_tables, table_stride, out, ldo, requests,
+                                               tile_bound, heads, kv_heads, head_dim, page_size, num_pages, scale,
+                                               min_query_len, window, keep_first, sinks, slopes, chunk, softcap,
+                                               head_dim, status, stream);
 }

@@ -343,6 +343,9 @@ def _declare(library: ctypes.CDLL) -> None:
     library.hx_prefill_attention_tc_packed_tokens.argtypes = [_c_int, _c_int, _c_int, _c_int]
     library.hx_prefill_attention_tc_packed_tokens.restype = _c_int
     library.hx_prefill_attention_tc_packed.argtypes = library.hx_prefill_attention_tc_biased.argtypes
+    library.hx_prefill_attention_tc_packed_values.argtypes = [
+        *library.hx_prefill_attention_tc_biased.argtypes[:-2], _c_int, _c_ptr, _c_ptr]
+    library.hx_prefill_attention_tc_packed_values.restype = _c_int
     library.hx_prefill_attention_tc_packed.restype = _c_int
     library.hx_delta_chunks_supports.argtypes = [_c_int, _c_int]
     library.hx_delta_chunks_supports.restype = _c_int
@@ -892,7 +895,7 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
                       keep_first: int = 0, packed: bool = False,
                       sinks: Optional[torch.Tensor] = None,
                       slopes: Optional[torch.Tensor] = None, chunk: int = 0,
-                      softcap: float = 0.0) -> None:
+                      softcap: float = 0.0, value_dim: int = 0) -> None:
     """Tensor-core attention (bfloat16) of every request that brings at least
     ``min_query_len`` tokens; ``tile_bound`` bounds the number of query tiles of 64 tokens
     (the tensor-memory kernel, whose tiles hold 256 tokens, needs no more).  A CTA that finds
@@ -908,7 +911,8 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
     for heads of 160 to 256 (unless ``tensor_memory`` is False), else the ``mma.sync`` kernel
     (``prefill_attention_packed_tokens`` tokens a tile).  ``sinks``,
     ``slopes``, ``chunk`` and ``softcap`` as in :func:`paged_attention`; all three kernels take
-    them."""
+    them.  ``value_dim`` > 0: the caller reads so many leading coordinates of a head's output only;
+    the packed tcgen05 kernel leaves the others as they are."""
     biased = sinks is not None or slopes is not None or chunk > 0 or softcap > 0.0
     for per_head in (sinks, slopes):
         if per_head is not None:
@@ -939,9 +943,10 @@ def prefill_attention(q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Ten
         block_tables.stride(0), out.data_ptr(), out.stride(0), requests, tile_bound, heads,
         kv_heads, head_dim, page_size, num_pages, float(scale), min_query_len)
     if packed_tokens:
-        _check(lib().hx_prefill_attention_tc_packed(*arguments, int(window), int(keep_first),
-                                                    _ptr(sinks), _ptr(slopes), int(chunk),
-                                                    float(softcap), _ptr(status), _stream()))
+        wanted = min(head_dim, -(-value_dim // 32) * 32) if value_dim > 0 else head_dim
+        _check(lib().hx_prefill_attention_tc_packed_values(
+            *arguments, int(window), int(keep_first), _ptr(sinks), _ptr(slopes), int(chunk),
+            float(softcap), wanted, _ptr(status), _stream()))
     elif biased and tensor_memory:
         _check(lib().hx_prefill_attention_tc_biased(*arguments, int(window), int(keep_first),
                                                     _ptr(sinks), _ptr(slopes), int(chunk),

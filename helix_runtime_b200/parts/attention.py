@@ -102,6 +102,7 @@ def rotary_row_permutation(heads: int, head_dim: int, rotary_dim: int) -> torch.
 class PagedAttention(Mixer):
     pack_heads = False      # subclasses whose heads share few cached rows set this
     pack_always = True      # ... for every step; False: only for steps of single tokens
+    value_columns = 0       # subclasses that read only so many columns of a head's output set this
 
     def __init__(self, spec: PartSpec, hidden_size: int) -> None:
         super().__init__(spec, hidden_size)
@@ -375,7 +376,7 @@ class PagedAttention(Mixer):
                                   ctx.status, query_lengths=ctx.host_query_lengths,
                                   window=window, keep_first=kept, packed=True,
                                   sinks=self.sinks, slopes=self.slopes, chunk=chunk,
-                                  softcap=self.softcap)
+                                  softcap=self.softcap, value_dim=self.value_columns)
             return
         if tensor_cores:
             ops.prefill_attention(qkv, cache.keys, cache.values, ctx.request_start,
@@ -678,6 +679,8 @@ class LatentAttention(PagedAttention):
         self.head_dim = self.kv_rank + self.rotated_dim        # of the one cached key head
         self.row_dim = row_width(self.head_dim)
         self.row_dim += self.row_dim % 2                       # the append moves pairs
+        # the values' up-projection reads the latent's columns, 64 at a time; zeros lie behind them
+        self.value_columns = min(self.row_dim, -(-self.kv_rank // 64) * 64)
         self.q_size = self.heads * self.row_dim
         self.rows_size = self.q_size + 2 * self.row_dim
         self.q_width = self.heads * (self.plain_dim + self.rotated_dim)

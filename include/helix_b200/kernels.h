@@ -724,6 +724,18 @@ int hx_prefill_attention_tc_packed(const void* q, int ldq, const void* k_cache,
                                    int min_query_len, int window, int keep_first,
                                    const float* sinks, const float* slopes, int chunk,
                                    float softcap, int* status, cudaStream_t stream);
+/* the same where only the leading value_dim coordinates of the values are wanted (a multiple of 32); the
+ * others of a row of `out` are not written */
+int hx_prefill_attention_tc_packed_values(const void* q, int ldq, const void* k_cache,
+                                   const void* v_cache, const int* request_start,
+                                   const int* request_context, const int* request_table_row,
+                                   const int* block_tables, int table_stride, void* out, int ldo,
+                                   int requests, int tile_bound, int heads, int kv_heads,
+                                   int head_dim, int page_size, int num_pages, float scale,
+                                   int min_query_len, int window, int keep_first,
+                                   const float* sinks, const float* slopes, int chunk,
+                                   float softcap, int value_dim,
+                                   int* status, cudaStream_t stream);
 /* the tcgen05 kernel with a window and kept first keys (see hx_prefill_attention_windowed) */
 int hx_prefill_attention_tc_windowed(const void* q, int ldq, const void* k_cache,
                                      const void* v_cache, const int* request_start,

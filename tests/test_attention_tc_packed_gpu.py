@@ -138,3 +138,39 @@ def test_the_same_heads_are_packed_as_before():
         before = ops.prefill_attention_packed_tokens(heads, kv_heads)
         assert tokens(heads, kv_heads, 256, 16) == (128 // (heads // kv_heads) if before else 0)
     assert tokens(32, 1, 128, 16) == tokens(32, 1, 240, 16) == tokens(32, 1, 256, 8) == 0
+
+
+@pytest.mark.parametrize("head_dim,value_dim", [(160, 32), (160, 96), (192, 160), (256, 192), (256, 224)])
+@pytest.mark.parametrize("page_size", [16, 32])
+def test_leading_columns_of_the_values(head_dim, value_dim, page_size):
+    """So many columns as are asked for are those of the whole call, bit for bit; the others stay.  (Contexts
+    of one tile, of an odd and an even number of tiles, and a window that begins inside one.)"""
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(head_dim + value_dim)
+    heads, lengths, contexts = 8, (70, 3, 20), (0, 130, 61)
+    pages_of = [-(-(length + context) // page_size) for length, context in zip(lengths, contexts)]
+    pages = sum(pages_of)
+    q = torch.randn(sum(lengths), heads * head_dim, device="cuda").bfloat16()
+    keys = torch.randn(pages, 1, page_size * head_dim, device="cuda").bfloat16()
+    values = torch.randn_like(keys)
+    table = torch.zeros(len(lengths), max(pages_of), dtype=torch.int32)
+    order, at = torch.randperm(pages).int(), 0
+    for request, count in enumerate(pages_of):
+        table[request, :count] = order[at:at + count]
+        at += count
+    starts = torch.tensor([0, *torch.tensor(lengths).cumsum(0)], dtype=torch.int32).cuda()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for window in (0, 50):
+        outs = []
+        for wanted in (0, value_dim):
+            out = torch.full((sum(lengths), heads * head_dim), 5.0, device="cuda").bfloat16()
+            ops.prefill_attention(q, keys, values, starts, torch.tensor(contexts, dtype=torch.int32).cuda(),
+                                  torch.arange(len(lengths), dtype=torch.int32).cuda(), table.cuda(), out,
+                                  len(lengths), sum(lengths), heads, 1, head_dim, page_size, pages,
+                                  head_dim ** -0.5, 1, status, query_lengths=lengths, window=window,
+                                  packed=True, value_dim=wanted)
+            outs.append(out.view(-1, heads, head_dim))
+        whole, part = outs
+        assert torch.equal(part[..., :value_dim], whole[..., :value_dim])
+        assert (part[..., value_dim:] == 5.0).all() and whole.float().abs().max() < 5.0
+    assert int(status.item()) == 0
