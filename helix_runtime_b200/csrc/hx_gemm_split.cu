@@ -306,7 +306,7 @@ __global__ __launch_bounds__(THREADS, 1) void gemm_split_kernel(const SplitArgs 
   }
 }
 
-// ------------------------------------------------------------------ many tokens: pairs of CTAs
+// ------------------------------------------------------------------ with scratch: pairs of CTAs
 //
 // Above, every tile cuts its tokens again, for each of its 128 features once: with 512 tokens by [17,280 x
 // 3,200] the conversion of the tokens is done 135 times.  Here split_cut_kernel cuts the tokens once (6 bytes a
@@ -608,7 +608,7 @@ HX_API int hx_gemm_split_supports(const void* x, int ldx, const void* w, int ldw
          ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
 }
 
-// Whether it is the faster road for this many tokens: with few tiles either road is one round of CTAs that
+// Whether it is the faster road for this many tokens, without scratch: with few tiles either road is one round of CTAs that
 // walk the depth alone, 2.0 us a block of 64 k on the CUDA cores (32 x 32 a tile, several CTAs an SM) against
 // 2.2 here, so the CUDA cores need more than two such tiles an SM to be slower.  Measured (us, CUDA cores / here):
 // 9,600 features of 3,200 17 tokens 141 / 111; 4,096 of 4,096 64 tokens 131 / 143, 100 188 / 146; 3,200 of 8,640 64
@@ -618,10 +618,19 @@ HX_API int hx_gemm_split_pays(int tokens, int features) {
   return tokens > 16 && small >= 2ll * hx_device_sm_count();
 }
 
-// Numbers of bfloat16 scratch (on 16 bytes) with which hx_gemm_split_scratch is the faster road, 0 where it has
-// no use for any: a tile of 128 tokens that are fewer is for the kernel that cuts its own.
+// The same for a caller with scratch: the pairs' kernel beats the CUDA cores from 17 tokens on wherever the latter's
+// tiles of 32 x 32 are not a handful (two launches against one).  Measured (us, CUDA cores / one CTA a tile /
+// here): 17 tokens by [17,280 x 3,200] 152 / 123 / 120, by [3,200 x 8,640] 248 / 291 / 151, by [4,096 x 4,096] 123 / 145 /
+// 79, by [1,024 x 4,096] 123 / 148 / 75; 64 tokens 265 / 131 / 126, 272 / 297 / 153, 137 / 152 / 85, 125 / 150 / 77;
+// 16 tokens are the CUDA cores' (123, 131, 68, 64 against 120, 153, 79, 75 here).
+HX_API int hx_gemm_split_scratch_pays(int tokens, int features) {
+  const long long small = static_cast<long long>((tokens + 31) / 32) * ((features + 31) / 32);
+  return tokens > 16 && small >= 32;
+}
+
+// Numbers of bfloat16 scratch (on 16 bytes) that hx_gemm_split_scratch has a use for.
 HX_API long long hx_gemm_split_terms(int tokens, int depth) {
-  return tokens > TILE && hx_device_sm_count() >= 2 ? 3ll * tokens * terms_row(depth) : 0;
+  return tokens > 0 && hx_device_sm_count() >= 2 ? 3ll * tokens * terms_row(depth) : 0;
 }
 
 // float32 x [tokens, ldx], w [features, ldw], out [tokens, ldo]; epilogues and softcap as hx_gemm_simt_softcapped.

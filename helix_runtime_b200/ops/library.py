@@ -317,6 +317,8 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
     library.hx_gemm_split_supports.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int]
     library.hx_gemm_split_pays.argtypes = [_c_int, _c_int]
+    library.hx_gemm_split_scratch_pays.argtypes = [_c_int, _c_int]
+    library.hx_gemm_split_scratch_pays.restype = _c_int
     library.hx_gemm_split.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int,
                                       _c_int, _c_int, _c_float, _c_ptr, _c_ptr]
     library.hx_gemm_split_scratch.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int,
@@ -652,7 +654,7 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, 
 def gemm_split_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int) -> bool:
     """Whether a float32 product runs, and is faster, as :func:`gemm_split`."""
     return (x.dtype == w.dtype == out.dtype == torch.float32
-            and bool(lib().hx_gemm_split_pays(tokens, w.shape[0]))
+            and bool(lib().hx_gemm_split_scratch_pays(tokens, w.shape[0]))
             and bool(lib().hx_gemm_split_supports(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
                                                   w.shape[0], w.shape[1])))
 

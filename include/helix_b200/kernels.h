@@ -536,8 +536,9 @@ int hx_gemm_split_pays(int tokens, int features);
 int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
                   int features, int depth, int epilogue, float softcap, int* status,
                   cudaStream_t stream);
-/* the same with scratch for the terms of x (hx_gemm_split_terms() bfloat16 numbers on 16 bytes; 0: none are
- * wanted; null: the product does without) */
+/* the same with scratch for the terms of x (hx_gemm_split_terms() bfloat16 numbers on 16 bytes; null: the
+ * product does without), and whether it is then the faster road */
+int hx_gemm_split_scratch_pays(int tokens, int features);
 long long hx_gemm_split_terms(int tokens, int depth);
 int hx_gemm_split_scratch(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
                           int features, int depth, int epilogue, float softcap, void* terms,

@@ -110,6 +110,7 @@ def test_which_products_take_it():
 
 @pytest.mark.parametrize("tokens,features,depth", [
     (129, 129, 68), (256, 128, 64), (257, 300, 132), (300, 63, 4), (520, 9700, 196), (130, 40, 1000),
+    (17, 130, 132), (1, 5, 64), (128, 129, 200),
 ])
 def test_pairs_have_the_sums_of_single_tiles(tokens, features, depth):
     """More tokens than a tile, with scratch for their terms and without: the same order of the same sums.
@@ -117,16 +118,16 @@ def test_pairs_have_the_sums_of_single_tiles(tokens, features, depth):
     from helix_runtime_b200.ops import library as ops
     torch.manual_seed(tokens)
     x, w = torch.randn(tokens, depth + 4, device="cuda")[:, :depth], torch.randn(features, depth, device="cuda")
-    x[7, 3], w[5, 1] = float("inf"), float("nan")
+    x[tokens // 2, 3], w[features // 2, 1] = float("inf"), float("nan")
     status = torch.zeros(1, dtype=torch.int32, device="cuda")
     size = ops.gemm_split_terms(tokens, depth)
-    assert size >= 3 * tokens * depth and ops.gemm_split_terms(128, depth) == 0
+    assert size >= 3 * tokens * depth
     terms = torch.full((size + 64,), float("nan"), dtype=torch.bfloat16, device="cuda")
     for epilogue in (ops.EPI_STORE_F32, ops.EPI_ADD_F32):
         out, plain = torch.full((2, tokens + 1, features + 3), 2.0, device="cuda")
         ops.gemm_split(x, w, out, tokens, epilogue, status, terms=terms[:size])
-        parts = [slice(begin, min(begin + 100, tokens)) for begin in range(0, tokens, 100)]
-        for part in parts:
-            ops.gemm_split(x[part], w, plain[part], part.stop - part.start, epilogue, status)
+        ops._check(ops.lib().hx_gemm_split(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), plain.data_ptr(),
+                                           plain.stride(0), tokens, features, depth, epilogue, 0.0,
+                                           status.data_ptr(), ops._stream()))
         torch.testing.assert_close(out, plain, rtol=0, atol=0, equal_nan=True)
     assert terms[size:].isnan().all() and int(status.item()) == 0
