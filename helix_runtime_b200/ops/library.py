@@ -1935,21 +1935,19 @@ def latent_queries(q: torch.Tensor, rot_offset: int, rows: torch.Tensor, positio
                                    _stream()))
 
 
-# Fewer tokens than this are a stream of the heads' matrices either way; 2,048 tokens of 32 heads,
-# 192 by 128 and 128 by 192: 234 us for both products on the CUDA cores, 28 on the tensor cores.
-HEAD_PRODUCTS_TC_FROM = 33
+# 32 heads, 192 by 128 and 128 by 192, both products: 2,048 tokens 234 us on the CUDA cores, 28 on the
+# tensor cores; one token 37 and 10.
 
 
 def head_products(x: torch.Tensor, x_stride: int, w: torch.Tensor, out: torch.Tensor,
                   out_stride: int, tokens: int, status: Optional[torch.Tensor] = None) -> None:
     """out[t, h * out_stride + o] = sum_i w[h, o, i] * x[t, h * x_stride + i]: one small product
     per head, ``w`` ``[heads, out_dim, in_dim]``, everything in the compute dtype.  With a
-    ``status`` word products of many bfloat16 tokens run on the tensor cores where sizes and
-    strides allow (:data:`HEAD_PRODUCTS_TC_FROM`)."""
+    ``status`` word bfloat16 products run on the tensor cores where sizes and strides allow."""
     heads, out_dim, in_dim = w.shape
     assert x.dtype == w.dtype == out.dtype and w.is_contiguous()
     assert x.stride(-1) == 1 and out.stride(-1) == 1
-    if (status is not None and tokens >= HEAD_PRODUCTS_TC_FROM and x.dtype == torch.bfloat16
+    if (status is not None and tokens > 0 and x.dtype == torch.bfloat16
             and lib().hx_gemm_tc_heads_supports(in_dim, x_stride, x.stride(0))
             and (x.data_ptr() | w.data_ptr()) % 16 == 0):
         _check(lib().hx_gemm_tc_heads(x.data_ptr(), x.stride(0), x.shape[0], x_stride, w.data_ptr(),
