@@ -153,7 +153,57 @@ struct GemmArgs {
   const float* gate_bias = nullptr;
   const float* up_bias = nullptr;
   float softcap = 0.0f;       // float32 store: see level_off
+  // Store epilogues: > 1 where the CTAs of a tile, one for each run of k-blocks, are a cluster that adds its
+  // sums up (see gather_parts).
+  int cluster = 1;
 };
+
+// A product that is stored cannot be cut along the reduction into atomic adds, and one with few tiles (a
+// router of 16 features, a projection of 1,280) was a few CTAs that walked the whole depth, 0.25 us a block
+// of 64.  Here the CTAs that share a tile's depth form a cluster: each leaves its sums in its own shared memory
+// (the ring is empty by then), [column][feature], and every 16 columns are added up by one of them, in the order of
+// the ranks, and stored.  Measured (us, in a chain of launches, a CTA a tile before): 1 token by [16 x 4,096] 13.1 ->
+// 7.2, 64 16.0 -> 8.6, 100 20.4 -> 10.4, 1,024 13.8 -> 11.6; by [1,280 x 4,096] 13.2 -> 7.6, 16.3 -> 9.9, 25.7 -> 12.5
+// (1, 64, 100 tokens); by [4,096 x 4,096] 13.2 -> 8.8, 15.4 -> 11.6, 22.4 -> 15.8.
+template <int BN>
+__device__ __forceinline__ void leave_part(float* part, uint32_t lane_address, int row, int columns) {
+#pragma unroll 1
+  for (int column = 0; column < columns; column += 16) {
+    float acc[16];
+    tmem_load16(lane_address + column, acc);
+#pragma unroll
+    for (int j = 0; j < 16; ++j) part[(column + j) * BM + row] = acc[j];
+  }
+}
+
+template <int BN, int EPI>
+__device__ __forceinline__ void gather_parts(const GemmArgs& a, const float* part, int rank, int row, int feature,
+                                             int token0) {
+#pragma unroll 1
+  for (int column = 16 * rank; column < BN && token0 + column < a.tokens; column += 16 * a.cluster) {
+    float sums[16];
+#pragma unroll
+    for (int j = 0; j < 16; ++j) sums[j] = 0.0f;
+    for (int r = 0; r < a.cluster; ++r) {
+      const uint32_t from = cluster_address(part + column * BM + row, r);
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        float x;
+        asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(from + j * BM * 4));
+        sums[j] += x;
+      }
+    }
+    if (feature >= a.features) continue;
+#pragma unroll
+    for (int j = 0; j < 16; ++j) {
+      const int token = token0 + column + j;
+      if (token >= a.tokens) break;
+      const size_t index = static_cast<size_t>(token) * a.ldo + feature;
+      if (EPI == EPI_STORE_BF16) static_cast<__nv_bfloat16*>(a.out)[index] = __float2bfloat16_rn(sums[j]);
+      else static_cast<float*>(a.out)[index] = level_off(sums[j], a.softcap);
+    }
+  }
+}
 
 template <int BN, int EPI>
 __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
@@ -162,6 +212,8 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   constexpr bool DUAL = EPI == EPI_SWIGLU;
   using Config = TileConfig<BN, DUAL>;
   constexpr int STAGES = Config::kStages;
+  constexpr bool CLUSTERS = (EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32) && BN <= 128;
+  static_assert(!CLUSTERS || BN * BM * 4 <= STAGES * Config::kStageBytes, "a part lies where the ring was");
 
   hx_pdl_trigger();
   extern __shared__ uint8_t smem_raw[];
@@ -288,11 +340,24 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       } else {
         tc_fence_after();
         const uint32_t lane_address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-        write_tile<BN, EPI>(args.out, args.ldo, args.tokens, args.features, lane_address, feature,
-                            token0, args.activation, args.gate_limit, args.gate_bias, args.up_bias,
-                            args.softcap);
+        if (CLUSTERS && args.cluster > 1)
+          leave_part<BN>(reinterpret_cast<float*>(smem), lane_address, quarter * 32 + lane,
+                         min(BN, args.tokens - token0));
+        else
+          write_tile<BN, EPI>(args.out, args.ldo, args.tokens, args.features, lane_address, feature,
+                              token0, args.activation, args.gate_limit, args.gate_bias, args.up_bias,
+                              args.softcap);
       }
     }
+  }
+  if (CLUSTERS && args.cluster > 1) {      // (every CTA of a cluster comes here, whatever went wrong)
+    __syncthreads();
+    cluster_sync();
+    if (warp >= 2)
+      gather_parts<BN, EPI>(args, reinterpret_cast<const float*>(smem), static_cast<int>(cluster_rank()),
+                            (warp & 3) * 32 + lane, feature0 + (warp & 3) * 32 + lane, token0);
+    __syncthreads();
+    cluster_sync();      // nobody's part is read any more
   }
 
   tc_fence_before();
@@ -1124,6 +1189,23 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& a
     }
     configured = true;
   }
+  if (args.cluster > 1) {
+    cudaLaunchConfig_t config = {};
+    config.gridDim = grid;
+    config.blockDim = THREADS;
+    config.dynamicSmemBytes = Config::kSmemBytes;
+    config.stream = stream;
+    cudaLaunchAttribute attributes[2];
+    attributes[0].id = cudaLaunchAttributeClusterDimension;
+    attributes[0].val.clusterDim.x = attributes[0].val.clusterDim.y = 1;
+    attributes[0].val.clusterDim.z = args.cluster;
+    attributes[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attributes[1].val.programmaticStreamSerializationAllowed = 1;
+    config.attrs = attributes;
+    config.numAttrs = hx_pdl_enabled() ? 2 : 1;
+    cudaLaunchKernelEx(&config, gemm_tc_kernel<BN, EPI>, map_w, map_x, args);
+    return HX_OK;
+  }
   hx_launch(gemm_tc_kernel<BN, EPI>, grid, THREADS, Config::kSmemBytes, stream, map_w, map_x, args);
   return HX_OK;
 }
@@ -1335,15 +1417,34 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
              "hx_gemm_tc: features exceed the weight matrix");
   HX_REQUIRE(ldo >= features, "hx_gemm_tc: output stride too small");
 
-  const int bn = hx_gemm_tc_token_tile(tokens);
+  int bn = hx_gemm_tc_token_tile(tokens);
   // prompt portions: the persistent kernel, whose tiles have 128 tokens on the M side.  A sum
   // into a float32 output over at most 128 tokens is a weight stream even when it is not cut
   // along the reduction (the fused gate/up matrix has tiles enough as it is) and stays with
   // the streaming kernel: 128 weight rows per CTA, two CTAs an SM (measured: steps of 65 to
   // 128 tokens take 6 to 8 % less time than with that one product on the persistent kernel).
-  const bool persistent = bn >= 128 && k_splits == 1 && !(epilogue == EPI_ADD_F32 && tokens <= 128);
-  CUtensorMap map_w, map_x;
   const int total_k_blocks = (depth + BK - 1) / BK;
+  // Products that are stored, deep and of few tiles: as many CTAs a tile, each with a run of k-blocks of its own, as
+  // fill a wave of two CTAs an SM to four fifths (see gather_parts).  A cluster costs about 4 us of its own, so it
+  // needs a depth of 2,048 and four runs (two of 32 blocks for 97 tiles: 17 us without, 18 with); with more
+  // than 128 tokens the persistent kernels have tiles enough unless the features are a handful (300 tokens by
+  // [1,280 x 4,096] 16.0 and 16.4).
+  const bool stores = epilogue == EPI_STORE_BF16 || epilogue == EPI_STORE_F32;
+  int cluster = 1;
+  if (stores && total_k_blocks >= 32) {
+    const long long tiles = static_cast<long long>((tokens + 127) / 128) * ((features + BM - 1) / BM);
+    const long long fit = static_cast<long long>(0.8 * 2 * hx_device_sm_count()) / tiles;
+    if (fit >= 4 && (tokens <= 128 || tiles <= 16)) {
+      cluster = static_cast<int>(fit < 8 ? fit : 8);
+      const int per = (total_k_blocks + cluster - 1) / cluster;
+      cluster = (total_k_blocks + per - 1) / per;      // none without a block
+      if (bn > 128) bn = 128;
+    }
+  }
+  const bool persistent =
+      cluster <= 1 && bn >= 128 && k_splits == 1 && !(epilogue == EPI_ADD_F32 && tokens <= 128);
+  if (cluster > 1) k_splits = cluster;
+  CUtensorMap map_w, map_x;
   const int k_tiles = weight_tiles ? total_k_blocks : 0;
   const WeightBoxes boxes = weight_boxes(w, weight_rows, depth, ldw, k_tiles);
   int rc = get_tensor_map(boxes.base, boxes.rows, boxes.depth, boxes.ld, BM, &map_w);
@@ -1364,7 +1465,7 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
   const int per_split = (total_k_blocks + k_splits - 1) / k_splits;
   k_splits = (total_k_blocks + per_split - 1) / per_split;
   GemmArgs args{out, ldo, tokens, features, depth, up_row_offset, per_split, k_tiles, status,
-                activation, nullptr, 0, gate_limit, gate_bias, up_bias, softcap};
+                activation, nullptr, 0, gate_limit, gate_bias, up_bias, softcap, cluster > 1 ? k_splits : 1};
   const dim3 grid((tokens + bn - 1) / bn, (features + BM - 1) / BM, k_splits);
   HX_REQUIRE(grid.y <= 65535, "hx_gemm_tc: too many features (%d)", features);
 
