@@ -385,13 +385,18 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
 // matrix: gate and up of a feature sit side by side in the thread's own lane.
 //
 // The add epilogue does not add at the memory side here (float32 reductions reach only about
-// 1.8 TB/s in the L2, a quarter of what this product would need): while the MMA warp works on
-// one accumulator, the epilogue warps load the output tile of the unit after it INTO the other
-// accumulator (tcgen05.st), the products then accumulate on top of it, and the epilogue
-// stores the sum.  One writer per element: the result is deterministic.
+// 1.8 TB/s in the L2, a quarter of what this product would need): it reads the output's old values, the
+// first of them while the unit's products run, adds and stores.  One writer per element: the result is
+// deterministic.  Old values loaded INTO the accumulator before the products took 65.6 us at 2,048 x 4,096 x 4,096,
+// 137.2 at depth 11,008 and 201.5 at 1,900 x 5,120 x 13,824 (weights and inputs out of the L2); so it is 61.4,
+// 131.0 and 194.6, and depths of 64 and 512 take 32.8 and 35.6 us after 33.6 and 35.6.
 //
 // Tiles are dealt round-robin with the token tile varying fastest, so the CTAs that run side
 // by side read the same weight tiles at the same time, once from DRAM.
+
+// Floats between rows, and bytes, of what the add epilogue's warps exchange (see add_tile).
+constexpr int ADD_STRIDE = 36;
+constexpr int ADD_BYTES = 4 * 32 * ADD_STRIDE * 4;      // of the four epilogue warps
 
 struct PersistentConfig {
   static constexpr int kRowsA = BM;              // tokens
@@ -400,7 +405,7 @@ struct PersistentConfig {
   static constexpr int kBytesB = kRowsB * BK * 2;
   static constexpr int kStageBytes = kBytesA + kBytesB;
   static constexpr int kStages = 200 * 1024 / kStageBytes;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment*/ + 256 /*barriers*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment*/ + 256 /*barriers*/ + ADD_BYTES;
   static constexpr int kBufferColumns = 256;     // one accumulator per half of tensor memory
   static constexpr int kTmemColumns = 512;
 };
@@ -520,38 +525,74 @@ __device__ __forceinline__ bool unit_at(const PersistentArgs& a, int iteration, 
   return true;
 }
 
-// The add epilogue's preparation: this thread's token, 256 columns of the float32 output
-// into its lane of the accumulator (zeros where the tile hangs over the output's edge).
-__device__ __forceinline__ void load_row_into_accumulator(const float* out, int ldo, int features,
-                                                          uint32_t lane_address, int token,
-                                                          int tokens, int feature0) {
-  const bool wide = (ldo % 4 == 0) && ((reinterpret_cast<uintptr_t>(out) & 15) == 0);
-  const float* row = out + static_cast<size_t>(token < tokens ? token : 0) * ldo + feature0;
-#pragma unroll 1
-  for (int group = 0; group < 2 * BM; group += 64) {
-    float v[4][16];
+// The add epilogue of a warp's 32 tokens, 32 columns at a time, the next 32 on their way.  A thread finds a token's
+// sums in its lane of tensor memory; in the output 32 columns of a token are a line of 128 bytes, which eight threads
+// read and write with 16 bytes each.  So the sums change places in shared memory (rows ADD_STRIDE floats apart use
+// different banks).  With a token a thread, every access 32 lines, 2,048 x 4,096 took 35.8 us at a depth of 64 and
+// 39.7 at 512, so 32.8 and 35.6; at 4,096 64.5, so 61.4.
+
+// Old values: four columns from `column` on of tokens first + 4 i + lane / 8 (zeros behind the output's edges).
+__device__ __forceinline__ void load_old(const float* out, int ldo, int features, int first, int tokens, int column,
+                                         bool wide, float4 (&v)[8]) {
+  const int lane = threadIdx.x & 31, at = column + 4 * (lane & 7);
 #pragma unroll
-    for (int c = 0; c < 4; ++c) {
-      const int column = group + c * 16;
-      if (token < tokens && wide && feature0 + column + 16 <= features) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          const float4 x = *reinterpret_cast<const float4*>(row + column + 4 * j);
-          v[c][4 * j] = x.x;
-          v[c][4 * j + 1] = x.y;
-          v[c][4 * j + 2] = x.z;
-          v[c][4 * j + 3] = x.w;
-        }
+  for (int i = 0; i < 8; ++i) {
+    const int token = first + 4 * i + (lane >> 3);
+    v[i] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (token < tokens) {
+      const float* from = out + static_cast<size_t>(token) * ldo + at;
+      if (wide && at + 4 <= features) {
+        v[i] = *reinterpret_cast<const float4*>(from);
       } else {
-#pragma unroll
-        for (int j = 0; j < 16; ++j)
-          v[c][j] = (token < tokens && feature0 + column + j < features) ? row[column + j] : 0.0f;
+        if (at < features) v[i].x = from[0];
+        if (at + 1 < features) v[i].y = from[1];
+        if (at + 2 < features) v[i].z = from[2];
+        if (at + 3 < features) v[i].w = from[3];
       }
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) tmem_store16(lane_address + group + c * 16, v[c]);
   }
-  asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+}
+
+// 256 columns from feature0 on; `old` holds the first 32.  All lanes of the warp, with the same arguments.
+__device__ __forceinline__ void add_tile(float* out, int ldo, int features, uint32_t lane_address, int first,
+                                         int tokens, int feature0, bool wide, float* exchange, float4 (&old)[8]) {
+  const int lane = threadIdx.x & 31;
+#pragma unroll 1
+  for (int column = 0; column < 2 * BM; column += 32) {
+    if (feature0 + column >= features) break;      // uniform over the warp
+    float4 next[8];
+    if (column + 32 < 2 * BM) load_old(out, ldo, features, first, tokens, feature0 + column + 32, wide, next);
+    uint32_t acc[2][16];
+    tmem_load16_issue(lane_address + column, acc[0]);
+    tmem_load16_issue(lane_address + column + 16, acc[1]);
+    tmem_load_wait();
+    __syncwarp();      // (the last columns are read)
+#pragma unroll
+    for (int j = 0; j < 8; ++j)
+      *reinterpret_cast<uint4*>(exchange + lane * ADD_STRIDE + 4 * j) =
+          make_uint4(acc[j / 4][4 * j % 16], acc[j / 4][4 * j % 16 + 1], acc[j / 4][4 * j % 16 + 2],
+                     acc[j / 4][4 * j % 16 + 3]);
+    __syncwarp();
+    const int at = feature0 + column + 4 * (lane & 7);
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int row = 4 * i + (lane >> 3), token = first + row;
+      const float4 sum = *reinterpret_cast<const float4*>(exchange + row * ADD_STRIDE + 4 * (lane & 7));
+      const float4 v = make_float4(old[i].x + sum.x, old[i].y + sum.y, old[i].z + sum.z, old[i].w + sum.w);
+      if (token < tokens) {
+        float* to = out + static_cast<size_t>(token) * ldo + at;
+        if (wide && at + 4 <= features) {
+          *reinterpret_cast<float4*>(to) = v;
+        } else {
+          if (at < features) to[0] = v.x;
+          if (at + 1 < features) to[1] = v.y;
+          if (at + 2 < features) to[2] = v.z;
+          if (at + 3 < features) to[3] = v.w;
+        }
+      }
+      old[i] = next[i];
+    }
+  }
 }
 
 // This thread's token: `columns` features starting at feature0, 16 at a time, from its lane of
@@ -846,7 +887,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
         const uint32_t use = static_cast<uint32_t>(iteration >> 1);
         // the epilogue must have read this accumulator's previous unit (and, for the add
         // epilogue, have loaded this unit's old output into it: one more arrival)
-        if (!mbar_wait(&tmem_empty_bar[buffer], EPI == EPI_ADD_F32 ? (use & 1u) : (use & 1u) ^ 1u)) {
+        if (!mbar_wait(&tmem_empty_bar[buffer], (use & 1u) ^ 1u)) {
           atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
           break;
@@ -871,7 +912,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
             // a whole tile of the add epilogue starts from the old output in the accumulator
             const uint32_t accumulate =
-                ((EPI == EPI_ADD_F32 && !unit.partial) || kb > unit.kb_begin || k > 0) ? 1u : 0u;
+                (kb > unit.kb_begin || k > 0) ? 1u : 0u;
             umma_bf16(accumulator, desc_a + step, desc_b + step, idesc, accumulate);
           }
           umma_commit(&empty_bar[s]);
@@ -885,26 +926,17 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     const int quarter = warp & 3;     // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     Unit unit;
-    // add epilogue: the old output of unit `iteration` goes into its accumulator, which is
-    // then handed to the MMA warp
-    auto prepare = [&](int iteration) {
-      if (EPI != EPI_ADD_F32 || !unit_at(args, iteration, unit, worker, workers)) return;
-      const int buffer = iteration & 1;
-      if (!unit.partial)      // a piece starts from zero and is added to the output afterwards
-        load_row_into_accumulator(static_cast<const float*>(args.out), args.ldo, args.features,
-                                  lane_base + buffer * Config::kBufferColumns,
-                                  unit.token_tile * BM + quarter * 32 + lane, args.tokens,
-                                  unit.feature_tile * FEATURES);
-      tc_fence_before();
-      __syncwarp();
-      if (lane == 0) mbar_arrive(&tmem_empty_bar[buffer]);
-    };
-    prepare(0);
-    prepare(1);
+    // add epilogue
+    const bool wide = args.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0;
+    float* exchange = reinterpret_cast<float*>(smem + STAGES * Config::kStageBytes + 256);
     for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
       const int buffer = iteration & 1;
       const uint32_t use = static_cast<uint32_t>(iteration >> 1);
       bool ok = true;
+      float4 old[8];
+      if (EPI == EPI_ADD_F32 && !unit.partial)      // on their way while the unit's products run
+        load_old(static_cast<const float*>(args.out), args.ldo, args.features, unit.token_tile * BM + quarter * 32,
+                 args.tokens, unit.feature_tile * FEATURES, wide, old);
       if (lane == 0) ok = mbar_wait(&tmem_full_bar[buffer], use & 1u);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) {
@@ -918,7 +950,11 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       if constexpr (EPI == EPI_ROPE_APPEND) {
         write_row_rope(FEATURES, args, lane_base + buffer * Config::kBufferColumns,
                        unit.token_tile * BM + quarter * 32 + lane, unit.feature_tile * FEATURES);
-      } else if (EPI == EPI_ADD_F32 && unit.partial) {
+      } else if (EPI == EPI_ADD_F32 && !unit.partial) {
+        add_tile(static_cast<float*>(args.out), args.ldo, args.features, lane_base + buffer * Config::kBufferColumns,
+                 unit.token_tile * BM + quarter * 32, args.tokens, unit.feature_tile * FEATURES, wide,
+                 exchange + quarter * 32 * ADD_STRIDE, old);
+      } else if (EPI == EPI_ADD_F32) {
         add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features,
                            lane_base + buffer * Config::kBufferColumns,
                            unit.token_tile * BM + quarter * 32 + lane, args.tokens,
@@ -939,13 +975,9 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       }
       // every lane's tcgen05.ld has completed (the loads are waited for where they are
       // issued): hand the accumulator back
-      if (EPI == EPI_ADD_F32) {
-        prepare(iteration + 2);
-      } else {
-        tc_fence_before();
-        __syncwarp();
-        if (lane == 0) mbar_arrive(&tmem_empty_bar[buffer]);
-      }
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&tmem_empty_bar[buffer]);
     }
   }
 
@@ -975,7 +1007,7 @@ struct PairConfig {
   static constexpr int kBytesB = BM * BK * 2;    // its half of the weight rows
   static constexpr int kStageBytes = kBytesA + kBytesB;
   static constexpr int kStages = 6;
-  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment*/ + 256 /*barriers*/;
+  static constexpr int kSmemBytes = kStages * kStageBytes + 1024 /*alignment*/ + 256 /*barriers*/ + ADD_BYTES;
 };
 
 template <int EPI>
@@ -1072,7 +1104,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
         const int buffer = iteration & 1;
         const uint32_t use = static_cast<uint32_t>(iteration >> 1);
         if (!mbar_wait_cluster(&tmem_empty_bar[buffer],
-                               EPI == EPI_ADD_F32 ? (use & 1u) : (use & 1u) ^ 1u)) {
+                               (use & 1u) ^ 1u)) {
           atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
           break;
@@ -1095,7 +1127,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
             const uint32_t accumulate =
-                ((EPI == EPI_ADD_F32 && !unit.partial) || kb > unit.kb_begin || k > 0) ? 1u : 0u;
+                (kb > unit.kb_begin || k > 0) ? 1u : 0u;
             umma_bf16_pair(accumulator, desc_a + step, desc_b + step, idesc, accumulate);
           }
           umma_commit_pair(&empty_bar[s]);
@@ -1115,21 +1147,17 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(cluster_address(&tmem_empty_bar[buffer], 0));
     };
-    auto prepare = [&](int iteration) {
-      if (EPI != EPI_ADD_F32 || !unit_at(args, iteration, unit, worker, workers)) return;
-      const int buffer = iteration & 1;
-      if (!unit.partial)
-        load_row_into_accumulator(static_cast<const float*>(args.out), args.ldo, args.features,
-                                  lane_base + buffer * kBufferColumns, unit.token_tile * 2 * BM + row,
-                                  args.tokens, unit.feature_tile * FEATURES);
-      hand_over(buffer);
-    };
-    prepare(0);
-    prepare(1);
+    // add epilogue
+    const bool wide = args.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0;
+    float* exchange = reinterpret_cast<float*>(smem + STAGES * Config::kStageBytes + 256);
     for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
       const int buffer = iteration & 1;
       const uint32_t use = static_cast<uint32_t>(iteration >> 1);
       bool ok = true;
+      float4 old[8];
+      if (EPI == EPI_ADD_F32 && !unit.partial)      // on their way while the unit's products run
+        load_old(static_cast<const float*>(args.out), args.ldo, args.features,
+                 unit.token_tile * 2 * BM + row - lane, args.tokens, unit.feature_tile * FEATURES, wide, old);
       if (lane == 0) ok = mbar_wait_cluster(&tmem_full_bar[buffer], use & 1u);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) {
@@ -1146,15 +1174,17 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       const int feature0 = unit.feature_tile * FEATURES + unit.piece * columns;
       if constexpr (EPI == EPI_ROPE_APPEND) {
         write_row_rope(columns, args, accumulator, token, feature0);
-      } else if (EPI == EPI_ADD_F32 && unit.partial) {
+      } else if (EPI == EPI_ADD_F32 && !unit.partial) {
+        add_tile(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token - lane, args.tokens,
+                 feature0, wide, exchange + quarter * 32 * ADD_STRIDE, old);
+      } else if (EPI == EPI_ADD_F32) {
         add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
                            args.tokens, feature0);
       } else {
         write_row<EPI>(columns, args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
                        args.activation, args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
       }
-      if (EPI == EPI_ADD_F32) prepare(iteration + 2);
-      else hand_over(buffer);
+      hand_over(buffer);
     }
   }
 
