@@ -36,6 +36,7 @@ SOURCES = (
     "hx_normed_residual.cu",
     "hx_routed_experts.cu",
     "hx_latent.cu",
+    "hx_gemm_few.cu",
     "hx_gemm_simt.cu",
     "hx_gemm_split.cu",
     "hx_gemm_tc.cu",

@@ -1,12 +1,12 @@
 // Matrix product on the CUDA cores: out[t, o] (+)= sum_k x[t, k] * w[o, k].
 //
 // This is the true 32-bit path (float32 storage, float32 fused multiply-adds, no
-// reduced-precision matrix mode; many tokens take hx_gemm_split.cu, whose sums are closer
-// still) and also the bfloat16 path for shapes the tensor
+// reduced-precision matrix mode; few tokens take hx_gemm_few.cu and many hx_gemm_split.cu, whose sums are
+// closer still) and also the bfloat16 path for shapes the tensor
 // core kernel refuses.  Each output element is one sequential sum over k in
 // ascending order, so in this kernel its value never depends on how many rows the call has or
-// on which tile it falls into (a product that hx_gemm_split.cu takes for its many rows is another
-// order of the same sums).  The reference's counterpart is its 16x16 tiled kernel
+// on which tile it falls into (a product that one of those two takes for its number of rows is
+// another order of the same sums).  The reference's counterpart is its 16x16 tiled kernel
 // (src/kernels/cuda/matmul.cu:36-71).
 //
 // Prompt portions are bound by the multiply-adds and by the 16-byte loads from shared memory
@@ -18,7 +18,8 @@
 //
 // Measured (one B200, float32, alone): 512 tokens by [17,280 x 3,200] 2,243 -> 1,573 us (36
 // TFLOP/s), by [3,200 x 8,640] 2,287 -> 1,071 us, by [4,096 x 4,096] 1,262 -> 512 us; one token
-// by the same 667 -> 68 us (3.2 TB/s of weights), 770 -> 100 us, 296 -> 52 us.
+// by the same 667 -> 68 us (3.2 TB/s of weights), 770 -> 100 us, 296 -> 52 us (a few float32 tokens of
+// a depth from 256 on whose rows begin on 16 bytes are hx_gemm_few.cu's: 51, 29 and 21 us).
 #include "hx_mma.cuh"
 
 #include <mutex>

@@ -622,7 +622,7 @@ HX_API int hx_gemm_split_pays(int tokens, int features) {
 // tiles of 32 x 32 are not a handful (two launches against one).  Measured (us, CUDA cores / one CTA a tile /
 // here): 17 tokens by [17,280 x 3,200] 152 / 123 / 120, by [3,200 x 8,640] 248 / 291 / 151, by [4,096 x 4,096] 123 / 145 /
 // 79, by [1,024 x 4,096] 123 / 148 / 75; 64 tokens 265 / 131 / 126, 272 / 297 / 153, 137 / 152 / 85, 125 / 150 / 77;
-// 16 tokens are the CUDA cores' (123, 131, 68, 64 against 120, 153, 79, 75 here).
+// (Up to 16 tokens, and up to 128 of few features, are hx_gemm_few.cu's.)
 HX_API int hx_gemm_split_scratch_pays(int tokens, int features) {
   const long long small = static_cast<long long>((tokens + 31) / 32) * ((features + 31) / 32);
   return tokens > 16 && small >= 32;

@@ -326,8 +326,11 @@ def _declare(library: ctypes.CDLL) -> None:
                                               _c_ptr, _c_ptr]
     library.hx_gemm_split_terms.argtypes = [_c_int, _c_int]
     library.hx_gemm_split_terms.restype = _c_longlong
-    for name in ("hx_gemm_split_supports", "hx_gemm_split_pays", "hx_gemm_split",
-                 "hx_gemm_split_scratch"):
+    library.hx_gemm_few_takes.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int, _c_int]
+    library.hx_gemm_few.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int,
+                                    _c_int, _c_int, _c_float, _c_ptr]
+    for name in ("hx_gemm_few_takes", "hx_gemm_few", "hx_gemm_split_supports", "hx_gemm_split_pays",
+                 "hx_gemm_split", "hx_gemm_split_scratch"):
         getattr(library, name).restype = _c_int
     library.hx_gemm_tc_ordered.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr,
                                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr]
@@ -649,6 +652,25 @@ def gemm_simt(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, 
     _check(lib().hx_gemm_simt_softcapped(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
                                          out.data_ptr(), out.stride(0), dtype_code(x.dtype), tokens,
                                          features, depth, epilogue, float(softcap), _stream()))
+
+
+def gemm_few_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int) -> bool:
+    """Whether a float32 product runs, and is faster, as :func:`gemm_few`."""
+    return (x.dtype == w.dtype == out.dtype == torch.float32
+            and bool(lib().hx_gemm_few_takes(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
+                                             tokens, w.shape[0], w.shape[1])))
+
+
+def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, epilogue: int,
+             softcap: float = 0.0) -> None:
+    """:func:`gemm_simt` for a few float32 tokens, as a stream of the weights: the same multiply-adds,
+    the depth of a sum split over the lanes of two warps.  A value does not depend on the other rows."""
+    for tensor, name in ((x, "x"), (w, "w"), (out, "out")):
+        _need(tensor, torch.float32, name)
+    assert x.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1
+    features, depth = w.shape
+    _check(lib().hx_gemm_few(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0), out.data_ptr(),
+                             out.stride(0), tokens, features, depth, epilogue, float(softcap), _stream()))
 
 
 def gemm_split_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int) -> bool:

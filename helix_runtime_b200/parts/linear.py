@@ -81,7 +81,9 @@ def _gemm_simt(x, w: Weight, out, tokens, epilogue, status, softcap: float = 0.0
         raise RuntimeError("this product needs the CUDA-core kernel, but the weight is held as "
                            "tiles for the tensor cores")
     matrix = w.matrix if features is None else w.matrix[:features]
-    if ops.gemm_split_takes(x, matrix, out, tokens):
+    if ops.gemm_few_takes(x, matrix, out, tokens):
+        ops.gemm_few(x, matrix, out, tokens, epilogue, softcap)
+    elif ops.gemm_split_takes(x, matrix, out, tokens):
         size = ops.gemm_split_terms(tokens, w.depth) if workspace is not None else 0
         terms = workspace.at_least("split.terms", size, torch.bfloat16) if size > 0 else None
         ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap, terms)
