@@ -521,6 +521,11 @@ int hx_gemm_simt(const void* x, int ldx, const void* w, int ldw, void* out, int 
 int hx_gemm_simt_softcapped(const void* x, int ldx, const void* w, int ldw, void* out, int ldo,
                             int dtype, int tokens, int features, int depth, int epilogue,
                             float softcap, cudaStream_t stream);
+/* float32, a few tokens: a stream of the weights, each sum over the lanes of two warps in a fixed order;
+ * whether the product runs there and is the faster road (rows from 256 on, on 16 bytes) */
+int hx_gemm_few_takes(const void* x, int ldx, const void* w, int ldw, int tokens, int features, int depth);
+int hx_gemm_few(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
+                int features, int depth, int epilogue, float softcap, cudaStream_t stream);
 int hx_gemm_tc_softcapped(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,
                           int weight_rows, float* out, int ldo, int tokens, int features,
                           int depth, float softcap, int weight_tiles, int* status,
