@@ -618,14 +618,24 @@ HX_API int hx_gemm_split_pays(int tokens, int features) {
   return tokens > 16 && small >= 2ll * hx_device_sm_count();
 }
 
-// The same for a caller with scratch: the pairs' kernel beats the CUDA cores from 17 tokens on wherever the latter's
-// tiles of 32 x 32 are not a handful (two launches against one).  Measured (us, CUDA cores / one CTA a tile /
-// here): 17 tokens by [17,280 x 3,200] 152 / 123 / 120, by [3,200 x 8,640] 248 / 291 / 151, by [4,096 x 4,096] 123 / 145 /
-// 79, by [1,024 x 4,096] 123 / 148 / 75; 64 tokens 265 / 131 / 126, 272 / 297 / 153, 137 / 152 / 85, 125 / 150 / 77;
-// (Up to 16 tokens, and up to 128 of few features, are hx_gemm_few.cu's.)
-HX_API int hx_gemm_split_scratch_pays(int tokens, int features) {
+// The same for a caller with scratch.  The cut is a launch of its own, and a pair's way through its first blocks is
+// longer: 6 to 8 us more than the CUDA cores take for a shallow product, 2 more than one CTA a tile, which a deep
+// product or several rounds of tiles bring back.  Measured (us, the road without scratch / here):
+//   fewer tiles of 32 x 32 than SMs: 129 tokens by [700 x 64] 3.6 / 12.2, x 512 17.0 / 18.3, x 768 24.3 / 23.0;
+//   fewer than two an SM: 256 by [700 x 256] 11.9 / 18.3, 129 by [1,500 x 256] 13.4 / 16.1, x 512 24.6 / 19.1, 64 by [4,000 x
+//   128] 8.4 / 10.1, x 256 14.5 / 12.2;
+//   more (without scratch one CTA a tile): 256 by [9,000 x 64] 9.7 / 12.7, 512 18.6 / 17.2, 512 by [4,000 x 128] 12.4 / 13.7, 1,024
+//   23.6 / 20.0, 256 by [4,000 x 256] 16.8 / 14.6, 2,048 by [300 x 256] 15.7 / 16.5, x 512 23.3 / 20.2.
+// 17 tokens by [17,280 x 3,200] 123 / 120, by [3,200 x 8,640] 248 / 151.  (Up to 16 tokens, and up to 128 of few
+// features, are hx_gemm_few.cu's.)
+HX_API int hx_gemm_split_scratch_pays(int tokens, int features, int depth) {
   const long long small = static_cast<long long>((tokens + 31) / 32) * ((features + 31) / 32);
-  return tokens > 16 && small >= 32;
+  const int sms = hx_device_sm_count();
+  if (tokens <= 16 || small < 32) return 0;
+  if (small < 2ll * sms) return depth >= (small < sms ? 640 : tokens > 64 ? 512 : 256);
+  const long long units = static_cast<long long>((tokens + PAIR_TOKENS - 1) / PAIR_TOKENS) *
+                          ((features + TILE - 1) / TILE);
+  return depth >= 512 || units > sms / 2 || (depth >= 256 && tokens <= 4ll * features);
 }
 
 // Numbers of bfloat16 scratch (on 16 bytes) that hx_gemm_split_scratch has a use for.

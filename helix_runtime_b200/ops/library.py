@@ -317,7 +317,7 @@ def _declare(library: ctypes.CDLL) -> None:
         _c_ptr, _c_ptr, _c_int, _c_ptr, _c_ptr, _c_ptr, _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr]
     library.hx_gemm_split_supports.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int]
     library.hx_gemm_split_pays.argtypes = [_c_int, _c_int]
-    library.hx_gemm_split_scratch_pays.argtypes = [_c_int, _c_int]
+    library.hx_gemm_split_scratch_pays.argtypes = [_c_int, _c_int, _c_int]
     library.hx_gemm_split_scratch_pays.restype = _c_int
     library.hx_gemm_split.argtypes = [_c_ptr, _c_int, _c_ptr, _c_int, _c_ptr, _c_int, _c_int, _c_int,
                                       _c_int, _c_int, _c_float, _c_ptr, _c_ptr]
@@ -676,7 +676,8 @@ def gemm_few(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, e
 def gemm_split_takes(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int) -> bool:
     """Whether a float32 product runs, and is faster, as :func:`gemm_split`."""
     return (x.dtype == w.dtype == out.dtype == torch.float32
-            and bool(lib().hx_gemm_split_scratch_pays(tokens, w.shape[0]))
+            and bool(lib().hx_gemm_split_pays(tokens, w.shape[0]) or
+                     lib().hx_gemm_split_scratch_pays(tokens, *w.shape))
             and bool(lib().hx_gemm_split_supports(x.data_ptr(), x.stride(0), w.data_ptr(), w.stride(0),
                                                   w.shape[0], w.shape[1])))
 
@@ -686,19 +687,25 @@ def gemm_split_terms(tokens: int, depth: int) -> int:
     return int(lib().hx_gemm_split_terms(tokens, depth))
 
 
+def gemm_split_scratch_pays(tokens: int, features: int, depth: int) -> bool:
+    """Whether :func:`gemm_split` is faster with scratch (a launch more) than without."""
+    return bool(lib().hx_gemm_split_scratch_pays(tokens, features, depth))
+
+
 def gemm_split(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, epilogue: int,
                status: torch.Tensor, softcap: float = 0.0,
-               terms: Optional[torch.Tensor] = None) -> None:
+               terms: Optional[torch.Tensor] = None, scratch: bool = True) -> None:
     """:func:`gemm_simt` for many float32 tokens, on the tensor cores: both operands as three
     bfloat16 terms, 24 bits, sums of 64 products added in float32.  Closer to the sum of 64 bits than
     the chain of multiply-adds; like that one, the same from call to call.  ``terms``: contiguous
-    scratch of :func:`gemm_split_terms` numbers (allocated here if there is none)."""
+    scratch of :func:`gemm_split_terms` numbers (allocated here if there is none); ``scratch``
+    False: the road that needs none, with the same bits."""
     for tensor, name in ((x, "x"), (w, "w"), (out, "out")):
         _need(tensor, torch.float32, name)
     assert x.stride(-1) == 1 and w.stride(-1) == 1 and out.stride(-1) == 1
     features, depth = w.shape
     if terms is None:
-        size = gemm_split_terms(tokens, depth)
+        size = gemm_split_terms(tokens, depth) if scratch else 0
         terms = torch.empty(size, dtype=torch.bfloat16, device=x.device) if size > 0 else None
     else:
         _need(terms, torch.bfloat16, "terms")

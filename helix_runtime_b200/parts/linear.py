@@ -84,9 +84,10 @@ def _gemm_simt(x, w: Weight, out, tokens, epilogue, status, softcap: float = 0.0
     if ops.gemm_few_takes(x, matrix, out, tokens):
         ops.gemm_few(x, matrix, out, tokens, epilogue, softcap)
     elif ops.gemm_split_takes(x, matrix, out, tokens):
-        size = ops.gemm_split_terms(tokens, w.depth) if workspace is not None else 0
+        scratch = ops.gemm_split_scratch_pays(tokens, *matrix.shape)
+        size = ops.gemm_split_terms(tokens, w.depth) if scratch and workspace is not None else 0
         terms = workspace.at_least("split.terms", size, torch.bfloat16) if size > 0 else None
-        ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap, terms)
+        ops.gemm_split(x, matrix, out, tokens, epilogue, status, softcap, terms, scratch)
     else:
         ops.gemm_simt(x, matrix, out, tokens, epilogue, softcap)
 

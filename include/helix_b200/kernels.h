@@ -543,7 +543,7 @@ int hx_gemm_split(const float* x, int ldx, const float* w, int ldw, float* out, 
                   cudaStream_t stream);
 /* the same with scratch for the terms of x (hx_gemm_split_terms() bfloat16 numbers on 16 bytes; null: the
  * product does without), and whether it is then the faster road */
-int hx_gemm_split_scratch_pays(int tokens, int features);
+int hx_gemm_split_scratch_pays(int tokens, int features, int depth);
 long long hx_gemm_split_terms(int tokens, int depth);
 int hx_gemm_split_scratch(const float* x, int ldx, const float* w, int ldw, float* out, int ldo, int tokens,
                           int features, int depth, int epilogue, float softcap, void* terms,

@@ -131,3 +131,28 @@ def test_pairs_have_the_sums_of_single_tiles(tokens, features, depth):
                                            status.data_ptr(), ops._stream()))
         torch.testing.assert_close(out, plain, rtol=0, atol=0, equal_nan=True)
     assert terms[size:].isnan().all() and int(status.item()) == 0
+
+
+@pytest.mark.parametrize("tokens,features,depth,scratch", [
+    (129, 700, 64, 0), (129, 1500, 256, 0), (256, 300, 256, 0), (2048, 16, 64, 0), (100, 300, 128, 0),
+    (129, 700, 512, 0), (256, 9000, 64, 0), (512, 4000, 128, 0), (2048, 300, 256, 0),
+    (129, 1500, 512, 1), (129, 700, 640, 1), (64, 4000, 256, 1), (512, 9000, 64, 1), (256, 4000, 256, 1),
+])
+def test_shallow_products_do_not_pay_for_the_cut(tokens, features, depth, scratch):
+    """Where the cut of the tokens costs more than it gives the product takes none, and has the bits of the road
+    that it takes instead."""
+    from helix_runtime_b200.ops import library as ops
+    from helix_runtime_b200.parts.base import Workspace
+    from helix_runtime_b200.parts.linear import Weight, project
+    torch.manual_seed(tokens)
+    x, w = torch.randn(tokens, depth, device="cuda"), torch.randn(features, depth, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    workspace = Workspace(torch.device("cuda"))
+    out, want = torch.zeros((2, tokens, features), device="cuda")
+    project(x, Weight(w), out, tokens, ops.EPI_STORE_F32, status, workspace=workspace)
+    assert (workspace.bytes() > 0) == bool(scratch)
+    if ops.gemm_split_takes(x, w, out, tokens):
+        ops.gemm_split(x, w, want, tokens, ops.EPI_STORE_F32, status, scratch=False)
+    else:
+        ops.gemm_simt(x, w, want, tokens, ops.EPI_STORE_F32)
+    assert torch.equal(out, want) and int(status.item()) == 0
