@@ -1456,16 +1456,19 @@ static int gemm_tc(const void* x, int ldx, int x_capacity_rows, const void* w, i
   const int total_k_blocks = (depth + BK - 1) / BK;
   // Products that are stored, deep and of few tiles: as many CTAs a tile, each with a run of k-blocks of its own, as
   // fill a wave of two CTAs an SM to four fifths (see gather_parts).  A cluster costs about 4 us of its own, so it
-  // needs a depth of 2,048 and four runs (two of 32 blocks for 97 tiles: 17 us without, 18 with); with more
-  // than 128 tokens the persistent kernels have tiles enough unless the features are a handful (300 tokens by
-  // [1,280 x 4,096] 16.0 and 16.4).
+  // needs a depth of 2,048 and four runs (two of 32 blocks for 97 tiles: 17 us without, 18 with).  More than 128
+  // tokens have the persistent kernels, 0.17 us a block of 64 against 0.25, and the epilogues of several tiles of 128
+  // tokens: from a depth of 3,072 on, and four runs up to 6,144 (us, without / four runs / eight: 300 tokens by [16 x
+  // 2,048] 9.0 / 9.9 / 10.9, x 3,072 11.8 / 11.2 / 11.4, x 5,120 17.4 / 13.7 / 12.9; 1,500 by [16 x 3,072] 11.6 / 11.4 / 15.0, x 4,096
+  // 14.5 / 12.9 / 15.8; 700 by [256 x 4,096] 15.3 / 13.0 / 15.8; eight runs, 1,500 by [16 x 6,144] 19.8 / 17.0).
   const bool stores = epilogue == EPI_STORE_BF16 || epilogue == EPI_STORE_F32;
   int cluster = 1;
-  if (stores && total_k_blocks >= 32) {
+  if (stores && total_k_blocks >= (tokens <= 128 ? 32 : 48)) {
     const long long tiles = static_cast<long long>((tokens + 127) / 128) * ((features + BM - 1) / BM);
     const long long fit = static_cast<long long>(0.8 * 2 * hx_device_sm_count()) / tiles;
     if (fit >= 4 && (tokens <= 128 || tiles <= 16)) {
-      cluster = static_cast<int>(fit < 8 ? fit : 8);
+      cluster = fit < 8 ? static_cast<int>(fit) : 8;
+      if (tokens > 128 && total_k_blocks < 96) cluster = 4;
       const int per = (total_k_blocks + cluster - 1) / cluster;
       cluster = (total_k_blocks + per - 1) / per;      // none without a block
       if (bn > 128) bn = 128;

@@ -38,3 +38,21 @@ def test_clusters_add_up_their_parts(tokens, features, depth):
     ops.gemm_tc(x, w, out, tokens, features, ops.EPI_STORE_F32, status, softcap=5.0)
     assert ((out - 5.0 * torch.tanh(want / 5.0)).abs() <= bound + 1e-5).all()
     assert int(status.item()) == 0
+
+
+@pytest.mark.parametrize("tokens,features,depth,cut", [
+    (129, 16, 2048, 0), (300, 512, 2560, 0), (1500, 16, 2048, 0), (2048, 100, 3008, 0), (700, 256, 2048, 0),
+    (129, 16, 3072, 1), (1500, 16, 4096, 1), (2048, 100, 6144, 1), (128, 16, 2048, 1),
+])
+def test_shallow_prompts_keep_one_chain(tokens, features, depth, cut):
+    """More than 128 tokens of a depth below 3,072 are faster as one chain over the depth: the bits of a sum
+    that is added up by one writer, which is never cut."""
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(tokens)
+    x = torch.randn(tokens, depth, device="cuda").bfloat16()
+    w = torch.randn(features, depth, device="cuda").bfloat16()
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    out, chain = torch.zeros((2, tokens, features), device="cuda")
+    ops.gemm_tc(x, w, out, tokens, features, ops.EPI_STORE_F32, status)
+    ops.gemm_tc(x, w, chain, tokens, features, ops.EPI_ADD_F32, status, ordered=True)
+    assert torch.equal(out, chain) == (not cut) and int(status.item()) == 0
