@@ -335,6 +335,10 @@ def _declare(library: ctypes.CDLL) -> None:
     library.hx_gemm_tc_ordered.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr,
                                            _c_int, _c_int, _c_int, _c_int, _c_int, _c_ptr, _c_ptr]
     library.hx_gemm_tc_ordered.restype = _c_int
+    library.hx_gemm_tc_stored_ordered.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr,
+                                                  _c_int, _c_int, _c_int, _c_int, _c_int, _c_float, _c_int,
+                                                  _c_ptr, _c_ptr]
+    library.hx_gemm_tc_stored_ordered.restype = _c_int
     library.hx_gemm_tc_runs_supports.argtypes = [_c_int] * 6
     library.hx_gemm_tc_runs.argtypes = [_c_ptr, _c_int, _c_int, _c_ptr, _c_int, _c_int, _c_ptr, _c_int,
                                         _c_int, _c_int, _c_int, _c_int, _c_float, _c_int, _c_ptr, _c_ptr,
@@ -743,7 +747,9 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, fe
     the epilogue is that gated activation of ``[gate; up]`` whatever ``epilogue`` says, with the
     optional float32 biases ``gate_bias`` and ``up_bias`` ``[features]`` added first.
     ``softcap`` > 0 with ``EPI_STORE_F32``: softcap * tanh(product / softcap) is stored.
-    ``ordered`` with ``EPI_ADD_F32``: one writer per sum, so that a call repeats bit for bit."""
+    ``ordered`` with ``EPI_ADD_F32``: one writer per sum, so that a call repeats bit for bit; with
+    ``EPI_STORE`` and ``EPI_STORE_F32``: one chain over the depth, so that a sum does not depend on the
+    number of tokens (else a few tiles' depth is shared by clusters of CTAs)."""
     _need(x, torch.bfloat16, "x")
     _need(w, torch.bfloat16, "w")
     tiled = w.dim() == 4
@@ -769,9 +775,15 @@ def gemm_tc(x: torch.Tensor, w: torch.Tensor, out: torch.Tensor, tokens: int, fe
                                       _ptr(up_bias), up_row_offset, 1 if tiled else 0,
                                       status.data_ptr(), _stream()))
         return
+    if softcap > 0.0 and (epilogue != EPI_STORE_F32 or k_splits != 1):
+        raise ValueError("a softcap belongs to a float32 store")
+    if ordered and epilogue in (EPI_STORE, EPI_STORE_F32) and k_splits == 1:
+        _check(lib().hx_gemm_tc_stored_ordered(
+            x.data_ptr(), x.stride(0), x.shape[0], w.data_ptr(), ldw, rows, out.data_ptr(), out.stride(0),
+            tokens, features, depth, epilogue, float(softcap), 1 if tiled else 0, status.data_ptr(),
+            _stream()))
+        return
     if softcap > 0.0:
-        if epilogue != EPI_STORE_F32 or k_splits != 1:
-            raise ValueError("a softcap belongs to a float32 store")
         _check(lib().hx_gemm_tc_softcapped(x.data_ptr(), x.stride(0), x.shape[0], w.data_ptr(), ldw,
                                            rows, out.data_ptr(), out.stride(0), tokens, features,
                                            depth, float(softcap), 1 if tiled else 0,

@@ -320,7 +320,8 @@ class PagedAttention(Mixer):
         else:
             raw = ctx.workspace.get(f"attention.projected/{self.projected_size}",
                                     (ctx.capacity, self.projected_size), ctx.dtype)
-            project(x, self.w_qkv, raw, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+            project(x, self.w_qkv, raw, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                    workspace=ctx.workspace)
         ops.short_conv_append(raw, accumulator, qkv, self.conv_filter, cache.state, ctx.positions,
                               ctx.token_request, ctx.request_slot, ctx.request_start,
                               cache.block_tables if appends else None,
@@ -432,7 +433,8 @@ class PagedAttention(Mixer):
             self.position.apply(ctx, cache, qkv, self.heads, self.kv_heads, accum=accumulator)
         elif not self.position.project_and_apply(ctx, cache, x, self.w_qkv, qkv, self.heads,
                                                  self.kv_heads):
-            project(x, self.w_qkv, qkv, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+            project(x, self.w_qkv, qkv, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                    workspace=ctx.workspace)
             self.position.apply(ctx, cache, qkv, self.heads, self.kv_heads)
 
         self.attend(ctx, cache, qkv, context)
@@ -445,7 +447,8 @@ class PagedAttention(Mixer):
             else:
                 gate = ctx.workspace.get(f"attention.gate/{self.q_size}",
                                          (ctx.capacity, self.q_size), ctx.dtype)
-                project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+                project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                        workspace=ctx.workspace)
             ops.sigmoid_gate(context, gate, n, self.q_size, clear=uncleared)
         elif uncleared is not None:
             uncleared[:n].zero_()
@@ -591,7 +594,7 @@ class NormedProjectionAttention(PagedAttention):
         else:
             projected = get(f"attention.projected_sums/{self.projected_size}",
                             (ctx.capacity, self.projected_size), torch.float32)
-            project(x, self.w_proj, projected, n, ops.EPI_STORE_F32, ctx.status,
+            project(x, self.w_proj, projected, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
                     workspace=ctx.workspace)
             clear = False
         ops.biased_normed_rows(projected, clear, qkv, n, self.heads, self.kv_heads, self.head_dim,
@@ -762,12 +765,14 @@ class LatentAttention(PagedAttention):
         rows = get(f"latent.rows/{self.rows_size}", (ctx.capacity, self.rows_size), ctx.dtype)
         context = get(f"attention.context/{self.q_size}", (ctx.capacity, self.q_size), ctx.dtype)
         heads_out = get(f"latent.heads/{self.o_columns}", (ctx.capacity, self.o_columns), ctx.dtype)
-        project(x, self.w_down, down, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_down, down, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         ops.latent_prepare(down, self.q_norm, self.kv_norm, self.eps, ctx.positions, self.freq,
                            self.freq_exact, self.rotary_dims, self.rotary_layout, latent, rows,
                            self.q_size, n, self.q_rank, self.kv_rank, self.rotated_dim,
                            self.row_dim, amplitude=self.amplitude)
-        project(latent, self.w_q_up, q, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+        project(latent, self.w_q_up, q, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         # [Uk_h' q_h | rot(qr_h) | 0] per head
         ops.head_products(q, self.plain_dim, self.w_k_up, rows, self.row_dim, n, ctx.status)
         ops.latent_queries(q, self.heads * self.plain_dim, rows, ctx.positions, self.freq,
@@ -785,7 +790,8 @@ class LatentAttention(PagedAttention):
                           ctx.status)
         if self.gated:
             gate = get(f"attention.gate/{self.o_columns}", (ctx.capacity, self.o_columns), ctx.dtype)
-            project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+            project(x, self.w_g, gate, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                    workspace=ctx.workspace)
             ops.sigmoid_gate(heads_out, gate, n, self.o_columns)
         project(heads_out, self.w_o, residual, n, ops.EPI_ADD_F32, ctx.status, ctx.ordered_sums,
                 workspace=ctx.workspace)
@@ -947,7 +953,7 @@ class DifferentialAttention(PagedAttention):
         else:
             size = -(-self.projected_size // 8) * 8
             projected = get(f"attention.projected/{size}", (ctx.capacity, size), ctx.dtype)
-            project(x, self.w_proj, projected, n, ops.EPI_STORE, ctx.status,
+            project(x, self.w_proj, projected, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
                     workspace=ctx.workspace)
         table = self.table
         write = not self.shared_cache

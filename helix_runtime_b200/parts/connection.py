@@ -135,7 +135,7 @@ class GatedConnection(Part):
         n = ctx.n_tokens
         norm.forward(ctx, streams, normed)
         project(normed, self.weight, self._gate(ctx), n, ops.EPI_STORE_F32, ctx.status,
-                workspace=ctx.workspace)
+                ctx.ordered_sums, workspace=ctx.workspace)
         output[:n].zero_()
 
     def write_back(self, ctx: StepContext, streams: torch.Tensor, output: torch.Tensor) -> None:
@@ -173,7 +173,7 @@ class LinearRejoin(Part):
         n, h = ctx.n_tokens, self.hidden_size
         joined = ctx.workspace.get(f"linear_rejoin.joined/{h}", (ctx.capacity, 2 * h), ctx.dtype)
         ops.join_rows(residual, embedded, joined, n)
-        project(joined, self.weight, residual, n, ops.EPI_STORE_F32, ctx.status,
+        project(joined, self.weight, residual, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
                 workspace=ctx.workspace)
         ops.add_bias(residual, self.step, n)
 
@@ -271,10 +271,12 @@ class TokenSideInput(Part):
         sums = get(f"token_side.sums/{self.dim}", (ctx.capacity, self.dim), torch.float32)
         gated = get(f"token_side.gated/{self.dim}", (ctx.capacity, self.dim), ctx.dtype)
         y = get(f"token_side.output/{h}", (ctx.capacity, h), torch.float32)
-        project(x, self.w_gate, sums, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_gate, sums, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         ops.token_gate(sums, False, self.table, self.offset, ctx.token_ids, gated, n, self.dim,
                        ctx.status)
-        project(gated, self.w_proj, y, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
+        project(gated, self.w_proj, y, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         ops.norm_residual_add(residual, y, self.norm, self.eps, self.scale, n)
 
 

@@ -105,8 +105,8 @@ class LmHead(Part):
         return self.weight.nbytes()
 
     def forward(self, ctx: StepContext, x: torch.Tensor, logits: torch.Tensor, rows: int) -> None:
-        project(x, self.weight, logits, rows, ops.EPI_STORE_F32, ctx.status, softcap=self.softcap,
-                workspace=ctx.workspace)
+        project(x, self.weight, logits, rows, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                softcap=self.softcap, workspace=ctx.workspace)
 
 
 register_part("embedding", "token_table", TokenEmbedding)

@@ -152,7 +152,8 @@ class DenseMlp(FeedForward):
                                  torch.float32)
         act = ctx.workspace.get(f"mlp.act/{self.intermediate}", (ctx.capacity, self.intermediate),
                                 ctx.dtype)
-        project(x, self.w_up, sums, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_up, sums, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         ops.biased_activation(sums, self.up_bias, act, n, ops.ACT_XIELU, *self.constants)
         if self.down_bias is not None and not bias_in_place:
             ops.add_bias(residual, self.down_bias, n)
@@ -270,7 +271,8 @@ class RoutedExperts(FeedForward):
         weights = get(f"experts.weights/{self.top}", (ctx.capacity, self.top), torch.float32)
         act = get(f"experts.act/{self.top}x{self.intermediate}",
                   (ctx.capacity * self.top, self.intermediate), ctx.dtype)
-        project(x, self.w_router, sums, n, ops.EPI_STORE_F32, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_router, sums, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         ops.route_top(sums, chosen, weights, n, self.router_outputs, self.top, self.scale,
                       softmax=self.softmax, correction=self.correction, normalize=self.normalize,
                       chosen_softmax=self.chosen_softmax, bias=self.router_bias)

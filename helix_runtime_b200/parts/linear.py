@@ -122,7 +122,8 @@ def project(x: torch.Tensor, w: Weight, out: torch.Tensor, tokens: int, epilogue
             features: Optional[int] = None, workspace=None) -> None:
     """``out[:tokens] (op)= x[:tokens] @ w.T``; epilogue is one of ops.EPI_STORE,
     ops.EPI_STORE_F32, ops.EPI_ADD_F32.  ``features``: only the first so many rows of ``w``.
-    ``ordered``: one writer per sum, no split-K (see ``split_k_for``) and no shared last round.
+    ``ordered``: one writer per sum, no split-K (see ``split_k_for``), no shared last round and no
+    clusters: one chain over the depth, whatever the number of tokens.
     ``softcap`` > 0 (ops.EPI_STORE_F32 only): ``softcap * tanh(product / softcap)``.
     ``workspace``: where a product that wants scratch takes it from (else it allocates)."""
     if tokens == 0:
@@ -197,7 +198,7 @@ def project_gated(x: torch.Tensor, w_gate_up: Weight, intermediate: int, act: to
     else:
         sums = workspace.get(f"mlp.gate_up/{intermediate}", (capacity, 2 * intermediate),
                              torch.float32)
-        project(x, w_gate_up, sums, tokens, ops.EPI_STORE_F32, status, workspace=workspace)
+        project(x, w_gate_up, sums, tokens, ops.EPI_STORE_F32, status, ordered, workspace=workspace)
         clear = False
     ops.swiglu(sums[:tokens], act[:tokens], zero_input=clear, activation=activation,
                gate_bias=gate_bias, up_bias=up_bias, limit=limit)

@@ -150,7 +150,8 @@ class StateSpaceMixer(Mixer):
                               torch.float32)
         gated = ctx.workspace.get(f"state_space.gated/{self.inner}", (ctx.capacity, self.inner),
                                   ctx.dtype)
-        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         inner, bc = self.inner, self.groups * self.state_size
         ops.causal_filter(rows[:, inner:inner + self.filtered], filtered, self.filter,
                           self.filter_bias,
@@ -227,13 +228,13 @@ class TimeMix(Mixer):
                         ctx.request_slot, ctx.request_start)
         for index, role in enumerate(("r", "k", "v", "g")):
             project(mixes[index], self.weights[role], projected[index], n, ops.EPI_STORE, ctx.status,
-                    workspace=ctx.workspace)
+                    ctx.ordered_sums, workspace=ctx.workspace)
         project(mixes[4], self.weights["w1"], low_sums, n, ops.EPI_STORE_F32, ctx.status,
-                workspace=ctx.workspace)
+                ctx.ordered_sums, workspace=ctx.workspace)
         ops.biased_activation(low_sums[:, :self.decay_rank], None, low[:, :self.decay_rank], n,
                               ops.ACT_TANH)
         project(low[:, :self.decay_rank], self.weights["w2"], decay_log, n, ops.EPI_STORE_F32,
-                ctx.status, workspace=ctx.workspace)
+                ctx.status, ctx.ordered_sums, workspace=ctx.workspace)
         ops.outer_product_scan(projected[0], projected[1], projected[2], decay_log, self.w0,
                                self.bonus, _state_piece(cache, h, self.matrix_state), o,
                                ctx.request_start, ctx.request_slot, ctx.n_requests, self.heads,
@@ -416,7 +417,8 @@ class LinearState(Mixer):
                               torch.float32)
         gated = ctx.workspace.get(f"linear_state.gated/{self.v_width}",
                                   (ctx.capacity, self.v_width), ctx.dtype)
-        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+        project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                workspace=ctx.workspace)
         qkv = rows
         if self.taps is not None:
             qkv = ctx.workspace.get(f"linear_state.filtered/{self.filtered}",
@@ -532,7 +534,8 @@ class GatedRecurrence(Mixer):
             project_into_accumulator(x, self.w_in, rows, n, ctx.status, ctx.ordered_sums)
         else:
             rows = get(f"gated_recurrence.rows/{w}", (ctx.capacity, -(-2 * w // 8) * 8), ctx.dtype)
-            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, workspace=ctx.workspace)
+            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                    workspace=ctx.workspace)
         # rows of a width that keeps them 16-byte aligned
         wide = -(-w // 8) * 8
         u = get(f"gated_recurrence.filtered/{w}", (ctx.capacity, wide), ctx.dtype)
@@ -645,11 +648,11 @@ class MatrixLstm(Mixer):
         else:
             size = -(-self.rows_size // 8) * 8
             rows = get(f"matrix_lstm.rows/{size}", (ctx.capacity, size), ctx.dtype)
-            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, features=self.rows_size,
-                    workspace=ctx.workspace)
+            project(x, self.w_in, rows, n, ops.EPI_STORE, ctx.status, ctx.ordered_sums,
+                    features=self.rows_size, workspace=ctx.workspace)
             width = -(-2 * heads // 4) * 4
             gate_sums = get(f"matrix_lstm.gate_sums/{width}", (ctx.capacity, width), torch.float32)
-            project(x, self.w_gates, gate_sums, n, ops.EPI_STORE_F32, ctx.status,
+            project(x, self.w_gates, gate_sums, n, ops.EPI_STORE_F32, ctx.status, ctx.ordered_sums,
                     workspace=ctx.workspace)
         batch = (ctx.request_start, ctx.request_slot, ctx.n_requests, n, heads, self.head_dim,
                  self.value_dim)

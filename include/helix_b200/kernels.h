@@ -534,6 +534,12 @@ int hx_gemm_tc_softcapped(const void* x, int ldx, int x_capacity_rows, const voi
 int hx_gemm_tc_ordered(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,
                        int weight_rows, float* out, int ldo, int tokens, int features, int depth,
                        int weight_tiles, int* status, cudaStream_t stream);
+/* out = x w^T (epilogue 0 or 1; softcap as above) as one chain over the depth: a sum does not depend on the
+ * number of tokens, where hx_gemm_tc shares the depth of a few tiles out to clusters of CTAs */
+int hx_gemm_tc_stored_ordered(const void* x, int ldx, int x_capacity_rows, const void* w, int ldw,
+                              int weight_rows, void* out, int ldo, int tokens, int features, int depth,
+                              int epilogue, float softcap, int weight_tiles, int* status,
+                              cudaStream_t stream);
 /* the float32 product on the tensor cores: operands as three bfloat16 terms (24 bits), sums of 64 k added
  * in float32 registers; rows of a multiple of four that begin on 16 bytes */
 int hx_gemm_split_supports(const void* x, int ldx, const void* w, int ldw, int features, int depth);

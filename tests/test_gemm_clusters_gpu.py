@@ -56,3 +56,24 @@ def test_shallow_prompts_keep_one_chain(tokens, features, depth, cut):
     ops.gemm_tc(x, w, out, tokens, features, ops.EPI_STORE_F32, status)
     ops.gemm_tc(x, w, chain, tokens, features, ops.EPI_ADD_F32, status, ordered=True)
     assert torch.equal(out, chain) == (not cut) and int(status.item()) == 0
+
+
+@pytest.mark.parametrize("features,depth", [(16, 4096), (300, 2120), (1280, 8192)])
+def test_ordered_products_do_not_depend_on_the_number_of_tokens(features, depth):
+    """One token, a weight stream, a prompt's few tiles and many: the same bits of a token's sums, through the
+    entry that every layer uses."""
+    from helix_runtime_b200.ops import library as ops
+    from helix_runtime_b200.parts.linear import Weight, project
+    torch.manual_seed(features)
+    x = torch.randn(700, depth, device="cuda").bfloat16()
+    w = Weight(torch.randn(features, depth, device="cuda").bfloat16())
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    for epilogue, dtype in ((ops.EPI_STORE_F32, torch.float32), (ops.EPI_STORE, torch.bfloat16)):
+        for softcap in (0.0, 30.0) if epilogue == ops.EPI_STORE_F32 else (0.0,):
+            want = torch.zeros(700, features, dtype=dtype, device="cuda")
+            project(x, w, want, 700, epilogue, status, ordered=True, softcap=softcap)
+            for tokens in (1, 16, 17, 64, 100, 128, 129, 300):
+                out = torch.zeros(tokens, features, dtype=dtype, device="cuda")
+                project(x, w, out, tokens, epilogue, status, ordered=True, softcap=softcap)
+                assert torch.equal(out, want[:tokens])
+    assert int(status.item()) == 0
