@@ -63,6 +63,28 @@ __device__ __forceinline__ float level_off(float x, float cap) {
   return cap > 0.0f ? cap * tanhf(x / cap) : x;
 }
 
+// This thread's feature of 16 tokens from token0 on, as the epilogue stores it.
+template <int EPI>
+__device__ __forceinline__ void store_columns(void* out, int ldo, int tokens, int token0, int feature,
+                                              const float (&acc)[16], float softcap) {
+#pragma unroll
+  for (int j = 0; j < 16; ++j) {
+    const int token = token0 + j;
+    if (token < tokens) {
+      const size_t index = static_cast<size_t>(token) * ldo + feature;
+      if (EPI == EPI_STORE_BF16 || EPI == EPI_SWIGLU) {
+        static_cast<__nv_bfloat16*>(out)[index] = __float2bfloat16_rn(acc[j]);
+      } else if (EPI == EPI_STORE_F32) {
+        static_cast<float*>(out)[index] = level_off(acc[j], softcap);
+      } else {
+        // a reduction at the memory side: nothing to wait for.  With one writer per
+        // element the sum is still deterministic.
+        atomicAdd(static_cast<float*>(out) + index, acc[j]);
+      }
+    }
+  }
+}
+
 // One epilogue warp's share of a finished tile: its 32 features (tensor-memory lanes) for all
 // BN token columns, 16 columns at a time.  With SwiGLU the up accumulator sits BN columns on.
 template <int BN, int EPI>
@@ -87,24 +109,7 @@ __device__ __forceinline__ void write_tile(void* out, int ldo, int tokens, int f
       for (int j = 0; j < 16; ++j)
         acc[j] = hx_gated_fast(acc[j] + gate_b, up[j] + up_b, activation, gate_limit);
     }
-    if (feature_ok) {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const int token = token0 + column + j;
-        if (token < tokens) {
-          const size_t index = static_cast<size_t>(token) * ldo + feature;
-          if (EPI == EPI_STORE_BF16 || EPI == EPI_SWIGLU) {
-            static_cast<__nv_bfloat16*>(out)[index] = __float2bfloat16_rn(acc[j]);
-          } else if (EPI == EPI_STORE_F32) {
-            static_cast<float*>(out)[index] = level_off(acc[j], softcap);
-          } else {
-            // a reduction at the memory side: nothing to wait for.  With one writer per
-            // element the sum is still deterministic.
-            atomicAdd(static_cast<float*>(out) + index, acc[j]);
-          }
-        }
-      }
-    }
+    if (feature_ok) store_columns<EPI>(out, ldo, tokens, token0 + column, feature, acc, softcap);
   }
 }
 
@@ -156,6 +161,7 @@ struct GemmArgs {
   // Store epilogues: > 1 where the CTAs of a tile, one for each run of k-blocks, are a cluster that adds its
   // sums up (see gather_parts).
   int cluster = 1;
+  bool in_blocks = false;     // tiles of 16 tokens, float32 store: see sum_blocks
 };
 
 // A product that is stored cannot be cut along the reduction into atomic adds, and one with few tiles (a
@@ -205,6 +211,57 @@ __device__ __forceinline__ void gather_parts(const GemmArgs& a, const float* par
   }
 }
 
+// A grouped product of a few tiles of 16 tokens (experts of one to three tokens) with float32 sums leaves them in
+// tensor memory for one block of 64 k only: the tensor cores do not round to nearest, and a chain over a depth of
+// 2,816 is off by 3.0e-6 (relative 2-norm), where a product a pair on the CUDA cores (hx_expert_down), which such
+// experts would else take, is off by 8.6e-8.  Four blocks are a turn, two turns share tensor memory; the blocks are
+// added here in registers, with what each addition rounds away: 7.0e-8.  Measured (us, the chain / here): 4 tiles by
+// [4,096 x 2,816] 20.0 / 21.6, 2 by [4,096 x 4,096] 20.0 / 23.4; turns of one block 23.8 and 30.2.
+constexpr int TURN_BLOCKS = 4, TURN_COLUMNS = 16 * TURN_BLOCKS, TURNS = 2;
+
+__device__ __forceinline__ void sum_blocks(const GemmArgs& a, uint32_t lane_address, uint64_t* turn_full_bar,
+                                           uint64_t* turn_empty_bar, int blocks, int feature, int token0) {
+  const int lane = threadIdx.x & 31;
+  float sum[16], lost[16];
+#pragma unroll
+  for (int j = 0; j < 16; ++j) sum[j] = lost[j] = 0.0f;
+  for (int turn = 0; turn * TURN_BLOCKS < blocks; ++turn) {
+    const int buffer = turn % TURNS;
+    bool ok = true;
+    if (lane == 0) ok = mbar_wait(&turn_full_bar[buffer], static_cast<uint32_t>(turn / TURNS) & 1u);
+    ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
+    if (!ok) {
+      if (lane == 0) atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
+      return;
+    }
+    tc_fence_after();
+    uint32_t block[TURN_BLOCKS][16];
+#pragma unroll
+    for (int b = 0; b < TURN_BLOCKS; ++b)
+      tmem_load16_issue(lane_address + buffer * TURN_COLUMNS + 16 * b, block[b]);
+    tmem_load_wait();
+    tc_fence_before();
+    __syncwarp();
+    if (lane == 0) mbar_arrive(&turn_empty_bar[buffer]);
+#pragma unroll
+    for (int b = 0; b < TURN_BLOCKS; ++b) {
+      if (turn * TURN_BLOCKS + b >= blocks) break;
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float x = __uint_as_float(block[b][j]), before = sum[j];
+        sum[j] = before + x;
+        const float added = sum[j] - before;
+        lost[j] += (before - (sum[j] - added)) + (x - added);
+      }
+    }
+  }
+  if (feature >= a.features) return;
+#pragma unroll
+  for (int j = 0; j < 16; ++j)
+    if (isfinite(sum[j])) sum[j] += lost[j];      // (an infinite sum has lost what is no number)
+  store_columns<EPI_STORE_F32>(a.out, a.ldo, a.tokens, token0, feature, sum, a.softcap);
+}
+
 template <int BN, int EPI>
 __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
@@ -212,6 +269,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   constexpr bool DUAL = EPI == EPI_SWIGLU;
   using Config = TileConfig<BN, DUAL>;
   constexpr int STAGES = Config::kStages;
+  constexpr bool BLOCKS = BN == 16 && EPI == EPI_STORE_F32;      // see sum_blocks
   constexpr bool CLUSTERS = (EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32) && BN <= 128;
   static_assert(!CLUSTERS || BN * BM * 4 <= STAGES * Config::kStageBytes, "a part lies where the ring was");
 
@@ -222,7 +280,12 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   uint64_t* full_bar = reinterpret_cast<uint64_t*>(smem + STAGES * Config::kStageBytes);
   uint64_t* empty_bar = full_bar + STAGES;
   uint64_t* accum_bar = empty_bar + STAGES;
-  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(accum_bar + 1);
+  uint64_t* turn_full_bar = accum_bar + 1;      // [TURNS] a turn's sums are complete
+  uint64_t* turn_empty_bar = turn_full_bar + TURNS;      // [TURNS] they are read
+  uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(turn_empty_bar + TURNS);
+  static_assert((2 * STAGES + 1 + 2 * TURNS) * 8 + 4 <= 256, "the barriers' place");
+  const bool in_blocks = BLOCKS && args.in_blocks;
+  const int tmem_columns = in_blocks ? TURNS * TURN_COLUMNS : Config::kTmemColumns;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -249,10 +312,16 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(accum_bar, 1);
+    if (BLOCKS) {
+      for (int b = 0; b < TURNS; ++b) {
+        mbar_init(&turn_full_bar[b], 1);
+        mbar_init(&turn_empty_bar[b], 4);      // one arrival per epilogue warp
+      }
+    }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tmem_holder, Config::kTmemColumns);
+  if (warp == 1) tmem_alloc(tmem_holder, tmem_columns);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -305,12 +374,16 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
         for (int i = 0; i < n_k_blocks && ok; ++i) {
           const int s = i % STAGES;
           const uint32_t round = static_cast<uint32_t>(i / STAGES);
-          if (!mbar_wait(&full_bar[s], round & 1u)) {
+          const int turn = i / TURN_BLOCKS;
+          if (!mbar_wait(&full_bar[s], round & 1u) ||
+              (in_blocks && i % TURN_BLOCKS == 0 &&
+               !mbar_wait(&turn_empty_bar[turn % TURNS], (static_cast<uint32_t>(turn / TURNS) & 1u) ^ 1u))) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
             ok = false;
             break;
           }
           tc_fence_after();
+          const uint32_t sums = tmem_base + (in_blocks ? i % (TURNS * TURN_BLOCKS) * 16 : 0);
           const uint32_t stage = smem_u32(smem + s * Config::kStageBytes);
           const uint64_t desc_w = make_smem_desc(stage);
           const uint64_t desc_w2 = make_smem_desc(stage + BM * BK * 2);
@@ -319,11 +392,13 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // stepping 16 k-elements = 32 bytes inside the swizzle span: +2 in 16-byte units
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
-            const uint32_t accumulate = (i > 0 || k > 0) ? 1u : 0u;
-            umma_bf16(tmem_base, desc_w + step, desc_x + step, idesc, accumulate);
-            if (DUAL) umma_bf16(tmem_base + BN, desc_w2 + step, desc_x + step, idesc, accumulate);
+            const uint32_t accumulate = ((i > 0 && !in_blocks) || k > 0) ? 1u : 0u;
+            umma_bf16(sums, desc_w + step, desc_x + step, idesc, accumulate);
+            if (DUAL) umma_bf16(sums + BN, desc_w2 + step, desc_x + step, idesc, accumulate);
           }
           umma_commit(&empty_bar[s]);   // the stage may be refilled once these MMAs have read it
+          if (in_blocks && (i % TURN_BLOCKS == TURN_BLOCKS - 1 || i + 1 == n_k_blocks))
+            umma_commit(&turn_full_bar[turn % TURNS]);
         }
         umma_commit(accum_bar);         // the accumulator is complete
       }
@@ -332,14 +407,18 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       hx_pdl_wait();                    // the output may be something the last kernel read
       const int quarter = warp & 3;     // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
       const int feature = feature0 + quarter * 32 + lane;
+      const uint32_t lane_address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
+      if constexpr (BLOCKS) {
+        if (in_blocks)
+          sum_blocks(args, lane_address, turn_full_bar, turn_empty_bar, n_k_blocks, feature, token0);
+      }
       bool ok = true;
       if (lane == 0) ok = mbar_wait(accum_bar, 0);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) {
         if (lane == 0) atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
-      } else {
+      } else if (!in_blocks) {
         tc_fence_after();
-        const uint32_t lane_address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
         if (CLUSTERS && args.cluster > 1)
           leave_part<BN>(reinterpret_cast<float*>(smem), lane_address, quarter * 32 + lane,
                          min(BN, args.tokens - token0));
@@ -364,7 +443,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, Config::kTmemColumns);
+    tmem_dealloc(tmem_base, tmem_columns);
   }
 }
 
@@ -1630,6 +1709,7 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
   }
   GemmArgs args{out, ldo, tokens, features, depth, up_row_offset, total_k_blocks, 0, status,
                 activation, tile_group, group_rows, gate_limit};
+  args.in_blocks = token_tile == 16 && tokens < 16 * 16 && epilogue == EPI_STORE_F32;
   const dim3 grid((tokens + token_tile - 1) / token_tile, (features + BM - 1) / BM, 1);
   HX_REQUIRE(grid.y <= 65535, "hx_gemm_tc_grouped: too many features (%d)", features);
   switch (token_tile) {

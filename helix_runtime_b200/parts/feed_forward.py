@@ -282,20 +282,19 @@ class RoutedExperts(FeedForward):
             # router outputs behind the experts return the input; the experts' kernels leave
             # such choices out
             ops.expert_identity_add(x, chosen, weights, residual, n, self.top, self.experts)
-        if self.grouped(ctx, n):
+        if self.grouped(ctx):
             self.forward_grouped(ctx, x, chosen, weights, residual)
             return
         ops.expert_gate_up(x, self.w_gate_up, chosen, act, n, self.top, self.activation,
                            self.limit)
         ops.expert_down(act, self.w_down, chosen, weights, residual, n, self.top)
 
-    # Fewer pairs than this and an expert's matrices are read about once anyway: a product
-    # per pair streams them; from here on the pairs are sorted by expert.
-    GROUPED_FROM_PAIRS = 1
-
-    def grouped(self, ctx: StepContext, tokens: int) -> bool:
-        return (ctx.dtype == torch.bfloat16 and tokens * self.top >= self.GROUPED_FROM_PAIRS
-                and self.hidden_size % 8 == 0 and self.intermediate % 8 == 0)
+    def grouped(self, ctx: StepContext) -> bool:
+        """Whether the pairs go sorted by expert through the tensor cores, however few they are (one
+        token of 16 experts of 2,816 by 4,096: 90 us, 319 with a product a pair); float32 and
+        sizes that are no multiple of eight take the product a pair."""
+        return (ctx.dtype == torch.bfloat16 and self.hidden_size % 8 == 0
+                and self.intermediate % 8 == 0)
 
     def forward_grouped(self, ctx: StepContext, x: torch.Tensor, chosen: torch.Tensor,
                         weights: torch.Tensor, residual: torch.Tensor) -> None:

@@ -259,7 +259,9 @@ def test_experts_against_the_plain_sum(width, ff, experts, top, tokens, dtype):
 
 @pytest.mark.parametrize("width,ff,experts,top,tokens", [(40, 24, 5, 2, 37), (136, 64, 9, 1, 70),
                                                          (256, 136, 7, 3, 300), (64, 200, 3, 3, 11),
-                                                         (128, 128, 20, 2, 1500)])
+                                                         (128, 128, 20, 2, 1500),
+                                                         (256, 136, 7, 3, 1), (4096, 2816, 5, 4, 3),
+                                                         (136, 64, 40, 1, 2), (520, 328, 3, 2, 1)])
 def test_experts_sorted_for_grouped_products(width, ff, experts, top, tokens):
     """The same sum through the pairs sorted by expert and two grouped tensor-core products:
     experts with no token, with less than a tile and with several tiles; the sorted order
@@ -309,6 +311,36 @@ def test_experts_sorted_for_grouped_products(width, ff, experts, top, tokens):
     ops.expert_combine(rows_out, pair_row, weights, out, tokens, top, width)
     assert int(status.item()) == 0
     close(as_double(out) - rounded(start, torch.float32), want, 2e-2, 1e-2)
+
+
+@pytest.mark.parametrize("depth", [1408, 2816, 4096, 4104])
+def test_sums_of_a_few_pairs_keep_their_bits(depth):
+    """The float32 sums of experts of one to three tokens are no further from those of 64 bits than a product
+    a pair on the CUDA cores makes them (the layers' depths; a product that is not finite stays so)."""
+    from helix_runtime_b200.ops import library as ops
+    tokens, width = 3, 1000
+    status = torch.zeros((1,), dtype=torch.int32, device="cuda")
+    chosen = torch.arange(tokens, dtype=torch.int32, device="cuda")
+    errors = [0.0, 0.0]
+    for seed in range(4):
+        torch.manual_seed(seed)
+        act = torch.randn(tokens, depth, device="cuda").bfloat16()
+        down = (torch.randn(tokens, width, depth, device="cuda") * 0.02).bfloat16()
+        want = torch.einsum("td,twd->tw", act.double(), down.double())
+        pair, grouped = torch.zeros(tokens, width, device="cuda"), torch.zeros(16 * tokens, width, device="cuda")
+        ops.expert_down(act, down, chosen, torch.ones(tokens, 1, device="cuda"), pair, tokens, 1)
+        rows = torch.zeros(16 * tokens, depth, dtype=torch.bfloat16, device="cuda")
+        rows[::16] = act
+        ops.gemm_tc_grouped(rows, down, grouped, 16 * tokens, width, ops.EPI_STORE_F32, 0, 16, chosen, status)
+        for i, got in enumerate((pair, grouped[::16])):
+            errors[i] += float((got - want).norm() / want.norm())
+    assert errors[1] <= errors[0], errors
+    down[1, 7, 3], down[1, 8, 3], act[1, 3] = float("inf"), float("nan"), 1.0
+    rows[::16] = act
+    ops.gemm_tc_grouped(rows, down, grouped, 16 * tokens, width, ops.EPI_STORE_F32, 0, 16, chosen, status)
+    odd = ~grouped[::16].isfinite()
+    assert odd.sum() == 2 and grouped[16, 7] == float("inf") and grouped[16, 8].isnan()
+    assert int(status.item()) == 0
 
 
 # ------------------------------------------------- gated connection, rows joined for a pass
