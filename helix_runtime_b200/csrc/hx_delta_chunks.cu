@@ -79,6 +79,7 @@ struct DeltaArgs {
   int min_query_len;         // requests with fewer tokens are left alone;
   int portions;              // so many have as many
   int* status;               // may be null
+  uint32_t polls;            // of a wait for copies, before it gives up
 };
 
 // two neighbouring values in three bfloat16 terms, a word each
@@ -688,14 +689,20 @@ __global__ __launch_bounds__(STATES_THREADS, 1) void delta_states_kernel(const _
   const int chunks = (count + CHUNK - 1) / CHUNK;
   // Whether the chunk's rows are there; behind it nobody reads the other stage any more.
   auto arrived = [&](int chunk) {
-    const bool there = mbar_wait(&bars[chunk & 1], (chunk >> 1) & 1u);
+    const bool there = mbar_wait(&bars[chunk & 1], (chunk >> 1) & 1u, a.polls);
     return __syncthreads_or(!there) == 0;
   };
   if (threadIdx.x >= 2 * 32 * BLOCKS) {
     asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(COPY_REGISTERS));
     fetch(0, 0);
-    for (int chunk = 0; chunk < chunks && arrived(chunk); ++chunk)
+    for (int chunk = 0; chunk < chunks; ++chunk) {
+      if (!arrived(chunk)) {
+        // what was asked for lands in memory that the CTA is about to give back
+        mbar_wait(&bars[chunk & 1], (chunk >> 1) & 1u);
+        return;
+      }
       if (chunk + 1 < chunks) fetch(chunk + 1, (chunk + 1) & 1);
+    }
     return;
   }
   asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(WORK_REGISTERS));
@@ -968,15 +975,16 @@ HX_API long long hx_delta_chunks_scratch(int heads, int tokens) {
 // counted request by request.
 // Requests that bring fewer than min_query_len tokens are left alone (hx_linear_state_scan_below takes
 // them); portions: how many bring as many, tiles: the chunks of those.  status: the device status word, or
-// null; a wait that runs out leaves NaN in the outputs besides.
-HX_API int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+// null; a wait for a chunk's rows that runs out (after `polls` polls) leaves NaN in the outputs from there on
+// besides, and the portion's state as it was.
+HX_API int hx_delta_chunks_limited(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
                                 const void* decay_in, const void* beta_in, int ld_gates,
                                 const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
                                 int unit_norm, float unit_eps, float q_scale, float k_scale,
                                 void* scratch, float* state, long long state_stride, int head_stride,
                                 float* o, const int* request_start, const int* request_slot,
                                 int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
-                                int vdim, int min_query_len, int portions, int* status,
+                                int vdim, int min_query_len, int portions, int* status, unsigned polls,
                                 cudaStream_t stream) {
   HX_REQUIRE(hx_delta_chunks_supports(dim, vdim), "hx_delta_chunks: heads of %d by %d are not supported",
              dim, vdim);
@@ -1006,7 +1014,7 @@ HX_API int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int l
                     ld_gates, a_log, dt_bias, fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, weights,
                     factors, total, tokens, state, state_stride, head_stride, o, request_start, request_slot,
                     requests, heads, qk_heads, dim, vdim, parts_for(dim), min_query_len,
-                    portions, status};
+                    portions, status, polls};
   int rc;
   switch ((dim + 15) / 16) {
     case 1: case 2: rc = launch_delta<2>(a, tiles, stream); break;
@@ -1018,6 +1026,21 @@ HX_API int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int l
   hx_count_launches(1);
   HX_CHECK_LAUNCH("hx_delta_chunks");
   return HX_OK;
+}
+
+HX_API int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                                const void* decay_in, const void* beta_in, int ld_gates,
+                                const float* a_log, const float* dt_bias, const float* fixed_decay_m1,
+                                int unit_norm, float unit_eps, float q_scale, float k_scale,
+                                void* scratch, float* state, long long state_stride, int head_stride,
+                                float* o, const int* request_start, const int* request_slot,
+                                int requests, int tokens, int tiles, int heads, int qk_heads, int dim,
+                                int vdim, int min_query_len, int portions, int* status,
+                                cudaStream_t stream) {
+  return hx_delta_chunks_limited(q, ld_q, k, ld_k, v, ld_v, decay_in, beta_in, ld_gates, a_log, dt_bias,
+                                 fixed_decay_m1, unit_norm, unit_eps, q_scale, k_scale, scratch, state, state_stride,
+                                 head_stride, o, request_start, request_slot, requests, tokens, tiles, heads,
+                                 qk_heads, dim, vdim, min_query_len, portions, status, WAIT_LIMIT, stream);
 }
 
 HX_API int hx_delta_chunks_from(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,

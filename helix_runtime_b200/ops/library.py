@@ -369,7 +369,9 @@ def _declare(library: ctypes.CDLL) -> None:
     library.hx_delta_chunks.restype = library.hx_delta_chunks_from.restype = _c_int
     library.hx_delta_chunks_checked.argtypes = \
         library.hx_delta_chunks.argtypes[:-1] + [_c_int, _c_int, _c_ptr, _c_ptr]
-    library.hx_delta_chunks_checked.restype = _c_int
+    library.hx_delta_chunks_limited.argtypes = \
+        library.hx_delta_chunks.argtypes[:-1] + [_c_int, _c_int, _c_ptr, ctypes.c_uint, _c_ptr]
+    library.hx_delta_chunks_checked.restype = library.hx_delta_chunks_limited.restype = _c_int
     library.hx_linear_state_scan_below.argtypes = \
         library.hx_linear_state_scan.argtypes[:-1] + [_c_int, _c_int, _c_ptr]
     library.hx_linear_state_scan_below.restype = _c_int
@@ -1459,7 +1461,7 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
                  fixed_decay_m1: Optional[torch.Tensor] = None, unit_norm: bool = False,
                  unit_eps: float = 0.0, q_scale: float = 1.0, k_scale: float = 1.0,
                  min_query_len: int = 1, portions: Optional[int] = None,
-                 status: Optional[torch.Tensor] = None) -> None:
+                 status: Optional[torch.Tensor] = None, polls: Optional[int] = None) -> None:
     """The ``delta`` rule of :func:`linear_state_scan` without a rotation, 64 tokens at a time on
     the tensor cores (bfloat16 rows on 16 bytes); arguments as there.  ``scratch``:
     :func:`delta_chunks_scratch` bytes; ``tiles``: :func:`recurrence_tiles` of the step.
@@ -1479,14 +1481,18 @@ def delta_chunks(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, state: torch
         if tensor is not None:
             _need(tensor, torch.float32, name)
     assert scratch.numel() * scratch.element_size() >= delta_chunks_scratch(heads, tokens)
-    _check(lib().hx_delta_chunks_checked(
+    arguments = (
         q.data_ptr(), q.stride(0), k.data_ptr(), k.stride(0), v.data_ptr(), v.stride(0),
         _ptr(decay_in), beta_in.data_ptr(), beta_in.stride(0), _ptr(a_log), _ptr(dt_bias),
         _ptr(fixed_decay_m1), 1 if unit_norm else 0, float(unit_eps), float(q_scale),
         float(k_scale), scratch.data_ptr(), state.data_ptr(), state.stride(0), head_stride,
         o.data_ptr(), request_start.data_ptr(), request_slot.data_ptr(), requests, tokens, tiles,
         heads, qk_heads, dim, vdim, min_query_len, requests if portions is None else portions,
-        _ptr(status), _stream()))
+        _ptr(status))
+    if polls is None:
+        _check(lib().hx_delta_chunks_checked(*arguments, _stream()))
+    else:
+        _check(lib().hx_delta_chunks_limited(*arguments, int(polls), _stream()))
 
 
 # ------------------------------------------------------------- gated residual connection

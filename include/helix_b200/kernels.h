@@ -446,6 +446,16 @@ int hx_delta_chunks_checked(const void* q, int ld_q, const void* k, int ld_k, co
                             const int* request_slot, int requests, int tokens, int tiles, int heads,
                             int qk_heads, int dim, int vdim, int min_query_len,
                             int portions, int* status, cudaStream_t stream);
+/* and with the number of polls after which a wait for rows gives up */
+int hx_delta_chunks_limited(const void* q, int ld_q, const void* k, int ld_k, const void* v, int ld_v,
+                            const void* decay_in, const void* beta_in, int ld_gates, const float* a_log,
+                            const float* dt_bias, const float* fixed_decay_m1, int unit_norm,
+                            float unit_eps, float q_scale, float k_scale, void* scratch, float* state,
+                            long long state_stride, int head_stride, float* o, const int* request_start,
+                            const int* request_slot, int requests, int tokens, int tiles, int heads,
+                            int qk_heads, int dim, int vdim, int min_query_len,
+                            int portions, int* status, unsigned polls,
+                            cudaStream_t stream);
 
 /* ---- attention over a cached latent ----------------------------------------------------- */
 /* down [tokens][q_rank + kv_rank + rot] float32: both latents RMS-normed with a weight; the

@@ -330,3 +330,42 @@ def test_refusals():
     assert ops.delta_chunks_supports(128, 8) and ops.delta_chunks_supports(8, 512)
     assert not ops.delta_chunks_supports(136, 8) and not ops.delta_chunks_supports(20, 8)
     assert not ops.delta_chunks_supports(16, 12)
+
+
+@pytest.mark.parametrize("heads,qk_heads,dim,vdim", [(4, 2, 128, 128), (3, 1, 48, 136), (2, 2, 8, 8)])
+def test_a_wait_that_runs_out_is_reported(heads, qk_heads, dim, vdim):
+    """No polls for the rows of a portion: its status bit, NaN in every output of the portions that take chunks
+    and nowhere else, the state as it was; and the next call goes on as ever."""
+    from helix_runtime_b200.ops import library as ops
+    torch.manual_seed(vdim)
+    lengths, shortest = (70, 3, 128, 1, 65), 16
+    tokens, per_head = sum(lengths), ops.scan_state_floats(vdim, dim)
+    q, k = torch.randn(2, tokens, qk_heads * dim, device="cuda").bfloat16()
+    v = torch.randn(tokens, heads * vdim, device="cuda").bfloat16()
+    beta = torch.randn(tokens, heads, device="cuda").bfloat16()
+    starts = torch.tensor(np.concatenate([[0], np.cumsum(lengths)]), dtype=torch.int32).cuda()
+    slots = torch.arange(len(lengths), dtype=torch.int32, device="cuda")
+    state = torch.randn(len(lengths), heads * per_head, device="cuda")
+    before = state.clone()
+    o = torch.full((tokens, heads * vdim), 7.0, device="cuda")
+    scratch = torch.empty(ops.delta_chunks_scratch(heads, tokens) // 4 + 1, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    taken = [n for n in lengths if n >= shortest]
+
+    def call(**options):
+        ops.delta_chunks(q, k, v, state, o, scratch, starts, slots, len(lengths), tokens,
+                         ops.recurrence_tiles(taken), heads, qk_heads, dim, vdim, beta_in=beta,
+                         fixed_decay_m1=torch.full((heads,), -0.01, device="cuda"), unit_norm=True,
+                         min_query_len=shortest, portions=len(taken), status=status, **options)
+
+    call(polls=0)
+    assert int(status.item()) == ops.FLAG_WAIT_TIMEOUT
+    assert torch.equal(state, before)
+    for r, n in enumerate(lengths):
+        rows = o[starts[r]:starts[r + 1]]
+        assert rows.isnan().all() if n >= shortest else (rows == 7.0).all()
+    status.zero_()
+    call()
+    assert int(status.item()) == 0 and o.isfinite().all() and state.isfinite().all()
+    changed = [not torch.equal(state[r], before[r]) for r in range(len(lengths))]
+    assert changed == [n >= shortest for n in lengths]
