@@ -157,14 +157,18 @@ __device__ __forceinline__ uint64_t float_pair(float low, float high) {
 __device__ __forceinline__ void float_pair_halves(uint64_t pair, float& low, float& high) {
   asm("mov.b64 {%0, %1}, %2;" : "=f"(low), "=f"(high) : "l"(pair));
 }
+__device__ __forceinline__ uint64_t float_pair_add(uint64_t x, uint64_t y) {
+  uint64_t r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(x), "l"(y));
+  return r;
+}
 __device__ __forceinline__ uint64_t float_pair_fma(uint64_t x, uint64_t y, uint64_t z) {
   uint64_t r;
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(x), "l"(y), "l"(z));
   return r;
 }
 
-// BIASED: inputs have a bias, which the state holds and the rows do not; the first tokens of a portion then
-// go a road of their own.
+// BIASED: inputs have a bias, which the state holds and the rows do not: it is added as a row is unpacked.
 template <int TAPS, bool SUMS, bool BIASED>
 __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const FilterArgs<__nv_bfloat16> a,
                                                                    int tokens, int run) {
@@ -216,8 +220,7 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
   };
   // rows[j]: the inputs of batch row token - REACH + j, used only by tokens that lie at least
   // REACH tokens into their portion (rows of another request are never used: not fetched).
-  // A row of raw inputs is kept packed; sums (few tokens) are rounded into the same form.  The
-  // input bias of a row inside the portion is part of the sum's start value.
+  // A row of raw inputs is kept packed; sums (few tokens) are rounded into the same form.
   auto packed_input = [&](int token) {
     if constexpr (!SUMS) {
       return *reinterpret_cast<const uint4*>(a.raw + static_cast<size_t>(token) * a.ld_raw + c);
@@ -235,26 +238,21 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
     }
   };
   // two channels an instruction, each rounded as its scalar form
-  uint64_t w2[TAPS][4], inside[4];
+  uint64_t w2[TAPS][4], b2[4], in_bias2[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    float sums[2];
-#pragma unroll
-    for (int k = 0; k < 2; ++k) {
-      float sum = 0.0f;
-#pragma unroll
-      for (int j = 0; j < TAPS; ++j) sum += w[j][2 * i + k];
-      sums[k] = fmaf(sum, in_bias[2 * i + k], b[2 * i + k]);
-    }
-    inside[i] = float_pair(sums[0], sums[1]);
+    b2[i] = float_pair(b[2 * i], b[2 * i + 1]);
+    in_bias2[i] = float_pair(in_bias[2 * i], in_bias[2 * i + 1]);
 #pragma unroll
     for (int j = 0; j < TAPS; ++j) w2[j][i] = float_pair(w[j][2 * i], w[j][2 * i + 1]);
   }
-  auto unpack = [](const uint4& packed, uint64_t (&x)[4]) {
+  auto unpack = [&](const uint4& packed, uint64_t (&x)[4]) {
     const uint32_t words[4] = {packed.x, packed.y, packed.z, packed.w};
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i) {
       x[i] = float_pair(__uint_as_float(words[i] << 16), __uint_as_float(words[i] & 0xffff0000u));
+      if (BIASED) x[i] = float_pair_add(x[i], in_bias2[i]);
+    }
   };
   int token = first;
   while (token < last) {
@@ -265,12 +263,12 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
       slot = a.request_slot[request];
     }
     const int index = token - start;
-    if (index >= REACH || (!BIASED && index == 0 && end - start > 1)) {
+    if (index >= REACH || (index == 0 && end - start > 1)) {
       // RING tokens at a time: a row is unpacked once, and the rows of the RING tokens behind are on their way
       // meanwhile.  The thread of a portion's first token begins with the state's rows, takes all the tokens
       // that these reach, and writes the new state.
       constexpr int RING = 4;
-      const bool from_state = !BIASED && REACH > 0 && index == 0;
+      const bool from_state = REACH > 0 && index == 0;
       const int stop = min(end, from_state ? max(last, start + REACH) : last);
       uint4 ahead[RING];
       uint64_t rows[REACH + RING][4];
@@ -335,7 +333,7 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
             float y[8];
 #pragma unroll
             for (int i = 0; i < 4; ++i) {
-              uint64_t sum = inside[i];
+              uint64_t sum = b2[i];
 #pragma unroll
               for (int j = 0; j < TAPS; ++j) sum = float_pair_fma(w2[j][i], rows[k + j][i], sum);
               float_pair_halves(sum, y[2 * i], y[2 * i + 1]);
@@ -351,71 +349,41 @@ __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const Filt
       token = stop;
       continue;
     }
-    if (index == 0 && (BIASED || end - start == 1)) {
-      // A portion of one token, or (BIASED) the first tokens of any portion: their filter reaches behind the
-      // portion.  Then the new state (see the scalar kernel).
-      const int count = end - start;
+    if (index == 0) {
+      // a decoded token, a portion by itself: its filter reads the state and itself, and the state moves up by one
       float* state = a.state + static_cast<size_t>(slot) * a.state_stride + c;
-      // the input at a place of the portion, or in front of it the state's
-      auto input_at = [&](int place, float (&x)[8]) {
-        if (place >= 0) {
-          filter_input8(a, start + place, c, in_bias, x);
-        } else if (wide_state) {
-          const float4* source = reinterpret_cast<const float4*>(
-              state + static_cast<size_t>(place + REACH) * a.channels);
-          const float4 lo = source[0], hi = source[1];
-          x[0] = lo.x; x[1] = lo.y; x[2] = lo.z; x[3] = lo.w;
-          x[4] = hi.x; x[5] = hi.y; x[6] = hi.z; x[7] = hi.w;
+      float x[TAPS][8], y[8];
+#pragma unroll
+      for (int j = 0; j < REACH; ++j) {
+        const float* source = state + static_cast<size_t>(j) * a.channels;
+        if (wide_state) {
+          const float4 lo = reinterpret_cast<const float4*>(source)[0], hi = reinterpret_cast<const float4*>(source)[1];
+          x[j][0] = lo.x; x[j][1] = lo.y; x[j][2] = lo.z; x[j][3] = lo.w;
+          x[j][4] = hi.x; x[j][5] = hi.y; x[j][6] = hi.z; x[j][7] = hi.w;
         } else {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) x[i] = state[static_cast<size_t>(place + REACH) * a.channels + i];
+          for (int i = 0; i < 8; ++i) x[j][i] = source[i];
         }
-      };
-      if (!BIASED || count == 1) {
-        // a decoded token: its filter reads the state and itself, and the state moves up by one
-        float x[TAPS][8], y[8];
+      }
+      filter_input8(a, start, c, in_bias, x[REACH]);
 #pragma unroll
-        for (int j = 0; j < TAPS; ++j) input_at(j - REACH, x[j]);
+      for (int i = 0; i < 8; ++i) {
+        y[i] = b[i];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          y[i] = b[i];
+        for (int j = 0; j < TAPS; ++j) y[i] = fmaf(w[j][i], x[j][i], y[i]);
+      }
+      emit(token, y);
 #pragma unroll
-          for (int j = 0; j < TAPS; ++j) y[i] = fmaf(w[j][i], x[j][i], y[i]);
-        }
-        emit(token, y);
+      for (int r = 0; r < REACH; ++r) {
+        float* target = state + static_cast<size_t>(r) * a.channels;
+        if (wide_state) {
+          reinterpret_cast<float4*>(target)[0] =
+              make_float4(x[r + 1][0], x[r + 1][1], x[r + 1][2], x[r + 1][3]);
+          reinterpret_cast<float4*>(target)[1] =
+              make_float4(x[r + 1][4], x[r + 1][5], x[r + 1][6], x[r + 1][7]);
+        } else {
 #pragma unroll
-        for (int r = 0; r < REACH; ++r) {
-          float* target = state + static_cast<size_t>(r) * a.channels;
-          if (wide_state) {
-            reinterpret_cast<float4*>(target)[0] =
-                make_float4(x[r + 1][0], x[r + 1][1], x[r + 1][2], x[r + 1][3]);
-            reinterpret_cast<float4*>(target)[1] =
-                make_float4(x[r + 1][4], x[r + 1][5], x[r + 1][6], x[r + 1][7]);
-          } else {
-#pragma unroll
-            for (int i = 0; i < 8; ++i) target[i] = x[r + 1][i];
-          }
-        }
-      } else {
-        const int behind = count < REACH ? count : REACH;
-        for (int t = 0; t < behind; ++t) {
-          float y[8];
-#pragma unroll
-          for (int i = 0; i < 8; ++i) y[i] = b[i];
-#pragma unroll
-          for (int j = 0; j < TAPS; ++j) {
-            float x[8];
-            input_at(t - REACH + j, x);
-#pragma unroll
-            for (int i = 0; i < 8; ++i) y[i] = fmaf(w[j][i], x[i], y[i]);
-          }
-          emit(start + t, y);
-        }
-        for (int r = 0; r < REACH; ++r) {
-          float x[8];
-          input_at(count - REACH + r, x);
-#pragma unroll
-          for (int i = 0; i < 8; ++i) state[static_cast<size_t>(r) * a.channels + i] = x[i];
+          for (int i = 0; i < 8; ++i) target[i] = x[r + 1][i];
         }
       }
     }
