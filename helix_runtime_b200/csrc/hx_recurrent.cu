@@ -168,7 +168,9 @@ __device__ __forceinline__ uint64_t float_pair_fma(uint64_t x, uint64_t y, uint6
   return r;
 }
 
-// BIASED: inputs have a bias, which the state holds and the rows do not: it is added as a row is unpacked.
+// BIASED: inputs have a bias, which the state holds and the rows do not: it is added as a row is unpacked.  (As part
+// of the sum's start value, with a road of its own for the tokens whose filter reaches behind the portion, four taps,
+// 300 tokens of 4,096 channels took 7.9 us and two portions of 1,657 tokens of 512 channels 7.9: 5.3 and 6.5.)
 template <int TAPS, bool SUMS, bool BIASED>
 __global__ __launch_bounds__(256, 2) void causal_filter_pieces_kernel(const FilterArgs<__nv_bfloat16> a,
                                                                    int tokens, int run) {
