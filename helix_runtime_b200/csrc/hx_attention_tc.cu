@@ -831,7 +831,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
         // values were (every product is done), 16 bytes apart more than they are long, so that a warp's rows
         // use different banks (a thread's own row, 16 bytes at a time, is half a sector a store).  With two CTAs
         // an SM they leave with whole rows side by side, with one by a bulk copy each (the other way round: heads
-        // of 128 67 -> 70 us, heads of 256 96 -> 101).
+        // of 128 67 -> 70 us, heads of 256 over pages of 16 96 -> 101; pages of 32, 32 heads of 224 over one cached row,
+        // 2,048 tokens 127 -> 137, eight decoded tokens behind 500 19.5 -> 21.9).
         constexpr int SHARE = D / GROUPS, ROW_BYTES = SHARE * 2 + 16;
         static_assert(4 * GROUPS * 32 * ROW_BYTES <= Config::kQBytes + (K_STAGES + V_STAGES) * Config::kHalfBytes,
                       "the rows' place");
@@ -858,7 +859,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
               *reinterpret_cast<uint4*>(gathered + (d0 + h * 16 + d) * 2) = packed;
             }
         }
-        if constexpr (GROUPS > 1) {
+        if constexpr (Config::kCtas == 1) {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           if (row < rows_here && share > 0) {
             __nv_bfloat16* out = a.out + static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
