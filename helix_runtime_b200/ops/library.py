@@ -1982,15 +1982,14 @@ def latent_queries(q: torch.Tensor, rot_offset: int, rows: torch.Tensor, positio
                                    _stream()))
 
 
-# 32 heads, 192 by 128 and 128 by 192, both products: 2,048 tokens 234 us on the CUDA cores, 28 on the
-# tensor cores; one token 37 and 10.
-
-
 def head_products(x: torch.Tensor, x_stride: int, w: torch.Tensor, out: torch.Tensor,
                   out_stride: int, tokens: int, status: Optional[torch.Tensor] = None) -> None:
     """out[t, h * out_stride + o] = sum_i w[h, o, i] * x[t, h * x_stride + i]: one small product
     per head, ``w`` ``[heads, out_dim, in_dim]``, everything in the compute dtype.  With a
     ``status`` word bfloat16 products run on the tensor cores where sizes and strides allow."""
+    # Measured, 32 heads, 192 by 128 and 128 by 192, both products: 2,048 tokens 234 us on the CUDA cores,
+    # 28 on the tensor cores; one token 37 and 10.  The results, stored in bfloat16, are as far from 64 bits
+    # either way (1.660e-3 and 1.652e-3 at one token, 1.6557e-3 and 1.6582e-3 at 16).
     heads, out_dim, in_dim = w.shape
     assert x.dtype == w.dtype == out.dtype and w.is_contiguous()
     assert x.stride(-1) == 1 and out.stride(-1) == 1

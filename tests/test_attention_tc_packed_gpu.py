@@ -107,6 +107,8 @@ def test_wide_heads_against_the_formula(head_dim, heads, kv_heads, page, lengths
     (33, 3, 64, 40, 72, 40), (129, 2, 192, 128, 256, 128), (300, 5, 128, 300, 128, 304),
     (1100, 40, 64, 256, 64, 256),      # more tiles than SMs
     (257, 1, 64, 500, 72, 512),        # one head: pairs of CTAs, tiles in pieces
+    (1, 32, 128, 192, 128, 256), (1, 1, 64, 8, 64, 8), (5, 3, 192, 128, 256, 128), (16, 40, 64, 40, 72, 48),
+    (17, 2, 128, 300, 136, 304), (32, 32, 192, 128, 256, 128),
 ])
 def test_products_per_head_on_the_tensor_cores(tokens, heads, in_dim, out_dim, x_stride, out_stride):
     from helix_runtime_b200.ops import library as ops
