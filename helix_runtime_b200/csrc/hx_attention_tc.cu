@@ -123,10 +123,11 @@ struct TcConfig {
   static constexpr int kSoftmaxGroups = D > 128 && GATHER ? 2 : 1;
   static constexpr int kScoreBuffers = 2 * kSoftmaxGroups;      // score tiles in tensor memory
   static constexpr int kThreads = kRewriters <= 1 && kSoftmaxGroups == 1 ? 256 : 384;
+  static constexpr int kBarrierBytes = 256;
   static constexpr int kQBytes = BLOCK_M * D * 2;
   static constexpr int kHalfBytes = BLOCK_N * D * 2;          // keys (or values) of a tile
   static constexpr int kSmemBytes = kQBytes + (kKeyStages + kValueStages + kKeyBuffers) * kHalfBytes +
-                                    128 /*alignment*/ + 256 /*barriers*/ +
+                                    128 /*alignment*/ + kBarrierBytes +
                                     (kSoftmaxGroups > 1 ? 2 * kSoftmaxGroups * BLOCK_M * 4 : 0);
   static constexpr int kScoreColumns = BLOCK_N;               // per score buffer
   static constexpr int kLowTermColumn = BLOCK_N / 2;          // P: hi in columns [0, 32), lo after
@@ -230,7 +231,7 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
   uint64_t* k_empty = k_full + K_STAGES;
   uint64_t* v_full = k_empty + K_STAGES;
   uint64_t* v_empty = v_full + V_STAGES;       // the product has read it
-  uint64_t* s_full = v_empty + V_STAGES;       // [S_BUFFERS] scores of tile t in buffer t % 2
+  uint64_t* s_full = v_empty + V_STAGES;       // [S_BUFFERS] scores of tile t in buffer t % S_BUFFERS
   uint64_t* p_full = s_full + S_BUFFERS;       // [S_BUFFERS] its probabilities are in place
   uint64_t* o_full = p_full + S_BUFFERS;       // [S_BUFFERS] its output product is done
   uint64_t* k_ready = o_full + S_BUFFERS;      // [KEY_BUFFERS] the tile's keys are rewritten
@@ -239,8 +240,11 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
   uint64_t* told_bar = q_ready + 1;            // [GROUPS][4] a group's warp has told its reference
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(told_bar + (GROUPS > 1 ? 4 * GROUPS : 0));
   volatile int* failed = reinterpret_cast<volatile int*>(tmem_holder + 1);
+  constexpr int kBarriers = 2 * K_STAGES + 2 * V_STAGES + 3 * S_BUFFERS + 2 * KEY_BUFFERS + 1 +
+                            (GROUPS > 1 ? 4 * GROUPS : 0);
+  static_assert(kBarriers * 8 + 8 <= Config::kBarrierBytes, "the place of barriers, tensor memory's address and flag");
   // two groups of softmax warps: [GROUPS][BLOCK_M] references they tell each other, then their sums
-  float* told = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(k_full) + 256);
+  float* told = reinterpret_cast<float*>(reinterpret_cast<uint8_t*>(k_full) + Config::kBarrierBytes);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -531,8 +535,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
         atomicOr(a.status, HX_FLAG_WAIT_TIMEOUT);
         *failed = 1;
       }
-      // S[tile % 2] = Q K_tile^T: one product of 64 keys per 16 coordinates.  The buffer held the
-      // probabilities of tile - 2, which the output product must have read.
+      // S[tile % S_BUFFERS] = Q K_tile^T: one product of 64 keys per 16 coordinates.  The buffer held the
+      // probabilities of tile - S_BUFFERS, which the output product must have read.
       for (int tile = 0; tile < n_tiles && !*failed; ++tile) {
         const int b = tile % S_BUFFERS;
         if (!mbar_wait(&k_ready[tile % KEY_BUFFERS], static_cast<uint32_t>(tile / KEY_BUFFERS) & 1u) ||
@@ -706,8 +710,8 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
       if (raised) {
         // ---- a new reference: what O holds was taken against the old one.  The
         // product of the previous tile must have landed; the product of this tile waits for
-        // this warp's arrival below.  (o_full[b] completes a phase for every other tile; its
-        // previous phase was complete before the scores of the previous tile were.)
+        // this warp's arrival below.  (o_full[b] completes a phase for every S_BUFFERS-th tile;
+        // its previous phase was complete before the scores of the previous tile were.)
         const float correction = old_max == -INFINITY ? 0.0f : fast_exp2(old_max - row_max);
         if (GROUPS == 1) row_sum *= correction;
         ok = wait_for(&o_full[(tile - 1) % S_BUFFERS],

@@ -14,14 +14,17 @@
 // A sum that is not finite (an operand is not, or 2^16 times it leaves float32, or 2^32 times a block's
 // sum does: operands from 2^112 and sums from 2^96 on) is taken again as that chain, which says what it is.
 //
-// What bounds it: the conversion.  A block of 64 k of a tile of 128 x 128 takes about 4,000 cycles; with one
+// Two kernels: one CTA a tile, for shallow products and callers without scratch, and below, with scratch, pairs of
+// CTAs (hx_gemm_split_scratch_pays says where the line lies).
+//
+// What bounds the first: the conversion.  A block of 64 k of a tile of 128 x 128 takes about 4,000 cycles; with one
 // of the six products it takes as long, without the loads 3,300 (ncu: issue slots 54 % busy, tensor pipe 38 %):
 // eight warps that load, cut and store 16 pieces of four numbers each a block, two warps a scheduler.
 // Slower: sixteen such warps (too few registers for loads in flight: 463 -> 502 us), all warps converting
 // and summing in turn (539), the weights' lines asked for ahead (4 % faster alone, 3 % slower in place).
-// Measured (us, tiles of multiply-adds before): 512 tokens by [17,280 x 3,200] 1,581 -> 434, by [3,200 x 8,640] 947 ->
-// 287, by [4,096 x 4,096] 522 -> 157; 33 by the first 248 -> 117.  (With the next block's tokens asked for in front
-// of the proxy fence, which waits for loads too: 459 and 311.)
+// Measured (us, tiles of multiply-adds / one CTA a tile; deep products, which pairs take now): 512 tokens by
+// [17,280 x 3,200] 1,581 / 434, by [3,200 x 8,640] 947 / 287, by [4,096 x 4,096] 522 / 157; 33 by the first 248 / 117.
+// (With the next block's tokens asked for in front of the proxy fence, which waits for loads too: 459 and 311.)
 //
 // Every wait on an mbarrier is bounded; a wait that runs out sets a status bit, the CTA skips its
 // remaining work, frees its tensor memory and returns.
@@ -328,12 +331,9 @@ constexpr int PAIR_ROWS = TILE / 2;                     // weight rows of a CTA
 constexpr int PAIR_X_BYTES = TILE * BK * 2, PAIR_W_BYTES = PAIR_ROWS * BK * 2;      // a term
 constexpr int PAIR_STAGE_BYTES = 3 * (PAIR_X_BYTES + PAIR_W_BYTES);
 constexpr int PAIR_STAGES = 3;
-#ifndef GROUPS
-#define GROUPS 2
-#endif
 constexpr int PAIR_BUFFERS = 4;                         // of a block's sums
 constexpr int PAIR_TMEM_COLUMNS = PAIR_BUFFERS * TILE;
-constexpr int PAIR_GROUPS = GROUPS, PAIR_GROUP_WARPS = 8 / PAIR_GROUPS;
+constexpr int PAIR_GROUPS = 2, PAIR_GROUP_WARPS = 8 / PAIR_GROUPS;
 constexpr int PAIR_TMA_WARP = SUM_WARPS + PAIR_GROUPS * PAIR_GROUP_WARPS, PAIR_MMA_WARP = PAIR_TMA_WARP + 1;
 constexpr int PAIR_THREADS = 32 * (PAIR_TMA_WARP + 4);      // whole warpgroups, whose registers are dealt anew
 // At launch 96 a thread; those that issue copies and products need few, the others take what they leave.
@@ -512,7 +512,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) void gem
             }
             if (rank == 0) mbar_expect_tx(&full_bar[s], 2 * 3 * PAIR_X_BYTES);
             const uint32_t bar = cluster_address(&full_bar[s], 0);
-  #pragma unroll
+#pragma unroll
             for (int term = 0; term < 3; ++term)
               tma_load_2d_pair(smem + s * PAIR_STAGE_BYTES + term * PAIR_X_BYTES, &map_terms, bar, kb * BK,
                                term * a.tokens + token0);
@@ -535,11 +535,11 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(PAIR_THREADS, 1) void gem
         tc_fence_after();
         const uint32_t stage = smem_u32(smem + s * PAIR_STAGE_BYTES);
         const uint32_t sums = tmem_base + buffer * TILE;
-  #pragma unroll
+#pragma unroll
         for (int i = 0; i < 6; ++i) {
           const uint64_t desc_x = make_smem_desc(stage + TERM_OF_X[i] * PAIR_X_BYTES);
           const uint64_t desc_w = make_smem_desc(stage + 3 * PAIR_X_BYTES + TERM_OF_W[i] * PAIR_W_BYTES);
-  #pragma unroll
+#pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
             umma_bf16_pair(sums, desc_x + step, desc_w + step, idesc, i > 0 || k > 0 ? 1u : 0u);

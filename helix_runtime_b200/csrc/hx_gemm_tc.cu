@@ -722,7 +722,6 @@ __device__ __forceinline__ void write_row(int columns, void* out, int ldo, int f
         reinterpret_cast<uint4*>(row)[0] = packed[0];
         reinterpret_cast<uint4*>(row)[1] = packed[1];
       } else {
-        // the add epilogue too: the accumulator began as the output's old value
 #pragma unroll
         for (int j = 0; j < 4; ++j)
           reinterpret_cast<float4*>(row)[j] =
@@ -964,8 +963,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
         const int buffer = iteration & 1;
         const uint32_t use = static_cast<uint32_t>(iteration >> 1);
-        // the epilogue must have read this accumulator's previous unit (and, for the add
-        // epilogue, have loaded this unit's old output into it: one more arrival)
+        // the epilogue must have read this accumulator's previous unit
         if (!mbar_wait(&tmem_empty_bar[buffer], (use & 1u) ^ 1u)) {
           atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
@@ -989,9 +987,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
-            // a whole tile of the add epilogue starts from the old output in the accumulator
-            const uint32_t accumulate =
-                (kb > unit.kb_begin || k > 0) ? 1u : 0u;
+            const uint32_t accumulate = (kb > unit.kb_begin || k > 0) ? 1u : 0u;
             umma_bf16(accumulator, desc_a + step, desc_b + step, idesc, accumulate);
           }
           umma_commit(&empty_bar[s]);
@@ -1005,7 +1001,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
     const int quarter = warp & 3;     // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
     const uint32_t lane_base = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
     Unit unit;
-    // add epilogue
+    // the add epilogue's: whether output rows take 16-byte accesses, and where sums change places
     const bool wide = args.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0;
     float* exchange = reinterpret_cast<float*>(smem + STAGES * Config::kStageBytes + 256);
     for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
@@ -1029,15 +1025,16 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_persistent_kernel(
       if constexpr (EPI == EPI_ROPE_APPEND) {
         write_row_rope(FEATURES, args, lane_base + buffer * Config::kBufferColumns,
                        unit.token_tile * BM + quarter * 32 + lane, unit.feature_tile * FEATURES);
-      } else if (EPI == EPI_ADD_F32 && !unit.partial) {
-        add_tile(static_cast<float*>(args.out), args.ldo, args.features, lane_base + buffer * Config::kBufferColumns,
-                 unit.token_tile * BM + quarter * 32, args.tokens, unit.feature_tile * FEATURES, wide,
-                 exchange + quarter * 32 * ADD_STRIDE, old);
-      } else if (EPI == EPI_ADD_F32) {
-        add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features,
-                           lane_base + buffer * Config::kBufferColumns,
-                           unit.token_tile * BM + quarter * 32 + lane, args.tokens,
-                           unit.feature_tile * FEATURES);
+      } else if constexpr (EPI == EPI_ADD_F32) {
+        if (!unit.partial)
+          add_tile(static_cast<float*>(args.out), args.ldo, args.features,
+                   lane_base + buffer * Config::kBufferColumns, unit.token_tile * BM + quarter * 32, args.tokens,
+                   unit.feature_tile * FEATURES, wide, exchange + quarter * 32 * ADD_STRIDE, old);
+        else
+          add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features,
+                             lane_base + buffer * Config::kBufferColumns,
+                             unit.token_tile * BM + quarter * 32 + lane, args.tokens,
+                             unit.feature_tile * FEATURES);
       } else if (EPI == EPI_STORE_BF16 && args.heads > 1) {
         const int head = unit.feature_tile / args.head_tiles;
         write_row<EPI>(FEATURES, static_cast<__nv_bfloat16*>(args.out) + static_cast<size_t>(head) * args.head_out,
@@ -1182,8 +1179,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
         const int buffer = iteration & 1;
         const uint32_t use = static_cast<uint32_t>(iteration >> 1);
-        if (!mbar_wait_cluster(&tmem_empty_bar[buffer],
-                               (use & 1u) ^ 1u)) {
+        if (!mbar_wait_cluster(&tmem_empty_bar[buffer], (use & 1u) ^ 1u)) {
           atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
           *failed = 1;
           break;
@@ -1205,8 +1201,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
 #pragma unroll
           for (int k = 0; k < BK / UMMA_K; ++k) {
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
-            const uint32_t accumulate =
-                (kb > unit.kb_begin || k > 0) ? 1u : 0u;
+            const uint32_t accumulate = (kb > unit.kb_begin || k > 0) ? 1u : 0u;
             umma_bf16_pair(accumulator, desc_a + step, desc_b + step, idesc, accumulate);
           }
           umma_commit_pair(&empty_bar[s]);
@@ -1226,7 +1221,7 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       __syncwarp();
       if (lane == 0) mbar_arrive_cluster(cluster_address(&tmem_empty_bar[buffer], 0));
     };
-    // add epilogue
+    // the add epilogue's: whether output rows take 16-byte accesses, and where sums change places
     const bool wide = args.ldo % 4 == 0 && (reinterpret_cast<uintptr_t>(args.out) & 15) == 0;
     float* exchange = reinterpret_cast<float*>(smem + STAGES * Config::kStageBytes + 256);
     for (int iteration = 0; unit_at(args, iteration, unit, worker, workers) && !*failed; ++iteration) {
@@ -1253,12 +1248,13 @@ __global__ __cluster_dims__(2, 1, 1) __launch_bounds__(THREADS) void gemm_tc_pai
       const int feature0 = unit.feature_tile * FEATURES + unit.piece * columns;
       if constexpr (EPI == EPI_ROPE_APPEND) {
         write_row_rope(columns, args, accumulator, token, feature0);
-      } else if (EPI == EPI_ADD_F32 && !unit.partial) {
-        add_tile(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token - lane, args.tokens,
-                 feature0, wide, exchange + quarter * 32 * ADD_STRIDE, old);
-      } else if (EPI == EPI_ADD_F32) {
-        add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
-                           args.tokens, feature0);
+      } else if constexpr (EPI == EPI_ADD_F32) {
+        if (!unit.partial)
+          add_tile(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token - lane, args.tokens,
+                   feature0, wide, exchange + quarter * 32 * ADD_STRIDE, old);
+        else
+          add_row_atomically(static_cast<float*>(args.out), args.ldo, args.features, accumulator, token,
+                             args.tokens, feature0);
       } else {
         write_row<EPI>(columns, args.out, args.ldo, args.features, accumulator, token, args.tokens, feature0,
                        args.activation, args.gate_limit, args.gate_bias, args.up_bias, args.softcap);
