@@ -161,7 +161,6 @@ struct GemmArgs {
   // Store epilogues: > 1 where the CTAs of a tile, one for each run of k-blocks, are a cluster that adds its
   // sums up (see gather_parts).
   int cluster = 1;
-  bool in_blocks = false;     // tiles of 16 tokens, float32 store: see sum_blocks
 };
 
 // A product that is stored cannot be cut along the reduction into atomic adds, and one with few tiles (a
@@ -216,7 +215,7 @@ __device__ __forceinline__ void gather_parts(const GemmArgs& a, const float* par
 // 2,816 is off by 3.0e-6 (relative 2-norm), where a product a pair on the CUDA cores (hx_expert_down), which such
 // experts would else take, is off by 8.6e-8.  Four blocks are a turn, two turns share tensor memory; the blocks are
 // added here in registers, with what each addition rounds away: 7.0e-8.  Measured (us, the chain / here): 4 tiles by
-// [4,096 x 2,816] 20.0 / 21.6, 2 by [4,096 x 4,096] 20.0 / 23.4; turns of one block 23.8 and 30.2.
+// [4,096 x 2,816] 20.0 / 21.5, 2 by [4,096 x 4,096] 20.0 / 22.7; turns of one block 23.8 and 30.2.
 constexpr int TURN_BLOCKS = 4, TURN_COLUMNS = 16 * TURN_BLOCKS, TURNS = 2;
 
 __device__ __forceinline__ void sum_blocks(const GemmArgs& a, uint32_t lane_address, uint64_t* turn_full_bar,
@@ -235,23 +234,27 @@ __device__ __forceinline__ void sum_blocks(const GemmArgs& a, uint32_t lane_addr
       return;
     }
     tc_fence_after();
-    uint32_t block[TURN_BLOCKS][16];
 #pragma unroll
-    for (int b = 0; b < TURN_BLOCKS; ++b)
-      tmem_load16_issue(lane_address + buffer * TURN_COLUMNS + 16 * b, block[b]);
-    tmem_load_wait();
-    tc_fence_before();
-    __syncwarp();
-    if (lane == 0) mbar_arrive(&turn_empty_bar[buffer]);
+    for (int half = 0; half < TURN_BLOCKS; half += 2) {
+      uint32_t block[2][16];
+      tmem_load16_issue(lane_address + buffer * TURN_COLUMNS + 16 * half, block[0]);
+      tmem_load16_issue(lane_address + buffer * TURN_COLUMNS + 16 * half + 16, block[1]);
+      tmem_load_wait();
+      if (half + 2 == TURN_BLOCKS) {
+        tc_fence_before();
+        __syncwarp();
+        if (lane == 0) mbar_arrive(&turn_empty_bar[buffer]);
+      }
 #pragma unroll
-    for (int b = 0; b < TURN_BLOCKS; ++b) {
-      if (turn * TURN_BLOCKS + b >= blocks) break;
+      for (int b = 0; b < 2; ++b) {
+        if (turn * TURN_BLOCKS + half + b >= blocks) break;
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float x = __uint_as_float(block[b][j]), before = sum[j];
-        sum[j] = before + x;
-        const float added = sum[j] - before;
-        lost[j] += (before - (sum[j] - added)) + (x - added);
+        for (int j = 0; j < 16; ++j) {
+          const float x = __uint_as_float(block[b][j]), before = sum[j];
+          sum[j] = before + x;
+          const float added = sum[j] - before;
+          lost[j] += (before - (sum[j] - added)) + (x - added);
+        }
       }
     }
   }
@@ -262,14 +265,15 @@ __device__ __forceinline__ void sum_blocks(const GemmArgs& a, uint32_t lane_addr
   store_columns<EPI_STORE_F32>(a.out, a.ldo, a.tokens, token0, feature, sum, a.softcap);
 }
 
-template <int BN, int EPI>
+// IN_BLOCKS: see sum_blocks; a kernel of its own because of its registers (79 a thread, 40 without).
+template <int BN, int EPI, bool IN_BLOCKS = false>
 __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
     const __grid_constant__ CUtensorMap map_w, const __grid_constant__ CUtensorMap map_x,
     const GemmArgs args) {
   constexpr bool DUAL = EPI == EPI_SWIGLU;
   using Config = TileConfig<BN, DUAL>;
   constexpr int STAGES = Config::kStages;
-  constexpr bool BLOCKS = BN == 16 && EPI == EPI_STORE_F32;      // see sum_blocks
+  static_assert(!IN_BLOCKS || (BN == 16 && EPI == EPI_STORE_F32), "sum_blocks is for tiles of 16 tokens");
   constexpr bool CLUSTERS = (EPI == EPI_STORE_BF16 || EPI == EPI_STORE_F32) && BN <= 128;
   static_assert(!CLUSTERS || BN * BM * 4 <= STAGES * Config::kStageBytes, "a part lies where the ring was");
 
@@ -284,8 +288,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   uint64_t* turn_empty_bar = turn_full_bar + TURNS;      // [TURNS] they are read
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(turn_empty_bar + TURNS);
   static_assert((2 * STAGES + 1 + 2 * TURNS) * 8 + 4 <= 256, "the barriers' place");
-  const bool in_blocks = BLOCKS && args.in_blocks;
-  const int tmem_columns = in_blocks ? TURNS * TURN_COLUMNS : Config::kTmemColumns;
+  constexpr int TMEM_COLUMNS = IN_BLOCKS ? TURNS * TURN_COLUMNS : Config::kTmemColumns;
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -312,7 +315,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       mbar_init(&empty_bar[s], 1);
     }
     mbar_init(accum_bar, 1);
-    if (BLOCKS) {
+    if (IN_BLOCKS) {
       for (int b = 0; b < TURNS; ++b) {
         mbar_init(&turn_full_bar[b], 1);
         mbar_init(&turn_empty_bar[b], 4);      // one arrival per epilogue warp
@@ -321,7 +324,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
-  if (warp == 1) tmem_alloc(tmem_holder, tmem_columns);
+  if (warp == 1) tmem_alloc(tmem_holder, TMEM_COLUMNS);
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
@@ -376,14 +379,14 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
           const uint32_t round = static_cast<uint32_t>(i / STAGES);
           const int turn = i / TURN_BLOCKS;
           if (!mbar_wait(&full_bar[s], round & 1u) ||
-              (in_blocks && i % TURN_BLOCKS == 0 &&
+              (IN_BLOCKS && i % TURN_BLOCKS == 0 &&
                !mbar_wait(&turn_empty_bar[turn % TURNS], (static_cast<uint32_t>(turn / TURNS) & 1u) ^ 1u))) {
             atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
             ok = false;
             break;
           }
           tc_fence_after();
-          const uint32_t sums = tmem_base + (in_blocks ? i % (TURNS * TURN_BLOCKS) * 16 : 0);
+          const uint32_t sums = tmem_base + (IN_BLOCKS ? i % (TURNS * TURN_BLOCKS) * 16 : 0);
           const uint32_t stage = smem_u32(smem + s * Config::kStageBytes);
           const uint64_t desc_w = make_smem_desc(stage);
           const uint64_t desc_w2 = make_smem_desc(stage + BM * BK * 2);
@@ -392,12 +395,12 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
           for (int k = 0; k < BK / UMMA_K; ++k) {
             // stepping 16 k-elements = 32 bytes inside the swizzle span: +2 in 16-byte units
             const uint64_t step = static_cast<uint64_t>(k * UMMA_K * 2 >> 4);
-            const uint32_t accumulate = ((i > 0 && !in_blocks) || k > 0) ? 1u : 0u;
+            const uint32_t accumulate = ((i > 0 && !IN_BLOCKS) || k > 0) ? 1u : 0u;
             umma_bf16(sums, desc_w + step, desc_x + step, idesc, accumulate);
             if (DUAL) umma_bf16(sums + BN, desc_w2 + step, desc_x + step, idesc, accumulate);
           }
           umma_commit(&empty_bar[s]);   // the stage may be refilled once these MMAs have read it
-          if (in_blocks && (i % TURN_BLOCKS == TURN_BLOCKS - 1 || i + 1 == n_k_blocks))
+          if (IN_BLOCKS && (i % TURN_BLOCKS == TURN_BLOCKS - 1 || i + 1 == n_k_blocks))
             umma_commit(&turn_full_bar[turn % TURNS]);
         }
         umma_commit(accum_bar);         // the accumulator is complete
@@ -408,16 +411,14 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
       const int quarter = warp & 3;     // tensor-memory lanes [32 * quarter, 32 * quarter + 32)
       const int feature = feature0 + quarter * 32 + lane;
       const uint32_t lane_address = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16);
-      if constexpr (BLOCKS) {
-        if (in_blocks)
-          sum_blocks(args, lane_address, turn_full_bar, turn_empty_bar, n_k_blocks, feature, token0);
-      }
+      if constexpr (IN_BLOCKS)
+        sum_blocks(args, lane_address, turn_full_bar, turn_empty_bar, n_k_blocks, feature, token0);
       bool ok = true;
       if (lane == 0) ok = mbar_wait(accum_bar, 0);
       ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
       if (!ok) {
         if (lane == 0) atomicOr(args.status, HX_FLAG_WAIT_TIMEOUT);
-      } else if (!in_blocks) {
+      } else if (!IN_BLOCKS) {
         tc_fence_after();
         if (CLUSTERS && args.cluster > 1)
           leave_part<BN>(reinterpret_cast<float*>(smem), lane_address, quarter * 32 + lane,
@@ -443,7 +444,7 @@ __global__ __launch_bounds__(THREADS) void gemm_tc_kernel(
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
-    tmem_dealloc(tmem_base, tmem_columns);
+    tmem_dealloc(tmem_base, TMEM_COLUMNS);
   }
 }
 
@@ -1280,13 +1281,13 @@ int get_tensor_map(const void* base, uint64_t rows, uint64_t depth, uint64_t ld,
   return hx_tensor_map("hx_gemm_tc", base, rows, depth, ld, box_rows, BK, true, out);
 }
 
-template <int BN, int EPI>
+template <int BN, int EPI, bool IN_BLOCKS = false>
 int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& args, dim3 grid,
            cudaStream_t stream) {
   using Config = TileConfig<BN, EPI == EPI_SWIGLU>;
   static bool configured = false;
   if (!configured) {
-    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, EPI>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(gemm_tc_kernel<BN, EPI, IN_BLOCKS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              Config::kSmemBytes) != cudaSuccess) {
       hx_set_error("hx_gemm_tc: cannot reserve %d bytes of shared memory", Config::kSmemBytes);
       cudaGetLastError();
@@ -1308,10 +1309,10 @@ int launch(const CUtensorMap& map_w, const CUtensorMap& map_x, const GemmArgs& a
     attributes[1].val.programmaticStreamSerializationAllowed = 1;
     config.attrs = attributes;
     config.numAttrs = hx_pdl_enabled() ? 2 : 1;
-    cudaLaunchKernelEx(&config, gemm_tc_kernel<BN, EPI>, map_w, map_x, args);
+    cudaLaunchKernelEx(&config, gemm_tc_kernel<BN, EPI, IN_BLOCKS>, map_w, map_x, args);
     return HX_OK;
   }
-  hx_launch(gemm_tc_kernel<BN, EPI>, grid, THREADS, Config::kSmemBytes, stream, map_w, map_x, args);
+  hx_launch(gemm_tc_kernel<BN, EPI, IN_BLOCKS>, grid, THREADS, Config::kSmemBytes, stream, map_w, map_x, args);
   return HX_OK;
 }
 
@@ -1705,11 +1706,16 @@ static int gemm_tc_grouped(const void* x, int ldx, int x_capacity_rows, const vo
   }
   GemmArgs args{out, ldo, tokens, features, depth, up_row_offset, total_k_blocks, 0, status,
                 activation, tile_group, group_rows, gate_limit};
-  args.in_blocks = token_tile == 16 && tokens < 16 * 16 && epilogue == EPI_STORE_F32;
   const dim3 grid((tokens + token_tile - 1) / token_tile, (features + BM - 1) / BM, 1);
   HX_REQUIRE(grid.y <= 65535, "hx_gemm_tc_grouped: too many features (%d)", features);
   switch (token_tile) {
-    case 16: rc = launch_epilogue<16>(epilogue, map_w, map_x, args, grid, stream); break;
+    case 16:
+      // fewer than 16 tiles: experts of one to three tokens, whose float32 sums are those of products a pair
+      if (epilogue == EPI_STORE_F32 && tokens < 16 * 16)
+        rc = launch<16, EPI_STORE_F32, true>(map_w, map_x, args, grid, stream);
+      else
+        rc = launch_epilogue<16>(epilogue, map_w, map_x, args, grid, stream);
+      break;
     case 32: rc = launch_epilogue<32>(epilogue, map_w, map_x, args, grid, stream); break;
     case 64: rc = launch_epilogue<64>(epilogue, map_w, map_x, args, grid, stream); break;
     default: rc = launch_epilogue<256>(epilogue, map_w, map_x, args, grid, stream); break;
