@@ -836,11 +836,15 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
         // use different banks (a thread's own row, 16 bytes at a time, is half a sector a store).  With two CTAs
         // an SM they leave with whole rows side by side, with one by a bulk copy each (the other way round: heads
         // of 128 67 -> 70 us, heads of 256 over pages of 16 96 -> 101; pages of 32, 32 heads of 224 over one cached row,
-        // 2,048 tokens 127 -> 137, eight decoded tokens behind 500 19.5 -> 21.9).
+        // 2,048 tokens 127 -> 137, eight decoded tokens behind 500 19.5 -> 21.9).  Heads of 64 over pages of 16, a line of
+        // 128 bytes each, go straight from the registers (2,048 tokens of 32 heads 57.0 -> 55.6; over pages of 32 72 -> 76).
+        constexpr bool LINE_ROWS = D == 64 && GATHER;
         constexpr int SHARE = D / GROUPS, ROW_BYTES = SHARE * 2 + 16;
         static_assert(4 * GROUPS * 32 * ROW_BYTES <= Config::kQBytes + (K_STAGES + V_STAGES) * Config::kHalfBytes,
                       "the rows' place");
         uint8_t* gathered = q_tile + ((4 * softmax_group + quarter) * 32 + lane) * ROW_BYTES;
+        __nv_bfloat16* own_row = a.out + static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
+                                 static_cast<size_t>(head) * D;
         const int share = min(SHARE, a.value_dim - softmax_group * SHARE);      // coordinates that are wanted
 #pragma unroll
         for (int d0 = 0; d0 < SHARE; d0 += 32) {
@@ -860,21 +864,24 @@ prefill_attention_tc_kernel(const __grid_constant__ CUtensorMap key_pages, const
               for (int i = 0; i < 4; ++i)
                 pairs[i] = __floats2bfloat162_rn(__uint_as_float(r[h][d + 2 * i]) * inverse,
                                                  __uint_as_float(r[h][d + 2 * i + 1]) * inverse);
-              *reinterpret_cast<uint4*>(gathered + (d0 + h * 16 + d) * 2) = packed;
+              if constexpr (LINE_ROWS) {
+                if (row < rows_here) *reinterpret_cast<uint4*>(own_row + d0 + h * 16 + d) = packed;
+              } else {
+                *reinterpret_cast<uint4*>(gathered + (d0 + h * 16 + d) * 2) = packed;
+              }
             }
         }
         if constexpr (Config::kCtas == 1) {
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           if (row < rows_here && share > 0) {
-            __nv_bfloat16* out = a.out + static_cast<size_t>(q_begin + token0 + my_token) * a.ldo +
-                                 static_cast<size_t>(head) * D + softmax_group * SHARE;
-            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(out),
+            asm volatile("cp.async.bulk.global.shared::cta.bulk_group [%0], [%1], %2;" ::"l"(
+                             own_row + softmax_group * SHARE),
                          "r"(smem_u32(gathered)), "r"(2 * share)
                          : "memory");
             asm volatile("cp.async.bulk.commit_group;" ::: "memory");
             asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
           }
-        } else {
+        } else if constexpr (!LINE_ROWS) {
           __syncwarp();
           constexpr int PIECES = SHARE / 8;
           const uint8_t* of_warp = q_tile + quarter * 32 * ROW_BYTES;
