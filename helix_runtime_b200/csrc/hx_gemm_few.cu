@@ -219,7 +219,8 @@ int launch_tokens(const FewArgs& a, cudaStream_t stream) {
 // behind 16 tokens only while the tiles are few rounds of the SMs.  Measured (us, tensor cores / here): 9,600 features of
 // 3,200 with 32 tokens, 5 rounds, 111 / 94, 48, 7 rounds, 111 / 129; 17,280 with 17, 8 rounds, 120 / 150; 4,096 of 4,096 with
 // 48, 3 rounds, 81 / 72, 64, 4 rounds, 81 / 92; 3,200 of 8,640 with 64, 3 rounds, 150 / 137; 1,024 of 4,096 with 128, 2
-// rounds, 77 / 50.  A depth below a stage is mostly zeros here (9,000 of 128 with 16 tokens 10 / 12).
+// rounds, 77 / 50.  A depth below a stage is mostly zeros here (9,000 of 128 with 16 tokens 10 / 12).  The line at 128 tokens is
+// only where the measurements end: 16 of 2,048 take 7.2 us with 128 tokens and, as one chain, 58 with 129.
 HX_API int hx_gemm_few_takes(const void* x, int ldx, const void* w, int ldw, int tokens, int features, int depth) {
   if (tokens <= 0 || tokens > 128 || features <= 0 || depth < FEW_DEPTH || ldx % 4 != 0 || ldw % 4 != 0 ||
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w)) & 15) != 0)

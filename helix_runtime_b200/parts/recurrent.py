@@ -371,15 +371,16 @@ class LinearState(Mixer):
                           and ops.delta_chunks_supports(self.head_dim, self.value_dim))
 
     # What the recurrence takes, alone (us, 32 heads of 128 by 128): one portion of 32 / 64 / 128
-    # tokens 45 / 46 / 56 in chunks (two launches) and 42 / 76 / 144 by the scan, 16 portions of 32 152
-    # and 272; a decoding request in chunks costs a whole one, 82 for 8 of them and 473 for 64, where
-    # the scan takes 19 and 100.  So a step without decoding requests goes in chunks from a portion of
-    # 32 tokens and 48 tokens in all on.  Beside decoding requests the portions (SHORT_TOKENS and
-    # more) go in chunks and the others by the scan, one behind the other.  With few decoding requests
-    # and a portion of fewer than 64 tokens the scan takes both in the time of the portion.  A layer:
-    # 64 decoding requests and a portion of 32 / 128 / 512 tokens 567 / 599 / 733 all in chunks, 319 /
-    # 461 / 937 all by the scan, 241 / 266 / 352 so; 8 and 32 / 64 / 512 158 / 163 / 336, 129 / 169 /
-    # 726, 125 / 149 / 261.
+    # tokens 30 / 31 / 37 in chunks (two launches) and 36 / 67 / 130 by the scan (16 tokens 29 and 21),
+    # 16 portions of 32 126 and 250; a decoding request in chunks costs a whole one, 69 for 8 of them
+    # and 430 for 64, where the scan takes 15 and 96.  So a step without decoding requests goes in
+    # chunks from a portion of 32 tokens and 48 tokens in all on.  Beside decoding requests the portions
+    # (SHORT_TOKENS and more) go in chunks and the others by the scan, one behind the other.  With few
+    # decoding requests and a portion of fewer than 64 tokens the scan takes both in the time of the
+    # portion.  A layer: 64 decoding requests and a portion of 32 / 128 / 512 tokens 525 / 548 / 661 all in
+    # chunks, 319 / 451 / 912 all by the scan, 232 / 250 / 327 so; 8 and 32 / 64 / 512 132 / 133 / 259,
+    # 117 / 158 / 680, 117 / 113 / 214.  (The lines were drawn for chunks of 19,000 cycles and are at most 15 %
+    # off for 11,800: 8 and 48 tokens 136 by the scan, 116 in two.)
     CHUNKS_FROM_TOKENS, CHUNKS_FROM_TOKENS_IN_ALL = 32, 48
     SHORT_TOKENS = 16
     MIXED_CHUNKS_FROM_TOKENS = 64
