@@ -379,8 +379,9 @@ class LinearState(Mixer):
     # decoding requests and a portion of fewer than 64 tokens the scan takes both in the time of the
     # portion.  A layer: 64 decoding requests and a portion of 32 / 128 / 512 tokens 525 / 548 / 661 all in
     # chunks, 319 / 451 / 912 all by the scan, 232 / 250 / 327 so; 8 and 32 / 64 / 512 132 / 133 / 259,
-    # 117 / 158 / 680, 117 / 113 / 214.  (The lines were drawn for chunks of 19,000 cycles and are at most 15 %
-    # off for 11,800: 8 and 48 tokens 136 by the scan, 116 in two.)
+    # 117 / 158 / 680, 117 / 113 / 214.  (The lines were drawn for chunks of 19,000 cycles; a chunk takes 11,800
+    # now, and below them two launches would be faster: 8 requests and 48 tokens 136 by the scan, 116 in
+    # two, 64 and 24 307 and 230.)
     CHUNKS_FROM_TOKENS, CHUNKS_FROM_TOKENS_IN_ALL = 32, 48
     SHORT_TOKENS = 16
     MIXED_CHUNKS_FROM_TOKENS = 64
